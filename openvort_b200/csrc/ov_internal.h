@@ -97,10 +97,13 @@ struct OvTree {
   DevBuf scan_part;     // block sums of the exclusive scans
   DevBuf mom_part;      // per-chunk partial moments of the largest cells
   DevBuf walk_order;    // the walk's target list when nodes lie outside the root box
-  // the multi-image walk's groups of 32 targets by decreasing time in the
-  // last walk (wvals after the sort), their times, and the sort's buffers
+  DevBuf walk_part;     // partial sums of a walk split over several warps per group
+  DevBuf pkeys, pvals;  // point queries: sort keys and order
+  // the multi-image walk's units (groups of 32 targets, or their parts) by
+  // decreasing time in the last walk (wvals after the sort), their times,
+  // and the sort's buffers
   DevBuf warp_cost, wkeys, wkeys2, wvals, wvals2, whist, wscan;
-  int n_perm_warps = 0;   // groups the order in wvals covers (0: none yet)
+  int n_perm_warps = 0;   // units the order in wvals covers (0: none yet)
 };
 
 // ---------------------------------------------------------------- state
@@ -180,10 +183,11 @@ bool ov_shard_unpack(ov_state_impl* s, const double* xbuf, size_t xcap);
 bool ov_tree_walk_points(ov_state_impl* s, OvTree* tree, int npts, const double* pts,
                          const int* skip, double theta, double* out_nl, double* out_img);
 
-// stable LSD radix sort of 64-bit keys with int values (ov_tree.cu); the
-// result ends in (ka, va), (kb, vb) are scratch of the same sizes
-bool ov_radix_sort_u64(uint64_t* ka, int* va, uint64_t* kb, int* vb, int n, DevBuf& hist, DevBuf& scan_part,
-                       cudaStream_t st);
+// stable LSD radix sort of keys by their low `bits` bits, with int values
+// (ov_tree.cu); the result ends in (ka, va), (kb, vb) are scratch of the same
+// sizes
+bool ov_radix_sort_u64(uint64_t* ka, int* va, uint64_t* kb, int* vb, int n, int bits, DevBuf& hist,
+                       DevBuf& scan_part, cudaStream_t st);
 // direct sums for all nodes -> v_nl, v_img
 bool ov_direct_nodes(ov_state_impl* s, const double* pos, double* v_nl, double* v_img);
 // direct sums at arbitrary points (device arrays), sources = all segments or

@@ -386,7 +386,7 @@ bool find_candidates(RecState& R, const tangle_state* t, double rec_dist, double
   OV_TRY_CUDA(cudaGetLastError());
   // the tree build's radix sort; the sorted keys and ids end in keys / ids
   if (!ov_radix_sort_u64(R.keys.as<uint64_t>(), R.ids.as<int>(), R.keys2.as<uint64_t>(), R.ids2.as<int>(), n,
-                         R.hist, R.scan_part, s->stream))
+                         64, R.hist, R.scan_part, s->stream))
     return false;
   int cap = std::max(1024, n / 4);
   const double cos_angle = cos(rec_angle);

@@ -782,9 +782,10 @@ void ov_tree_release(OvTree* t) {
   DevBuf* bufs[] = {&t->keys, &t->keys_alt, &t->vals, &t->vals_alt, &t->stop, &t->hist,
                     &t->perm, &t->bnode, &t->cstart_cnt, &t->cbase, &t->cell_of, &t->cells,
                     &t->cell_lm, &t->cell_range, &t->nodes64, &t->nodeids, &t->nodes32, &t->counters,
-                    &t->scratch, &t->scan_part, &t->mom_part};
+                    &t->scratch, &t->scan_part, &t->mom_part, &t->walk_order, &t->walk_part, &t->pkeys,
+                    &t->pvals, &t->warp_cost, &t->wkeys, &t->wkeys2, &t->wvals, &t->wvals2, &t->whist, &t->wscan};
   for (DevBuf* b : bufs) b->release();
-  t->n_nodes = t->n_cells = t->built = 0;
+  t->n_nodes = t->n_cells = t->built = t->n_perm_warps = 0;
 }
 
 // exclusive scan of v[0..m) in place (block sums in `part`)
@@ -802,16 +803,17 @@ static bool scan_excl(unsigned* v, int m, DevBuf& part, cudaStream_t st) {
   return ov_cuda_ok(cudaGetLastError(), "scan");
 }
 
-// Stable LSD radix sort of n 64-bit keys with int values, 8 passes of 8
-// bits (k_rs_hist, the three-launch scan, k_rs_scatter).  (kb, vb) are the
-// alternate buffers; after the even number of passes the sorted keys and
-// values are back in (ka, va).
-bool ov_radix_sort_u64(uint64_t* ka, int* va, uint64_t* kb, int* vb, int n, DevBuf& hist, DevBuf& scan_part,
-                       cudaStream_t st) {
+// Stable LSD radix sort of n keys by their low `bits` bits, with int values,
+// in passes of 8 bits (k_rs_hist, the three-launch scan, k_rs_scatter), an
+// even number of them.  (kb, vb) are the alternate buffers; after the even
+// number of passes the sorted keys and values are back in (ka, va).
+bool ov_radix_sort_u64(uint64_t* ka, int* va, uint64_t* kb, int* vb, int n, int bits, DevBuf& hist,
+                       DevBuf& scan_part, cudaStream_t st) {
   if (n <= 0) return true;
   const int nb = (n + kRsTile - 1) / kRsTile;
   if (!hist.reserve(sizeof(unsigned) * 256 * (size_t)nb)) return false;
-  for (int pass = 0; pass < 8; ++pass) {
+  const int passes = 2 * ((bits + 15) / 16);
+  for (int pass = 0; pass < passes; ++pass) {
     const int shift = 8 * pass;
     k_rs_hist<<<nb, kRsThreads, 0, st>>>(ka, n, shift, hist.as<unsigned>(), nb);
     OV_LAUNCHED();
@@ -875,7 +877,7 @@ bool ov_tree_build(ov_state_impl* s, const double* pos, OvTree* T) {
   uint64_t* ka = khi;
   int* va = vals;
   if (!T->scratch.reserve(sizeof(int) * (size_t)n + 16)) return false;
-  if (!ov_radix_sort_u64(khi, vals, khi_alt, T->scratch.as<int>(), n, T->hist, T->scan_part, st)) return false;
+  if (!ov_radix_sort_u64(khi, vals, khi_alt, T->scratch.as<int>(), n, 64, T->hist, T->scan_part, st)) return false;
   if (!T->perm.reserve(sizeof(int) * (size_t)(n > 0 ? n : 1))) return false;
   int* perm = T->perm.as<int>();
   if (n > 0) {

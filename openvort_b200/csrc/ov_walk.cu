@@ -227,7 +227,6 @@ constexpr int kPrimary = 13;
 constexpr int kFewImages = 4;
 constexpr unsigned kAllImages = (1u << 27) - 1;
 constexpr int kLevelSlots = 34;
-constexpr int kMultiWarps = 4;
 
 // Parameters of the walk's shortcut decisions (every image from the
 // target's own distance): on = no image shifts along a non-periodic axis
@@ -663,42 +662,68 @@ __device__ __forceinline__ void cell_fp64(const OvParams& P, const Cell* cp, dou
                 fma(g[0], py, fma(-g[1], px, fma(m02, qy, -m12 * qx))));
 }
 
-// resident blocks per SM the register allocation must allow, measured at
+// resident warps per SM the register allocation must allow, measured at
 // 1M points, ms per launch:
-//   mixed 47.6 / 40.6 / 43.8 / 44.8 for 3 / 4 / 5 / 6 blocks (136 and 128
+//   mixed 47.6 / 40.6 / 43.8 / 44.8 for 12 / 16 / 20 / 24 warps (136 and 128
 //   registers without spills, 96 registers and 56 bytes spilled, 80
 //   registers and 272 bytes spilled)
-//   FP64 87.6 / 79.8 / 78.5 for 4 / 5 / 6 blocks (110 registers without
+//   FP64 87.6 / 79.8 / 78.5 for 16 / 20 / 24 warps (110 registers without
 //   spills, 96 registers and 48 bytes spilled, 80 registers and 88 bytes
 //   spilled)
-#ifndef OV_WALK_MULTI_MIN_BLOCKS_MIXED
-#define OV_WALK_MULTI_MIN_BLOCKS_MIXED 4
+// Blocks are one warp each: a block of four kept its place until its slowest
+// warp ended (200k nodes FP64, two parts, a first walk: 16.9 ms against 15.9;
+// 1M mixed 35.8 against 35.1).
+#ifndef OV_WALK_MULTI_MIN_WARPS_MIXED
+#define OV_WALK_MULTI_MIN_WARPS_MIXED 16
 #endif
-#ifndef OV_WALK_MULTI_MIN_BLOCKS_FP64
-#define OV_WALK_MULTI_MIN_BLOCKS_FP64 6
+#ifndef OV_WALK_MULTI_MIN_WARPS_FP64
+#define OV_WALK_MULTI_MIN_WARPS_FP64 24
 #endif
 
-template <bool kMixed>
-__global__ void __launch_bounds__(kMultiWarps * 32, kMixed ? OV_WALK_MULTI_MIN_BLOCKS_MIXED
-                                                           : OV_WALK_MULTI_MIN_BLOCKS_FP64)
+// A group's walk split over `parts` warps (a power of two), for launches with
+// too few groups to fill the GPU.  Every part traverses the cells whose
+// subtree holds more than `frontier` cells and takes their decisions; those
+// cells' evaluations and the smaller subtrees below them are dealt to the
+// parts by their place in the preorder, a stretch of 2^deal cells each in
+// turn.  Cells near the targets, where most of the work lies, are close
+// together in the preorder, so dealing them in turn spreads them.  A target's
+// terms are thus dealt by the cells alone, whatever group it is in.  Part p
+// of target i writes its sums to nl[p * n_t + i]; k_walk_reduce adds the
+// parts in order, so the result depends on neither the grouping nor the
+// scheduling.
+struct WalkSplit {
+  int parts;       // 1, 2, 4, ...
+  int frontier;    // cells
+  int deal;        // log2 of the stretch of cells dealt at a time
+  const int* skip; // points: slot skipped per point (null: none); nodes: unused
+  double* nl;      // partial sums, 3 doubles per part and target
+  double* im;
+};
+
+template <bool kMixed, bool kSplit>
+__global__ void __launch_bounds__(32, kMixed ? OV_WALK_MULTI_MIN_WARPS_MIXED : OV_WALK_MULTI_MIN_WARPS_FP64)
     k_walk_multi(
     OvParams P, TreeView T, const int* __restrict__ order, const int2* __restrict__ status,
     const double* __restrict__ pos, int n_t, unsigned combos, ImageShortcut S, double near2,
     double* v_nl, double* v_img, unsigned long long* counters, const int* __restrict__ warp_perm,
-    unsigned* __restrict__ warp_cost) {
-  __shared__ unsigned sh_mask[kMultiWarps][kLevelSlots][32];
+    unsigned* __restrict__ warp_cost, WalkSplit W) {
+  __shared__ unsigned sh_mask[kLevelSlots][32];
   const unsigned FULL = 0xffffffffu;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int lane = threadIdx.x;
   const long long t_start = clock64();
-  const int slot = blockIdx.x * kMultiWarps + warp;
-  if (slot * 32 >= n_t) return;   // whole warp out of range
-  // the group of 32 consecutive targets this warp takes: launch slot
-  // `slot` runs group warp_perm[slot] (the groups by decreasing time in the
-  // previous evaluation), or group `slot`
-  const int gw = warp_perm ? warp_perm[slot] : slot;
+  // the group of 32 consecutive targets this warp takes (and its part of a
+  // split group): block b runs unit warp_perm[b] (the units by decreasing
+  // time in the previous evaluation), or unit b
+  const int unit = warp_perm ? warp_perm[blockIdx.x] : blockIdx.x;
+  const int gw = kSplit ? unit / W.parts : unit;
   const int i = gw * 32 + lane;
   const int k = i < n_t ? (order ? order[i] : i) : -1;
-  const bool live = k >= 0 && status[k].x != OV_PINNED && status[k].x != OV_EMPTY;
+  const bool live =
+      k >= 0 && ((kSplit && !status) || (status[k].x != OV_PINNED && status[k].x != OV_EMPTY));
+  // the slot whose own segments the tangle's sum leaves out
+  const int skip = kSplit && !status ? (W.skip && live ? W.skip[k] : -1) : k;
+  const int part = kSplit ? unit % W.parts : 0;
+  int own_end = 0;   // end of the subtree this part walks
   const d3 r = live ? ld3(pos, k) : mk3(0, 0, 0);
   // the shortcuts' bound on rounding holds for targets within a quarter box
   // of the box (a node further out takes every decision in full)
@@ -708,7 +733,7 @@ __global__ void __launch_bounds__(kMultiWarps * 32, kMixed ? OV_WALK_MULTI_MIN_B
     const double v = a == 0 ? r.x : (a == 1 ? r.y : r.z);
     sane = sane && v >= P.lo[a] - 0.25 * P.L[a] && v <= P.hi[a] + 0.25 * P.L[a];
   }
-  unsigned* lvl_mask = &sh_mask[warp][0][lane];   // level l at lvl_mask[32 l]
+  unsigned* lvl_mask = &sh_mask[0][lane];   // level l at lvl_mask[32 l]
   lvl_mask[0] = combos;
   d3 nl = mk3(0, 0, 0), im = mk3(0, 0, 0);
   unsigned n_p2p = 0, n_far = 0, n_iter = 0;
@@ -724,19 +749,30 @@ __global__ void __launch_bounds__(kMultiWarps * 32, kMixed ? OV_WALK_MULTI_MIN_B
     const double2 t1 = *reinterpret_cast<const double2*>(&cp->x[1]);
     const int kind = cell_kind(h.w);
     if (lane == 1 && h.z < T.n_cells) prefetch_l1(T.cells + h.z);
+    bool mine = true;   // whether this part evaluates the cell
+    if (kSplit && q >= own_end) {
+      mine = ((q >> W.deal) & (W.parts - 1)) == part;
+      if (h.z - q <= W.frontier) {
+        if (!mine) {   // a subtree of another part
+          if (next == q) next = max(h.z, q + 1);
+          continue;
+        }
+        own_end = h.z;
+      }
+    }
     unsigned p2p_mask = 0;   // images summing this cell's node range directly
     if (next == q) {
       const unsigned m = lvl_mask[32 * cell_ltop(h.w)];
       unsigned open = 0;
       if (kind == CELL_LEAF1) {
         if (kMixed && __popc(m) >= kColumnImages)
-          p2p_mixed_columns(P, m, r, mk3(t0.y, t1.x, t1.y), mk3(cp->y[0], cp->y[1], cp->y[2]), h.x, h.y, k,
+          p2p_mixed_columns(P, m, r, mk3(t0.y, t1.x, t1.y), mk3(cp->y[0], cp->y[1], cp->y[2]), h.x, h.y, skip,
                             near2, nl, n_p2p);
         else
           p2p_images<kMixed>(P, m, r, mk3(t0.y, t1.x, t1.y), mk3(cp->y[0], cp->y[1], cp->y[2]), h.x,
-                             h.y, k, near2, nl, im, n_p2p);
+                             h.y, skip, near2, nl, im, n_p2p);
       } else if (kind == CELL_LEAFN) {
-        p2p_mask = m;
+        p2p_mask = mine ? m : 0;
       } else {
         // opening test per image (octree_get_vs, src/octree.c:284-296)
         const double cx = t0.y, cy = t1.x, cz = t1.y;
@@ -789,8 +825,8 @@ __global__ void __launch_bounds__(kMultiWarps * 32, kMixed ? OV_WALK_MULTI_MIN_B
         pass &= m;
         const unsigned fail = m & ~pass;
         if (kind == CELL_OPEN) open = fail;
-        else if (kind == CELL_OPEN_P2P) p2p_mask = fail;
-        if (pass) {
+        else if (kind == CELL_OPEN_P2P) p2p_mask = mine ? fail : 0;
+        if (pass && mine) {
           n_far += __popc(pass);
           // expansion at every accepting image: R = r - L s - com, unwrapped
           if (kMixed) {
@@ -815,14 +851,19 @@ __global__ void __launch_bounds__(kMultiWarps * 32, kMixed ? OV_WALK_MULTI_MIN_B
         const double* nd = T.nodes64 + 6 * (size_t)j;
         if (kMixed && __popc(p2p_mask) >= kColumnImages)
           p2p_mixed_columns(P, p2p_mask, r, mk3(nd[0], nd[1], nd[2]), mk3(nd[3], nd[4], nd[5]), id.x, id.y,
-                            k, near2, nl, n_p2p);
+                            skip, near2, nl, n_p2p);
         else
           p2p_images<kMixed>(P, p2p_mask, r, mk3(nd[0], nd[1], nd[2]), mk3(nd[3], nd[4], nd[5]), id.x,
-                             id.y, k, near2, nl, im, n_p2p);
+                             id.y, skip, near2, nl, im, n_p2p);
       }
     }
   }
-  if (live) {
+  if (kSplit) {
+    if (i < n_t) {
+      st3(W.nl + 3 * (size_t)part * n_t, i, nl);
+      st3(W.im + 3 * (size_t)part * n_t, i, im);
+    }
+  } else if (live) {
     st3(v_nl, k, nl);
     st3(v_img, k, im);
   }
@@ -836,11 +877,28 @@ __global__ void __launch_bounds__(kMultiWarps * 32, kMixed ? OV_WALK_MULTI_MIN_B
     atomicAdd(&counters[0], a);
     atomicAdd(&counters[1], b);
     atomicAdd(&counters[2], (unsigned long long)n_iter);
-    // this group's time in SM cycles / 64, for the next evaluation's order
-    if (warp_cost) warp_cost[gw] = (unsigned)min((clock64() - t_start) >> 6, 0xffffffffll);
+    // this unit's time in SM cycles / 64, for the next evaluation's order
+    if (warp_cost) warp_cost[unit] = (unsigned)min((clock64() - t_start) >> 6, 0xffffffffll);
   }
 }
 
+// the parts of a split walk added in order: target i's sums into slot
+// order[i] (or i)
+__global__ void k_walk_reduce(const int* __restrict__ order, const int2* __restrict__ status, int n_t, int parts,
+                              const double* __restrict__ nl, const double* __restrict__ im, double* v_nl,
+                              double* v_img) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n_t) return;
+  const int k = order ? order[i] : i;
+  if (k < 0 || (status && (status[k].x == OV_PINNED || status[k].x == OV_EMPTY))) return;
+  d3 a = ld3(nl, i), b = ld3(im, i);
+  for (int p = 1; p < parts; ++p) {
+    a = a + ld3(nl + 3 * (size_t)p * n_t, i);
+    b = b + ld3(im + 3 * (size_t)p * n_t, i);
+  }
+  st3(v_nl, k, a);
+  if (v_img) st3(v_img, k, b);
+}
 
 // All nodes: warp w handles sorted targets 32w .. 32w+31, every image.
 // Targets in `order` (the tree's key order, so a warp's targets are close in
@@ -937,13 +995,63 @@ static __global__ void k_drop_first(const int* __restrict__ perm, int nin, int n
   out[i] = i < pad ? ((i & 31) == 0 ? perm[nin + (i >> 5)] : -1) : perm[i - pad];
 }
 
-// sort keys for the groups' order: decreasing time first
+// sort keys for the units' order: decreasing time first, to 8 significant
+// bits (the time as an FP32 number, its sign and low 15 bits dropped), so two
+// passes of the radix sort order them
+constexpr int kCostBits = 16;
 static __global__ void k_cost_keys(const unsigned* __restrict__ cost, int n, uint64_t* keys, int* vals) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
-  keys[i] = (uint64_t)(0xffffffffu - cost[i]);
+  keys[i] = 0xffffu - ((unsigned)__float_as_int((float)cost[i]) >> 15);
   vals[i] = i;
 }
+
+// Hilbert keys of points in the box, kCurveBits per axis (J. Skilling,
+// "Programming the Hilbert curve", AIP Conf. Proc. 707, 2004: the transform
+// of the axes into the curve's transposed index).  Points outside the box,
+// whose coordinates clamp, and NaN, which converts to 0, sort somewhere: the
+// order only decides which targets share a warp.  Value i of the sort is
+// slots[i] (or i).
+constexpr int kCurveBits = 10;
+static __global__ void k_curve_keys(OvParams P, const double* __restrict__ pts, const int* __restrict__ slots, int n,
+                                    uint64_t* keys, int* vals) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const int k = slots ? slots[i] : i;
+  unsigned x[3];
+#pragma unroll
+  for (int a = 0; a < 3; ++a) {
+    const double f = (pts[3 * (size_t)k + a] - P.lo[a]) / P.L[a] * (1 << kCurveBits);
+    x[a] = (unsigned)fmin(fmax(f, 0.0), (double)((1 << kCurveBits) - 1));
+  }
+  for (unsigned q = 1u << (kCurveBits - 1); q > 1; q >>= 1) {
+    const unsigned m = q - 1;
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+      if (x[a] & q) {
+        x[0] ^= m;
+      } else {
+        const unsigned t = (x[0] ^ x[a]) & m;
+        x[0] ^= t;
+        x[a] ^= t;
+      }
+    }
+  }
+  x[1] ^= x[0];
+  x[2] ^= x[1];
+  unsigned t = 0;
+  for (unsigned q = 1u << (kCurveBits - 1); q > 1; q >>= 1)
+    if (x[2] & q) t ^= q - 1;
+  unsigned key = 0;
+#pragma unroll
+  for (int b = kCurveBits - 1; b >= 0; --b)
+#pragma unroll
+    for (int a = 0; a < 3; ++a) key = (key << 1) | (((x[a] ^ t) >> b) & 1u);
+  keys[i] = key;
+  vals[i] = k;
+}
+
+constexpr int kMaxParts = 32;   // warps a group's walk is split over, at most
 
 static bool read_counters(ov_state_impl* s, OvTree* t) {
   unsigned long long c[3] = {0, 0, 0};
@@ -954,6 +1062,148 @@ static bool read_counters(ov_state_impl* s, OvTree* t) {
   st.interactions = (double)c[0];
   st.cell_interactions = (double)c[1];
   st.warp_iterations = (double)c[2];
+  return true;
+}
+
+// The image table as a set of periodic shifts in {-1,0,1}^3 (bit 9 (sx+1) +
+// 3 (sy+1) + (sz+1), the tangle itself included); false for a table with
+// mirrors or repeated shifts, which the multi-image walk does not take.
+static bool image_combos(const OvParams& P, int n_img, unsigned& combos) {
+  combos = 1u << kPrimary;
+  for (int j = 0; j < n_img; ++j) {
+    const int* im = P.img[j];
+    if (im[3] != -1 || im[0] < -1 || im[0] > 1 || im[1] < -1 || im[1] > 1 || im[2] < -1 || im[2] > 1)
+      return false;
+    const unsigned bit = 1u << (9 * (im[0] + 1) + 3 * (im[1] + 1) + (im[2] + 1));
+    if (combos & bit) return false;
+    combos |= bit;
+  }
+  return true;
+}
+
+// shortcut parameters: see ImageShortcut and mac_margin (the rounding
+// allowance 8 u B with B the bound on magnitudes of mac_margin)
+static ImageShortcut image_shortcut(const OvParams& P, unsigned combos) {
+  ImageShortcut sc;
+  double B = 0;
+  for (int a = 0; a < 3; ++a) B = std::max(B, std::fabs(P.lo[a]) + std::fabs(P.hi[a]));
+  const double allowance = 8 * 0x1p-53 * 3.5 * B;
+  sc.on = 1;
+  for (int a = 0; a < 3; ++a) {
+    bool shifted = false;
+    for (int c = 0; c < kCombos; ++c) {
+      const int sa = a == 0 ? c / 9 : (a == 1 ? (c / 3) % 3 : c % 3);
+      if (((combos >> c) & 1u) && sa != 1) shifted = true;
+    }
+    if (shifted && !P.periodic[a]) sc.on = 0;
+    sc.hw[a] = shifted ? 0.5 * P.L[a] - allowance : DBL_MAX;
+    sc.half[a] = P.periodic[a] ? P.L[a] * 0.5 : DBL_MAX;
+  }
+  return sc;
+}
+
+// warps of one wave of a walk kernel: resident blocks on every SM
+template <class K>
+static int walk_wave(K kernel) {
+  int dev = 0, sms = 0, nb = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, kernel, 32, 0) != cudaSuccess) {
+    cudaGetLastError();
+    return 1;
+  }
+  return std::max(1, sms * nb);
+}
+
+// The multi-image walk of n_t targets at pos: nodes (status given: slots of
+// `order`) or points (status null: order sorts them, skip per point).
+// n_rule: the targets the split rule counts (a rank's share of a sharded
+// evaluation counts all of them, so every rank adds its sums in the order
+// one GPU would).  v_img null: no image sums wanted.
+static bool launch_multi(ov_state_impl* s, OvTree* t, const OvParams& P, const int* order, const int2* status,
+                         const int* skip, const double* pos, int n_t, int n_rule, unsigned combos, double* v_nl,
+                         double* v_img, bool timed) {
+  unsigned long long* ctr = reinterpret_cast<unsigned long long*>(t->counters.as<char>() + 64);
+  const bool mixed = P.precision == OV_PREC_MIXED;
+  const ImageShortcut sc = image_shortcut(P, combos);
+  const TreeView tv = view_of(t);
+  static const int wave_mixed = walk_wave(k_walk_multi<true, true>);
+  static const int wave_fp64 = walk_wave(k_walk_multi<false, true>);
+  const int wave = mixed ? wave_mixed : wave_fp64;
+  // Parts per group: enough that the units make two waves, so the last wave's
+  // slow units are short.  Measured, ms per walk of a tangle stepped on, at 1
+  // / 2 / 4 / 8 / 16 parts, 26 images.  Mixed (a wave is 2368 warps), theta =
+  // 0.4: 22.4k nodes 3.07 / 2.03 / 1.54 / 1.25 / 1.35, 60k 4.36 / 3.16 / 3.08
+  // / 3.22 / 3.76, 200k 10.7 / 10.6 / 11.0 / 12.0 / 14.0.  FP64 (3552):
+  // 22.4k 7.12 / 4.9 / 3.4 / 2.6 / 2.4, 200k at theta = 0.5 14.1 / 12.6 /
+  // 12.6 / 13.1; a first walk, without times to order it by, takes 15.8 / 15.9
+  // / 16.7 / 17.8 there.
+  int parts = 1;
+  const int groups = (n_t + 31) / 32;
+  const long long groups_rule = (n_rule + 31) / 32;
+  while (parts < kMaxParts && groups_rule * parts < 2LL * wave) parts *= 2;
+  // Frontier: a smaller one deals the work out more evenly, but its cells'
+  // decisions are taken again in every part.  1/64 of the cells, for few
+  // groups (16 parts and more) and for points, whose groups are wider, 1/256:
+  // mixed 22.4k nodes at 8 parts 1.25 ms against 1.39 at 1/128; FP64 3000
+  // nodes at 32 parts 0.49 ms against 0.81 at 1/64; 512 points over 50k nodes
+  // 2.4 ms a query.
+  const int frontier = std::max(1, t->n_cells / (status && parts < 16 ? 64 : 256));
+  // stretches of a quarter of the frontier (22.4k nodes FP64, 8 parts: 2.52
+  // ms, against 2.66 with a sixteenth)
+  int deal = 0;
+  while ((8 << deal) <= frontier) ++deal;
+  const bool split = parts > 1 || !status;
+  const int warps = groups * parts;
+  WalkSplit W{parts, frontier, deal, skip, nullptr, nullptr};
+  if (split) {
+    const size_t per = 3 * (size_t)n_t * parts;
+    if (!t->walk_part.reserve(sizeof(double) * 2 * per)) return false;
+    W.nl = t->walk_part.as<double>();
+    W.im = W.nl + per;
+  }
+  // Longest first: the launch runs the warps' units (groups of 32 targets,
+  // or their parts) in the order of their times in the previous walk of this
+  // tree (the same regions of the key order, a few node moves apart), so the
+  // slow ones do not start in the last wave.  The sums do not depend on the
+  // order.  A launch within one wave starts every unit at once and needs no
+  // order.  A rank's share of a sharded evaluation is the same key range at
+  // every evaluation, so its units are ordered the same way.
+  timed = timed && warps > wave;
+  const int* wperm = timed && t->n_perm_warps == warps ? t->wvals.as<int>() : nullptr;
+  unsigned* wcost = nullptr;
+  if (timed) {
+    if (!t->warp_cost.reserve(sizeof(unsigned) * (size_t)warps)) return false;
+    wcost = t->warp_cost.as<unsigned>();
+  } else {
+    t->n_perm_warps = 0;
+  }
+  auto kernel = split ? (mixed ? k_walk_multi<true, true> : k_walk_multi<false, true>)
+                      : (mixed ? k_walk_multi<true, false> : k_walk_multi<false, false>);
+  kernel<<<warps, 32, 0, s->stream>>>(P, tv, order, status, pos, n_t, combos, sc, P.near2, v_nl, v_img, ctr, wperm,
+                                      wcost, W);
+  OV_LAUNCHED();
+  OV_TRY_CUDA(cudaGetLastError());
+  if (split) {
+    k_walk_reduce<<<(n_t + 127) / 128, 128, 0, s->stream>>>(order, status, n_t, parts, W.nl, W.im, v_nl, v_img);
+    OV_LAUNCHED();
+    OV_TRY_CUDA(cudaGetLastError());
+  }
+  cudaEventRecord(s->ev2, s->stream);
+  if (timed) {
+    // the order for the next walk (after the timed kernel)
+    const size_t nw = (size_t)warps;
+    if (!t->wkeys.reserve(sizeof(uint64_t) * nw) || !t->wkeys2.reserve(sizeof(uint64_t) * nw) ||
+        !t->wvals.reserve(sizeof(int) * nw) || !t->wvals2.reserve(sizeof(int) * nw))
+      return false;
+    k_cost_keys<<<(warps + 255) / 256, 256, 0, s->stream>>>(wcost, warps, t->wkeys.as<uint64_t>(),
+                                                              t->wvals.as<int>());
+    OV_LAUNCHED();
+    if (!ov_radix_sort_u64(t->wkeys.as<uint64_t>(), t->wvals.as<int>(), t->wkeys2.as<uint64_t>(),
+                           t->wvals2.as<int>(), warps, kCostBits, t->whist, t->wscan, s->stream))
+      return false;
+    t->n_perm_warps = warps;
+  }
   return true;
 }
 
@@ -1002,7 +1252,6 @@ bool ov_tree_walk_nodes(ov_state_impl* s, OvTree* t, const double* pos, bool own
     order = t->walk_order.as<int>();
     n_t = m;
   }
-  TreeView tv = view_of(t);
   OvParams P = t->P;
   // image table and precision of this call; geometry of the tree's build
   P.n_img = s->P.n_img;
@@ -1010,96 +1259,27 @@ bool ov_tree_walk_nodes(ov_state_impl* s, OvTree* t, const double* pos, bool own
     for (int c = 0; c < 4; ++c) P.img[j][c] = s->P.img[j][c];
   P.precision = s->P.precision;
   const bool mixed = s->P.precision == OV_PREC_MIXED;
-  // images as a set of periodic shifts in {-1,0,1}^3 without mirrors or
-  // repeats: one multi-image walk per target
-  unsigned combos = 1u << 13;
-  bool multi = true;
-  for (int j = 0; j < P.n_img && multi; ++j) {
-    const int* im = P.img[j];
-    if (im[3] != -1 || im[0] < -1 || im[0] > 1 || im[1] < -1 || im[1] > 1 || im[2] < -1 ||
-        im[2] > 1) {
-      multi = false;
-      break;
-    }
-    unsigned bit = 1u << (9 * (im[0] + 1) + 3 * (im[1] + 1) + (im[2] + 1));
-    if (combos & bit) multi = false;
-    combos |= bit;
-  }
-  const double near2 = s->P.near2;
-  // shortcut parameters: see ImageShortcut and mac_margin (the rounding
-  // allowance 8 u B with B the bound on magnitudes of mac_margin)
-  ImageShortcut sc;
-  {
-    double B = 0;
-    for (int a = 0; a < 3; ++a) B = std::max(B, std::fabs(P.lo[a]) + std::fabs(P.hi[a]));
-    const double allowance = 8 * 0x1p-53 * 3.5 * B;
-    sc.on = 1;
-    for (int a = 0; a < 3; ++a) {
-      bool shifted = false;
-      for (int c = 0; c < kCombos; ++c) {
-        const int sa = a == 0 ? c / 9 : (a == 1 ? (c / 3) % 3 : c % 3);
-        if (((combos >> c) & 1u) && sa != 1) shifted = true;
-      }
-      if (shifted && !P.periodic[a]) sc.on = 0;
-      sc.hw[a] = shifted ? 0.5 * P.L[a] - allowance : DBL_MAX;
-      sc.half[a] = P.periodic[a] ? P.L[a] * 0.5 : DBL_MAX;
-    }
-  }
-  cudaEventRecord(s->ev1, s->stream);
-  if (multi) {
-    int warps = (n_t + 31) / 32;
-    int blocks = (warps + kMultiWarps - 1) / kMultiWarps;
-    // Longest groups first: the launch runs the groups of 32 targets in the
-    // order of their times in the previous walk of this tree (the same
-    // regions of the key order, a few node moves apart), so the slow ones
-    // do not start in the last wave.  The sums do not depend on the order.
-    // A rank's share of a sharded evaluation is the same key range at every
-    // evaluation, so its groups are ordered the same way.
-    const bool timed = own_tree;
-    const int* wperm = timed && t->n_perm_warps == warps ? t->wvals.as<int>() : nullptr;
-    unsigned* wcost = nullptr;
-    if (timed) {
-      if (!t->warp_cost.reserve(sizeof(unsigned) * (size_t)warps)) return false;
-      wcost = t->warp_cost.as<unsigned>();
-    }
-    if (mixed) {
-      k_walk_multi<true><<<blocks, kMultiWarps * 32, 0, s->stream>>>(
-          P, tv, order, s->status.as<int2>(), pos, n_t, combos, sc, near2, v_nl, v_img, ctr, wperm, wcost);
-      OV_LAUNCHED();
-    } else {
-      k_walk_multi<false><<<blocks, kMultiWarps * 32, 0, s->stream>>>(
-          P, tv, order, s->status.as<int2>(), pos, n_t, combos, sc, near2, v_nl, v_img, ctr, wperm, wcost);
-      OV_LAUNCHED();
-    }
-    OV_TRY_CUDA(cudaGetLastError());
-    cudaEventRecord(s->ev2, s->stream);
-    if (timed) {
-      // the order for the next walk (after the timed kernel)
-      const size_t nw = (size_t)warps;
-      if (!t->wkeys.reserve(sizeof(uint64_t) * nw) || !t->wkeys2.reserve(sizeof(uint64_t) * nw) ||
-          !t->wvals.reserve(sizeof(int) * nw) || !t->wvals2.reserve(sizeof(int) * nw))
-        return false;
-      k_cost_keys<<<(warps + 255) / 256, 256, 0, s->stream>>>(wcost, warps, t->wkeys.as<uint64_t>(),
-                                                                t->wvals.as<int>());
-      OV_LAUNCHED();
-      if (!ov_radix_sort_u64(t->wkeys.as<uint64_t>(), t->wvals.as<int>(), t->wkeys2.as<uint64_t>(),
-                             t->wvals2.as<int>(), warps, t->whist, t->wscan, s->stream))
-        return false;
-      t->n_perm_warps = warps;
-    }
+  unsigned combos = 0;
+  if (image_combos(P, P.n_img, combos)) {
+    cudaEventRecord(s->ev1, s->stream);
+    P.near2 = s->P.near2;
+    if (!launch_multi(s, t, P, order, s->status.as<int2>(), nullptr, pos, n_t, own_tree ? t->n_nodes : n_t, combos,
+                      v_nl, v_img, own_tree))
+      return false;
     return read_counters(s, t);
+  }
+  const TreeView tv = view_of(t);
+  cudaEventRecord(s->ev1, s->stream);
+  const int warps = (n_t + 31) / 32;
+  const int blocks = (warps * 32 + 127) / 128;
+  if (mixed) {
+    k_walk_nodes<true><<<blocks, 128, 0, s->stream>>>(P, tv, order, s->status.as<int2>(), pos, n_t,
+                                                       v_nl, v_img, ctr);
+    OV_LAUNCHED();
   } else {
-    int warps = (n_t + 31) / 32;
-    int blocks = (warps * 32 + 127) / 128;
-    if (mixed) {
-      k_walk_nodes<true><<<blocks, 128, 0, s->stream>>>(P, tv, order, s->status.as<int2>(), pos, n_t,
-                                                         v_nl, v_img, ctr);
-      OV_LAUNCHED();
-    } else {
-      k_walk_nodes<false><<<blocks, 128, 0, s->stream>>>(P, tv, order, s->status.as<int2>(), pos, n_t,
-                                                          v_nl, v_img, ctr);
-      OV_LAUNCHED();
-    }
+    k_walk_nodes<false><<<blocks, 128, 0, s->stream>>>(P, tv, order, s->status.as<int2>(), pos, n_t,
+                                                        v_nl, v_img, ctr);
+    OV_LAUNCHED();
   }
   OV_TRY_CUDA(cudaGetLastError());
   cudaEventRecord(s->ev2, s->stream);
@@ -1116,14 +1296,38 @@ bool ov_tree_walk_points(ov_state_impl* s, OvTree* t, int npts, const double* pt
   }
   unsigned long long* ctr = reinterpret_cast<unsigned long long*>(t->counters.as<char>() + 64);
   OV_TRY_CUDA(cudaMemsetAsync(ctr, 0, 24, s->stream));
-  int warps = (npts + 31) / 32;
-  int blocks = (warps * 32 + 127) / 128;
-  TreeView tv = view_of(t);
   OvParams P = t->P;
   P.n_img = s->P.n_img;
   for (int j = 0; j < P.n_img; ++j)
     for (int c = 0; c < 4; ++c) P.img[j][c] = s->P.img[j][c];
-  int use_thr = theta == t->theta;
+  const int use_thr = theta == t->theta;
+  unsigned combos = 0;
+  // One traversal per point for all its images, the points in Hilbert order
+  // of the box so a warp's 32 are close together: 4096 probes of a 50k-node
+  // tangle with 26 images take 2.9 ms, against 129 ms with one walk per image
+  // and the points as given.  FP64 in the mixed form too (a query's cost is
+  // its traversal).  A table with mirrors, or an opening angle other than the
+  // tree's, takes the walk per image.
+  if (use_thr && image_combos(P, out_img ? P.n_img : 0, combos)) {
+    const int* order = nullptr;
+    if (npts > 32) {
+      const size_t np = (size_t)npts;
+      if (!t->pkeys.reserve(sizeof(uint64_t) * 2 * np) || !t->pvals.reserve(sizeof(int) * 2 * np)) return false;
+      uint64_t* keys = t->pkeys.as<uint64_t>();
+      int* vals = t->pvals.as<int>();
+      k_curve_keys<<<(npts + 255) / 256, 256, 0, s->stream>>>(P, pts, nullptr, npts, keys, vals);
+      OV_LAUNCHED();
+      if (!ov_radix_sort_u64(keys, vals, keys + np, vals + np, npts, 3 * kCurveBits, t->whist, t->wscan, s->stream))
+        return false;
+      order = vals;
+    }
+    P.precision = OV_PREC_FP64;
+    if (!launch_multi(s, t, P, order, nullptr, skip, pts, npts, npts, combos, out_nl, out_img, false)) return false;
+    return read_counters(s, t);
+  }
+  const int warps = (npts + 31) / 32;
+  const int blocks = (warps * 32 + 127) / 128;
+  const TreeView tv = view_of(t);
   if (s->P.precision == OV_PREC_MIXED) {
     k_walk_points<true><<<blocks, 128, 0, s->stream>>>(P, tv, pts, skip, npts, use_thr, theta,
                                                         out_nl, out_img, ctr);

@@ -399,6 +399,32 @@ def test_bh_tree_beyond_one_million_nodes(ov, oracle):
     st.close()
 
 
+@pytest.mark.parametrize("boundary", ["open", "periodic-26", "periodic-z-open-xy"])
+@pytest.mark.parametrize("rings,grain", [(1, 1e-8), (12, 1e-8), (40, 3e-3)])
+def test_split_walk_vs_oracle(ov, oracle, boundary, rings, grain):
+    """Walks whose groups of 32 targets are split over several warps, and
+    point queries around the group size, some points outside the box, with
+    leaves of several nodes (grain 3e-3): node velocities in both forms and
+    FP64 points against the oracle's recursive tree."""
+    from openvort_b200.tangle import IMAGE_TABLES
+    t = G.random_ring_tangle(40 + rings, rings, 0.1, boundary=boundary, empty_slots=3)
+    p = Params(core_a=1.3e-8, alpha=0.098, alpha_p=0.016, dl_max=1e-3, use_bh=1, bh_theta=0.4, bh_grain=grain,
+               vn=Flow("simple", {"external_v": (0.5, 0, 0)}))
+    ref = oracle.update_tangle(t, p)
+    assert rel_err(gpu_update(ov, t, p).vels, ref.vels, t.active) < TOL_V64
+    assert rel_err(gpu_update(ov, t, p, precision=1).vels, ref.vels, t.active) < TOL_MIXED
+    ov.configure(p, 0)
+    st = ov.DeviceState(t.copy())
+    rng = np.random.default_rng(rings)
+    for npts in (1, 31, 33, 200):
+        pts = rng.uniform(-0.01, 0.11, size=(npts, 3))
+        want = oracle.bh_at(t, p, pts)
+        for sh, _ in IMAGE_TABLES[boundary]:
+            want = want + oracle.bh_at(t, p, pts - 0.1 * np.array(sh))
+        assert rel_err(st.eval_points(pts, method=1), want) < TOL_V64
+    st.close()
+
+
 def _ring5():
     from openvort_b200.tangle import ring_points
     r = ring_points(np.array([0.05, 0.05, 0.05]), (0.3, 0.2, 0.9), 0.004, 5)
