@@ -152,50 +152,132 @@ __device__ __forceinline__ d3 seg_vel64(double f4pi, d3 r1, d3 r2, d3 r, double 
 }
 
 // 1/sqrt(x) and 1/x in FP64 from the hardware approximations
-// (rsqrt.approx.f64, rcp.approx.ftz.f64, relative error ~2^-22) refined by
-// two Newton-Raphson steps each, which square the relative error per step:
-//   1/sqrt(x):  y <- y + y (1 - x y^2) / 2
-//   1/x:        y <- y + y (1 - x y)
-// The results are within a few ulps of the correctly rounded values
-// (ov_check_fast_math measures this on the device); positive normal x only.
+// (rsqrt.approx.ftz.f64, rcp.approx.ftz.f64, relative error ~2^-21) refined by
+// one third-order step each (Householder's method): with r = 1 - x y^2,
+// e = 1 - x y,
+//   1/sqrt(x) = y (1 - r)^(-1/2) ~ y + y r (1/2 + 3 r / 8)    remainder 5 r^3 / 16
+//   1/x       = y / (1 - e)      ~ y + y (e + e^2)            remainder e^3
+// 5 and 3 operations against 8 and 4 for two Newton-Raphson steps, with
+// remainders below 2^-59.  The results are within an ulp of the correctly
+// rounded values (ov_check_fast_math measures this on the device); positive
+// normal x only.
 __device__ __forceinline__ double rsqrt_nr(double x) {
   double y;
-  asm("rsqrt.approx.f64 %0, %1;" : "=d"(y) : "d"(x));
-#pragma unroll
-  for (int i = 0; i < 2; ++i) {
-    const double r = fma(-(x * y), y, 1.0);
-    y = fma(0.5 * y, r, y);
-  }
-  return y;
+  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+  const double r = fma(-(x * y), y, 1.0);
+  return fma(y * r, fma(0.375, r, 0.5), y);
 }
 __device__ __forceinline__ double rcp_nr(double x) {
   double y;
   asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-#pragma unroll
-  for (int i = 0; i < 2; ++i) {
-    const double e = fma(-x, y, 1.0);
-    y = fma(y, e, y);
-  }
-  return y;
+  const double e = fma(-x, y, 1.0);
+  return fma(y, fma(e, e, e), y);
 }
+
+// The colinearity cut-off |cos - 1| < col decided from den = 1 + cos as the
+// refined reciprocals give it.  That den and the reference's quotient both
+// carry a few ulps (errors below 2e-15); outside a band of 1e-14 (or 1e-6 of
+// the cut-off) around 2 - col they decide alike: den < lo adds the segment,
+// den > hi drops it, and in between the reference's own operations decide.
+// col = 0 (the cut-off off): every segment is added.
+struct ColCut {
+  double lo, hi, col;
+};
+__host__ __device__ __forceinline__ ColCut col_cut_of(double col) {
+  const double m = col * 1e-6 > 1e-14 ? col * 1e-6 : 1e-14;
+  const double inf = 1.7976931348623157e308;
+  return ColCut{col > 0 ? 2.0 - (col + m) : inf, col > m ? 2.0 - (col - m) : inf, col};
+}
+// an endpoint nearer than 1.5e-8, where the reference's distance cut-off
+// (1e-8) could decide: a test on the high word, an integer operation
+__device__ __forceinline__ bool near_end(double R2) { return __double2hiint(R2) <= 0x3cb03684; }
 
 // The reference's segment formula without IEEE square roots and divisions:
 // with u = 1/(|R||R'|) from two refined reciprocal square roots,
 //   f (|R| + |R'|) / (|R||R'| (|R||R'| + R.R')) = f (1/|R| + 1/|R'|) u / (1 + R.R' u).
 // R' = R + d (d = r2 - r1, staged per segment) differs from r2 - r by an ulp
-// of |R'|.  Where either cut-off could decide (|R| or |R'| within 1.5x of
-// 1e-8, or cos within 2e-8 of 1) the reference's own operations decide
-// (seg_vel64), so every cut-off decision is the reference's.
-__device__ __forceinline__ d3 seg_vel64_nr(double f4pi, d3 r1, d3 r2, d3 d, d3 r, double col = 1e-8) {
+// of |R'|.  Where either cut-off could decide (near_end, ColCut) the
+// reference's own operations decide (seg_vel64), so every cut-off decision is
+// the reference's.
+__device__ __forceinline__ d3 seg_vel64_nr(double f4pi, d3 r1, d3 r2, d3 d, d3 r,
+                                           ColCut cut = col_cut_of(1e-8)) {
   const d3 R = r1 - r;
   const d3 Rp = R + d;
   const double R2 = dot3(R, R), Rp2 = dot3(Rp, Rp), RRp = dot3(R, Rp);
-  if (R2 < 2.25e-16 || Rp2 < 2.25e-16) return seg_vel64(f4pi, r1, r2, r, col);
+  const bool near = near_end(R2) || near_end(Rp2);
   const double ia = rsqrt_nr(R2), ib = rsqrt_nr(Rp2);
   const double u = ia * ib;
-  if (fabs(fma(RRp, u, -1.0)) < 2.0 * col) return seg_vel64(f4pi, r1, r2, r, col);
-  const double s = f4pi * (ia + ib) * (u * rcp_nr(fma(RRp, u, 1.0)));
-  return cross3(R, Rp) * s;
+  const double den = fma(RRp, u, 1.0);
+  if (!near && den < cut.lo) return cross3(R, Rp) * (f4pi * (ia + ib) * (u * rcp_nr(den)));
+  if (!near && den > cut.hi) return mk3(0, 0, 0);
+  return seg_vel64(f4pi, r1, r2, r, cut.col);
+}
+
+// The chain sweep: cnt staged slots, the segment from node i to node i + 1
+// where bit i of `chain` (words of 32) is set, summed at r without the factor
+// kappa/4pi.  Each node's R = r_node - r and refined 1/|R| are formed once
+// and serve both segments that touch it; R' is r2 - r itself, as the
+// reference forms it (src/tangle.c:490-491).  A segment then costs 32 FP64
+// operations: R, |R|^2, R.R' 9; the reciprocals 5 and 3; the weight 5; cross
+// product and sum 9; the cut-off 1.  Slots whose segment does not run to the
+// next slot have their bit in `other` and take other_seg(i), in place, so the
+// terms are added in slot order whatever the staging.  kSkip: segments from
+// or to node `skip` (an index into the staged nodes) are left out.
+// Groups of kChainGroup segments are summed without a branch (a segment left
+// out has weight zero), so their dependency chains overlap; the segments the
+// reference's own operations decide follow the group.  Groups of 1 / 2 / 4:
+// 42.6 / 36.3 / 35.7 ms at 22.4k nodes and 26 images; two targets per thread
+// took 35.7 to 40 ms.
+constexpr int kChainGroup = 4;
+template <bool kSkip, class Other>
+__device__ __forceinline__ void chain64_sweep(const double (*nd)[3], const unsigned* chain, const unsigned* other,
+                                              int cnt, int skip, d3 r, const ColCut& cut, d3& acc,
+                                              Other&& other_seg) {
+  d3 Ra = mk3(nd[0][0], nd[0][1], nd[0][2]) - r;
+  const double Ra2 = dot3(Ra, Ra);
+  double ia = rsqrt_nr(Ra2);
+  bool na = near_end(Ra2);
+  for (int i0 = 0; i0 < cnt; i0 += kChainGroup) {
+    const unsigned bits = chain[i0 >> 5] >> (i0 & 31), rest = other[i0 >> 5] >> (i0 & 31);
+    bool slow[kChainGroup];
+    bool any = false;
+#pragma unroll
+    for (int q = 0; q < kChainGroup; ++q) {
+      const int i = i0 + q;
+      const d3 Rb = mk3(nd[i + 1][0], nd[i + 1][1], nd[i + 1][2]) - r;
+      const double Rb2 = dot3(Rb, Rb);
+      const double ib = rsqrt_nr(Rb2);
+      const bool nb = near_end(Rb2);
+      const double u = ia * ib;
+      const double den = fma(dot3(Ra, Rb), u, 1.0);
+      bool on = (bits >> q) & 1u;
+      if (kSkip) on = on && i != skip && i + 1 != skip;
+      const bool fast = !na && !nb && den < cut.lo;
+      slow[q] = on && !fast && (na || nb || !(den > cut.hi));
+      any = any || slow[q];
+      const double w = on && fast ? (ia + ib) * (u * rcp_nr(den)) : 0.0;
+      const d3 c = cross3(Ra, Rb);
+      acc.x = fma(c.x, w, acc.x);
+      acc.y = fma(c.y, w, acc.y);
+      acc.z = fma(c.z, w, acc.z);
+      Ra = Rb;
+      ia = ib;
+      na = nb;
+    }
+    if (any) {
+#pragma unroll
+      for (int q = 0; q < kChainGroup; ++q) {
+        const int i = i0 + q;
+        if (slow[q])
+          acc = acc + seg_vel64(1.0, mk3(nd[i][0], nd[i][1], nd[i][2]),
+                                mk3(nd[i + 1][0], nd[i + 1][1], nd[i + 1][2]), r, cut.col);
+      }
+    }
+    if (rest & ((1u << kChainGroup) - 1)) {
+      for (int q = 0; q < kChainGroup; ++q)
+        if ((rest >> q) & 1u) acc = acc + other_seg(i0 + q);
+    }
+  }
 }
 
 // FP32 far-field form: R and the segment vector ds are formed in FP64 by the

@@ -70,6 +70,7 @@ __global__ void __launch_bounds__(kTB) k_direct64(OvParams P, SegTab S, int n_sr
   }
   double ax = 0, ay = 0, az = 0;
   const double f4pi = P.f4pi;
+  const ColCut cut = col_cut_of(P.col_cut);
   const int s_lo = blockIdx.z * chunk, s_hi = min(n_src, s_lo + chunk);
   for (int base = s_lo; base < s_hi; base += kTS) {
     __syncthreads();
@@ -97,7 +98,7 @@ __global__ void __launch_bounds__(kTB) k_direct64(OvParams P, SegTab S, int n_sr
       if (fw == -1 || id == skip || fw == skip) continue;
       d3 v = seg_vel64_nr(f4pi, mk3(sh_r[q][0], sh_r[q][1], sh_r[q][2]),
                           mk3(sh_r[q][3], sh_r[q][4], sh_r[q][5]),
-                          mk3(sh_r[q][6], sh_r[q][7], sh_r[q][8]), r, P.col_cut);
+                          mk3(sh_r[q][6], sh_r[q][7], sh_r[q][8]), r, cut);
       ax += v.x; ay += v.y; az += v.z;
     }
   }
@@ -109,17 +110,18 @@ __global__ void __launch_bounds__(kTB) k_direct64(OvParams P, SegTab S, int n_sr
 
 // FP64 in chain order: sources in slot order, where a loop's segments
 // follow one another (segment m runs from node m to its forward node m + 1
-// for all but one segment per loop).  Each node's R = r_node - r, |R|^2 and
-// refined 1/|R| are formed once per target and serve both segments that
-// touch it, so a chained segment costs its R.R', one refined reciprocal and
-// the cross product: about 42 FP64 operations against 55 for seg_vel64_nr.
-// R' is r2 - r itself, as the reference forms it (src/tangle.c:490-491).
-// The cut-offs are decided as in seg_vel64_nr: where |R| or |R'| is within
-// 1.5e-8 or cos within 2e-8 of 1, the reference's own operations decide
-// (seg_vel64).  Segments that do not chain (a loop's closing segment, one
-// wrapped across a periodic face) take seg_vel64_nr from a list.  Block =
-// kTB targets x one image; targets are node slots (status-filtered, skip =
-// the slot) or explicit points (kPoints, skip from tskip).
+// for all but one segment per loop), through chain64_sweep, which forms each
+// node's terms once for the two segments that touch it.  Segments that do
+// not chain (a loop's closing segment, one wrapped across a periodic face)
+// take seg_vel64_nr in place.  Block = kTB targets x one image; targets
+// are node slots (status-filtered) or explicit points (kPoints, skip from
+// tskip).  A node's own two chained segments end at the target itself, where
+// the reference's distance cut-off returns zero, so the skip rule needs no
+// test of its own there.
+// Bound by the FP64 pipe.  22.4k nodes, 26 images: 36.4 ms,
+// 47% of the FP64 FMA peak by the 43-flop count (54 ms when the reciprocals
+// took two Newton-Raphson steps each, every segment branched and the sum was
+// scaled term by term); the FP64 pipe is 71% busy, 4 resident blocks.
 constexpr int kCS = 128;   // chained segments per shared-memory tile
 static_assert(kCS == kTS, "the chain sweep splits sources as k_direct64 does");
 
@@ -131,9 +133,7 @@ __global__ void __launch_bounds__(kTB) k_direct64_chain(OvParams P, SegTab S, in
                                                         const int* __restrict__ tskip, int n_t,
                                                         double* __restrict__ part, int chunk) {
   __shared__ double sh_node[kCS + 1][3];
-  __shared__ int sh_kind[kCS];   // 1: chained, 0: no segment or in the list
-  __shared__ int sh_irr[kCS];
-  __shared__ int sh_nirr;
+  __shared__ unsigned sh_chain[kCS / 32], sh_other[kCS / 32];   // chained and other segments
   const int j = blockIdx.y;   // 0: the tangle itself, j >= 1: image j-1
   const int k = blockIdx.x * kTB + threadIdx.x;
   bool act = k < n_t;
@@ -145,12 +145,10 @@ __global__ void __launch_bounds__(kTB) k_direct64_chain(OvParams P, SegTab S, in
     if (j > 0) r = image_point(P, j - 1, r);
     else skip = kPoints ? (tskip ? tskip[k] : -1) : k;
   }
-  double ax = 0, ay = 0, az = 0;
-  const double f4pi = P.f4pi;
+  d3 acc = mk3(0, 0, 0);
+  const ColCut cut = col_cut_of(P.col_cut);
   const int s_lo = blockIdx.z * chunk, s_hi = min(n_src, s_lo + chunk);
   for (int sb = s_lo; sb < s_hi; sb += kCS) {
-    __syncthreads();
-    if (threadIdx.x == 0) sh_nirr = 0;
     __syncthreads();
     // nodes sb .. sb + kCS (positions; a slot beyond the range or EMPTY is
     // used by no chained segment)
@@ -164,74 +162,41 @@ __global__ void __launch_bounds__(kTB) k_direct64_chain(OvParams P, SegTab S, in
     for (int i = threadIdx.x; i < kCS; i += kTB) {
       const int m = sb + i;
       const int fw = m < s_hi ? S.fwd[m] : -1;
-      int kind = 0;
+      bool chained = false;
       if (fw >= 0) {
         const double* sg = S.r1r2 + 6 * (size_t)m;
-        bool chained = fw == m + 1;
+        chained = fw == m + 1;
         if (chained) {
           const d3 e = ld3(pos, fw);
           chained = e.x == sg[3] && e.y == sg[4] && e.z == sg[5];
         }
-        if (chained) kind = 1;
-        else sh_irr[atomicAdd(&sh_nirr, 1)] = m;
       }
-      sh_kind[i] = kind;
+      const unsigned bits = __ballot_sync(0xffffffffu, chained);
+      const unsigned rest = __ballot_sync(0xffffffffu, fw >= 0 && !chained);
+      if ((i & 31) == 0) {
+        sh_chain[i >> 5] = bits;
+        sh_other[i >> 5] = rest;
+      }
     }
     __syncthreads();
     if (!act) continue;
-    // node 0 of the tile
-    d3 Ra = mk3(sh_node[0][0], sh_node[0][1], sh_node[0][2]) - r;
-    double Ra2 = dot3(Ra, Ra);
-    double ia = Ra2 >= 2.25e-16 ? rsqrt_nr(Ra2) : 0.0;
-    const int cnt = min(kCS, s_hi - sb);
-#pragma unroll 2
-    for (int i = 0; i < cnt; ++i) {
-      const d3 nb = mk3(sh_node[i + 1][0], sh_node[i + 1][1], sh_node[i + 1][2]);
-      const d3 Rb = nb - r;
-      const double Rb2 = dot3(Rb, Rb);
-      const double ib = Rb2 >= 2.25e-16 ? rsqrt_nr(Rb2) : 0.0;
-      const int m = sb + i;
-      // skip rule of calculate_vs_shift (src/tangle.c:567-569): segment m
-      // runs from m to m + 1
-      if (sh_kind[i] && m != skip && m + 1 != skip) {
-        d3 v;
-        const double RRp = dot3(Ra, Rb);
-        const double u = ia * ib;
-        if (Ra2 < 2.25e-16 || Rb2 < 2.25e-16 || fabs(fma(RRp, u, -1.0)) < 2.0 * P.col_cut) {
-          v = seg_vel64(f4pi, mk3(sh_node[i][0], sh_node[i][1], sh_node[i][2]), nb, r, P.col_cut);
-        } else {
-          const double sc = f4pi * (ia + ib) * (u * rcp_nr(fma(RRp, u, 1.0)));
-          v = cross3(Ra, Rb) * sc;
-        }
-        ax += v.x;
-        ay += v.y;
-        az += v.z;
-      }
-      Ra = Rb;
-      Ra2 = Rb2;
-      ia = ib;
-    }
-    // the segments that do not chain
-    const int nirr = sh_nirr;
-    for (int q = 0; q < nirr; ++q) {
-      const int m = sh_irr[q];
-      const int fw = S.fwd[m];
-      if (m == skip || fw == skip) continue;
-      const double* sg = S.r1r2 + 6 * (size_t)m;
-      const d3 r1 = mk3(sg[0], sg[1], sg[2]), r2 = mk3(sg[3], sg[4], sg[5]);
-      const d3 v = seg_vel64_nr(f4pi, r1, r2, r2 - r1, r, P.col_cut);
-      ax += v.x;
-      ay += v.y;
-      az += v.z;
-    }
+    chain64_sweep<kPoints>(sh_node, sh_chain, sh_other, min(kCS, s_hi - sb), skip >= 0 ? skip - sb : -2, r, cut, acc,
+                           [&](int i) {
+                             const int m = sb + i;
+                             if (m == skip || S.fwd[m] == skip) return mk3(0, 0, 0);
+                             const double* sg = S.r1r2 + 6 * (size_t)m;
+                             const d3 r1 = mk3(sg[0], sg[1], sg[2]), r2 = mk3(sg[3], sg[4], sg[5]);
+                             return seg_vel64_nr(1.0, r1, r2, r2 - r1, r, cut);
+                           });
   }
   if (k < n_t) {
     double* o = part + ((size_t)blockIdx.z * gridDim.y + j) * 3 * (size_t)n_t + 3 * (size_t)k;
-    o[0] = act ? ax : 0;
-    o[1] = act ? ay : 0;
-    o[2] = act ? az : 0;
+    o[0] = act ? P.f4pi * acc.x : 0;
+    o[1] = act ? P.f4pi * acc.y : 0;
+    o[2] = act ? P.f4pi * acc.z : 0;
   }
 }
+static_assert(kCS == kTB, "every thread stages one segment (the ballot needs whole warps)");
 
 // Mixed form, two sources per instruction.  Block = kPB threads x kTT
 // targets (the tree's key order, so close in space) x one image.  The
@@ -285,7 +250,9 @@ __global__ void __launch_bounds__(kPB, OV_DIRECT_PAIRS_MIN_BLOCKS) k_direct_mixe
   for (int u = 0; u < kTT; ++u) acc[u][0] = acc[u][1] = acc[u][2] = 0;
   const double f4pi = P.f4pi;
   // FP64 evaluation of segment id at target u (skip rule of
-  // calculate_vs_shift, src/tangle.c:567-569, for the tangle itself)
+  // calculate_vs_shift, src/tangle.c:567-569, for the tangle itself), out of
+  // the way in IEEE operations: seg_vel64_nr inlined here costs the main loop
+  // registers (18.0 against 17.2 ms at 22.4k nodes)
   auto special = [&](int u, int id) {
 #pragma unroll
     for (int v = 0; v < kTT; ++v) {
@@ -297,7 +264,8 @@ __global__ void __launch_bounds__(kPB, OV_DIRECT_PAIRS_MIN_BLOCKS) k_direct_mixe
       d3 r = ld3(pos, k);
       if (j > 0) r = image_point(P, j - 1, r);
       const double* sg = S.r1r2 + 6 * (size_t)id;
-      const d3 vv = seg_vel64(f4pi, mk3(sg[0], sg[1], sg[2]), mk3(sg[3], sg[4], sg[5]), r);
+      const d3 r1 = mk3(sg[0], sg[1], sg[2]), r2 = mk3(sg[3], sg[4], sg[5]);
+      const d3 vv = seg_vel64(f4pi, r1, r2, r);
       acc[v][0] += vv.x;
       acc[v][1] += vv.y;
       acc[v][2] += vv.z;
@@ -397,6 +365,8 @@ __global__ void __launch_bounds__(kPB, OV_DIRECT_CHAIN_MIN_BLOCKS) k_direct_mixe
 #pragma unroll
   for (int u = 0; u < kTT; ++u) acc[u][0] = acc[u][1] = acc[u][2] = 0;
   const double f4pi = P.f4pi;
+  // near pairs in FP64, a large share of a small sum: refined reciprocals
+  // (2000 open nodes 0.074 ms, against 0.100 with IEEE operations)
   auto special = [&](int u, int id) {
 #pragma unroll
     for (int v = 0; v < kTT; ++v) {
@@ -408,7 +378,8 @@ __global__ void __launch_bounds__(kPB, OV_DIRECT_CHAIN_MIN_BLOCKS) k_direct_mixe
       d3 r = ld3(pos, k);
       if (j > 0) r = image_point(P, j - 1, r);
       const double* sg = S.r1r2 + 6 * (size_t)id;
-      const d3 vv = seg_vel64(f4pi, mk3(sg[0], sg[1], sg[2]), mk3(sg[3], sg[4], sg[5]), r);
+      const d3 r1 = mk3(sg[0], sg[1], sg[2]), r2 = mk3(sg[3], sg[4], sg[5]);
+      const d3 vv = seg_vel64_nr(f4pi, r1, r2, r2 - r1, r);
       acc[v][0] += vv.x;
       acc[v][1] += vv.y;
       acc[v][2] += vv.z;
@@ -574,7 +545,8 @@ __global__ void __launch_bounds__(kPB) k_direct_mixed_points(OvParams P, SegTab 
       const int fw = S.fwd[id];
       if (j == 0 && (id == kk[v] || fw == kk[v])) return;
       const double* sg = S.r1r2 + 6 * (size_t)id;
-      const d3 vv = seg_vel64(f4pi, mk3(sg[0], sg[1], sg[2]), mk3(sg[3], sg[4], sg[5]), rr[v]);
+      const d3 r1 = mk3(sg[0], sg[1], sg[2]), r2 = mk3(sg[3], sg[4], sg[5]);
+      const d3 vv = seg_vel64(f4pi, r1, r2, rr[v]);
       acc[v][0] += vv.x;
       acc[v][1] += vv.y;
       acc[v][2] += vv.z;

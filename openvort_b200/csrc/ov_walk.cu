@@ -70,7 +70,7 @@ __device__ __forceinline__ double mac_dist2(const OvParams& P, d3 r, double cx, 
 // m = (M21, M02, M12, M22).
 __device__ __forceinline__ d3 expansion64(const double* g, const double* m, d3 R) {
   const double R2 = dot3(R, R);
-  const double inv = rsqrt(R2);
+  const double inv = rsqrt_nr(R2);
   const double inv2 = inv * inv;
   const double i3 = inv2 * inv;
   const double w = R.z * inv2;
@@ -116,7 +116,7 @@ __device__ __forceinline__ void p2p_one(const OvParams& P, d3 r1, d3 r2, d3 rp, 
       return;
     }
   }
-  d3 v = seg_vel64(P.f4pi, r1, r2, rp);
+  const d3 v = seg_vel64_nr(P.f4pi, r1, r2, r2 - r1, rp);
   ax += v.x; ay += v.y; az += v.z;
 }
 
@@ -259,7 +259,9 @@ __device__ __forceinline__ float sel3f(int i, float a, float b, float c) {
 // expansion at one image offset.  Inlined: out of line (__noinline__) the
 // calls' register saves made the mixed walk 52.1 ms per launch at 1M points
 // against 37.9 ms.
-__device__ __forceinline__ d3 seg64_at(double f4pi, d3 r1, d3 r2, d3 t) { return seg_vel64(f4pi, r1, r2, t); }
+__device__ __forceinline__ d3 seg64_at(double f4pi, d3 r1, d3 r2, d3 t) {
+  return seg_vel64_nr(f4pi, r1, r2, r2 - r1, t);
+}
 __device__ __forceinline__ d3 expansion64_at(const Cell* cp, d3 R) { return expansion64(cp->y, cp->m, R); }
 
 // One segment r1 -> r2 for every image in `mask`: FP64 with the reference's
@@ -640,7 +642,7 @@ __device__ __forceinline__ void cell_fp64(const OvParams& P, const Cell* cp, dou
     for (int iz = 0; iz < 3; ++iz) {
       if (!((bits >> iz) & 1u)) continue;
       const double Z = Rz[iz];
-      const double inv = rsqrt(fma(Z, Z, XY2));
+      const double inv = rsqrt_nr(fma(Z, Z, XY2));
       const double inv2 = inv * inv;
       const double i3 = inv2 * inv;
       const double i5 = (i3 * inv2) * Z;
