@@ -484,20 +484,20 @@ __device__ __forceinline__ void cell_mixed(const OvParams& P, const Cell* cp, fl
     // P_x, P_y, Q_x, Q_y take each column's sums of i3 and i5 once.
     f2 px = f2_splat(0.f), py = px, pz = px, qx = px, qy = px, qz = px, sv = px;
     // All 27 images accept (the usual case: the wrapped opening test
-    // treats every image point like the target) and none is near:
-    // no per-image masks or near-field tests.  An image shifted
+    // treats every image point like the target) and none but the tangle's own
+    // is near: no per-image masks or near-field tests.  An image shifted
     // along an axis has |R|^2 >= that axis offset squared (FP32
     // rounding of sums of non-negative terms is monotonic), so when
-    // every shifted offset and the target's own |R|^2 reach the near
-    // radius, no image takes the FP64 path.
-    bool all_far = pass == kAllImages;
-    if (all_far && test_near) {
+    // every shifted offset reaches the near radius, only the tangle's own
+    // image can take the FP64 path; its weight here is then zero.
+    bool all = pass == kAllImages, near0 = false;
+    if (all && test_near) {
       const float X = Fx[1], Y = Fy[1], Z = Fz[1];
-      all_far = fmaf(Z, Z, fmaf(X, X, Y * Y)) >= fnear2 && Fx[0] * Fx[0] >= fnear2 &&
-                Fx[2] * Fx[2] >= fnear2 && Fy[0] * Fy[0] >= fnear2 && Fy[2] * Fy[2] >= fnear2 &&
-                Fz[0] * Fz[0] >= fnear2 && Fz[2] * Fz[2] >= fnear2;
+      near0 = fmaf(Z, Z, fmaf(X, X, Y * Y)) < fnear2;
+      all = Fx[0] * Fx[0] >= fnear2 && Fx[2] * Fx[2] >= fnear2 && Fy[0] * Fy[0] >= fnear2 &&
+            Fy[2] * Fy[2] >= fnear2 && Fz[0] * Fz[0] >= fnear2 && Fz[2] * Fz[2] >= fnear2;
     }
-    if (all_far) {
+    if (all) {
       // unrolled: the column offsets are chosen at compile time
 #pragma unroll
       for (int grp = 0; grp < 5; ++grp) {
@@ -516,6 +516,7 @@ __device__ __forceinline__ void cell_mixed(const OvParams& P, const Cell* cp, fl
           const f2 Zs = f2_splat(Fz[iz]);
           f2 inv = f2_rsqrt(f2_fma(Zs, Zs, XY2));
           if (grp == 4) inv = inv * keep;
+          if (grp == 2 && iz == 1) inv = inv * f2_pack(near0 ? 0.f : 1.f, 1.f);
           const f2 inv2 = inv * inv;
           const f2 i3 = inv2 * inv;
           const f2 i5 = (i3 * inv2) * Zs;
@@ -530,6 +531,8 @@ __device__ __forceinline__ void cell_mixed(const OvParams& P, const Cell* cp, fl
         qy = f2_fma(c5, Y, qy);
         sv = sv + c3;
       }
+      if (near0)
+        nl = nl + expansion64_at(cp, mk3(__dsub_rn(r.x, cx), __dsub_rn(r.y, cy), __dsub_rn(r.z, cz)));
     } else {
 #pragma unroll 1
     for (int grp = 0; grp < 5; ++grp) {
