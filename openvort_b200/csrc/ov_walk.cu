@@ -235,6 +235,7 @@ constexpr int kLevelSlots = 34;
 // (half a box less a rounding allowance; DBL_MAX on axes without shifts).
 struct ImageShortcut {
   double hw[3];
+  double wr[3];     // the smallest |c - r| at which the target's own image surely wraps (DBL_MAX: no shifts)
   double half[3];   // L / 2 on periodic axes (the reference's wrap test), DBL_MAX otherwise
   int on;
 };
@@ -298,6 +299,46 @@ __device__ __forceinline__ unsigned mac_exact(const OvParams& P, d3 r, double cx
     }
   }
   return pass;
+}
+
+// The images of a cell whose opening test the target's own image fails by
+// the margin E, from two distances per axis (dx = cx - r.x and so on, not
+// wrapped).  Along an axis where |d| <= hw every image's wrapped distance is
+// |d|.  Where |d| >= wr the target's own image wraps, to |d| - L: the image
+// shifted towards the cell has that distance too, and the one shifted away
+// wraps back to |d|.  So the images fall into the products of "same" and
+// "away" along the wrapped axes.  Each product's squared distance is formed
+// here within the rounding that E covers (mac_margin: every component within
+// e of its exact value), so it decides its images when it is E away from the
+// threshold.  False when a product is not, or an axis lies between hw and wr:
+// the caller then takes the images' decisions in full.
+// (22.4k nodes, theta = 0.4: 248 of a group's 1478 visits took mac_exact for
+// such cells.)
+__device__ __forceinline__ bool wrapped_decisions(const OvParams& P, const ImageShortcut& S, d3 r, double cx,
+                                                  double cy, double cz, double dx, double dy, double dz, double thr,
+                                                  double E, unsigned& pass) {
+  const double ax = fabs(dx), ay = fabs(dy), az = fabs(dz);
+  const bool wx = ax > S.hw[0], wy = ay > S.hw[1], wz = az > S.hw[2];
+  pass = 0;
+  if (!(wx || wy || wz)) return true;   // every image as near as the target
+  if ((wx && ax < S.wr[0]) || (wy && ay < S.wr[1]) || (wz && az < S.wr[2])) return false;
+  // images shifted away along a wrapped axis: shift index 2 for d > 0
+  const unsigned mx = wx ? (dx > 0 ? 0x1ffu << 18 : 0x1ffu) : 0u;
+  const unsigned my = wy ? (dy > 0 ? 0x1c0e07u << 6 : 0x1c0e07u) : 0u;
+  const unsigned mz = wz ? (dz > 0 ? 0x1249249u << 2 : 0x1249249u) : 0u;
+  const double qx = wrapped_sq(P, 0, r.x, cx), qy = wrapped_sq(P, 1, r.y, cy), qz = wrapped_sq(P, 2, r.z, cz);
+  const double hi = thr + E, lo = thr - E;
+  bool clear = true;
+#pragma unroll
+  for (int b = 1; b < 8; ++b) {
+    const unsigned set = ((b & 4) ? mx : ~mx) & ((b & 2) ? my : ~my) & ((b & 1) ? mz : ~mz);
+    if (!(set & kAllImages) || ((b & 4) && !wx) || ((b & 2) && !wy) || ((b & 1) && !wz)) continue;
+    const double q = ((b & 4) ? dx * dx : qx) + ((b & 2) ? dy * dy : qy) + ((b & 1) ? dz * dz : qz);
+    if (q >= hi) pass |= set;
+    else if (q >= lo) clear = false;
+  }
+  pass &= kAllImages;
+  return clear;
 }
 
 template <bool kMixed>
@@ -443,6 +484,24 @@ __device__ __forceinline__ void p2p_mixed_columns(const OvParams& P, unsigned ma
 // images at which a segment is evaluated by columns rather than one by one
 constexpr int kColumnImages = 8;
 
+// images from which a product of shift sets takes the unrolled image loop
+// (1M nodes mixed, ms per walk: 27.7 from 4, 6 or 8 images, 28.0 from 12,
+// 28.5 from 18, 32.2 with only full masks; fewer images run only a few
+// groups of the masked loop, the tangle's own image alone just one)
+constexpr int kProductImages = 6;
+
+// Whether an image mask is a product of per-axis shift sets (bit i of
+// mx: shift i - 1 along x, and so on).  The masks of partly accepted cells
+// mostly are: an opening test's images differ along the axes where the
+// target's offset wraps.
+__device__ __forceinline__ bool product_mask(unsigned m, unsigned& mx, unsigned& my, unsigned& mz) {
+  const unsigned a = m & 511u, b = (m >> 9) & 511u, c = (m >> 18) & 511u, u = a | b | c;
+  mx = (a ? 1u : 0u) | (b ? 2u : 0u) | (c ? 4u : 0u);
+  my = (u & 7u ? 1u : 0u) | (u & 56u ? 2u : 0u) | (u & 448u ? 4u : 0u);
+  mz = (u | (u >> 3) | (u >> 6)) & 7u;
+  return __popc(m) == __popc(mx) * __popc(my) * __popc(mz);
+}
+
 // Mixed form of one accepted cell at every image in `pass` (a 27-bit mask
 // of the combos 9 (sx+1) + 3 (sy+1) + (sz+1)): FP32 expansions from the FP32
 // moments at R = r - L s - com formed in FP64 and rounded once, summed in
@@ -460,15 +519,15 @@ __device__ __forceinline__ void cell_mixed(const OvParams& P, const Cell* cp, fl
   float ax, ay, az;
   {
     // FP32 copies of the FP64-formed offsets r - L s - com per axis and shift
-    const float Fx[3] = {(float)__dsub_rn(img_coord(r.x, P.L[0], 0), cx),
-                         -(float)dc.x,
-                         (float)__dsub_rn(img_coord(r.x, P.L[0], 2), cx)};
-    const float Fy[3] = {(float)__dsub_rn(img_coord(r.y, P.L[1], 0), cy),
-                         -(float)dc.y,
-                         (float)__dsub_rn(img_coord(r.y, P.L[1], 2), cy)};
-    const float Fz[3] = {(float)__dsub_rn(img_coord(r.z, P.L[2], 0), cz),
-                         -(float)dc.z,
-                         (float)__dsub_rn(img_coord(r.z, P.L[2], 2), cz)};
+    float Fx[3] = {(float)__dsub_rn(img_coord(r.x, P.L[0], 0), cx),
+                   -(float)dc.x,
+                   (float)__dsub_rn(img_coord(r.x, P.L[0], 2), cx)};
+    float Fy[3] = {(float)__dsub_rn(img_coord(r.y, P.L[1], 0), cy),
+                   -(float)dc.y,
+                   (float)__dsub_rn(img_coord(r.y, P.L[1], 2), cy)};
+    float Fz[3] = {(float)__dsub_rn(img_coord(r.z, P.L[2], 0), cz),
+                   -(float)dc.z,
+                   (float)__dsub_rn(img_coord(r.z, P.L[2], 2), cz)};
     // an accepting image has |R|^2 >= its wrapped squared distance >=
     // thr, so a cell whose thr reaches the near radius needs no test
     const bool test_near = thr < near2;
@@ -484,13 +543,29 @@ __device__ __forceinline__ void cell_mixed(const OvParams& P, const Cell* cp, fl
     // P_x, P_y, Q_x, Q_y take each column's sums of i3 and i5 once.
     f2 px = f2_splat(0.f), py = px, pz = px, qx = px, qy = px, qz = px, sv = px;
     // All 27 images accept (the usual case: the wrapped opening test
-    // treats every image point like the target) and none but the tangle's own
-    // is near: no per-image masks or near-field tests.  An image shifted
+    // treats every image point like the target), or a product of per-axis
+    // shift sets, and none but the tangle's own image is near: no per-image
+    // masks or near-field tests.  A shift outside its set takes an offset of
+    // 1e18, whose |R|^-3 underflows to an exact zero.  An image shifted
     // along an axis has |R|^2 >= that axis offset squared (FP32
     // rounding of sums of non-negative terms is monotonic), so when
     // every shifted offset reaches the near radius, only the tangle's own
     // image can take the FP64 path; its weight here is then zero.
+    // (1M nodes: 922 visits of a group have a lane with all images, 246 one
+    // with 14 to 26 of them.)
     bool all = pass == kAllImages, near0 = false;
+    if (!all && __popc(pass) >= kProductImages) {
+      unsigned mx, my, mz;
+      all = product_mask(pass, mx, my, mz);
+      if (all) {
+#pragma unroll
+        for (int i = 0; i < 3; ++i) {
+          if (!((mx >> i) & 1u)) Fx[i] = 1e18f;
+          if (!((my >> i) & 1u)) Fy[i] = 1e18f;
+          if (!((mz >> i) & 1u)) Fz[i] = 1e18f;
+        }
+      }
+    }
     if (all && test_near) {
       const float X = Fx[1], Y = Fy[1], Z = Fz[1];
       near0 = fmaf(Z, Z, fmaf(X, X, Y * Y)) < fnear2;
@@ -621,44 +696,91 @@ __device__ __forceinline__ void cell_mixed(const OvParams& P, const Cell* cp, fl
 // factored form into im, as in cell_mixed: with i3 = |R|^-3 and
 // i5 = R_z |R|^-5 per image, the sum of ((g + m R_z/|R|^2) x R + (m21, 0, 0)) i3
 // is g x P + m x Q + (m21 S, 0, 0), P = sum i3 R, Q = sum i5 R, S = sum i3.
+// All images, or a product of shift sets: no branch per image, as in
+// cell_mixed (a shift outside its set takes an offset of 1e150, whose |R|^-3
+// underflows to an exact zero).
 __device__ __forceinline__ void cell_fp64(const OvParams& P, const Cell* cp, double cx, double cy, double cz, d3 r,
                                           unsigned pass, d3& nl, d3& im) {
   const double g[3] = {cp->y[0], cp->y[1], cp->y[2]};
   const double mm[4] = {cp->m[0], cp->m[1], cp->m[2], cp->m[3]};
-  const double Rz[3] = {__dsub_rn(img_coord(r.z, P.L[2], 0), cz), __dsub_rn(r.z, cz),
-                        __dsub_rn(img_coord(r.z, P.L[2], 2), cz)};
   if (pass & (1u << kPrimary))
-    nl = nl + expansion64(g, mm, mk3(__dsub_rn(r.x, cx), __dsub_rn(r.y, cy), Rz[1]));
+    nl = nl + expansion64(g, mm, mk3(__dsub_rn(r.x, cx), __dsub_rn(r.y, cy), __dsub_rn(r.z, cz)));
   const unsigned rest = pass & ~(1u << kPrimary);
   if (!rest) return;
+  double Rx[3] = {__dsub_rn(img_coord(r.x, P.L[0], 0), cx), __dsub_rn(r.x, cx),
+                  __dsub_rn(img_coord(r.x, P.L[0], 2), cx)};
+  double Ry[3] = {__dsub_rn(img_coord(r.y, P.L[1], 0), cy), __dsub_rn(r.y, cy),
+                  __dsub_rn(img_coord(r.y, P.L[1], 2), cy)};
+  double Rz[3] = {__dsub_rn(img_coord(r.z, P.L[2], 0), cz), __dsub_rn(r.z, cz),
+                  __dsub_rn(img_coord(r.z, P.L[2], 2), cz)};
   double px = 0, py = 0, pz = 0, qx = 0, qy = 0, qz = 0, sv = 0;
+  bool all = pass == kAllImages;
+  if (!all && __popc(pass) >= kProductImages) {
+    unsigned mx, my, mz;
+    all = product_mask(pass, mx, my, mz);
+    if (all) {
 #pragma unroll
-  for (int xy = 0; xy < 9; ++xy) {
-    const unsigned bits = (rest >> (3 * xy)) & 7u;
-    if (!bits) continue;
-    const int ix = (xy * 11) >> 5, iy = xy - 3 * ix;
-    const double X = __dsub_rn(img_coord(r.x, P.L[0], ix), cx);
-    const double Y = __dsub_rn(img_coord(r.y, P.L[1], iy), cy);
-    const double XY2 = fma(X, X, Y * Y);
-    double c3 = 0, c5 = 0;
-#pragma unroll
-    for (int iz = 0; iz < 3; ++iz) {
-      if (!((bits >> iz) & 1u)) continue;
-      const double Z = Rz[iz];
-      const double inv = rsqrt_nr(fma(Z, Z, XY2));
-      const double inv2 = inv * inv;
-      const double i3 = inv2 * inv;
-      const double i5 = (i3 * inv2) * Z;
-      c3 += i3;
-      c5 += i5;
-      pz = fma(i3, Z, pz);
-      qz = fma(i5, Z, qz);
+      for (int i = 0; i < 3; ++i) {
+        if (!((mx >> i) & 1u)) Rx[i] = 1e150;
+        if (!((my >> i) & 1u)) Ry[i] = 1e150;
+        if (!((mz >> i) & 1u)) Rz[i] = 1e150;
+      }
     }
-    px = fma(c3, X, px);
-    py = fma(c3, Y, py);
-    qx = fma(c5, X, qx);
-    qy = fma(c5, Y, qy);
-    sv += c3;
+  }
+  if (all) {
+#pragma unroll
+    for (int xy = 0; xy < 9; ++xy) {
+      const double X = Rx[xy / 3], Y = Ry[xy % 3];
+      const double XY2 = fma(X, X, Y * Y);
+      double c3 = 0, c5 = 0;
+#pragma unroll
+      for (int iz = 0; iz < 3; ++iz) {
+        if (3 * xy + iz == kPrimary) continue;
+        const double Z = Rz[iz];
+        const double inv = rsqrt_nr(fma(Z, Z, XY2));
+        const double inv2 = inv * inv;
+        const double i3 = inv2 * inv;
+        const double i5 = (i3 * inv2) * Z;
+        c3 += i3;
+        c5 += i5;
+        pz = fma(i3, Z, pz);
+        qz = fma(i5, Z, qz);
+      }
+      px = fma(c3, X, px);
+      py = fma(c3, Y, py);
+      qx = fma(c5, X, qx);
+      qy = fma(c5, Y, qy);
+      sv += c3;
+    }
+  } else {
+#pragma unroll 1
+    for (int xy = 0; xy < 9; ++xy) {
+      const unsigned bits = (rest >> (3 * xy)) & 7u;
+      if (!bits) continue;
+      const int ix = (xy * 11) >> 5, iy = xy - 3 * ix;
+      const double X = ix == 0 ? Rx[0] : (ix == 1 ? Rx[1] : Rx[2]);
+      const double Y = iy == 0 ? Ry[0] : (iy == 1 ? Ry[1] : Ry[2]);
+      const double XY2 = fma(X, X, Y * Y);
+      double c3 = 0, c5 = 0;
+#pragma unroll
+      for (int iz = 0; iz < 3; ++iz) {
+        if (!((bits >> iz) & 1u)) continue;
+        const double Z = Rz[iz];
+        const double inv = rsqrt_nr(fma(Z, Z, XY2));
+        const double inv2 = inv * inv;
+        const double i3 = inv2 * inv;
+        const double i5 = (i3 * inv2) * Z;
+        c3 += i3;
+        c5 += i5;
+        pz = fma(i3, Z, pz);
+        qz = fma(i5, Z, qz);
+      }
+      px = fma(c3, X, px);
+      py = fma(c3, Y, py);
+      qx = fma(c5, X, qx);
+      qy = fma(c5, Y, qy);
+      sv += c3;
+    }
   }
   // g x P + m x Q + (m21 S, 0, 0), m = (m02, m12, m22)
   const double m21 = mm[0], m02 = mm[1], m12 = mm[2], m22 = mm[3];
@@ -667,14 +789,11 @@ __device__ __forceinline__ void cell_fp64(const OvParams& P, const Cell* cp, dou
                 fma(g[0], py, fma(-g[1], px, fma(m02, qy, -m12 * qx))));
 }
 
-// resident warps per SM the register allocation must allow, measured at
-// 1M points, ms per launch:
-//   mixed 47.6 / 40.6 / 43.8 / 44.8 for 12 / 16 / 20 / 24 warps (136 and 128
-//   registers without spills, 96 registers and 56 bytes spilled, 80
-//   registers and 272 bytes spilled)
-//   FP64 87.6 / 79.8 / 78.5 for 16 / 20 / 24 warps (110 registers without
-//   spills, 96 registers and 48 bytes spilled, 80 registers and 88 bytes
-//   spilled)
+// resident warps per SM the register allocation must allow.  At 16 neither
+// form spills (128 registers).  Measured, ms per launch at 1M / 200k / 22.4k
+// nodes for 12 / 16 / 20 (24) warps: mixed 31.5 / 6.04 / 1.07, 27.7 / 5.42 /
+// 0.94, 28.0 / 5.69 / 1.67; FP64 (16, 20, 24) 53.4 / 10.4 / 1.70, 52.9 / 10.6
+// / 1.99, 53.2 / 9.87 / 2.03.
 // Blocks are one warp each: a block of four kept its place until its slowest
 // warp ended (200k nodes FP64, two parts, a first walk: 16.9 ms against 15.9;
 // 1M mixed 35.8 against 35.1).
@@ -682,7 +801,7 @@ __device__ __forceinline__ void cell_fp64(const OvParams& P, const Cell* cp, dou
 #define OV_WALK_MULTI_MIN_WARPS_MIXED 16
 #endif
 #ifndef OV_WALK_MULTI_MIN_WARPS_FP64
-#define OV_WALK_MULTI_MIN_WARPS_FP64 24
+#define OV_WALK_MULTI_MIN_WARPS_FP64 16
 #endif
 
 // A group's walk split over `parts` warps (a power of two), for launches with
@@ -787,9 +906,10 @@ __global__ void __launch_bounds__(32, kMixed ? OV_WALK_MULTI_MIN_WARPS_MIXED : O
         // image's single wrap then undoes its shift).  The cell's margin E
         // (mac_margin) bounds the FP64 rounding of every image's squared
         // distance, so when the target's q0 passes by E every image passes,
-        // and when q0 fails by E with no axis near half a box every image
-        // fails.  Otherwise (and at the root, whose centre of mass may lie
-        // outside the box) all decisions are taken in full.
+        // and when q0 fails by E the images' decisions follow from the
+        // per-axis distances (wrapped_decisions).  Otherwise (and at the
+        // root, whose centre of mass may lie outside the box) all decisions
+        // are taken in full.
         unsigned pass;
         // The reference wraps an axis when c - r lies outside [-L/2, L/2];
         // where no axis wraps its squared distance is that of c - r itself
@@ -804,9 +924,8 @@ __global__ void __launch_bounds__(32, kMixed ? OV_WALK_MULTI_MIN_WARPS_MIXED : O
         const bool shortcut = sane && q > 0;
         if (shortcut && q0 >= t0.x + E) {
           pass = m;
-        } else if (shortcut && q0 < t0.x - E && fabs(dx) <= S.hw[0] && fabs(dy) <= S.hw[1] &&
-                   fabs(dz) <= S.hw[2]) {
-          pass = 0;
+        } else if (shortcut && q0 < t0.x - E && wrapped_decisions(P, S, r, cx, cy, cz, dx, dy, dz, t0.x, E, pass)) {
+          // decided from the per-axis distances
         } else {
           // q0 is the target's own decision in mac_exact's operations; the
           // other images still open here are few below the top levels, so
@@ -1102,6 +1221,7 @@ static ImageShortcut image_shortcut(const OvParams& P, unsigned combos) {
     }
     if (shifted && !P.periodic[a]) sc.on = 0;
     sc.hw[a] = shifted ? 0.5 * P.L[a] - allowance : DBL_MAX;
+    sc.wr[a] = shifted ? 0.5 * P.L[a] + allowance : DBL_MAX;
     sc.half[a] = P.periodic[a] ? P.L[a] * 0.5 : DBL_MAX;
   }
   return sc;

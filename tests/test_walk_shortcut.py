@@ -126,3 +126,70 @@ def test_margin_scales_with_rounding():
     assert margin(lo, hi, 1e-6) < 1e-13 * 1.0
     assert margin(lo, hi, (1e-3 / 0.5) ** 2) / (1e-3 / 0.5) ** 2 < 1e-10
     assert margin(lo, hi, 1e-58) == math.inf
+
+
+def wrapped_decisions(r, c, L, lo, hi, thr, E):
+    """ov_walk.cu, wrapped_decisions: image -> decision, or None where the
+    walk takes the decisions in full."""
+    B = max(abs(a) + abs(b) for a, b in zip(lo, hi))
+    hw = half_width(lo, hi)
+    wr = [0.5 * (h - l) + 8 * U * 3.5 * B for l, h in zip(lo, hi)]
+    d = [c[a] - r[a] for a in range(3)]
+    wrap = [abs(d[a]) > hw[a] for a in range(3)]
+    if any(wrap[a] and abs(d[a]) < wr[a] for a in range(3)):
+        return None
+    same = [wrapped_sq(r[a], c[a], L[a], True) for a in range(3)]
+    away = [2 if d[a] > 0 else 0 for a in range(3)]
+    out = {}
+    for ix in range(3):
+        for iy in range(3):
+            for iz in range(3):
+                far = [wrap[a] and i == away[a] for a, i in enumerate((ix, iy, iz))]
+                if not any(far):
+                    out[ix, iy, iz] = False
+                    continue
+                q = ((d[0] * d[0] if far[0] else same[0]) + (d[1] * d[1] if far[1] else same[1])) \
+                    + (d[2] * d[2] if far[2] else same[2])
+                if thr - E <= q < thr + E:
+                    return None
+                out[ix, iy, iz] = q >= thr + E
+    return out
+
+
+def test_decisions_along_wrapped_axes_match_every_image():
+    """Cells the target's own image fails while one to three axes wrap: the
+    image products decided from two distances per axis, against every image
+    tested with the reference's operations; thresholds within rounding of one
+    image's distance, and axes about half a box away."""
+    rng = random.Random(77)
+    decided = [0, 0, 0, 0]
+    mixed = 0
+    for trial in range(12000):
+        off = rng.choice([0.0, -0.5, 3.0, -17.25])
+        size = rng.choice([0.1, 1.0, 2 * math.pi])
+        lo = [off * size] * 3
+        hi = [lo[a] + size * rng.uniform(0.8, 1.2) for a in range(3)]
+        L = [hi[a] - lo[a] for a in range(3)]
+        c = [rng.uniform(lo[a], hi[a]) for a in range(3)]
+        r = [rng.uniform(lo[a] - 0.25 * L[a], hi[a] + 0.25 * L[a]) for a in range(3)]
+        if rng.random() < 0.3:
+            ax = rng.randrange(3)
+            r[ax] = c[ax] + rng.choice([1, -1]) * 0.5 * L[ax] * (1 + rng.choice([1, -1]) * 10.0 ** rng.uniform(-17, -3))
+        if any(not (lo[a] - 0.25 * L[a] <= r[a] <= hi[a] + 0.25 * L[a]) for a in range(3)):
+            continue
+        q0 = image_q(r, c, L, (1, 1, 1))
+        # the threshold near some image's own distance, or anywhere
+        q1 = image_q(r, c, L, tuple(rng.randrange(3) for _ in range(3)))
+        thr = q1 * (1 + rng.choice([1, -1]) * 10.0 ** rng.uniform(-16, -6)) if rng.random() < 0.6 \
+            else q0 * rng.uniform(1.0, 4.0)
+        E = margin(lo, hi, thr)
+        if not q0 < thr - E:
+            continue
+        got = wrapped_decisions(r, c, L, lo, hi, thr, E)
+        if got is None:
+            continue
+        for im, passes in got.items():
+            assert passes == (image_q(r, c, L, im) >= thr), (trial, im)
+        decided[sum(abs(c[a] - r[a]) > 0.5 * L[a] for a in range(3))] += 1
+        mixed += 0 < sum(got.values()) < 27
+    assert all(n > 100 for n in decided) and mixed > 1000, (decided, mixed)
