@@ -118,16 +118,27 @@ __global__ void k_keys(OvParams P, const double* __restrict__ pos, const int2* _
     double c[3], Lh[3];
     split_params(lo, hi, c, Lh);
     int digit = kDigitDropped;
-    for (int ch = 0; ch < nch; ++ch) {
-      double clo[3], chi[3];
+    double clo[3], chi[3];
+    // The child on the node's side of every mid-plane.  A node further from
+    // each plane than the rounding of the children's faces (a few ulps of
+    // the coordinates) is in no other child, so if that child holds it, it
+    // is the first that does; otherwise every child is tested in order.
+    const double near = 0x1p-50 * (fabs(P.lo[0]) + fabs(P.hi[0]) + fabs(P.lo[1]) + fabs(P.hi[1]) + fabs(P.lo[2]) +
+                                   fabs(P.hi[2]));
+    const int own = (px > c[0] ? 1 : 0) | (py > c[1] ? 2 : 0) | (pz > c[2] ? 4 : 0);
+    if (!P.quadtree && fabs(px - c[0]) > near && fabs(py - c[1]) > near && fabs(pz - c[2]) > near) {
+      const int ch = own ^ 1;   // the reference's child order
+      child_box(lo, hi, c, Lh, ch, 0, clo, chi);
+      if (px > clo[0] && px < chi[0] && py > clo[1] && py < chi[1] && pz > clo[2] && pz < chi[2]) digit = ch;
+    }
+    for (int ch = 0; digit == kDigitDropped && ch < nch; ++ch) {
       child_box(lo, hi, c, Lh, ch, P.quadtree, clo, chi);
       // strict containment (in_box, src/vec3_maths.c:67-77)
-      if (px > clo[0] && px < chi[0] && py > clo[1] && py < chi[1] && pz > clo[2] && pz < chi[2]) {
-        digit = ch;
+      if (px > clo[0] && px < chi[0] && py > clo[1] && py < chi[1] && pz > clo[2] && pz < chi[2]) digit = ch;
+    }
+    if (digit != kDigitDropped) {
 #pragma unroll
-        for (int a = 0; a < 3; ++a) { lo[a] = clo[a]; hi[a] = chi[a]; }
-        break;
-      }
+      for (int a = 0; a < 3; ++a) { lo[a] = clo[a]; hi[a] = chi[a]; }
     }
     ++level;
     set_digit(h, l, level, digit);
@@ -145,22 +156,121 @@ __global__ void k_keys(OvParams P, const double* __restrict__ pos, const int2* _
 }
 
 // ---------------------------------------------------------------- 2. sort
+// A pass of 8 bits is two launches: k_rs_hist counts the digits of each tile
+// of kRsThreads * kItems keys (hist[tile][digit]), k_rs_scatter forms its
+// tile's offsets from those counts and moves the keys.  A tile's warps take
+// consecutive stretches of it, so the counts of the warps before, plus the
+// rank within the warp, keep the order stable with two block barriers.
+// With more than kRsFused tiles each block would read too many counts; the
+// offsets then come from three scan launches.  Tiles of 1024 keys up to 256k
+// keys, so a small sort fills the GPU: 22.4k keys take 4 + 3 us a pass on the
+// device, against 22 + 10 with 4096-key tiles ranked 256 at a time and 9 more
+// for the scans.
 constexpr int kRsThreads = 256;
-constexpr int kRsItems = 16;
-constexpr int kRsTile = kRsThreads * kRsItems;
+constexpr int kRsWarps = kRsThreads / 32;
+constexpr int kRsFused = 256;
+constexpr int kRsSmall = 4, kRsLarge = 16;   // keys per thread
 
-__global__ void k_rs_hist(const uint64_t* __restrict__ keys, int n, int shift, unsigned* hist,
-                          int nblocks) {
+template <int kItems>
+__global__ void __launch_bounds__(kRsThreads) k_rs_hist(const uint64_t* __restrict__ keys, int n, int shift,
+                                                        unsigned* hist) {
   __shared__ unsigned h[256];
   h[threadIdx.x] = 0;
   __syncthreads();
-  int base = blockIdx.x * kRsTile;
-  for (int t = 0; t < kRsItems; ++t) {
-    int i = base + t * kRsThreads + threadIdx.x;
+  const int base = blockIdx.x * kRsThreads * kItems;
+#pragma unroll
+  for (int t = 0; t < kItems; ++t) {
+    const int i = base + t * kRsThreads + threadIdx.x;
     if (i < n) atomicAdd(&h[(keys[i] >> shift) & 255], 1u);
   }
   __syncthreads();
-  hist[threadIdx.x * nblocks + blockIdx.x] = h[threadIdx.x];
+  hist[(size_t)blockIdx.x * 256 + threadIdx.x] = h[threadIdx.x];
+}
+
+// digit-major copy of the counts for the scans of a large sort
+__global__ void k_rs_transpose(const unsigned* __restrict__ hist, int tiles, unsigned* out) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= 256 * tiles) return;
+  out[(size_t)(i & 255) * tiles + (i >> 8)] = hist[i];
+}
+
+template <int kItems, bool kScanned>
+__global__ void __launch_bounds__(kRsThreads) k_rs_scatter(const uint64_t* __restrict__ kin,
+                                                           const int* __restrict__ vin, uint64_t* kout, int* vout,
+                                                           int n, int shift, const unsigned* __restrict__ hist,
+                                                           int tiles) {
+  __shared__ unsigned wcnt[kRsWarps][256];
+  __shared__ unsigned offs[256];
+  __shared__ unsigned wsum[kRsWarps];
+  const unsigned FULL = 0xffffffffu;
+  const int d0 = threadIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+#pragma unroll
+  for (int w = 0; w < kRsWarps; ++w) wcnt[w][d0] = 0;
+  __syncthreads();
+  // rank of every key among the equal digits of its warp's stretch
+  const int base = blockIdx.x * kRsThreads * kItems + warp * 32 * kItems;
+  const unsigned lt_mask = (1u << lane) - 1u;
+  uint64_t key[kItems];
+  int val[kItems];
+  unsigned rank[kItems];
+#pragma unroll
+  for (int t = 0; t < kItems; ++t) {
+    const int i = base + t * 32 + lane;
+    key[t] = i < n ? kin[i] : 0;
+    val[t] = i < n ? vin[i] : 0;
+  }
+#pragma unroll
+  for (int t = 0; t < kItems; ++t) {
+    const bool valid = base + t * 32 + lane < n;
+    const int d = valid ? (int)((key[t] >> shift) & 255) : 256;
+    const unsigned peers = __match_any_sync(FULL, d);
+    rank[t] = valid ? wcnt[warp][d] + __popc(peers & lt_mask) : 0;
+    __syncwarp();
+    if (valid && (peers & lt_mask) == 0) wcnt[warp][d] += __popc(peers);
+    __syncwarp();
+  }
+  // this digit's place: the keys of smaller digits, then the tiles before
+  unsigned before = 0, total = 0;
+  if (kScanned) {
+    before = hist[(size_t)d0 * tiles + blockIdx.x];
+  } else {
+#pragma unroll 8
+    for (int t = 0; t < tiles; ++t) {
+      const unsigned c = hist[(size_t)t * 256 + d0];
+      if (t < (int)blockIdx.x) before += c;
+      total += c;
+    }
+  }
+  unsigned inc = total;
+  if (!kScanned) {
+#pragma unroll
+    for (int off = 1; off < 32; off <<= 1) {
+      const unsigned y = __shfl_up_sync(FULL, inc, off);
+      if (lane >= off) inc += y;
+    }
+    if (lane == 31) wsum[warp] = inc;
+  }
+  __syncthreads();
+  unsigned place = before + inc - total;
+  if (!kScanned)
+    for (int w = 0; w < warp; ++w) place += wsum[w];
+  offs[d0] = place;
+  unsigned run = 0;
+#pragma unroll
+  for (int w = 0; w < kRsWarps; ++w) {
+    const unsigned c = wcnt[w][d0];
+    wcnt[w][d0] = run;
+    run += c;
+  }
+  __syncthreads();
+#pragma unroll
+  for (int t = 0; t < kItems; ++t) {
+    if (base + t * 32 + lane >= n) continue;
+    const int d = (int)((key[t] >> shift) & 255);
+    const unsigned r = offs[d] + wcnt[warp][d] + rank[t];
+    kout[r] = key[t];
+    vout[r] = val[t];
+  }
 }
 
 // Exclusive scan of m unsigned values in three launches: the sum of each
@@ -229,44 +339,6 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_apply(unsigned* v, int m,
   unsigned tot;
   const unsigned e = block_excl_scan(x, sh, tot);
   if (i < m) v[i] = sums[blockIdx.x] + e;
-}
-
-__global__ void k_rs_scatter(const uint64_t* __restrict__ kin, const int* __restrict__ vin,
-                             uint64_t* kout, int* vout, int n, int shift,
-                             const unsigned* __restrict__ hist, int nblocks) {
-  __shared__ unsigned offs[256];
-  __shared__ unsigned wcnt[kRsThreads / 32][256];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  offs[threadIdx.x] = hist[threadIdx.x * nblocks + blockIdx.x];
-  for (int w = 0; w < kRsThreads / 32; ++w) wcnt[w][threadIdx.x] = 0;
-  __syncthreads();
-  int base = blockIdx.x * kRsTile;
-  const unsigned lt_mask = (1u << lane) - 1u;
-  for (int t = 0; t < kRsItems; ++t) {
-    int i = base + t * kRsThreads + threadIdx.x;
-    bool valid = i < n;
-    uint64_t key = valid ? kin[i] : 0;
-    int val = valid ? vin[i] : 0;
-    int d = valid ? (int)((key >> shift) & 255) : 256;
-    unsigned peers = __match_any_sync(0xffffffffu, d);
-    unsigned rank_w = __popc(peers & lt_mask);
-    if (valid && rank_w == 0) wcnt[warp][d] = __popc(peers);
-    __syncthreads();
-    if (valid) {
-      unsigned r = offs[d] + rank_w;
-      for (int w = 0; w < warp; ++w) r += wcnt[w][d];
-      kout[r] = key;
-      vout[r] = val;
-    }
-    __syncthreads();
-    unsigned tot = 0;
-    for (int w = 0; w < kRsThreads / 32; ++w) {
-      tot += wcnt[w][threadIdx.x];
-      wcnt[w][threadIdx.x] = 0;
-    }
-    offs[threadIdx.x] += tot;
-    __syncthreads();
-  }
 }
 
 // gather the low key words and termination codes into sorted order
@@ -475,7 +547,7 @@ __global__ void k_write_cells(const BNode* __restrict__ nodes, const int* __rest
                               const CellInfo* __restrict__ info, const unsigned* __restrict__ base,
                               const uint64_t* __restrict__ khi, const uint64_t* __restrict__ klo,
                               const double* __restrict__ nodes64, const int2* __restrict__ nodeids,
-                              OvParams P, int n, Cell* cells, double* cell_lm, int2* cell_range,
+                              OvParams P, int n, int big, Cell* cells, double* cell_lm, int2* cell_range,
                               int* lists, int* list_counts) {
   int b = blockIdx.x * blockDim.x + threadIdx.x;
   if (b >= 2 * n - 1) return;
@@ -523,7 +595,7 @@ __global__ void k_write_cells(const BNode* __restrict__ nodes, const int* __rest
     // one atomic per class per warp (a list's order does not matter: each
     // cell's moments depend on its own nodes only)
     int count = last - first + 1;
-    int cls = count <= 16 ? 0 : (count <= 4096 ? 1 : 2);
+    int cls = count <= 16 ? 0 : (count <= big ? 1 : 2);
     const unsigned peers = __match_any_sync(__activemask(), cls);
     const int lane = threadIdx.x & 31, leader = __ffs(peers) - 1;
     int slot0 = 0;
@@ -597,7 +669,7 @@ __global__ void k_moments_thread(const int* __restrict__ list, const int* __rest
   write_moments(cells + c, com, g, m21, m02, m12, m22, f4pi);
 }
 
-// same, one warp per cell (17..4096 nodes): lane-strided sums, then a
+// same, one warp per cell (17 .. mom_big nodes): lane-strided sums, then a
 // butterfly over the warp
 __device__ void moments_warp(int c, Cell* cells, const int2* __restrict__ cell_range,
                              const double* __restrict__ nodes64,
@@ -642,14 +714,20 @@ __global__ void k_moments_warp(const int* __restrict__ list, const int* __restri
   moments_warp(list[w], cells, cell_range, nodes64, nodeids, f4pi);
 }
 
-// Cells of more than 4096 nodes: each cell's node range is cut into chunks of
+// Cells of more than mom_big nodes: each cell's node range is cut into chunks of
 // `chunk` nodes, one block of kMomThreads per (cell, chunk), so the largest
 // cells (the root holds every node) spread over the GPU.  Partial sums per
 // chunk land in part[(j * max_chunks + k) * 10 + ...] (3 position sums, then
 // the 7 moment sums) and are added in chunk order, so the result does not
 // depend on scheduling.
+// A small tree's build is as long as its largest warp or block: with cells
+// up to 1024 nodes to a warp and chunks of 1024 instead of 4096 and 8192,
+// 22.4k nodes' moments take 45 us on the device instead of 105.  Large trees keep the warp for the
+// many cells in between.
 constexpr int kMomThreads = 256;
-constexpr int kMomChunk = 8192;      // smallest chunk
+constexpr int kMomSmallTree = 1 << 18;
+inline int mom_big(int n) { return n <= kMomSmallTree ? 1024 : 4096; }
+inline int mom_chunk(int n) { return n <= kMomSmallTree ? 1024 : 8192; }   // smallest chunk
 constexpr int kMomMaxChunks = 64;    // chunks per cell at most
 
 // sum of v over the block's threads, in a fixed order; valid in thread 0
@@ -674,17 +752,13 @@ __device__ __forceinline__ void block_sum(double (&v)[kN], double* sh) {
   }
 }
 
-// centre of mass of list cell j from its chunk position sums
-__device__ __forceinline__ d3 chunked_com(const double* __restrict__ part, int j, int max_chunks,
-                                          int count, int chunk) {
-  const int nch = (count + chunk - 1) / chunk;
-  double s[3] = {0, 0, 0};
-  for (int k = 0; k < nch; ++k) {
-    const double* pk = part + ((size_t)j * max_chunks + k) * 10;
-    s[0] += pk[0]; s[1] += pk[1]; s[2] += pk[2];
-  }
-  const double inv = 1.0 / count;
-  return mk3(s[0] * inv, s[1] * inv, s[2] * inv);
+// sum q (0 .. 9) of list cell j over its chunks, in chunk order
+__device__ __forceinline__ double chunk_sum(const double* __restrict__ part, int j, int max_chunks, int nch, int q) {
+  const double* p = part + (size_t)j * max_chunks * 10 + q;
+  double s = 0;
+#pragma unroll 8
+  for (int k = 0; k < nch; ++k) s += p[10 * (size_t)k];
+  return s;
 }
 
 __global__ void __launch_bounds__(kMomThreads) k_moments_chunk_pos(
@@ -719,10 +793,8 @@ __global__ void __launch_bounds__(kMomThreads) k_moments_chunk_acc(
   const int lo = k * chunk;
   if (lo >= rg.y) return;
   const int hi = min(rg.y, lo + chunk);
-  if (threadIdx.x == 0) {
-    const d3 c = chunked_com(part, j, max_chunks, rg.y, chunk);
-    sh_com[0] = c.x; sh_com[1] = c.y; sh_com[2] = c.z;
-  }
+  if (threadIdx.x < 3)
+    sh_com[threadIdx.x] = chunk_sum(part, j, max_chunks, (rg.y + chunk - 1) / chunk, threadIdx.x) * (1.0 / rg.y);
   __syncthreads();
   const double cy = sh_com[1], cz = sh_com[2];
   double a[7] = {0, 0, 0, 0, 0, 0, 0};
@@ -741,22 +813,23 @@ __global__ void __launch_bounds__(kMomThreads) k_moments_chunk_acc(
   }
 }
 
-// one thread per list cell: chunk sums in chunk order into the cell record
+// one warp per list cell, a lane per sum: chunk sums in chunk order into the
+// cell record
 __global__ void k_moments_chunk_write(const int* __restrict__ list, const int* __restrict__ list_count,
                                       Cell* cells, const int2* __restrict__ cell_range, int chunk,
                                       int max_chunks, const double* __restrict__ part, double f4pi) {
-  const int j = blockIdx.x * blockDim.x + threadIdx.x;
+  const int j = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   if (j >= *list_count) return;
   const int c = list[j];
   const int count = cell_range[c].y;
-  const d3 com = chunked_com(part, j, max_chunks, count, chunk);
-  const int nch = (count + chunk - 1) / chunk;
-  double a[7] = {0, 0, 0, 0, 0, 0, 0};
-  for (int k = 0; k < nch; ++k) {
-    const double* pk = part + ((size_t)j * max_chunks + k) * 10 + 3;
-    for (int q = 0; q < 7; ++q) a[q] += pk[q];
-  }
-  write_moments(cells + c, com, mk3(a[0], a[1], a[2]), a[3], a[4], a[5], a[6], f4pi);
+  const double v = lane < 10 ? chunk_sum(part, j, max_chunks, (count + chunk - 1) / chunk, lane) : 0;
+  double s[10];
+#pragma unroll
+  for (int q = 0; q < 10; ++q) s[q] = __shfl_sync(0xffffffffu, v, q);
+  const double inv = 1.0 / count;
+  if (lane == 0)
+    write_moments(cells + c, mk3(s[0] * inv, s[1] * inv, s[2] * inv), mk3(s[3], s[4], s[5]), s[6], s[7], s[8], s[9],
+                  f4pi);
 }
 
 // a tangle of one node: the root is that node's leaf
@@ -803,22 +876,26 @@ static bool scan_excl(unsigned* v, int m, DevBuf& part, cudaStream_t st) {
   return ov_cuda_ok(cudaGetLastError(), "scan");
 }
 
-// Stable LSD radix sort of n keys by their low `bits` bits, with int values,
-// in passes of 8 bits (k_rs_hist, the three-launch scan, k_rs_scatter), an
-// even number of them.  (kb, vb) are the alternate buffers; after the even
-// number of passes the sorted keys and values are back in (ka, va).
-bool ov_radix_sort_u64(uint64_t* ka, int* va, uint64_t* kb, int* vb, int n, int bits, DevBuf& hist,
-                       DevBuf& scan_part, cudaStream_t st) {
-  if (n <= 0) return true;
-  const int nb = (n + kRsTile - 1) / kRsTile;
-  if (!hist.reserve(sizeof(unsigned) * 256 * (size_t)nb)) return false;
-  const int passes = 2 * ((bits + 15) / 16);
+template <int kItems>
+static bool rs_passes(uint64_t* ka, int* va, uint64_t* kb, int* vb, int n, int passes, DevBuf& hist, DevBuf& scan_part,
+                      cudaStream_t st) {
+  const int tiles = (n + kRsThreads * kItems - 1) / (kRsThreads * kItems);
+  const size_t counts = 256 * (size_t)tiles;
+  const bool fused = tiles <= kRsFused;
+  if (!hist.reserve(sizeof(unsigned) * counts * (fused ? 1 : 2))) return false;
+  unsigned* h = hist.as<unsigned>();
   for (int pass = 0; pass < passes; ++pass) {
     const int shift = 8 * pass;
-    k_rs_hist<<<nb, kRsThreads, 0, st>>>(ka, n, shift, hist.as<unsigned>(), nb);
+    k_rs_hist<kItems><<<tiles, kRsThreads, 0, st>>>(ka, n, shift, h);
     OV_LAUNCHED();
-    if (!scan_excl(hist.as<unsigned>(), 256 * nb, scan_part, st)) return false;
-    k_rs_scatter<<<nb, kRsThreads, 0, st>>>(ka, va, kb, vb, n, shift, hist.as<unsigned>(), nb);
+    if (fused) {
+      k_rs_scatter<kItems, false><<<tiles, kRsThreads, 0, st>>>(ka, va, kb, vb, n, shift, h, tiles);
+    } else {
+      k_rs_transpose<<<tiles, 256, 0, st>>>(h, tiles, h + counts);
+      OV_LAUNCHED();
+      if (!scan_excl(h + counts, (int)counts, scan_part, st)) return false;
+      k_rs_scatter<kItems, true><<<tiles, kRsThreads, 0, st>>>(ka, va, kb, vb, n, shift, h + counts, tiles);
+    }
     OV_LAUNCHED();
     OV_TRY_CUDA(cudaGetLastError());
     std::swap(ka, kb);
@@ -827,19 +904,29 @@ bool ov_radix_sort_u64(uint64_t* ka, int* va, uint64_t* kb, int* vb, int n, int 
   return true;
 }
 
+// Stable LSD radix sort of n keys by their low `bits` bits, with int values,
+// in passes of 8 bits, an even number of them.  (kb, vb) are the alternate
+// buffers; after the even number of passes the sorted keys and values are
+// back in (ka, va).
+bool ov_radix_sort_u64(uint64_t* ka, int* va, uint64_t* kb, int* vb, int n, int bits, DevBuf& hist,
+                       DevBuf& scan_part, cudaStream_t st) {
+  if (n <= 0) return true;
+  const int passes = 2 * ((bits + 15) / 16);
+  return n <= kRsFused * kRsThreads * kRsSmall ? rs_passes<kRsSmall>(ka, va, kb, vb, n, passes, hist, scan_part, st)
+                                               : rs_passes<kRsLarge>(ka, va, kb, vb, n, passes, hist, scan_part, st);
+}
+
 bool ov_tree_build(ov_state_impl* s, const double* pos, OvTree* T) {
   const int n = s->n;
   cudaStream_t st = s->stream;
   T->P = s->P;
   T->theta = s->P.theta;
   T->built = 0;
-  const int nb_rs = (n + kRsTile - 1) / kRsTile;
   // key/value double buffers + low words + termination codes
   if (!T->keys.reserve(sizeof(uint64_t) * 2 * (size_t)n) ||      // hi (slot order), lo (slot order)
       !T->keys_alt.reserve(sizeof(uint64_t) * 2 * (size_t)n) ||  // hi alt, lo sorted
       !T->vals.reserve(sizeof(int) * 2 * (size_t)n) ||           // vals, term (slot)
       !T->vals_alt.reserve(sizeof(int) * 2 * (size_t)n) ||       // vals alt, term (sorted)
-      !T->hist.reserve(sizeof(unsigned) * 256 * (size_t)(nb_rs > 0 ? nb_rs : 1)) ||
       !T->counters.reserve(128))
     return false;
   uint64_t* khi = T->keys.as<uint64_t>();
@@ -942,7 +1029,7 @@ bool ov_tree_build(ov_state_impl* s, const double* pos, OvTree* T) {
     if (!scan_excl(base, na + 1, T->scan_part, st)) return false;
     k_write_cells<<<(nbin + 255) / 256, 256, 0, st>>>(bn, leaf_parent, info, base, hi_sorted, klo,
                                                       T->nodes64.as<double>(), T->nodeids.as<int2>(),
-                                                      s->P, na, cells, cell_lm, cell_range, lists,
+                                                      s->P, na, mom_big(na), cells, cell_lm, cell_range, lists,
                                                       list_counts);
     OV_LAUNCHED();
     OV_TRY_CUDA(cudaGetLastError());
@@ -965,8 +1052,8 @@ bool ov_tree_build(ov_state_impl* s, const double* pos, OvTree* T) {
       OV_LAUNCHED();
     }
     if (lc[2] > 0) {
-      // chunks of at least kMomChunk nodes, at most kMomMaxChunks per cell
-      const int chunk = std::max(kMomChunk, (na + kMomMaxChunks - 1) / kMomMaxChunks);
+      // chunks of at least mom_chunk nodes, at most kMomMaxChunks per cell
+      const int chunk = std::max(mom_chunk(na), (na + kMomMaxChunks - 1) / kMomMaxChunks);
       const int max_chunks = (na + chunk - 1) / chunk;
       if (!T->mom_part.reserve(sizeof(double) * 10 * (size_t)lc[2] * max_chunks)) return false;
       const int* blist = lists + 4 * (size_t)na;
@@ -978,7 +1065,7 @@ bool ov_tree_build(ov_state_impl* s, const double* pos, OvTree* T) {
       k_moments_chunk_acc<<<grid, kMomThreads, 0, st>>>(blist, cell_range, T->nodes64.as<double>(),
                                                          T->nodeids.as<int2>(), chunk, max_chunks, part);
       OV_LAUNCHED();
-      k_moments_chunk_write<<<(lc[2] + 127) / 128, 128, 0, st>>>(blist, list_counts + 2, cells, cell_range,
+      k_moments_chunk_write<<<(lc[2] + 3) / 4, 128, 0, st>>>(blist, list_counts + 2, cells, cell_range,
                                                                   chunk, max_chunks, part, f4);
       OV_LAUNCHED();
     }

@@ -985,7 +985,7 @@ __global__ void __launch_bounds__(32, kMixed ? OV_WALK_MULTI_MIN_WARPS_MIXED : O
   if (kSplit) {
     if (i < n_t) {
       st3(W.nl + 3 * (size_t)part * n_t, i, nl);
-      st3(W.im + 3 * (size_t)part * n_t, i, im);
+      if (!kMixed) st3(W.im + 3 * (size_t)part * n_t, i, im);
     }
   } else if (live) {
     st3(v_nl, k, nl);
@@ -1007,7 +1007,7 @@ __global__ void __launch_bounds__(32, kMixed ? OV_WALK_MULTI_MIN_WARPS_MIXED : O
 }
 
 // the parts of a split walk added in order: target i's sums into slot
-// order[i] (or i)
+// order[i] (or i); im null: the mixed form, whose one sum is in nl
 __global__ void k_walk_reduce(const int* __restrict__ order, const int2* __restrict__ status, int n_t, int parts,
                               const double* __restrict__ nl, const double* __restrict__ im, double* v_nl,
                               double* v_img) {
@@ -1015,13 +1015,13 @@ __global__ void k_walk_reduce(const int* __restrict__ order, const int2* __restr
   if (i >= n_t) return;
   const int k = order ? order[i] : i;
   if (k < 0 || (status && (status[k].x == OV_PINNED || status[k].x == OV_EMPTY))) return;
-  d3 a = ld3(nl, i), b = ld3(im, i);
-  for (int p = 1; p < parts; ++p) {
-    a = a + ld3(nl + 3 * (size_t)p * n_t, i);
-    b = b + ld3(im + 3 * (size_t)p * n_t, i);
-  }
+  d3 a = ld3(nl, i);
+  for (int p = 1; p < parts; ++p) a = a + ld3(nl + 3 * (size_t)p * n_t, i);
   st3(v_nl, k, a);
-  if (v_img) st3(v_img, k, b);
+  if (!v_img) return;
+  d3 b = im ? ld3(im, i) : mk3(0, 0, 0);
+  for (int p = 1; im && p < parts; ++p) b = b + ld3(im + 3 * (size_t)p * n_t, i);
+  st3(v_img, k, b);
 }
 
 // All nodes: warp w handles sorted targets 32w .. 32w+31, every image.
@@ -1283,9 +1283,9 @@ static bool launch_multi(ov_state_impl* s, OvTree* t, const OvParams& P, const i
   WalkSplit W{parts, frontier, deal, skip, nullptr, nullptr};
   if (split) {
     const size_t per = 3 * (size_t)n_t * parts;
-    if (!t->walk_part.reserve(sizeof(double) * 2 * per)) return false;
+    if (!t->walk_part.reserve(sizeof(double) * (mixed ? 1 : 2) * per)) return false;
     W.nl = t->walk_part.as<double>();
-    W.im = W.nl + per;
+    W.im = mixed ? nullptr : W.nl + per;
   }
   // Longest first: the launch runs the warps' units (groups of 32 targets,
   // or their parts) in the order of their times in the previous walk of this

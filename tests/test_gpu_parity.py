@@ -399,6 +399,27 @@ def test_bh_tree_beyond_one_million_nodes(ov, oracle):
     st.close()
 
 
+@pytest.mark.parametrize("slots", [1023, 1025, 262144, 262145])
+def test_tree_sort_sizes_vs_oracle(ov, oracle, slots):
+    """Slot counts at the edges of the key sort's tiles (1024 keys, and 4096
+    from 262145 on), EMPTY slots among them: FP64 Barnes-Hut sums at points
+    against the oracle's recursive tree."""
+    D, dl = 0.4, 0.4 / 400
+    t = G.random_ring_tangle(slots, G.rings_for_points(int(0.9 * slots), D, dl=dl), D, dl=dl, boundary="periodic-26")
+    t = G.random_ring_tangle(slots, G.rings_for_points(int(0.9 * slots), D, dl=dl), D, dl=dl, boundary="periodic-26",
+                             empty_slots=slots - t.n)
+    assert t.n == slots
+    p = Params(core_a=1e-8, dl_max=2 * dl, use_bh=1, bh_theta=0.5, bh_grain=1e-8)
+    from openvort_b200.tangle import IMAGE_TABLES
+    ov.configure(p, 0)
+    st = ov.DeviceState(t.copy())
+    pts = np.random.default_rng(slots).uniform(0, D, size=(40, 3))
+    shifts = [(0, 0, 0)] + [sh for sh, _ in IMAGE_TABLES["periodic-26"]]
+    ref = oracle.bh_at(t, p, np.concatenate([pts - D * np.array(sh) for sh in shifts]))
+    assert rel_err(st.eval_points(pts, method=1), ref.reshape(len(shifts), len(pts), 3).sum(axis=0)) < TOL_V64
+    st.close()
+
+
 @pytest.mark.parametrize("boundary", ["open", "periodic-26", "periodic-z-open-xy"])
 @pytest.mark.parametrize("rings,grain", [(1, 1e-8), (12, 1e-8), (40, 3e-3)])
 def test_split_walk_vs_oracle(ov, oracle, boundary, rings, grain):
