@@ -502,6 +502,7 @@ static bool upload_tangle(ov_state_impl* s, const tangle_state* t, bool need_flo
   s->n_targets = nt;
   s->n_segments = ns;
   s->n_active = na;
+  s->stages_defined = false;
   for (int f = 0; f < 6; ++f) s->walls[f] = t->box.wall[f];
   if (n == 0) return true;
   return upload(s, t->vnodes, s->pos, 24 * n) && upload(s, t->connections, s->links, 8 * n) &&
@@ -545,6 +546,7 @@ static bool bs_sums(ov_state_impl* s, const double* pos, OvTree* external_tree, 
   cudaEventRecord(s->ev2, s->stream);
   double* v_nl = s->v_nl.as<double>();
   double* v_img = s->v_img.as<double>();
+  s->sums = OvSums{v_nl, v_img, nullptr, 0};
   if (!s->P.lia_only) {
     if (s->P.use_bh) {
       OvTree* tree = external_tree;
@@ -554,7 +556,7 @@ static bool bs_sums(ov_state_impl* s, const double* pos, OvTree* external_tree, 
       }
       if (!ov_tree_walk_nodes(s, tree, pos, tree == &s->tree, v_nl, v_img, k0, k_count)) return false;
     } else {
-      if (!ov_direct_nodes(s, pos, v_nl, v_img)) return false;
+      if (!ov_direct_partials(s, pos, v_nl, v_img, &s->sums)) return false;
       // every target against every segment, per image (src/tangle.c:612-636)
       tl_stats.interactions = (double)s->n_targets * (double)s->n_segments * (1 + s->P.n_img);
     }
@@ -564,8 +566,8 @@ static bool bs_sums(ov_state_impl* s, const double* pos, OvTree* external_tree, 
 
 // The epilogue of an evaluation over every node, and the state's counters.
 static bool finish_velocities(ov_state_impl* s, double t, const double* pos, const double* tan,
-                              const double* nrm, double* vels, double* vs) {
-  if (!ov_epilogue(s, t, pos, tan, nrm, s->v_nl.as<double>(), s->v_img.as<double>(), vels, vs, 0, s->n))
+                              const double* nrm, const OvStage& stage, double* vels, double* vs) {
+  if (!ov_epilogue(s, t, pos, tan, nrm, s->sums, stage, vels, vs, 0, s->n))
     return false;
   // the epilogue synchronised the stream: fold this evaluation into the
   // state's counters (device times from the events around the tree build and
@@ -588,9 +590,9 @@ static bool finish_velocities(ov_state_impl* s, double t, const double* pos, con
 
 bool ov_velocities(ov_state_impl* s, double t, const double* pos, const double* dxi,
                    const double* tan, const double* nrm, double* vels, double* vs,
-                   OvTree* external_tree) {
+                   OvTree* external_tree, const OvStage& stage) {
   (void)dxi;
-  return bs_sums(s, pos, external_tree, 0, -1) && finish_velocities(s, t, pos, tan, nrm, vels, vs);
+  return bs_sums(s, pos, external_tree, 0, -1) && finish_velocities(s, t, pos, tan, nrm, stage, vels, vs);
 }
 
 // ======================================================================
@@ -783,7 +785,7 @@ int ov_state_shard_end(ov_state* st, int q, double t, double dt) {
   if (!s->P.lia_only && !ov_shard_unpack(s, s->xbuf, s->xbytes / sizeof(double))) return tl_err;
   tl_last_state = s;
   tl_stats = OvStatsAcc{s->shard_inter, s->shard_cells, 0, 0, 0, 0, s->shard_warp_iter};
-  if (!finish_velocities(s, g.t, g.pos, g.tan, g.nrm, g.vels, g.vs)) return tl_err;
+  if (!finish_velocities(s, g.t, g.pos, g.tan, g.nrm, kNoStage, g.vels, g.vs)) return tl_err;
   if (q == 3 && !(ov_rk4_combine(s, dt) && sync(s))) return tl_err;
   return OV_OK;
 }
@@ -989,8 +991,8 @@ void update_velocity(struct tangle_state* tangle, int k, double t, struct octree
       ok = ov_direct_points(&s, s.pos.as<double>(), 1, pt, skip.as<int>(), nullptr, 0, nl, im);
   }
   ok = ok && ov_epilogue(&s, t, s.pos.as<double>(), s.tan.as<double>(), s.nrm.as<double>(),
-                         s.v_nl.as<double>(), s.v_img.as<double>(), s.vels.as<double>(),
-                         s.vs.as<double>(), k, k + 1);
+                         OvSums{s.v_nl.as<double>(), s.v_img.as<double>(), nullptr, 0}, kNoStage,
+                         s.vels.as<double>(), s.vs.as<double>(), k, k + 1);
   if (ok) {
     cudaMemcpyAsync(&tangle->vels[k], s.vels.as<double>() + 3 * (size_t)k, 24, cudaMemcpyDeviceToHost,
                     s.stream);

@@ -501,11 +501,12 @@ bool launch_near2(ov_batch* b, const double* pos) {
 
 // geometry + Biot-Savart + epilogue at positions pos (time t0 + *t_dev)
 bool enqueue_eval(ov_batch* b, const double* pos, double* dxi, double* tan, double* nrm, double* vels,
-                  double* vs, const double* t_dev, double t0, int* work, cudaEvent_t e0, cudaEvent_t e1) {
+                  double* vs, const double* t_dev, double t0, int* work, const OvStage& stage, cudaEvent_t e0,
+                  cudaEvent_t e1) {
   ov_state_impl* s = &b->s;
   int* flag = s->dflag.as<int>();
   if (!ov_launch_geometry(s->stream, s->P, s->links.as<int2>(), s->status.as<int2>(), pos, dxi, tan, nrm,
-                          s->n, flag))
+                          s->n, false, flag))
     return false;
   if (!s->P.lia_only) {
     if (e0) OV_TRY_CUDA(cudaEventRecord(e0, s->stream));
@@ -513,7 +514,8 @@ bool enqueue_eval(ov_batch* b, const double* pos, double* dxi, double* tan, doub
     if (e1) OV_TRY_CUDA(cudaEventRecord(e1, s->stream));
   }
   return ov_launch_epilogue(s->stream, s->P, s->links.as<int2>(), s->status.as<int2>(), t_dev, t0, pos,
-                            tan, nrm, s->v_nl.as<double>(), nullptr, vels, vs, 0, s->n, flag);
+                            tan, nrm, OvSums{s->v_nl.as<double>(), nullptr, nullptr, 0}, s->n, stage, vels, vs, 0,
+                            s->n, flag);
 }
 
 // one RK4 step (update_tangle + rk4_step2, src/vortex_dynamics.c:58-117) at
@@ -526,7 +528,7 @@ bool enqueue_step(ov_batch* b, double dt, bool classic) {
   ov_state_impl* s = &b->s;
   const int2* st = s->status.as<int2>();
   double* x0 = s->pos.as<double>();
-  double* xs = s->spos.as<double>();
+  double* xs[3] = {s->spos.as<double>(), s->pos0.as<double>(), s->spos.as<double>()};
   double* ks[3] = {s->k2.as<double>(), s->k3.as<double>(), s->k4.as<double>()};
   const double h[3] = {dt / 2, dt / 2, classic ? dt : dt / 2};
   const double toff[3] = {dt / 2, dt / 2, dt};
@@ -535,13 +537,13 @@ bool enqueue_step(ov_batch* b, double dt, bool classic) {
   OV_TRY_CUDA(cudaMemsetAsync(work, 0, 4 * sizeof(int), s->stream));
   if (!launch_near2(b, x0)) return false;
   if (!enqueue_eval(b, x0, s->dxi.as<double>(), s->tan.as<double>(), s->nrm.as<double>(),
-                    s->vels.as<double>(), s->vs.as<double>(), t_dev, 0.0, work, nullptr, nullptr))
+                    s->vels.as<double>(), s->vs.as<double>(), t_dev, 0.0, work, OvStage{x0, h[0], xs[0]}, nullptr,
+                    nullptr))
     return false;
   for (int q = 0; q < 3; ++q) {
-    const double* prev = q == 0 ? s->vels.as<double>() : ks[q - 1];
-    if (!ov_launch_euler(s->stream, st, x0, prev, h[q], xs, s->n)) return false;
-    if (!enqueue_eval(b, xs, s->sdxi.as<double>(), s->stan.as<double>(), s->snrm.as<double>(), ks[q],
-                      s->svs.as<double>(), t_dev, toff[q], work + q + 1, nullptr, nullptr))
+    if (!enqueue_eval(b, xs[q], s->sdxi.as<double>(), s->stan.as<double>(), s->snrm.as<double>(), ks[q],
+                      s->svs.as<double>(), t_dev, toff[q], work + q + 1,
+                      q < 2 ? OvStage{x0, h[q + 1], xs[q + 1]} : kNoStage, nullptr, nullptr))
       return false;
   }
   if (!ov_launch_rk4_combine(s->stream, st, s->vels.as<double>(), ks[0], ks[1], ks[2], dt, x0, s->n))
@@ -669,10 +671,11 @@ ov_batch* ov_batch_create(const struct tangle_state* all, int n_systems, const i
     ok = ok && ov_cuda_ok(cudaEventCreate(&b->ev_run0), "cudaEventCreate") &&
          ov_cuda_ok(cudaEventCreate(&b->ev_run1), "cudaEventCreate");
     // stage positions of EMPTY slots are never written: keep them defined
-    if (ok && all->N > 0)
-      ok = ov_cuda_ok(cudaMemcpyAsync(b->s.spos.p, b->s.pos.p, sizeof(double) * 3 * all->N,
-                                      cudaMemcpyDeviceToDevice, b->s.stream),
-                      "cudaMemcpyAsync");
+    for (DevBuf* x : {&b->s.spos, &b->s.pos0})
+      if (ok && all->N > 0)
+        ok = ov_cuda_ok(cudaMemcpyAsync(x->p, b->s.pos.p, sizeof(double) * 3 * all->N, cudaMemcpyDeviceToDevice,
+                                        b->s.stream),
+                        "cudaMemcpyAsync");
     ok = ok && ov_cuda_ok(cudaStreamSynchronize(b->s.stream), "cudaStreamSynchronize");
   }
   if (!ok) {
@@ -714,7 +717,7 @@ int ov_batch_update(ov_batch* b, double t) {
             launch_near2(b, s->pos.as<double>()) &&
             enqueue_eval(b, s->pos.as<double>(), s->dxi.as<double>(), s->tan.as<double>(),
                          s->nrm.as<double>(), s->vels.as<double>(), s->vs.as<double>(), nullptr, t,
-                         b->d_work.as<int>(), b->ev_bs[0], b->ev_bs[1]) &&
+                         b->d_work.as<int>(), kNoStage, b->ev_bs[0], b->ev_bs[1]) &&
             read_flag(b, "ov_batch_update");
   if (!ok) return ov_last_error();
   float ms = 0;

@@ -188,15 +188,20 @@ __host__ __device__ __forceinline__ ColCut col_cut_of(double col) {
   const double inf = 1.7976931348623157e308;
   return ColCut{col > 0 ? 2.0 - (col + m) : inf, col > m ? 2.0 - (col - m) : inf, col};
 }
-// an endpoint nearer than 1.5e-8, where the reference's distance cut-off
-// (1e-8) could decide: a test on the high word, an integer operation
-__device__ __forceinline__ bool near_end(double R2) { return __double2hiint(R2) <= 0x3cb03684; }
+// The distance cut-off |R| < 1e-8 from the high word of |R|^2 (integer
+// comparisons): 1e-16 has the high word kEndWord, so below it the endpoint is
+// surely inside (the segment adds nothing), above kEndWord + 1 surely
+// outside, and at these two words the reference's own square root decides.
+// A node's own two segments end at the node itself and are inside.
+constexpr int kEndWord = 0x3c9cd2b2;
+__device__ __forceinline__ bool end_inside(double R2) { return __double2hiint(R2) < kEndWord; }
+__device__ __forceinline__ bool end_near(double R2) { return __double2hiint(R2) <= kEndWord + 1; }
 
 // The reference's segment formula without IEEE square roots and divisions:
 // with u = 1/(|R||R'|) from two refined reciprocal square roots,
 //   f (|R| + |R'|) / (|R||R'| (|R||R'| + R.R')) = f (1/|R| + 1/|R'|) u / (1 + R.R' u).
 // R' = R + d (d = r2 - r1, staged per segment) differs from r2 - r by an ulp
-// of |R'|.  Where either cut-off could decide (near_end, ColCut) the
+// of |R'|.  Where a cut-off is too close to call (end_near, ColCut) the
 // reference's own operations decide (seg_vel64), so every cut-off decision is
 // the reference's.
 __device__ __forceinline__ d3 seg_vel64_nr(double f4pi, d3 r1, d3 r2, d3 d, d3 r,
@@ -204,7 +209,8 @@ __device__ __forceinline__ d3 seg_vel64_nr(double f4pi, d3 r1, d3 r2, d3 d, d3 r
   const d3 R = r1 - r;
   const d3 Rp = R + d;
   const double R2 = dot3(R, R), Rp2 = dot3(Rp, Rp), RRp = dot3(R, Rp);
-  const bool near = near_end(R2) || near_end(Rp2);
+  if (end_inside(R2) || end_inside(Rp2)) return mk3(0, 0, 0);
+  const bool near = end_near(R2) || end_near(Rp2);
   const double ia = rsqrt_nr(R2), ib = rsqrt_nr(Rp2);
   const double u = ia * ib;
   const double den = fma(RRp, u, 1.0);
@@ -236,7 +242,7 @@ __device__ __forceinline__ void chain64_sweep(const double (*nd)[3], const unsig
   d3 Ra = mk3(nd[0][0], nd[0][1], nd[0][2]) - r;
   const double Ra2 = dot3(Ra, Ra);
   double ia = rsqrt_nr(Ra2);
-  bool na = near_end(Ra2);
+  bool na = end_near(Ra2);
   for (int i0 = 0; i0 < cnt; i0 += kChainGroup) {
     const unsigned bits = chain[i0 >> 5] >> (i0 & 31), rest = other[i0 >> 5] >> (i0 & 31);
     bool slow[kChainGroup];
@@ -247,7 +253,7 @@ __device__ __forceinline__ void chain64_sweep(const double (*nd)[3], const unsig
       const d3 Rb = mk3(nd[i + 1][0], nd[i + 1][1], nd[i + 1][2]) - r;
       const double Rb2 = dot3(Rb, Rb);
       const double ib = rsqrt_nr(Rb2);
-      const bool nb = near_end(Rb2);
+      const bool nb = end_near(Rb2);
       const double u = ia * ib;
       const double den = fma(dot3(Ra, Rb), u, 1.0);
       bool on = (bits >> q) & 1u;
@@ -268,9 +274,11 @@ __device__ __forceinline__ void chain64_sweep(const double (*nd)[3], const unsig
 #pragma unroll
       for (int q = 0; q < kChainGroup; ++q) {
         const int i = i0 + q;
-        if (slow[q])
-          acc = acc + seg_vel64(1.0, mk3(nd[i][0], nd[i][1], nd[i][2]),
-                                mk3(nd[i + 1][0], nd[i + 1][1], nd[i + 1][2]), r, cut.col);
+        if (!slow[q]) continue;
+        const d3 a = mk3(nd[i][0], nd[i][1], nd[i][2]), b = mk3(nd[i + 1][0], nd[i + 1][1], nd[i + 1][2]);
+        // a node's own segments, in every warp: no square roots for them
+        const d3 Qa = a - r, Qb = b - r;
+        if (!end_inside(dot3(Qa, Qa)) && !end_inside(dot3(Qb, Qb))) acc = acc + seg_vel64(1.0, a, b, r, cut.col);
       }
     }
     if (rest & ((1u << kChainGroup) - 1)) {

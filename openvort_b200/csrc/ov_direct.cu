@@ -20,6 +20,7 @@
 #include <algorithm>
 
 #include "ov_internal.h"
+#include "ov_node.cuh"
 #include "ov_pair.cuh"
 
 namespace {
@@ -126,18 +127,20 @@ constexpr int kCS = 128;   // chained segments per shared-memory tile
 static_assert(kCS == kTS, "the chain sweep splits sources as k_direct64 does");
 
 template <bool kPoints>
-__global__ void __launch_bounds__(kTB) k_direct64_chain(OvParams P, SegTab S, int n_src,
-                                                        const double* __restrict__ pos,
+__global__ void __launch_bounds__(kTB) k_direct64_chain(OvParams P, int n_src, const double* __restrict__ pos,
+                                                        const int2* __restrict__ links,
+                                                        const int2* __restrict__ status,
                                                         const double* __restrict__ tpos,
-                                                        const int2* __restrict__ tstatus,
                                                         const int* __restrict__ tskip, int n_t,
                                                         double* __restrict__ part, int chunk) {
   __shared__ double sh_node[kCS + 1][3];
   __shared__ unsigned sh_chain[kCS / 32], sh_other[kCS / 32];   // chained and other segments
+  __shared__ double sh_end[kCS][3];                             // wrapped ends and forward
+  __shared__ int sh_fwd[kCS];                                   // slots of the other ones
   const int j = blockIdx.y;   // 0: the tangle itself, j >= 1: image j-1
   const int k = blockIdx.x * kTB + threadIdx.x;
   bool act = k < n_t;
-  if (act && !kPoints) act = tstatus[k].x != OV_EMPTY && tstatus[k].x != OV_PINNED;
+  if (act && !kPoints) act = status[k].x != OV_EMPTY && status[k].x != OV_PINNED;
   d3 r = mk3(0, 0, 0);
   int skip = -1;
   if (act) {
@@ -161,14 +164,16 @@ __global__ void __launch_bounds__(kTB) k_direct64_chain(OvParams P, SegTab S, in
     }
     for (int i = threadIdx.x; i < kCS; i += kTB) {
       const int m = sb + i;
-      const int fw = m < s_hi ? S.fwd[m] : -1;
+      const int fw = m < s_hi && status[m].x != OV_EMPTY ? links[m].x : -1;
       bool chained = false;
       if (fw >= 0) {
-        const double* sg = S.r1r2 + 6 * (size_t)m;
-        chained = fw == m + 1;
-        if (chained) {
-          const d3 e = ld3(pos, fw);
-          chained = e.x == sg[3] && e.y == sg[4] && e.z == sg[5];
+        const d3 e = ld3(pos, fw), w = pwrap(P, ld3(pos, m), e);
+        chained = fw == m + 1 && e.x == w.x && e.y == w.y && e.z == w.z;
+        if (!chained) {
+          sh_end[i][0] = w.x;
+          sh_end[i][1] = w.y;
+          sh_end[i][2] = w.z;
+          sh_fwd[i] = fw;
         }
       }
       const unsigned bits = __ballot_sync(0xffffffffu, chained);
@@ -182,10 +187,9 @@ __global__ void __launch_bounds__(kTB) k_direct64_chain(OvParams P, SegTab S, in
     if (!act) continue;
     chain64_sweep<kPoints>(sh_node, sh_chain, sh_other, min(kCS, s_hi - sb), skip >= 0 ? skip - sb : -2, r, cut, acc,
                            [&](int i) {
-                             const int m = sb + i;
-                             if (m == skip || S.fwd[m] == skip) return mk3(0, 0, 0);
-                             const double* sg = S.r1r2 + 6 * (size_t)m;
-                             const d3 r1 = mk3(sg[0], sg[1], sg[2]), r2 = mk3(sg[3], sg[4], sg[5]);
+                             if (sb + i == skip || sh_fwd[i] == skip) return mk3(0, 0, 0);
+                             const d3 r1 = mk3(sh_node[i][0], sh_node[i][1], sh_node[i][2]);
+                             const d3 r2 = mk3(sh_end[i][0], sh_end[i][1], sh_end[i][2]);
                              return seg_vel64_nr(1.0, r1, r2, r2 - r1, r, cut);
                            });
   }
@@ -614,25 +618,14 @@ __global__ void k_reduce_bounds(double f4pi, const double* __restrict__ bpart, i
   bound[i] = kMixedBoundU * f4pi * e;
 }
 
-// v_nl = part[0]; v_img = sum_j part[j] in image order (src/tangle.c:627-638);
-// mirror images reflect their velocity (src/tangle.c:633-634).  With source
-// splits, each image's partial sums are added split by split, in order.
+// the partials of each target added up (sum_partials)
 __global__ void k_reduce_images(OvParams P, const double* __restrict__ part, int n_t,
                                 double* v_nl, double* v_img, int splits) {
   int k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= n_t) return;
-  const size_t img_stride = 3 * (size_t)n_t, split_stride = img_stride * (P.n_img + 1);
-  d3 a = ld3(part, k);
-  for (int z = 1; z < splits; ++z) a = a + ld3(part + z * split_stride, k);
+  d3 a, s;
+  sum_partials(P, part, n_t, splits, k, a, s);
   if (v_nl) st3(v_nl, k, a);
-  d3 s = mk3(0, 0, 0);
-  for (int j = 1; j <= P.n_img; ++j) {
-    d3 v = ld3(part + (size_t)j * img_stride, k);
-    for (int z = 1; z < splits; ++z) v = v + ld3(part + z * split_stride + (size_t)j * img_stride, k);
-    int face = P.img[j - 1][3];
-    if (face > -1) v = mirror_dir(v, face);
-    s = s + v;
-  }
   if (v_img) st3(v_img, k, s);
 }
 
@@ -711,14 +704,14 @@ static int source_chunk(int n_src, long long blocks, int tile, int* splits, int 
   return chunk;
 }
 
-bool ov_direct_nodes(ov_state_impl* s, const double* pos, double* v_nl, double* v_img) {
+bool ov_direct_partials(ov_state_impl* s, const double* pos, double* v_nl, double* v_img, OvSums* out) {
+  *out = OvSums{v_nl, v_img, nullptr, 0};
   if (s->n == 0) return true;
-  if (!ensure_segtab(s, pos)) return false;
   int nimg = s->P.n_img;
-  SegTab S{s->seg64.as<double>(), s->segid.as<int>()};
-  OvStatsAcc& st = ov_stats_tls();
   int splits = 1;
   if (s->P.precision == OV_PREC_MIXED) {
+    if (!ensure_segtab(s, pos)) return false;
+    SegTab S{s->seg64.as<double>(), s->segid.as<int>()};
     // small sums: slot order, no key sort (k_direct_mixed_chain); otherwise
     // key order from the tree's sort (timed as the build)
     const double work = (double)s->n_targets * (double)s->n_segments * (1 + nimg);
@@ -760,20 +753,30 @@ bool ov_direct_nodes(ov_state_impl* s, const double* pos, double* v_nl, double* 
   } else {
     const int bx = (s->n + kTB - 1) / kTB;
     static const int res64 = resident_blocks(k_direct64_chain<false>, kTB);
-    const int chunk = source_chunk(s->n, (long long)bx * (nimg + 1), kCS, &splits, 4, 16, res64);
+    // small sums: pieces of a tile down to 32 sources (a 256-node ring is two
+    // target blocks: 16 blocks instead of 4)
+    const int chunk = source_chunk(s->n, (long long)bx * (nimg + 1), 32, &splits, 4, 64, res64);
     if (!s->img_part.reserve(sizeof(double) * 3 * (size_t)s->n * (nimg + 1) * splits)) return false;
     cudaEventRecord(s->ev1, s->stream);
     k_direct64_chain<false><<<dim3(bx, nimg + 1, splits), kTB, 0, s->stream>>>(
-        s->P, S, s->n, pos, nullptr, s->status.as<int2>(), nullptr, s->n, s->img_part.as<double>(), chunk);
+        s->P, s->n, pos, s->links.as<int2>(), s->status.as<int2>(), nullptr, nullptr, s->n, s->img_part.as<double>(),
+        chunk);
     OV_LAUNCHED();
     OV_TRY_CUDA(cudaGetLastError());
   }
   cudaEventRecord(s->ev2, s->stream);
-  k_reduce_images<<<(s->n + 255) / 256, 256, 0, s->stream>>>(s->P, s->img_part.as<double>(), s->n,
-                                                              v_nl, v_img, splits);
+  out->part = s->img_part.as<double>();
+  out->splits = splits;
+  return true;
+}
+
+bool ov_direct_nodes(ov_state_impl* s, const double* pos, double* v_nl, double* v_img) {
+  OvSums sums;
+  if (!ov_direct_partials(s, pos, v_nl, v_img, &sums)) return false;
+  if (!sums.part) return true;
+  k_reduce_images<<<(s->n + 255) / 256, 256, 0, s->stream>>>(s->P, sums.part, s->n, v_nl, v_img, sums.splits);
   OV_LAUNCHED();
   OV_TRY_CUDA(cudaGetLastError());
-  (void)st;
   return true;
 }
 
@@ -781,9 +784,7 @@ bool ov_direct_points(ov_state_impl* s, const double* pos, int npts, const doubl
                       const int* skip, const int* only, int n_only, double* out_nl,
                       double* out_img) {
   if (npts <= 0) return true;
-  if (!ensure_segtab(s, pos)) return false;
   int nimg = out_img ? s->P.n_img : 0;
-  SegTab S{s->seg64.as<double>(), s->segid.as<int>()};
   int n_src = only ? n_only : s->n;
   // few points over many sources: split the sources so the GPU fills, about
   // four waves of the kernel's 7 resident blocks per SM
@@ -795,12 +796,14 @@ bool ov_direct_points(ov_state_impl* s, const double* pos, int npts, const doubl
   if (!s->img_part.reserve(bytes)) return false;
   dim3 grid(bx, nimg + 1, splits);
   if (only) {
+    if (!ensure_segtab(s, pos)) return false;
+    SegTab S{s->seg64.as<double>(), s->segid.as<int>()};
     k_direct64<<<grid, kTB, 0, s->stream>>>(s->P, S, n_src, only, pts, nullptr, skip, npts,
                                             s->img_part.as<double>(), chunk);
   } else {
     // all segments: the chain sweep over slot order (kCS == kTS: same splits)
-    k_direct64_chain<true><<<grid, kTB, 0, s->stream>>>(s->P, S, n_src, pos, pts, nullptr, skip, npts,
-                                                        s->img_part.as<double>(), chunk);
+    k_direct64_chain<true><<<grid, kTB, 0, s->stream>>>(s->P, n_src, pos, s->links.as<int2>(), s->status.as<int2>(),
+                                                        pts, skip, npts, s->img_part.as<double>(), chunk);
   }
   OV_LAUNCHED();
   OV_TRY_CUDA(cudaGetLastError());

@@ -40,26 +40,78 @@ __global__ void k_tangents(OvParams P, Links L, const double* __restrict__ pos,
   st3(nrm, k, nn);
 }
 
-// velocity assembly per node (update_velocity, src/tangle.c:583-684)
+// dxi, tangents and normals of every slot in one launch: a node's stencil
+// takes the segment lengths it needs from the positions, in dxi_node's
+// operations, instead of waiting for a pass over dxi.  A node next to a pinned
+// one reads its neighbours' tangents and is left to k_tangents (pass 1).
+// Bound by launches up to ~100k nodes and by HBM above: 1M nodes 60 us,
+// against 93 us in three launches.
+__global__ void __launch_bounds__(kThreads) k_geometry(OvParams P, Links L, const double* __restrict__ pos,
+                                                       double* dxi, double* tan, double* nrm, int n, int* flag) {
+  const int k = blockIdx.x * blockDim.x + threadIdx.x;
+  if (k >= n) return;
+  const int2 st = L.st[k];
+  if (st.x == OV_EMPTY) return;
+  const int2 lk = L.lk[k];
+  d3 t, nn;
+  if (st.x == OV_FREE && lk.x >= 0 && lk.y >= 0) {
+    const int ff = L.lk[lk.x].x, rr = L.lk[lk.y].y;
+    if (ff >= 0 && rr >= 0 && L.st[lk.x].x != OV_PINNED && L.st[lk.y].x != OV_PINNED) {
+      const d3 s0 = ld3(pos, k);
+      const d3 p[4] = {ld3(pos, ff), ld3(pos, lk.x), ld3(pos, lk.y), ld3(pos, rr)};
+      const double d0 = norm_ref(s0 - pwrap(P, s0, p[1])), d1 = norm_ref(p[1] - pwrap(P, p[1], p[0]));
+      const double dm1 = norm_ref(p[2] - pwrap(P, p[2], s0)), dm2 = norm_ref(p[3] - pwrap(P, p[3], p[2]));
+      const double x[4] = {d0 + d1, d0, -dm1, -(dm1 + dm2)};
+      stencil4(P, s0, p, x, t, nn);
+      dxi[k] = d0;
+      st3(tan, k, t);
+      st3(nrm, k, nn);
+      return;
+    }
+  }
+  double d;
+  if (!dxi_node(P, L, pos, k, d)) { atomicOr(flag, 1); return; }
+  dxi[k] = d;
+  if (near_pinned(L, k)) return;
+  auto arc = [&](int kk, int dist, double& out) {
+    return arc_length_of(L, [&](int i, double& l) { return dxi_node(P, L, pos, i, l); }, kk, dist, out);
+  };
+  if (!tangent_node(P, L, pos, k, arc, tan, t, nn)) { atomicOr(flag, 1); return; }
+  st3(tan, k, t);
+  st3(nrm, k, nn);
+}
+
+// velocity assembly per node (update_velocity, src/tangle.c:583-684) from
+// its Biot-Savart sums, read from the walk's arrays or added up here from the
+// direct sum's partials (one launch and a round trip of 48 bytes per node
+// saved), and, when a stage follows, the node's position in it
+// (x0 + h v: euler_step2, src/vortex_dynamics.c:36-52)
 // time = t0 + (*t_dev when given: a graph replayed at advancing times)
 __global__ void k_epilogue(OvParams P, Links L, const double* __restrict__ t_dev, double t0,
                            const double* __restrict__ pos, const double* __restrict__ tan,
-                           const double* __restrict__ nrm, const double* __restrict__ v_nl,
-                           const double* __restrict__ v_img, double* vels, double* vs_out, int k0,
-                           int k1, const int* __restrict__ idx, int* flag) {
+                           const double* __restrict__ nrm, OvSums S, int n_slots, OvStage G, double* vels,
+                           double* vs_out, int k0, int k1, const int* __restrict__ idx, int* flag) {
   const int i = k0 + blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= k1) return;
   const int k = idx ? idx[i] : i;
   const double t = t_dev ? t0 + *t_dev : t0;
   if (L.st[k].x == OV_EMPTY) return;
-  const d3 vnl = P.lia_only ? mk3(0, 0, 0) : ld3(v_nl, k);
-  const d3 vim = (P.lia_only || P.n_img == 0) ? mk3(0, 0, 0) : ld3(v_img, k);
+  d3 vnl = mk3(0, 0, 0), vim = vnl;
+  if (!P.lia_only) {
+    if (S.part) {
+      sum_partials(P, S.part, n_slots, S.splits, k, vnl, vim);
+    } else {
+      vnl = ld3(S.nl, k);
+      if (P.n_img > 0) vim = ld3(S.img, k);
+    }
+  }
   d3 v, vs;
   const int err = epilogue_node(P, L, t, pos, k, ld3(tan, k), ld3(nrm, k), vnl, vim, v, vs);
   if (err & 1) { atomicOr(flag, 1); return; }
   if (err) atomicOr(flag, err);
   st3(vs_out, k, vs);
   st3(vels, k, v);
+  if (G.xs) st3(G.xs, k, ld3(G.x0, k) + v * G.h);
 }
 
 // x_s = x_0 + h v  (euler_step2, src/vortex_dynamics.c:36-52)
@@ -97,9 +149,17 @@ int blocks_for(int n) { return (n + kThreads - 1) / kThreads; }
 // a CUDA graph); link and finiteness errors accumulate in *flag.
 
 bool ov_launch_geometry(cudaStream_t st, const OvParams& P, const int2* links, const int2* status,
-                        const double* pos, double* dxi, double* tan, double* nrm, int n, int* flag) {
+                        const double* pos, double* dxi, double* tan, double* nrm, int n, bool pinned, int* flag) {
   if (n <= 0) return true;
-  return ov_launch_geometry_list(st, P, links, status, pos, dxi, tan, nrm, nullptr, n, flag);
+  Links L{links, status};
+  k_geometry<<<blocks_for(n), kThreads, 0, st>>>(P, L, pos, dxi, tan, nrm, n, flag);
+  OV_LAUNCHED();
+  if (pinned) {
+    k_tangents<<<blocks_for(n), kThreads, 0, st>>>(P, L, pos, dxi, tan, nrm, nullptr, n, 1, flag);
+    OV_LAUNCHED();
+  }
+  OV_TRY_CUDA(cudaGetLastError());
+  return true;
 }
 
 bool ov_launch_geometry_list(cudaStream_t st, const OvParams& P, const int2* links, const int2* status,
@@ -119,12 +179,12 @@ bool ov_launch_geometry_list(cudaStream_t st, const OvParams& P, const int2* lin
 
 bool ov_launch_epilogue(cudaStream_t st, const OvParams& P, const int2* links, const int2* status,
                         const double* t_dev, double t0, const double* pos, const double* tan,
-                        const double* nrm, const double* v_nl, const double* v_img, double* vels,
+                        const double* nrm, const OvSums& sums, int n_slots, const OvStage& stage, double* vels,
                         double* vs, int k0, int k1, int* flag) {
   if (k1 <= k0) return true;
   Links L{links, status};
-  k_epilogue<<<blocks_for(k1 - k0), kThreads, 0, st>>>(P, L, t_dev, t0, pos, tan, nrm, v_nl, v_img,
-                                                         vels, vs, k0, k1, nullptr, flag);
+  k_epilogue<<<blocks_for(k1 - k0), kThreads, 0, st>>>(P, L, t_dev, t0, pos, tan, nrm, sums, n_slots, stage, vels, vs,
+                                                         k0, k1, nullptr, flag);
   OV_LAUNCHED();
   OV_TRY_CUDA(cudaGetLastError());
   return true;
@@ -136,8 +196,8 @@ bool ov_launch_epilogue_list(cudaStream_t st, const OvParams& P, const int2* lin
                              const int* idx, int count, int* flag) {
   if (count <= 0) return true;
   Links L{links, status};
-  k_epilogue<<<blocks_for(count), kThreads, 0, st>>>(P, L, nullptr, t0, pos, tan, nrm, v_nl, v_img, vels,
-                                                     vs, 0, count, idx, flag);
+  k_epilogue<<<blocks_for(count), kThreads, 0, st>>>(P, L, nullptr, t0, pos, tan, nrm, OvSums{v_nl, v_img, nullptr, 0},
+                                                     0, OvStage{nullptr, 0, nullptr}, vels, vs, 0, count, idx, flag);
   OV_LAUNCHED();
   OV_TRY_CUDA(cudaGetLastError());
   return true;
@@ -185,19 +245,19 @@ bool ov_geometry(ov_state_impl* s, const double* pos, double* dxi, double* tan, 
   int* flag = s->dflag.as<int>();
   OV_TRY_CUDA(cudaMemsetAsync(flag, 0, sizeof(int), s->stream));
   if (!ov_launch_geometry(s->stream, s->P, s->links.as<int2>(), s->status.as<int2>(), pos, dxi, tan,
-                          nrm, s->n, flag))
+                          nrm, s->n, s->n_active > s->n_targets, flag))
     return false;
   return check_flag(s, "update_tangents_normals");
 }
 
 bool ov_epilogue(ov_state_impl* s, double t, const double* pos, const double* tan,
-                 const double* nrm, const double* v_nl, const double* v_img, double* vels,
+                 const double* nrm, const OvSums& sums, const OvStage& stage, double* vels,
                  double* vs, int k0, int k1) {
   if (k1 <= k0) return true;
   int* flag = s->dflag.as<int>();
   OV_TRY_CUDA(cudaMemsetAsync(flag, 0, sizeof(int), s->stream));
   if (!ov_launch_epilogue(s->stream, s->P, s->links.as<int2>(), s->status.as<int2>(), nullptr, t, pos,
-                          tan, nrm, v_nl, v_img, vels, vs, k0, k1, flag))
+                          tan, nrm, sums, s->n, stage, vels, vs, k0, k1, flag))
     return false;
   return check_flag(s, "update_velocities");
 }
@@ -212,6 +272,17 @@ bool ov_euler(ov_state_impl* s, double dt) {
   return true;
 }
 
+// EMPTY slots of the stage positions are used by nothing, but some kernels
+// load them: defined once per upload
+static bool define_stages(ov_state_impl* s) {
+  if (s->stages_defined) return true;
+  const size_t bytes = sizeof(double) * 3 * (size_t)s->n;
+  OV_TRY_CUDA(cudaMemcpyAsync(s->spos.p, s->pos.p, bytes, cudaMemcpyDeviceToDevice, s->stream));
+  OV_TRY_CUDA(cudaMemcpyAsync(s->pos0.p, s->pos.p, bytes, cudaMemcpyDeviceToDevice, s->stream));
+  s->stages_defined = true;
+  return true;
+}
+
 // Stage q = 1..3 positions of rk4_step2 (src/vortex_dynamics.c:76-92):
 // xs = x0 + h_q k_q, with k_1 = vels and k_2, k_3 the stage velocities; the
 // steps h are dt/2, dt/2 and, for the last stage, dt/2 like the reference
@@ -221,9 +292,7 @@ bool ov_rk4_stage_positions(ov_state_impl* s, int q, double dt, int classic) {
   const double h[3] = {dt / 2, dt / 2, classic ? dt : dt / 2};
   double* x0 = s->pos.as<double>();
   double* xs = s->spos.as<double>();
-  // EMPTY slots of the stage positions are never read, but keep them defined
-  if (q == 1)
-    OV_TRY_CUDA(cudaMemcpyAsync(xs, x0, sizeof(double) * 3 * s->n, cudaMemcpyDeviceToDevice, s->stream));
+  if (!define_stages(s)) return false;
   const double* prev = q == 1 ? s->vels.as<double>() : (q == 2 ? s->k2.as<double>() : s->k3.as<double>());
   k_euler<<<blocks_for(s->n), kThreads, 0, s->stream>>>(s->status.as<int2>(), x0, prev, h[q - 1], xs,
                                                          s->n);
@@ -244,18 +313,21 @@ bool ov_rk4_combine(ov_state_impl* s, double dt) {
 }
 
 // rk4_step2 (src/vortex_dynamics.c:58-117) on the device state.  Stage 4
-// advances dt/2 like the reference unless `classic`.
+// advances dt/2 like the reference unless `classic`.  Each evaluation's
+// epilogue forms the next stage's positions.
 bool ov_rk4(ov_state_impl* s, double t, double dt, int classic) {
   if (s->n == 0) return true;
   double* ks[3] = {s->k2.as<double>(), s->k3.as<double>(), s->k4.as<double>()};
   const double ts[3] = {t + dt / 2, t + dt / 2, t + dt};
-  const double* xs = s->spos.as<double>();
-  for (int q = 1; q <= 3; ++q) {
-    if (!ov_rk4_stage_positions(s, q, dt, classic)) return false;
-    if (!ov_geometry(s, xs, s->sdxi.as<double>(), s->stan.as<double>(), s->snrm.as<double>()))
+  const double h[3] = {dt / 2, dt / 2, classic ? dt : dt / 2};
+  const double* x0 = s->pos.as<double>();
+  double* xs[3] = {s->spos.as<double>(), s->pos0.as<double>(), s->spos.as<double>()};
+  if (!ov_rk4_stage_positions(s, 1, dt, classic)) return false;
+  for (int q = 0; q < 3; ++q) {
+    if (!ov_geometry(s, xs[q], s->sdxi.as<double>(), s->stan.as<double>(), s->snrm.as<double>()))
       return false;
-    if (!ov_velocities(s, ts[q - 1], xs, s->sdxi.as<double>(), s->stan.as<double>(),
-                       s->snrm.as<double>(), ks[q - 1], s->svs.as<double>(), nullptr))
+    if (!ov_velocities(s, ts[q], xs[q], s->sdxi.as<double>(), s->stan.as<double>(), s->snrm.as<double>(), ks[q],
+                       s->svs.as<double>(), nullptr, q < 2 ? OvStage{x0, h[q + 1], xs[q + 1]} : kNoStage))
       return false;
   }
   return ov_rk4_combine(s, dt);

@@ -106,6 +106,24 @@ struct OvTree {
   int n_perm_warps = 0;   // units the order in wvals covers (0: none yet)
 };
 
+// The Biot-Savart sums of an evaluation as the epilogue reads them: the
+// tangle's sum and the image sum per slot, or (part set) the direct sum's
+// partials per split, image and slot.
+struct OvSums {
+  const double* nl;
+  const double* img;
+  const double* part;
+  int splits;
+};
+// the stage that follows an evaluation: xs = x0 + h v (xs null: none; xs must
+// not be the positions the evaluation reads)
+struct OvStage {
+  const double* x0;
+  double h;
+  double* xs;
+};
+constexpr OvStage kNoStage = {nullptr, 0, nullptr};
+
 // ---------------------------------------------------------------- state
 struct ov_state_impl {
   int cap = 0;          // slot capacity of the device arrays
@@ -115,12 +133,15 @@ struct ov_state_impl {
   cudaEvent_t ev0 = nullptr, ev1 = nullptr, ev2 = nullptr;
   // slot-indexed (AoS, 3 doubles per vector, as struct vec3d)
   DevBuf pos, links, status, dxi, tan, nrm, vels, vs;
-  // RK4 scratch
+  // RK4 scratch (two stage positions: an evaluation reads one while its
+  // epilogue writes the other)
+  bool stages_defined = false;
   DevBuf pos0, spos, sdxi, stan, snrm, svs, k2, k3, k4;
   // Biot-Savart outputs: primary sum and image sum per slot
   DevBuf v_nl, v_img;
   // direct-sum per-image partials and segment table
   DevBuf img_part, seg64, segid;
+  OvSums sums = {nullptr, nullptr, nullptr, 0};   // of the evaluation under way
   // error flag written by kernels (bounded waits, broken links)
   DevBuf dflag;
   OvTree tree;
@@ -156,7 +177,7 @@ bool ov_geometry(ov_state_impl* s, const double* pos, double* dxi, double* tan, 
 // velocities at positions pos with tangents/normals -> vels, vs
 bool ov_velocities(ov_state_impl* s, double t, const double* pos, const double* dxi,
                    const double* tan, const double* nrm, double* vels, double* vs,
-                   OvTree* external_tree);
+                   OvTree* external_tree, const OvStage& stage = kNoStage);
 // one RK4 step on the state's pos using the state's vels as k1
 bool ov_rk4(ov_state_impl* s, double t, double dt, int classic);
 // its pieces: stage q = 1..3 positions into spos, and the final combination
@@ -190,6 +211,8 @@ bool ov_radix_sort_u64(uint64_t* ka, int* va, uint64_t* kb, int* vb, int n, int 
                        DevBuf& scan_part, cudaStream_t st);
 // direct sums for all nodes -> v_nl, v_img
 bool ov_direct_nodes(ov_state_impl* s, const double* pos, double* v_nl, double* v_img);
+// the same left as partials (in s->img_part) for the epilogue to add up
+bool ov_direct_partials(ov_state_impl* s, const double* pos, double* v_nl, double* v_img, OvSums* out);
 // direct sums at arbitrary points (device arrays), sources = all segments or
 // the slot list `only`: out_nl = the tangle's own sum, out_img = image sum
 // (nullptr: no images)
@@ -211,19 +234,20 @@ bool ov_segment_table(ov_state_impl* s, const double* pos);
 // out = a + b for n vectors of 3 doubles (device)
 bool ov_add3(cudaStream_t st, const double* a, const double* b, double* out, int n);
 
-// epilogue: LIA + external + v_nl + v_img + hyperfriction + mutual friction
-// for slots k0 <= k < k1
+// epilogue: LIA + external + Biot-Savart sums + hyperfriction + mutual
+// friction for slots k0 <= k < k1, and the following stage's positions
 bool ov_epilogue(ov_state_impl* s, double t, const double* pos, const double* tan,
-                 const double* nrm, const double* v_nl, const double* v_img,
+                 const double* nrm, const OvSums& sums, const OvStage& stage,
                  double* vels, double* vs, int k0, int k1);
 
 bool ov_state_reserve(ov_state_impl* s, int n);
 
 // Launches only, no host synchronisation (CUDA-graph capturable); link and
 // finiteness errors accumulate in *flag (bit 0 broken links, bit 1
-// non-finite velocity), read back later with ov_flag_status.
+// non-finite velocity), read back later with ov_flag_status.  pinned: the
+// tangle may have PINNED nodes (their neighbours take a second launch).
 bool ov_launch_geometry(cudaStream_t st, const OvParams& P, const int2* links, const int2* status,
-                        const double* pos, double* dxi, double* tan, double* nrm, int n, int* flag);
+                        const double* pos, double* dxi, double* tan, double* nrm, int n, bool pinned, int* flag);
 // the same for the slots idx[0 .. n-1] only (dxi of all of them first, then
 // the two tangent passes); the other slots' values are read as stored
 bool ov_launch_geometry_list(cudaStream_t st, const OvParams& P, const int2* links, const int2* status,
@@ -232,7 +256,7 @@ bool ov_launch_geometry_list(cudaStream_t st, const OvParams& P, const int2* lin
 // epilogue at time t0 + *t_dev (t_dev may be null: time t0)
 bool ov_launch_epilogue(cudaStream_t st, const OvParams& P, const int2* links, const int2* status,
                         const double* t_dev, double t0, const double* pos, const double* tan,
-                        const double* nrm, const double* v_nl, const double* v_img, double* vels,
+                        const double* nrm, const OvSums& sums, int n_slots, const OvStage& stage, double* vels,
                         double* vs, int k0, int k1, int* flag);
 // the epilogue of the slots idx[0 .. count-1] at time t0
 bool ov_launch_epilogue_list(cudaStream_t st, const OvParams& P, const int2* links, const int2* status,

@@ -50,21 +50,25 @@ __device__ bool step_node(const OvParams& P, const Links& L, const double* pos, 
   return true;
 }
 
-// Arc length `dist` links away along the stored segment lengths
-// (arc_length, src/tangle.c:208-243); reverses at a pinned end.
-__device__ bool arc_length(const Links& L, const double* dxi, int k, int dist, double& out) {
+// Arc length `dist` links away along the segment lengths seg(k, out) of the
+// nodes on the way (arc_length, src/tangle.c:208-243); reverses at a pinned
+// end.
+template <class Seg>
+__device__ __forceinline__ bool arc_length_of(const Links& L, Seg&& seg, int k, int dist, double& out) {
   double acc = 0;
   int cur = k, d = dist;
   for (int it = 0; it < 16 && d != 0; ++it) {
     bool pin = pinned_any(L.st[cur].x);
     int2 lk = L.lk[cur];
+    double l;
     if (d > 0) {
       if (lk.x < 0) {
         if (!pin) return false;
         d = -d;
         continue;
       }
-      acc += dxi[cur];
+      if (!seg(cur, l)) return false;
+      acc += l;
       cur = lk.x;
       --d;
     } else {
@@ -73,7 +77,8 @@ __device__ bool arc_length(const Links& L, const double* dxi, int k, int dist, d
         d = -d;
         continue;
       }
-      acc += dxi[lk.y];
+      if (!seg(lk.y, l)) return false;
+      acc += l;
       cur = lk.y;
       ++d;
     }
@@ -81,6 +86,17 @@ __device__ bool arc_length(const Links& L, const double* dxi, int k, int dist, d
   if (d != 0) return false;
   out = acc;
   return true;
+}
+
+// the same along the stored segment lengths
+__device__ bool arc_length(const Links& L, const double* dxi, int k, int dist, double& out) {
+  return arc_length_of(
+      L,
+      [&](int i, double& l) {
+        l = dxi[i];
+        return true;
+      },
+      k, dist, out);
 }
 
 }  // namespace
