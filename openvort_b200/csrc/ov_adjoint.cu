@@ -542,17 +542,16 @@ void ov_adjoint_destroy(ov_adjoint* a) {
   for (DevBuf* b : sb) b->release();
   ov_tree_release(&s->tree);
   if (s->stream) cudaStreamDestroy(s->stream);
-  if (s->ev0) cudaEventDestroy(s->ev0);
-  if (s->ev1) cudaEventDestroy(s->ev1);
-  if (s->ev2) cudaEventDestroy(s->ev2);
+  ov_events_release(s);
   delete a;
 }
 
 int ov_adjoint_velocity(ov_adjoint* a, const double* x, const double* vn, double t, double* v) {
   ov_clear_error();
   if (!a || !v) { ov_set_error(OV_ERR_INVALID, "null adjoint or output"); return ov_last_error(); }
-  if (!set_vn(a, vn) || !upload_pos(a, x, a->ybar.as<double>()) ||
+  if (!set_vn(a, vn) || !upload_pos(a, x, a->ybar.as<double>()) || !ov_eval_begin(&a->s) ||
       !velocity_at(a, a->ybar.as<double>(), t, a->tmp_v.as<double>()) ||
+      !ov_eval_collect(&a->s, "ov_adjoint_velocity") ||
       !sync_to(a, v, a->tmp_v.as<double>(), 3 * (size_t)a->n))
     return ov_last_error();
   return OV_OK;
@@ -591,7 +590,7 @@ int ov_adjoint_forward(ov_adjoint* a, const double* x0, const double* vn, double
   const int n_ckpt = (nsteps + every - 1) / every;
   if (!set_vn(a, vn) || !upload_pos(a, x0, s->pos.as<double>()) ||
       !a->ckpt.reserve(sizeof(double) * v3 * std::max(1, n_ckpt)) ||
-      !a->blk.reserve(sizeof(double) * v3 * every))
+      !a->blk.reserve(sizeof(double) * v3 * every) || !ov_eval_begin(s))
     return ov_last_error();
   for (int i = 0; i < nsteps; ++i) {
     if (i % every == 0 &&
@@ -601,7 +600,7 @@ int ov_adjoint_forward(ov_adjoint* a, const double* x0, const double* vn, double
       return ov_last_error();
     if (!forward_step(a, t0 + i * dt)) return ov_last_error();
   }
-  if (!sync_to(a, x_final, s->pos.as<double>(), v3)) return ov_last_error();
+  if (!ov_eval_collect(s, "ov_adjoint_forward") || !sync_to(a, x_final, s->pos.as<double>(), v3)) return ov_last_error();
   for (int c = 0; c < 3; ++c) a->fwd_vn[c] = a->vn[c];
   a->fwd_precision = s->P.precision;
   a->have_fwd = 1;
@@ -621,7 +620,7 @@ int ov_adjoint_backward(ov_adjoint* a, const double* x_final_bar, double* x0_bar
   // calls or precision changes came in between
   if (!set_vn(a, a->fwd_vn)) return ov_last_error();
   s->P.precision = a->fwd_precision;
-  if (!upload_pos(a, x_final_bar, a->xbar.as<double>()) ||
+  if (!upload_pos(a, x_final_bar, a->xbar.as<double>()) || !ov_eval_begin(s) ||
       !ov_cuda_ok(cudaMemsetAsync(a->vnbar.p, 0, 64, s->stream), "cudaMemsetAsync"))
     return ov_last_error();
   const int n_ckpt = (a->nsteps + a->every - 1) / a->every;
@@ -642,7 +641,7 @@ int ov_adjoint_backward(ov_adjoint* a, const double* x_final_bar, double* x0_bar
     for (int i = i1 - 1; i >= i0; --i)
       if (!reverse_step(a, a->blk.as<double>() + v3 * (i - i0), a->t0 + i * a->dt)) return ov_last_error();
   }
-  if (!sync_to(a, x0_bar, a->xbar.as<double>(), v3) || !sync_to(a, vn_bar, a->vnbar.as<double>(), vn_bar ? 3 : 0))
+  if (!ov_eval_collect(s, "ov_adjoint_backward") || !sync_to(a, x0_bar, a->xbar.as<double>(), v3) || !sync_to(a, vn_bar, a->vnbar.as<double>(), vn_bar ? 3 : 0))
     return ov_last_error();
   return OV_OK;
 }

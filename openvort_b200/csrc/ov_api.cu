@@ -396,13 +396,45 @@ bool ov_capture_params(const tangle_state* t, OvParams& P) { return capture_para
 // ======================================================================
 // state management
 
+// the events of slot i, created on its first use, as the evaluation's
+static bool use_slot(ov_state_impl* s, int i) {
+  OvEvalSlot& e = s->slots[i];
+  for (cudaEvent_t& ev : e.ev)
+    if (!ev) OV_TRY_CUDA(cudaEventCreate(&ev));
+  s->ev0 = e.ev[0];
+  s->ev1 = e.ev[1];
+  s->ev2 = e.ev[2];
+  return true;
+}
+
+void ov_events_release(ov_state_impl* s) {
+  for (OvEvalSlot& e : s->slots)
+    for (cudaEvent_t& ev : e.ev) {
+      if (ev) cudaEventDestroy(ev);
+      ev = nullptr;
+    }
+  s->ev0 = s->ev1 = s->ev2 = nullptr;
+  s->evctr.release();
+}
+
+void* ov_pinned_scratch() {
+  struct Pinned {
+    void* p = nullptr;
+    ~Pinned() {
+      if (p) cudaFreeHost(p);
+    }
+  };
+  static thread_local Pinned buf;
+  if (!buf.p && !ov_cuda_ok(cudaMallocHost(&buf.p, kPinnedScratch), "cudaMallocHost")) buf.p = nullptr;
+  return buf.p;
+}
+
 bool ov_state_reserve(ov_state_impl* s, int n) {
   if (!s->stream) {
     OV_TRY_CUDA(cudaStreamCreateWithFlags(&s->stream, cudaStreamNonBlocking));
-    OV_TRY_CUDA(cudaEventCreate(&s->ev0));
-    OV_TRY_CUDA(cudaEventCreate(&s->ev1));
-    OV_TRY_CUDA(cudaEventCreate(&s->ev2));
-    if (!s->dflag.reserve(64)) return false;
+    if (!s->dflag.reserve(64) || !s->evctr.reserve(sizeof(unsigned long long) * 3 * kEvalSlots) || !use_slot(s, 0))
+      return false;
+    OV_TRY_CUDA(cudaMemsetAsync(s->dflag.p, 0, 64, s->stream));
   }
   s->n = n;
   if (n <= s->cap) return true;
@@ -427,9 +459,8 @@ static void state_release(ov_state_impl* s) {
   for (DevBuf* b : bufs) b->release();
   ov_tree_release(&s->tree);
   if (s->stream) cudaStreamDestroy(s->stream);
-  if (s->ev0) cudaEventDestroy(s->ev0);
-  if (s->ev1) cudaEventDestroy(s->ev1);
-  if (s->ev2) cudaEventDestroy(s->ev2);
+  ov_events_release(s);
+  s->pending = 0;
   s->stream = nullptr;
   s->cap = s->n = 0;
 }
@@ -535,56 +566,100 @@ bool ov_download_fields(ov_state_impl* s, tangle_state* t, int what) {
   return ok && sync(s);
 }
 
-// The Biot-Savart sums of an evaluation into v_nl, v_img: the tree build and
+bool ov_eval_begin(ov_state_impl* s) {
+  s->pending = 0;
+  OV_TRY_CUDA(cudaMemsetAsync(s->dflag.p, 0, sizeof(int), s->stream));
+  return true;
+}
+
+bool ov_eval_collect(ov_state_impl* s, const char* where) {
+  char* host = static_cast<char*>(ov_pinned_scratch());
+  if (!host) return false;
+  int* flag = reinterpret_cast<int*>(host);
+  unsigned long long* ctr = reinterpret_cast<unsigned long long*>(host + 64);
+  static_assert(64 + sizeof(unsigned long long) * 3 * kEvalSlots <= kPinnedScratch, "read-back buffer");
+  bool walk = false;
+  for (int i = 0; i < s->pending; ++i) walk = walk || s->slots[i].walk;
+  OV_TRY_CUDA(cudaMemcpyAsync(flag, s->dflag.p, sizeof(int), cudaMemcpyDeviceToHost, s->stream));
+  if (walk)
+    OV_TRY_CUDA(cudaMemcpyAsync(ctr, s->evctr.p, sizeof(unsigned long long) * 3 * s->pending, cudaMemcpyDeviceToHost,
+                                s->stream));
+  OV_TRY_CUDA(cudaStreamSynchronize(s->stream));
+  const int pending = s->pending;
+  s->pending = 0;
+  // device times from the events around the tree build and the Biot-Savart
+  // kernel
+  for (int i = 0; i < pending; ++i) {
+    const OvEvalSlot& e = s->slots[i];
+    float build_ms = 0, bs_ms = 0;
+    if (!e.lia && (cudaEventElapsedTime(&build_ms, e.ev[0], e.ev[1]) != cudaSuccess ||
+                   cudaEventElapsedTime(&bs_ms, e.ev[1], e.ev[2]) != cudaSuccess))
+      (void)cudaGetLastError();
+    tl_stats.interactions = e.walk ? (double)ctr[3 * i] : e.inter;
+    tl_stats.cell_interactions = e.walk ? (double)ctr[3 * i + 1] : 0;
+    tl_stats.warp_iterations = e.walk ? (double)ctr[3 * i + 2] : 0;
+    tl_stats.build_ms = build_ms;
+    tl_stats.eval_ms = bs_ms;
+    tl_stats.total_ms = build_ms + bs_ms;
+    s->acc_evals += 1;
+    s->acc_build_ms += build_ms;
+    s->acc_bs_ms += bs_ms;
+    s->acc_bs_launches += e.lia ? 0 : 1;
+    s->acc_inter += tl_stats.interactions;
+    s->acc_cells += tl_stats.cell_interactions;
+    s->acc_warp_iter += tl_stats.warp_iterations;
+  }
+  return ov_flag_status(*flag, where);
+}
+
+// Evaluations a state launches between two waits.  A wait costs some 15 us,
+// so small evaluations go on for 16 (a 256-node ring's RK4 step 330 us with a
+// wait for each error flag, RING_NOW without); a direct sum of more than 2e7
+// interactions, over 50 us, is waited for each time, so positions that
+// have become NaN are not carried far.  The tree build reads the error flag
+// back with its cell count.
+static int max_pending(const ov_state_impl* s) {
+  if (s->P.lia_only || s->P.use_bh) return kEvalSlots;
+  return (double)s->n_targets * (double)s->n_segments * (1 + s->P.n_img) <= 2e7 ? kEvalSlots : 1;
+}
+
+// The Biot-Savart sums of an evaluation into s->sums: the tree build and
 // walk (for the targets at key positions [k0, k0 + k_count) of the tree; all
 // of them when k_count < 0), or the direct sum.
 static bool bs_sums(ov_state_impl* s, const double* pos, OvTree* external_tree, int k0, int k_count) {
   tl_last_state = s;
+  if (s->pending >= max_pending(s) && !ov_eval_collect(s, "update_velocities")) return false;
   tl_stats = OvStatsAcc{0, 0, 0, 0, 0, 0, 0};
-  cudaEventRecord(s->ev0, s->stream);
-  cudaEventRecord(s->ev1, s->stream);
-  cudaEventRecord(s->ev2, s->stream);
+  if (!use_slot(s, s->pending)) return false;
+  OvEvalSlot& slot = s->slots[s->pending];
+  slot.inter = 0;
+  slot.walk = false;
+  slot.lia = s->P.lia_only != 0;
   double* v_nl = s->v_nl.as<double>();
   double* v_img = s->v_img.as<double>();
   s->sums = OvSums{v_nl, v_img, nullptr, 0};
-  if (!s->P.lia_only) {
-    if (s->P.use_bh) {
-      OvTree* tree = external_tree;
-      if (!tree) {
-        if (!ov_tree_build(s, pos, &s->tree)) return false;
-        tree = &s->tree;
-      }
-      if (!ov_tree_walk_nodes(s, tree, pos, tree == &s->tree, v_nl, v_img, k0, k_count)) return false;
-    } else {
-      if (!ov_direct_partials(s, pos, v_nl, v_img, &s->sums)) return false;
-      // every target against every segment, per image (src/tangle.c:612-636)
-      tl_stats.interactions = (double)s->n_targets * (double)s->n_segments * (1 + s->P.n_img);
+  if (s->P.lia_only) return true;
+  cudaEventRecord(s->ev0, s->stream);
+  if (s->P.use_bh) {
+    OvTree* tree = external_tree;
+    if (!tree) {
+      if (!ov_tree_build(s, pos, &s->tree)) return false;
+      tree = &s->tree;
+      if (tree->flag_seen && !ov_flag_status(tree->flag_seen, "update_velocities")) return false;
     }
+    slot.walk = true;
+    return ov_tree_walk_nodes(s, tree, pos, tree == &s->tree, v_nl, v_img, k0, k_count);
   }
-  return true;
+  // every target against every segment, per image (src/tangle.c:612-636)
+  slot.inter = (double)s->n_targets * (double)s->n_segments * (1 + s->P.n_img);
+  return ov_direct_partials(s, pos, v_nl, v_img, &s->sums);
 }
 
-// The epilogue of an evaluation over every node, and the state's counters.
+// The epilogue of an evaluation over every node.
 static bool finish_velocities(ov_state_impl* s, double t, const double* pos, const double* tan,
                               const double* nrm, const OvStage& stage, double* vels, double* vs) {
-  if (!ov_epilogue(s, t, pos, tan, nrm, s->sums, stage, vels, vs, 0, s->n))
-    return false;
-  // the epilogue synchronised the stream: fold this evaluation into the
-  // state's counters (device times from the events around the tree build and
-  // the Biot-Savart kernel)
-  float build_ms = 0, bs_ms = 0;
-  cudaEventElapsedTime(&build_ms, s->ev0, s->ev1);
-  cudaEventElapsedTime(&bs_ms, s->ev1, s->ev2);
-  tl_stats.build_ms = build_ms;
-  tl_stats.eval_ms = bs_ms;
-  tl_stats.total_ms = build_ms + bs_ms;
-  s->acc_evals += 1;
-  s->acc_build_ms += build_ms;
-  s->acc_bs_ms += bs_ms;
-  s->acc_bs_launches += s->P.lia_only ? 0 : 1;
-  s->acc_inter += tl_stats.interactions;
-  s->acc_cells += tl_stats.cell_interactions;
-  s->acc_warp_iter += tl_stats.warp_iterations;
+  if (!ov_epilogue(s, t, pos, tan, nrm, s->sums, stage, vels, vs, 0, s->n)) return false;
+  ++s->pending;
   return true;
 }
 
@@ -635,16 +710,18 @@ int ov_state_download(ov_state* st, struct tangle_state* t, int what) {
   return OV_OK;
 }
 
+// update_tangle's launches on the state
+static bool launch_update(ov_state_impl* s, double t, const OvStage& stage) {
+  s->P.precision = g_precision;
+  return ov_geometry(s, s->pos.as<double>(), s->dxi.as<double>(), s->tan.as<double>(), s->nrm.as<double>()) &&
+         ov_velocities(s, t, s->pos.as<double>(), s->dxi.as<double>(), s->tan.as<double>(), s->nrm.as<double>(),
+                       s->vels.as<double>(), s->vs.as<double>(), nullptr, stage);
+}
+
 int ov_state_update_tangle(ov_state* st, double t) {
   ov_clear_error();
   ov_state_impl* s = &st->impl;
-  s->P.precision = g_precision;
-  if (!ov_geometry(s, s->pos.as<double>(), s->dxi.as<double>(), s->tan.as<double>(),
-                   s->nrm.as<double>()))
-    return tl_err;
-  if (!ov_velocities(s, t, s->pos.as<double>(), s->dxi.as<double>(), s->tan.as<double>(),
-                     s->nrm.as<double>(), s->vels.as<double>(), s->vs.as<double>(), nullptr))
-    return tl_err;
+  if (!ov_eval_begin(s) || !launch_update(s, t, kNoStage) || !ov_eval_collect(s, "update_tangle")) return tl_err;
   return OV_OK;
 }
 
@@ -652,7 +729,7 @@ int ov_state_rk4_step(ov_state* st, double t, double dt) {
   ov_clear_error();
   ov_state_impl* s = &st->impl;
   s->P.precision = g_precision;
-  if (!ov_rk4(s, t, dt, g_rk4_classic)) return tl_err;
+  if (!ov_eval_begin(s) || !ov_rk4(s, t, dt, g_rk4_classic) || !ov_eval_collect(s, "rk4_step")) return tl_err;
   return OV_OK;
 }
 
@@ -665,15 +742,14 @@ int ov_state_run(ov_state* st, double t0, double dt, int nsteps) {
   }
   cudaEventRecord(s->ev_run0, s->stream);
   double t = t0;
+  OvStage first = kNoStage;
+  if (!ov_eval_begin(s) || (s->n > 0 && !ov_rk4_first(s, dt, &first))) return tl_err;
   for (int i = 0; i < nsteps; ++i) {
-    int e = ov_state_update_tangle(st, t);
-    if (e) return e;
-    e = ov_state_rk4_step(st, t, dt);
-    if (e) return e;
+    if (!launch_update(s, t, first) || !ov_rk4(s, t, dt, g_rk4_classic, true)) return tl_err;
     t += dt;
   }
   cudaEventRecord(s->ev_run1, s->stream);
-  if (!sync(s)) return tl_err;
+  if (!ov_eval_collect(s, "ov_state_run")) return tl_err;
   float ms = 0;
   cudaEventElapsedTime(&ms, s->ev_run0, s->ev_run1);
   s->last_run_ms = ms;
@@ -761,18 +837,16 @@ int ov_state_shard_begin(ov_state* st, int q, double t, double dt) {
   ov_state_impl* s = &st->impl;
   s->P.precision = g_precision;
   if (!shard_ready(s, q)) return tl_err;
-  if (q > 0 && !ov_rk4_stage_positions(s, q, dt, g_rk4_classic)) return tl_err;
+  if (!ov_eval_begin(s) || (q > 0 && !ov_rk4_stage_positions(s, q, dt, g_rk4_classic))) return tl_err;
   const ShardStage g = shard_stage(s, q, t, dt);
   if (!ov_geometry(s, g.pos, g.dxi, g.tan, g.nrm)) return tl_err;
   const int c = shard_chunk(s, s->shard_world);
   if (!bs_sums(s, g.pos, nullptr, s->shard_rank * c, c)) return tl_err;
-  s->shard_inter = tl_stats.interactions;
-  s->shard_cells = tl_stats.cell_interactions;
-  s->shard_warp_iter = tl_stats.warp_iterations;
   if (!s->P.lia_only && !ov_shard_pack(s, s->shard_rank * c, c, s->xbuf, s->xbytes / sizeof(double)))
     return tl_err;
-  // the caller's exchange reads xbuf from another stream
-  if (!sync(s)) return tl_err;
+  // the caller's exchange reads xbuf from another stream; link errors are
+  // reported before it
+  if (!ov_eval_collect(s, "update_tangents_normals")) return tl_err;
   return OV_OK;
 }
 
@@ -784,9 +858,9 @@ int ov_state_shard_end(ov_state* st, int q, double t, double dt) {
   const ShardStage g = shard_stage(s, q, t, dt);
   if (!s->P.lia_only && !ov_shard_unpack(s, s->xbuf, s->xbytes / sizeof(double))) return tl_err;
   tl_last_state = s;
-  tl_stats = OvStatsAcc{s->shard_inter, s->shard_cells, 0, 0, 0, 0, s->shard_warp_iter};
   if (!finish_velocities(s, g.t, g.pos, g.tan, g.nrm, kNoStage, g.vels, g.vs)) return tl_err;
-  if (q == 3 && !(ov_rk4_combine(s, dt) && sync(s))) return tl_err;
+  if (q == 3 && !ov_rk4_combine(s, dt)) return tl_err;
+  if (!ov_eval_collect(s, "update_velocities")) return tl_err;
   return OV_OK;
 }
 
@@ -916,7 +990,9 @@ void update_tangents_normals(struct tangle_state* tangle) {
   ov_state_impl& s = tls_state();
   if (!upload_tangle(&s, tangle, false)) return;
   size_t n = (size_t)tangle->N;
-  if (!ov_geometry(&s, s.pos.as<double>(), s.dxi.as<double>(), s.tan.as<double>(), s.nrm.as<double>()))
+  if (!ov_eval_begin(&s) ||
+      !ov_geometry(&s, s.pos.as<double>(), s.dxi.as<double>(), s.tan.as<double>(), s.nrm.as<double>()) ||
+      !ov_eval_collect(&s, "update_tangents_normals"))
     return;
   if (download(&s, tangle->dxi, s.dxi, 8 * n) && download(&s, tangle->tangents, s.tan, 24 * n) &&
       download(&s, tangle->normals, s.nrm, 24 * n))
@@ -935,7 +1011,9 @@ void update_tangent_normal(struct tangle_state* tangle, size_t k) {
   }
   if (tangle->status[k].status == EMPTY) return;
   if (!upload_tangle(&s, tangle, false)) return;
-  if (!ov_geometry(&s, s.pos.as<double>(), s.dxi.as<double>(), s.tan.as<double>(), s.nrm.as<double>()))
+  if (!ov_eval_begin(&s) ||
+      !ov_geometry(&s, s.pos.as<double>(), s.dxi.as<double>(), s.tan.as<double>(), s.nrm.as<double>()) ||
+      !ov_eval_collect(&s, "update_tangent_normal"))
     return;
   cudaMemcpyAsync(&tangle->tangents[k], s.tan.as<double>() + 3 * k, 24, cudaMemcpyDeviceToHost, s.stream);
   cudaMemcpyAsync(&tangle->normals[k], s.nrm.as<double>() + 3 * k, 24, cudaMemcpyDeviceToHost, s.stream);
@@ -954,8 +1032,10 @@ void update_velocities(struct tangle_state* tangle, double t, struct octree* tre
     ov_set_error(OV_ERR_INVALID, "octree built for %d slots, tangle has %d", tree->h.st.n, tangle->N);
     return;
   }
-  if (!ov_velocities(&s, t, s.pos.as<double>(), s.dxi.as<double>(), s.tan.as<double>(),
-                     s.nrm.as<double>(), s.vels.as<double>(), s.vs.as<double>(), ext))
+  if (!ov_eval_begin(&s) ||
+      !ov_velocities(&s, t, s.pos.as<double>(), s.dxi.as<double>(), s.tan.as<double>(),
+                     s.nrm.as<double>(), s.vels.as<double>(), s.vs.as<double>(), ext) ||
+      !ov_eval_collect(&s, "update_velocities"))
     return;
   if (download(&s, tangle->vels, s.vels, 24 * n) && download(&s, tangle->vs, s.vs, 24 * n)) sync(&s);
 }
@@ -979,7 +1059,8 @@ void update_velocity(struct tangle_state* tangle, int k, double t, struct octree
   }
   DevBuf skip;
   if (!skip.reserve(sizeof(int))) return;
-  bool ok = ov_cuda_ok(cudaMemcpyAsync(skip.p, &k, sizeof(int), cudaMemcpyHostToDevice, s.stream),
+  bool ok = ov_eval_begin(&s) &&
+            ov_cuda_ok(cudaMemcpyAsync(skip.p, &k, sizeof(int), cudaMemcpyHostToDevice, s.stream),
                        "cudaMemcpyAsync");
   const double* pt = s.pos.as<double>() + 3 * (size_t)k;
   double* nl = s.v_nl.as<double>() + 3 * (size_t)k;
@@ -992,7 +1073,8 @@ void update_velocity(struct tangle_state* tangle, int k, double t, struct octree
   }
   ok = ok && ov_epilogue(&s, t, s.pos.as<double>(), s.tan.as<double>(), s.nrm.as<double>(),
                          OvSums{s.v_nl.as<double>(), s.v_img.as<double>(), nullptr, 0}, kNoStage,
-                         s.vels.as<double>(), s.vs.as<double>(), k, k + 1);
+                         s.vels.as<double>(), s.vs.as<double>(), k, k + 1) &&
+       ov_eval_collect(&s, "update_velocity");
   if (ok) {
     cudaMemcpyAsync(&tangle->vels[k], s.vels.as<double>() + 3 * (size_t)k, 24, cudaMemcpyDeviceToHost,
                     s.stream);
@@ -1063,7 +1145,7 @@ void rk4_step(struct tangle_state* tangle, double t, double dt) {
   size_t n = (size_t)tangle->N;
   if (n == 0) return;
   if (!upload(&s, tangle->vels, s.vels, 24 * n)) return;
-  if (ov_rk4(&s, t, dt, g_rk4_classic) && download(&s, tangle->vnodes, s.pos, 24 * n)) sync(&s);
+  if (ov_eval_begin(&s) && ov_rk4(&s, t, dt, g_rk4_classic) && ov_eval_collect(&s, "rk4_step") && download(&s, tangle->vnodes, s.pos, 24 * n)) sync(&s);
 }
 
 struct octree* octree_build(const struct tangle_state* tangle, int quadtree) {

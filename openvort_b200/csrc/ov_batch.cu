@@ -701,9 +701,7 @@ void ov_batch_destroy(ov_batch* b) {
                   &b->s.k2, &b->s.k3, &b->s.k4, &b->s.v_nl, &b->s.v_img, &b->s.dflag};
   for (DevBuf* d : sb) d->release();
   if (b->s.stream) cudaStreamDestroy(b->s.stream);
-  if (b->s.ev0) cudaEventDestroy(b->s.ev0);
-  if (b->s.ev1) cudaEventDestroy(b->s.ev1);
-  if (b->s.ev2) cudaEventDestroy(b->s.ev2);
+  ov_events_release(&b->s);
   delete b;
 }
 

@@ -706,7 +706,11 @@ static int source_chunk(int n_src, long long blocks, int tile, int* splits, int 
 
 bool ov_direct_partials(ov_state_impl* s, const double* pos, double* v_nl, double* v_img, OvSums* out) {
   *out = OvSums{v_nl, v_img, nullptr, 0};
-  if (s->n == 0) return true;
+  if (s->n == 0) {
+    cudaEventRecord(s->ev1, s->stream);
+    cudaEventRecord(s->ev2, s->stream);
+    return true;
+  }
   int nimg = s->P.n_img;
   int splits = 1;
   if (s->P.precision == OV_PREC_MIXED) {
@@ -718,7 +722,7 @@ bool ov_direct_partials(ov_state_impl* s, const double* pos, double* v_nl, doubl
     const bool slot_order = work <= kSlotOrderWork;
     int n_t = s->n;
     if (!slot_order) {
-      if (!ov_tree_build(s, pos, &s->tree)) return false;
+      if (!ov_tree_build(s, pos, &s->tree, true)) return false;
       n_t = s->tree.n_nodes;
     }
     if ((slot_order ? s->n_active : s->tree.n_nodes) == 0) {

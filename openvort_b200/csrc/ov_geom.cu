@@ -126,9 +126,10 @@ __global__ void k_euler(const int2* __restrict__ st, const double* __restrict__ 
 // x += dt/6 k1 + dt/3 k2 + dt/3 k3 + dt/6 k4 (src/vortex_dynamics.c:94-112)
 __global__ void k_rk4_combine(const int2* __restrict__ st, const double* __restrict__ k1,
                               const double* __restrict__ k2, const double* __restrict__ k3,
-                              const double* __restrict__ k4, double dt, double* x, int n) {
+                              const double* __restrict__ k4, double dt, double* x, int n,
+                              const int* __restrict__ flag) {
   int k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= n || st[k].x == OV_EMPTY) return;
+  if (k >= n || st[k].x == OV_EMPTY || (flag && *flag)) return;
 #pragma unroll
   for (int c = 0; c < 3; ++c) {
     int i = 3 * k + c;
@@ -213,9 +214,9 @@ bool ov_launch_euler(cudaStream_t st, const int2* status, const double* x0, cons
 }
 
 bool ov_launch_rk4_combine(cudaStream_t st, const int2* status, const double* k1, const double* k2,
-                           const double* k3, const double* k4, double dt, double* x, int n) {
+                           const double* k3, const double* k4, double dt, double* x, int n, const int* flag) {
   if (n <= 0) return true;
-  k_rk4_combine<<<blocks_for(n), kThreads, 0, st>>>(status, k1, k2, k3, k4, dt, x, n);
+  k_rk4_combine<<<blocks_for(n), kThreads, 0, st>>>(status, k1, k2, k3, k4, dt, x, n, flag);
   OV_LAUNCHED();
   OV_TRY_CUDA(cudaGetLastError());
   return true;
@@ -226,6 +227,10 @@ bool ov_flag_status(int h, const char* where) {
     ov_set_error(OV_ERR_INVALID, "%s: broken vortex links (a free node without a neighbour)", where);
     return false;
   }
+  if (h & 4) {
+    ov_set_error(OV_ERR_TREE_DEPTH, "%s: the box / BH_grain ratio needs more than %d octree levels", where, kTreeLevels);
+    return false;
+  }
   if (h & 2) {
     ov_set_error(OV_ERR_NONFINITE, "%s: non-finite velocity", where);
     return false;
@@ -233,33 +238,18 @@ bool ov_flag_status(int h, const char* where) {
   return true;
 }
 
-static bool check_flag(ov_state_impl* s, const char* where) {
-  int h = 0;
-  OV_TRY_CUDA(cudaMemcpyAsync(&h, s->dflag.p, sizeof(int), cudaMemcpyDeviceToHost, s->stream));
-  OV_TRY_CUDA(cudaStreamSynchronize(s->stream));
-  return ov_flag_status(h, where);
-}
-
 bool ov_geometry(ov_state_impl* s, const double* pos, double* dxi, double* tan, double* nrm) {
   if (s->n == 0) return true;
-  int* flag = s->dflag.as<int>();
-  OV_TRY_CUDA(cudaMemsetAsync(flag, 0, sizeof(int), s->stream));
-  if (!ov_launch_geometry(s->stream, s->P, s->links.as<int2>(), s->status.as<int2>(), pos, dxi, tan,
-                          nrm, s->n, s->n_active > s->n_targets, flag))
-    return false;
-  return check_flag(s, "update_tangents_normals");
+  return ov_launch_geometry(s->stream, s->P, s->links.as<int2>(), s->status.as<int2>(), pos, dxi, tan, nrm, s->n,
+                            s->n_active > s->n_targets, s->dflag.as<int>());
 }
 
 bool ov_epilogue(ov_state_impl* s, double t, const double* pos, const double* tan,
                  const double* nrm, const OvSums& sums, const OvStage& stage, double* vels,
                  double* vs, int k0, int k1) {
   if (k1 <= k0) return true;
-  int* flag = s->dflag.as<int>();
-  OV_TRY_CUDA(cudaMemsetAsync(flag, 0, sizeof(int), s->stream));
-  if (!ov_launch_epilogue(s->stream, s->P, s->links.as<int2>(), s->status.as<int2>(), nullptr, t, pos,
-                          tan, nrm, sums, s->n, stage, vels, vs, k0, k1, flag))
-    return false;
-  return check_flag(s, "update_velocities");
+  return ov_launch_epilogue(s->stream, s->P, s->links.as<int2>(), s->status.as<int2>(), nullptr, t, pos, tan, nrm,
+                            sums, s->n, stage, vels, vs, k0, k1, s->dflag.as<int>());
 }
 
 bool ov_euler(ov_state_impl* s, double dt) {
@@ -301,28 +291,32 @@ bool ov_rk4_stage_positions(ov_state_impl* s, int q, double dt, int classic) {
   return true;
 }
 
-// x0 += dt/6 k1 + dt/3 k2 + dt/3 k3 + dt/6 k4 (src/vortex_dynamics.c:95-112)
+// x0 += dt/6 k1 + dt/3 k2 + dt/3 k3 + dt/6 k4 (src/vortex_dynamics.c:95-112),
+// unless an evaluation of the step set the error flag
 bool ov_rk4_combine(ov_state_impl* s, double dt) {
   if (s->n == 0) return true;
-  k_rk4_combine<<<blocks_for(s->n), kThreads, 0, s->stream>>>(
-      s->status.as<int2>(), s->vels.as<double>(), s->k2.as<double>(), s->k3.as<double>(),
-      s->k4.as<double>(), dt, s->pos.as<double>(), s->n);
-  OV_LAUNCHED();
-  OV_TRY_CUDA(cudaGetLastError());
+  return ov_launch_rk4_combine(s->stream, s->status.as<int2>(), s->vels.as<double>(), s->k2.as<double>(),
+                               s->k3.as<double>(), s->k4.as<double>(), dt, s->pos.as<double>(), s->n,
+                               s->dflag.as<int>());
+}
+
+bool ov_rk4_first(ov_state_impl* s, double dt, OvStage* stage) {
+  if (!define_stages(s)) return false;
+  *stage = OvStage{s->pos.as<double>(), dt / 2, s->spos.as<double>()};
   return true;
 }
 
 // rk4_step2 (src/vortex_dynamics.c:58-117) on the device state.  Stage 4
 // advances dt/2 like the reference unless `classic`.  Each evaluation's
 // epilogue forms the next stage's positions.
-bool ov_rk4(ov_state_impl* s, double t, double dt, int classic) {
+bool ov_rk4(ov_state_impl* s, double t, double dt, int classic, bool have_stage1) {
   if (s->n == 0) return true;
   double* ks[3] = {s->k2.as<double>(), s->k3.as<double>(), s->k4.as<double>()};
   const double ts[3] = {t + dt / 2, t + dt / 2, t + dt};
   const double h[3] = {dt / 2, dt / 2, classic ? dt : dt / 2};
   const double* x0 = s->pos.as<double>();
   double* xs[3] = {s->spos.as<double>(), s->pos0.as<double>(), s->spos.as<double>()};
-  if (!ov_rk4_stage_positions(s, 1, dt, classic)) return false;
+  if (!have_stage1 && !ov_rk4_stage_positions(s, 1, dt, classic)) return false;
   for (int q = 0; q < 3; ++q) {
     if (!ov_geometry(s, xs[q], s->sdxi.as<double>(), s->stan.as<double>(), s->snrm.as<double>()))
       return false;

@@ -30,6 +30,7 @@ struct DevBuf {
 };
 
 // ---------------------------------------------------------------- BH tree
+constexpr int kTreeLevels = 32;   // octree levels a key holds
 // Octree cell kinds (what the walk does with a cell it reaches):
 //   CELL_LEAF1    : a single node (N == 1): its segment, inline in the record
 //   CELL_LEAFN    : several nodes in a box below BH_grain: direct sum over the
@@ -82,6 +83,7 @@ struct OvTree {
   int n_drop_root = 0;  // active nodes outside the root box (sorted last)
   int n_cells = 0;
   int built = 0;
+  int flag_seen = 0;    // the state's error flag when the build was read back
   double theta = 0;     // theta used for thr
   OvParams P;           // parameters at build time
   DevBuf keys, keys_alt, vals, vals_alt, stop, hist;   // sort
@@ -125,12 +127,27 @@ struct OvStage {
 constexpr OvStage kNoStage = {nullptr, 0, nullptr};
 
 // ---------------------------------------------------------------- state
+// Evaluations between two waits on the host, at most
+constexpr int kEvalSlots = 16;
+struct OvEvalSlot {
+  cudaEvent_t ev[3] = {nullptr, nullptr, nullptr};
+  double inter = 0;     // segment-point interactions (direct sums)
+  bool walk = false, lia = false;
+};
+
 struct ov_state_impl {
   int cap = 0;          // slot capacity of the device arrays
   int n = 0;            // slots in use
   OvParams P;           // captured at upload / call time
   cudaStream_t stream = nullptr;
+  // events of the evaluation under way (one of the slots'): around the tree
+  // build and around the Biot-Savart kernel
   cudaEvent_t ev0 = nullptr, ev1 = nullptr, ev2 = nullptr;
+  // evaluations launched since the last ov_eval_collect, which waits for them
+  // and takes their times, counters and error flags
+  OvEvalSlot slots[kEvalSlots];
+  int pending = 0;
+  DevBuf evctr;         // walk counters, 3 per slot
   // slot-indexed (AoS, 3 doubles per vector, as struct vec3d)
   DevBuf pos, links, status, dxi, tan, nrm, vels, vs;
   // RK4 scratch (two stage positions: an evaluation reads one while its
@@ -156,14 +173,12 @@ struct ov_state_impl {
   int walls[6] = {0, 0, 0, 0, 0, 0};   // box.wall of the uploaded tangle
   void* frames = nullptr;              // frame snapshot buffers (ov_frames.cu)
   // one tangle over several ranks (ov_state_shard): this rank's share of
-  // the targets, the exchange buffer, and the counters of the walk between
-  // ov_state_shard_begin and ov_state_shard_end
+  // the targets and the exchange buffer
   int n_active = 0;                    // non-EMPTY slots of the upload
   int shard_rank = 0, shard_world = 1;
   double* xbuf = nullptr;              // the caller's, or xown's when world is 1
   size_t xbytes = 0;
   DevBuf xown;
-  double shard_inter = 0, shard_cells = 0, shard_warp_iter = 0;
 };
 
 // the implementation behind a public ov_state handle
@@ -172,21 +187,38 @@ ov_state_impl* ov_state_impl_of(ov_state* s);
 void ov_frames_release(ov_state_impl* s);
 
 // ---------------------------------------------------------------- launchers
+// An entry point's evaluations: ov_eval_begin clears the error flag, the
+// evaluations below only launch (ov_geometry, ov_velocities, ov_rk4 and
+// ov_epilogue), and ov_eval_collect waits for them, adds their times and
+// counters to the state's and the thread's statistics and reports link and
+// finiteness errors.  ov_velocities collects by itself when its slots are
+// full, and before each evaluation large enough to hide the wait.
+bool ov_eval_begin(ov_state_impl* s);
+bool ov_eval_collect(ov_state_impl* s, const char* where);
+void ov_events_release(ov_state_impl* s);
+// pinned host memory of the calling thread for small read-backs (nullptr on
+// failure); every use waits for its copy before the next
+void* ov_pinned_scratch();
+constexpr size_t kPinnedScratch = 1024;
 // geometry: dxi, tangents, normals of all slots (pos/links/status -> dxi,tan,nrm)
 bool ov_geometry(ov_state_impl* s, const double* pos, double* dxi, double* tan, double* nrm);
 // velocities at positions pos with tangents/normals -> vels, vs
 bool ov_velocities(ov_state_impl* s, double t, const double* pos, const double* dxi,
                    const double* tan, const double* nrm, double* vels, double* vs,
                    OvTree* external_tree, const OvStage& stage = kNoStage);
-// one RK4 step on the state's pos using the state's vels as k1
-bool ov_rk4(ov_state_impl* s, double t, double dt, int classic);
+// one RK4 step on the state's pos using the state's vels as k1 (have_stage1:
+// the evaluation of vels has already formed the first stage's positions, as
+// ov_rk4_first's stage).  After an error (the flag set) the positions stay.
+bool ov_rk4(ov_state_impl* s, double t, double dt, int classic, bool have_stage1 = false);
+bool ov_rk4_first(ov_state_impl* s, double dt, OvStage* stage);
 // its pieces: stage q = 1..3 positions into spos, and the final combination
 bool ov_rk4_stage_positions(ov_state_impl* s, int q, double dt, int classic);
 bool ov_rk4_combine(ov_state_impl* s, double dt);
 bool ov_euler(ov_state_impl* s, double dt);
 
-// tree over the positions pos (slot-indexed); fills tree
-bool ov_tree_build(ov_state_impl* s, const double* pos, OvTree* tree);
+// tree over the positions pos (slot-indexed); fills tree.  order_only: just
+// the key order (perm), without waiting for anything
+bool ov_tree_build(ov_state_impl* s, const double* pos, OvTree* tree, bool order_only = false);
 void ov_tree_release(OvTree* tree);
 // Barnes-Hut nonlocal + image sums for every active node -> v_nl, v_img
 // own_tree: the tree was built from `pos` (targets in its key order); then
@@ -244,7 +276,8 @@ bool ov_state_reserve(ov_state_impl* s, int n);
 
 // Launches only, no host synchronisation (CUDA-graph capturable); link and
 // finiteness errors accumulate in *flag (bit 0 broken links, bit 1
-// non-finite velocity), read back later with ov_flag_status.  pinned: the
+// non-finite velocity; the tree's keys set bit 2 when the box needs more
+// levels than a key holds), read back later with ov_flag_status.  pinned: the
 // tangle may have PINNED nodes (their neighbours take a second launch).
 bool ov_launch_geometry(cudaStream_t st, const OvParams& P, const int2* links, const int2* status,
                         const double* pos, double* dxi, double* tan, double* nrm, int n, bool pinned, int* flag);
@@ -265,8 +298,10 @@ bool ov_launch_epilogue_list(cudaStream_t st, const OvParams& P, const int2* lin
                              const int* idx, int count, int* flag);
 bool ov_launch_euler(cudaStream_t st, const int2* status, const double* x0, const double* v,
                      double h, double* xs, int n);
+// flag given: nothing happens when it is set
 bool ov_launch_rk4_combine(cudaStream_t st, const int2* status, const double* k1, const double* k2,
-                           const double* k3, const double* k4, double dt, double* x, int n);
+                           const double* k3, const double* k4, double dt, double* x, int n,
+                           const int* flag = nullptr);
 // error for flag bits h (false and the error set when any bit is set)
 bool ov_flag_status(int h, const char* where);
 

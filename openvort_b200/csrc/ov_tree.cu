@@ -25,13 +25,14 @@
 #include <float.h>
 
 #include <algorithm>
+#include <cstring>
 #include <utility>
 
 #include "ov_internal.h"
 
 namespace {
 
-constexpr int kMaxLevels = 32;
+constexpr int kMaxLevels = kTreeLevels;
 constexpr int kDigitDropped = 8;
 enum { TERM_GRAIN = 0, TERM_BUILD = 1, TERM_DROP = 2 };
 
@@ -93,7 +94,7 @@ __device__ __forceinline__ void set_digit(uint64_t& hi, uint64_t& lo, int level,
 
 // ---------------------------------------------------------------- 1. keys
 __global__ void k_keys(OvParams P, const double* __restrict__ pos, const int2* __restrict__ status,
-                       int n, uint64_t* khi, uint64_t* klo, int* vals, int* term, int* counters) {
+                       int n, uint64_t* khi, uint64_t* klo, int* vals, int* term, int* counters, int* flag) {
   int k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= n) return;
   vals[k] = k;
@@ -114,7 +115,7 @@ __global__ void k_keys(OvParams P, const double* __restrict__ pos, const int2* _
     double Lmin = box_min(lo, hi);
     if (Lmin < P.grain) { tl = level; tk = TERM_GRAIN; break; }
     if (Lmin < build_min) { tl = level; tk = TERM_BUILD; break; }
-    if (level == kMaxLevels) { tl = level; tk = TERM_BUILD; atomicOr(&counters[1], 1); break; }
+    if (level == kMaxLevels) { tl = level; tk = TERM_BUILD; atomicOr(&counters[1], 1); atomicOr(flag, 4); break; }
     double c[3], Lh[3];
     split_params(lo, hi, c, Lh);
     int digit = kDigitDropped;
@@ -548,9 +549,13 @@ __global__ void k_write_cells(const BNode* __restrict__ nodes, const int* __rest
                               const uint64_t* __restrict__ khi, const uint64_t* __restrict__ klo,
                               const double* __restrict__ nodes64, const int2* __restrict__ nodeids,
                               OvParams P, int n, int big, Cell* cells, double* cell_lm, int2* cell_range,
-                              int* lists, int* list_counts) {
+                              int* lists, int* list_counts, const int* __restrict__ flag, int* tail) {
   int b = blockIdx.x * blockDim.x + threadIdx.x;
   if (b >= 2 * n - 1) return;
+  if (b == 0) {   // for the host's one read-back
+    tail[0] = (int)base[n];
+    tail[1] = *flag;
+  }
   CellInfo ci = info[b];
   if (!ci.is_cell) return;
   int first, last, dX, parent;
@@ -916,7 +921,21 @@ bool ov_radix_sort_u64(uint64_t* ka, int* va, uint64_t* kb, int* vb, int n, int 
                                                : rs_passes<kRsLarge>(ka, va, kb, vb, n, passes, hist, scan_part, st);
 }
 
-bool ov_tree_build(ov_state_impl* s, const double* pos, OvTree* T) {
+// the build's counters on the host (the build's one wait)
+static bool read_build(ov_state_impl* s, OvTree* T, const int* ctr, int (&hc)[16]) {
+  void* host = ov_pinned_scratch();
+  if (!host) return false;
+  OV_TRY_CUDA(cudaMemcpyAsync(host, ctr, sizeof(hc), cudaMemcpyDeviceToHost, s->stream));
+  OV_TRY_CUDA(cudaStreamSynchronize(s->stream));
+  memcpy(hc, host, sizeof(hc));
+  if (hc[1]) return ov_flag_status(4, "octree");
+  // a node outside the root box takes digit 8 at level 1, so these nodes
+  // sort after every node inside it: the last n_drop_root of the order
+  T->n_drop_root = hc[3];
+  return true;
+}
+
+bool ov_tree_build(ov_state_impl* s, const double* pos, OvTree* T, bool order_only) {
   const int n = s->n;
   cudaStream_t st = s->stream;
   T->P = s->P;
@@ -938,26 +957,18 @@ bool ov_tree_build(ov_state_impl* s, const double* pos, OvTree* T) {
   int* vals_alt = T->vals_alt.as<int>();
   int* term = vals_alt + n;
   int* ctr = T->counters.as<int>();
+  int hc[16];   // the device counters: active nodes, depth error, deepest level, nodes outside the
+                // box, cells per moment class (3), cells, the state's error flag
   OV_TRY_CUDA(cudaMemsetAsync(ctr, 0, sizeof(int) * 16, st));
   if (n > 0) {
     k_keys<<<(n + 255) / 256, 256, 0, st>>>(s->P, pos, s->status.as<int2>(), n, khi, klo_slot, vals,
-                                             term_slot, ctr);
+                                             term_slot, ctr, s->dflag.as<int>());
     OV_LAUNCHED();
     OV_TRY_CUDA(cudaGetLastError());
   }
-  int hc[4] = {0, 0, 0, 0};
-  OV_TRY_CUDA(cudaMemcpyAsync(hc, ctr, sizeof(hc), cudaMemcpyDeviceToHost, st));
-  OV_TRY_CUDA(cudaStreamSynchronize(st));
-  if (hc[1]) {
-    ov_set_error(OV_ERR_TREE_DEPTH,
-                 "octree: the box / BH_grain ratio needs more than %d levels", kMaxLevels);
-    return false;
-  }
-  const int na = hc[0];
+  const int na = s->n_active;   // as counted by the upload
   T->n_nodes = na;
-  // a node outside the root box takes digit 8 at level 1, so these nodes
-  // sort after every node inside it: the last n_drop_root of the order
-  T->n_drop_root = hc[3];
+  T->n_drop_root = T->flag_seen = 0;
   // radix sort over the high word (8 passes of 8 bits), stable; vals_alt's
   // second half holds the sorted term codes, so the values alternate with a
   // separate scratch.  The sorted data ends back in khi / vals.
@@ -976,6 +987,10 @@ bool ov_tree_build(ov_state_impl* s, const double* pos, OvTree* T) {
       OV_LAUNCHED();
     }
     OV_TRY_CUDA(cudaGetLastError());
+  }
+  if (order_only) {
+    T->n_cells = 0;
+    return true;
   }
   const uint64_t* hi_sorted = ka;
   // sorted node table for the walk
@@ -1019,6 +1034,7 @@ bool ov_tree_build(ov_state_impl* s, const double* pos, OvTree* T) {
                                    T->nodeids.as<int2>());
     OV_LAUNCHED();
     OV_TRY_CUDA(cudaGetLastError());
+    if (!read_build(s, T, ctr, hc)) return false;
     T->n_cells = 1;
   } else {
     k_karras<<<(na - 1 + 255) / 256, 256, 0, st>>>(hi_sorted, klo, na, bn, leaf_parent);
@@ -1030,15 +1046,13 @@ bool ov_tree_build(ov_state_impl* s, const double* pos, OvTree* T) {
     k_write_cells<<<(nbin + 255) / 256, 256, 0, st>>>(bn, leaf_parent, info, base, hi_sorted, klo,
                                                       T->nodes64.as<double>(), T->nodeids.as<int2>(),
                                                       s->P, na, mom_big(na), cells, cell_lm, cell_range, lists,
-                                                      list_counts);
+                                                      list_counts, s->dflag.as<int>(), ctr + 7);
     OV_LAUNCHED();
     OV_TRY_CUDA(cudaGetLastError());
-    unsigned nc = 0;
-    int lc[3] = {0, 0, 0};
-    OV_TRY_CUDA(cudaMemcpyAsync(&nc, base + na, sizeof(unsigned), cudaMemcpyDeviceToHost, st));
-    OV_TRY_CUDA(cudaMemcpyAsync(lc, list_counts, sizeof(lc), cudaMemcpyDeviceToHost, st));
-    OV_TRY_CUDA(cudaStreamSynchronize(st));
-    T->n_cells = (int)nc;
+    if (!read_build(s, T, ctr, hc)) return false;
+    T->n_cells = hc[7];
+    T->flag_seen = hc[8];
+    const int* lc = hc + 4;
     const double f4 = s->P.f4pi;
     if (lc[0] > 0) {
       k_moments_thread<<<(lc[0] + 127) / 128, 128, 0, st>>>(lists, list_counts, cells, cell_range,

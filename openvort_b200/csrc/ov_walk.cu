@@ -1247,8 +1247,7 @@ static int walk_wave(K kernel) {
 // one GPU would).  v_img null: no image sums wanted.
 static bool launch_multi(ov_state_impl* s, OvTree* t, const OvParams& P, const int* order, const int2* status,
                          const int* skip, const double* pos, int n_t, int n_rule, unsigned combos, double* v_nl,
-                         double* v_img, bool timed) {
-  unsigned long long* ctr = reinterpret_cast<unsigned long long*>(t->counters.as<char>() + 64);
+                         double* v_img, unsigned long long* ctr, bool timed) {
   const bool mixed = P.precision == OV_PREC_MIXED;
   const ImageShortcut sc = image_shortcut(P, combos);
   const TreeView tv = view_of(t);
@@ -1334,12 +1333,14 @@ static bool launch_multi(ov_state_impl* s, OvTree* t, const OvParams& P, const i
 
 bool ov_tree_walk_nodes(ov_state_impl* s, OvTree* t, const double* pos, bool own_tree,
                         double* v_nl, double* v_img, int k0, int k_count) {
-  unsigned long long* ctr = reinterpret_cast<unsigned long long*>(t->counters.as<char>() + 64);
+  unsigned long long* ctr = s->evctr.as<unsigned long long>() + 3 * s->pending;
   OV_TRY_CUDA(cudaMemsetAsync(ctr, 0, 24, s->stream));
   // a tree built from these positions: its key order; otherwise slot order
   const int* order = own_tree ? t->perm.as<int>() : nullptr;
   int n_t = own_tree ? t->n_nodes : s->n;
   if (n_t == 0 || t->n_cells == 0) {
+    cudaEventRecord(s->ev1, s->stream);
+    cudaEventRecord(s->ev2, s->stream);
     OV_TRY_CUDA(cudaMemsetAsync(v_nl, 0, sizeof(double) * 3 * s->n, s->stream));
     OV_TRY_CUDA(cudaMemsetAsync(v_img, 0, sizeof(double) * 3 * s->n, s->stream));
     return true;
@@ -1355,7 +1356,7 @@ bool ov_tree_walk_nodes(ov_state_impl* s, OvTree* t, const double* pos, bool own
     if (n_t <= 0) {
       cudaEventRecord(s->ev1, s->stream);
       cudaEventRecord(s->ev2, s->stream);
-      return read_counters(s, t);
+      return true;
     }
   }
   // Nodes outside the root box take key digit 8 at level 1 and sort after
@@ -1389,9 +1390,9 @@ bool ov_tree_walk_nodes(ov_state_impl* s, OvTree* t, const double* pos, bool own
     cudaEventRecord(s->ev1, s->stream);
     P.near2 = s->P.near2;
     if (!launch_multi(s, t, P, order, s->status.as<int2>(), nullptr, pos, n_t, own_tree ? t->n_nodes : n_t, combos,
-                      v_nl, v_img, own_tree))
+                      v_nl, v_img, ctr, own_tree))
       return false;
-    return read_counters(s, t);
+    return true;
   }
   const TreeView tv = view_of(t);
   cudaEventRecord(s->ev1, s->stream);
@@ -1408,7 +1409,7 @@ bool ov_tree_walk_nodes(ov_state_impl* s, OvTree* t, const double* pos, bool own
   }
   OV_TRY_CUDA(cudaGetLastError());
   cudaEventRecord(s->ev2, s->stream);
-  return read_counters(s, t);
+  return true;
 }
 
 bool ov_tree_walk_points(ov_state_impl* s, OvTree* t, int npts, const double* pts, const int* skip,
@@ -1447,7 +1448,8 @@ bool ov_tree_walk_points(ov_state_impl* s, OvTree* t, int npts, const double* pt
       order = vals;
     }
     P.precision = OV_PREC_FP64;
-    if (!launch_multi(s, t, P, order, nullptr, skip, pts, npts, npts, combos, out_nl, out_img, false)) return false;
+    if (!launch_multi(s, t, P, order, nullptr, skip, pts, npts, npts, combos, out_nl, out_img, ctr, false))
+      return false;
     return read_counters(s, t);
   }
   const int warps = (npts + 31) / 32;

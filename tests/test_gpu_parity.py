@@ -352,6 +352,33 @@ def test_broken_links_fail_loudly(ov, monkeypatch):
     assert e.value.code == 3
 
 
+@pytest.mark.parametrize("use_bh,precision", [(0, 0), (0, 1), (1, 0), (1, 1)])
+def test_nonfinite_run_stops_and_keeps_positions(ov, monkeypatch, use_bh, precision):
+    """Two neighbours at one place give a non-finite local term: a run of
+    several steps, whose evaluations are not waited for one by one, reports
+    it and leaves the positions it started from; the state then works again
+    with a sound tangle."""
+    monkeypatch.setenv("OV_QUIET", "1")
+    t = G.single_ring(64, 1e-2)
+    good = t.pos.copy()
+    ov.configure(Params(use_mf=0, hyperfriction=0, use_bh=use_bh, bh_theta=0.5), precision)
+    st = ov.DeviceState(t)
+    t.pos[7] = t.pos[6]
+    bad = t.pos.copy()
+    st.upload()
+    with pytest.raises(ov.OVError) as e:
+        st.run(0.0, 1e-6, 12)
+    assert e.value.code == 4
+    st.download(ov.OV_FIELD_POS)
+    assert np.array_equal(t.pos, bad)
+    t.pos[:] = good
+    st.upload()
+    st.run(0.0, 1e-6, 12)
+    st.download(ov.OV_FIELD_POS)
+    assert np.all(np.isfinite(t.pos)) and not np.array_equal(t.pos, good)
+    st.close()
+
+
 def test_unknown_flow_fails_loudly(ov, monkeypatch):
     monkeypatch.setenv("OV_QUIET", "1")
     t = G.single_ring(32, 1e-2)
