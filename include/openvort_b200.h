@@ -317,7 +317,8 @@ int ov_state_eval_points(ov_state *s, int npts, const double *pts, const int *sk
  * evaluations, segment-point interactions (direct and Barnes-Hut leaves),
  * multipole evaluations, device time of the Biot-Savart kernels and of the
  * tree builds, kernel launches by this library, and the device time of the
- * last ov_state_run (CUDA events on the state's stream). */
+ * last ov_state_run (CUDA events on the state's stream).  Of direct sums of
+ * up to 2e7 interactions one evaluation in 16 is timed for all of them. */
 typedef struct {
   double evals;
   double interactions;

@@ -396,9 +396,13 @@ bool ov_capture_params(const tangle_state* t, OvParams& P) { return capture_para
 // ======================================================================
 // state management
 
-// the events of slot i, created on its first use, as the evaluation's
-static bool use_slot(ov_state_impl* s, int i) {
+// the events of slot i, created on its first use, as the evaluation's; none
+// for an evaluation that is not timed
+static bool use_slot(ov_state_impl* s, int i, bool timed) {
   OvEvalSlot& e = s->slots[i];
+  e.timed = timed;
+  s->ev0 = s->ev1 = s->ev2 = nullptr;
+  if (!timed) return true;
   for (cudaEvent_t& ev : e.ev)
     if (!ev) OV_TRY_CUDA(cudaEventCreate(&ev));
   s->ev0 = e.ev[0];
@@ -432,7 +436,7 @@ void* ov_pinned_scratch() {
 bool ov_state_reserve(ov_state_impl* s, int n) {
   if (!s->stream) {
     OV_TRY_CUDA(cudaStreamCreateWithFlags(&s->stream, cudaStreamNonBlocking));
-    if (!s->dflag.reserve(64) || !s->evctr.reserve(sizeof(unsigned long long) * 3 * kEvalSlots) || !use_slot(s, 0))
+    if (!s->dflag.reserve(64) || !s->evctr.reserve(sizeof(unsigned long long) * 3 * kEvalSlots) || !use_slot(s, 0, true))
       return false;
     OV_TRY_CUDA(cudaMemsetAsync(s->dflag.p, 0, 64, s->stream));
   }
@@ -588,11 +592,12 @@ bool ov_eval_collect(ov_state_impl* s, const char* where) {
   const int pending = s->pending;
   s->pending = 0;
   // device times from the events around the tree build and the Biot-Savart
-  // kernel
+  // kernel; an evaluation that was not timed takes those of the one before
+  float build_ms = 0, bs_ms = 0;
   for (int i = 0; i < pending; ++i) {
     const OvEvalSlot& e = s->slots[i];
-    float build_ms = 0, bs_ms = 0;
-    if (!e.lia && (cudaEventElapsedTime(&build_ms, e.ev[0], e.ev[1]) != cudaSuccess ||
+    if (e.lia) build_ms = bs_ms = 0;
+    if (!e.lia && e.timed && (cudaEventElapsedTime(&build_ms, e.ev[0], e.ev[1]) != cudaSuccess ||
                    cudaEventElapsedTime(&bs_ms, e.ev[1], e.ev[2]) != cudaSuccess))
       (void)cudaGetLastError();
     tl_stats.interactions = e.walk ? (double)ctr[3 * i] : e.inter;
@@ -609,18 +614,23 @@ bool ov_eval_collect(ov_state_impl* s, const char* where) {
     s->acc_cells += tl_stats.cell_interactions;
     s->acc_warp_iter += tl_stats.warp_iterations;
   }
+  if (pending > 0 && !use_slot(s, 0, true)) return false;   // the timed one's, for ov_get_last_stats
   return ov_flag_status(*flag, where);
 }
 
-// Evaluations a state launches between two waits.  A wait costs some 15 us,
-// so small evaluations go on for 16 (a 256-node ring's RK4 step 330 us with a
-// wait for each error flag, RING_NOW without); a direct sum of more than 2e7
-// interactions, over 50 us, is waited for each time, so positions that
-// have become NaN are not carried far.  The tree build reads the error flag
-// back with its cell count.
+// Small direct sums (up to 2e7 interactions, some 50 us): a wait costs 15 us
+// and the three timing events of an evaluation 13 us, against 24 us for the
+// rest of a 256-node ring's (its RK4 step took 330 us with a wait for each
+// error flag, 150 us without, 95 us with one evaluation in 16 timed for all).
+static bool small_sum(const ov_state_impl* s) {
+  return !s->P.use_bh && (double)s->n_targets * (double)s->n_segments * (1 + s->P.n_img) <= 2e7;
+}
+
+// Evaluations a state launches between two waits: a larger direct sum is
+// waited for each time, so positions that have become NaN are not carried
+// far.  The tree build reads the error flag back with its cell count.
 static int max_pending(const ov_state_impl* s) {
-  if (s->P.lia_only || s->P.use_bh) return kEvalSlots;
-  return (double)s->n_targets * (double)s->n_segments * (1 + s->P.n_img) <= 2e7 ? kEvalSlots : 1;
+  return s->P.lia_only || s->P.use_bh || small_sum(s) ? kEvalSlots : 1;
 }
 
 // The Biot-Savart sums of an evaluation into s->sums: the tree build and
@@ -630,7 +640,7 @@ static bool bs_sums(ov_state_impl* s, const double* pos, OvTree* external_tree, 
   tl_last_state = s;
   if (s->pending >= max_pending(s) && !ov_eval_collect(s, "update_velocities")) return false;
   tl_stats = OvStatsAcc{0, 0, 0, 0, 0, 0, 0};
-  if (!use_slot(s, s->pending)) return false;
+  if (!use_slot(s, s->pending, s->pending == 0 || !small_sum(s))) return false;
   OvEvalSlot& slot = s->slots[s->pending];
   slot.inter = 0;
   slot.walk = false;
@@ -639,7 +649,7 @@ static bool bs_sums(ov_state_impl* s, const double* pos, OvTree* external_tree, 
   double* v_img = s->v_img.as<double>();
   s->sums = OvSums{v_nl, v_img, nullptr, 0};
   if (s->P.lia_only) return true;
-  cudaEventRecord(s->ev0, s->stream);
+  ov_mark(s, s->ev0);
   if (s->P.use_bh) {
     OvTree* tree = external_tree;
     if (!tree) {

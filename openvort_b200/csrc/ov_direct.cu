@@ -707,8 +707,8 @@ static int source_chunk(int n_src, long long blocks, int tile, int* splits, int 
 bool ov_direct_partials(ov_state_impl* s, const double* pos, double* v_nl, double* v_img, OvSums* out) {
   *out = OvSums{v_nl, v_img, nullptr, 0};
   if (s->n == 0) {
-    cudaEventRecord(s->ev1, s->stream);
-    cudaEventRecord(s->ev2, s->stream);
+    ov_mark(s, s->ev1);
+    ov_mark(s, s->ev2);
     return true;
   }
   int nimg = s->P.n_img;
@@ -727,8 +727,8 @@ bool ov_direct_partials(ov_state_impl* s, const double* pos, double* v_nl, doubl
     }
     if ((slot_order ? s->n_active : s->tree.n_nodes) == 0) {
       // every slot EMPTY: no targets and no segments
-      cudaEventRecord(s->ev1, s->stream);
-      cudaEventRecord(s->ev2, s->stream);
+      ov_mark(s, s->ev1);
+      ov_mark(s, s->ev2);
       OV_TRY_CUDA(cudaMemsetAsync(v_nl, 0, sizeof(double) * 3 * s->n, s->stream));
       OV_TRY_CUDA(cudaMemsetAsync(v_img, 0, sizeof(double) * 3 * s->n, s->stream));
       return true;
@@ -741,7 +741,7 @@ bool ov_direct_partials(ov_state_impl* s, const double* pos, double* v_nl, doubl
     const int chunk = source_chunk(n_src, (long long)bx * (nimg + 1), kPSrc, &splits, 4, 16,
                                    slot_order ? res_chain : res_pairs);
     if (!s->img_part.reserve(sizeof(double) * 3 * (size_t)s->n * (nimg + 1) * splits)) return false;
-    cudaEventRecord(s->ev1, s->stream);
+    ov_mark(s, s->ev1);
     if (slot_order) {
       k_direct_mixed_chain<<<dim3(bx, nimg + 1, splits), kPB, 0, s->stream>>>(
           s->P, S, n_src, pos, s->status.as<int2>(), n_t, s->img_part.as<double>(), chunk);
@@ -761,14 +761,14 @@ bool ov_direct_partials(ov_state_impl* s, const double* pos, double* v_nl, doubl
     // target blocks: 16 blocks instead of 4)
     const int chunk = source_chunk(s->n, (long long)bx * (nimg + 1), 32, &splits, 4, 64, res64);
     if (!s->img_part.reserve(sizeof(double) * 3 * (size_t)s->n * (nimg + 1) * splits)) return false;
-    cudaEventRecord(s->ev1, s->stream);
+    ov_mark(s, s->ev1);
     k_direct64_chain<false><<<dim3(bx, nimg + 1, splits), kTB, 0, s->stream>>>(
         s->P, s->n, pos, s->links.as<int2>(), s->status.as<int2>(), nullptr, nullptr, s->n, s->img_part.as<double>(),
         chunk);
     OV_LAUNCHED();
     OV_TRY_CUDA(cudaGetLastError());
   }
-  cudaEventRecord(s->ev2, s->stream);
+  ov_mark(s, s->ev2);
   out->part = s->img_part.as<double>();
   out->splits = splits;
   return true;

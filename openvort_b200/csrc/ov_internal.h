@@ -132,7 +132,7 @@ constexpr int kEvalSlots = 16;
 struct OvEvalSlot {
   cudaEvent_t ev[3] = {nullptr, nullptr, nullptr};
   double inter = 0;     // segment-point interactions (direct sums)
-  bool walk = false, lia = false;
+  bool walk = false, lia = false, timed = false;
 };
 
 struct ov_state_impl {
@@ -140,8 +140,8 @@ struct ov_state_impl {
   int n = 0;            // slots in use
   OvParams P;           // captured at upload / call time
   cudaStream_t stream = nullptr;
-  // events of the evaluation under way (one of the slots'): around the tree
-  // build and around the Biot-Savart kernel
+  // events of the evaluation under way (one of the slots', null when it is
+  // not timed): around the tree build and around the Biot-Savart kernel
   cudaEvent_t ev0 = nullptr, ev1 = nullptr, ev2 = nullptr;
   // evaluations launched since the last ov_eval_collect, which waits for them
   // and takes their times, counters and error flags
@@ -196,6 +196,10 @@ void ov_frames_release(ov_state_impl* s);
 bool ov_eval_begin(ov_state_impl* s);
 bool ov_eval_collect(ov_state_impl* s, const char* where);
 void ov_events_release(ov_state_impl* s);
+// records an event of the evaluation under way, if it is timed
+inline void ov_mark(ov_state_impl* s, cudaEvent_t ev) {
+  if (ev) cudaEventRecord(ev, s->stream);
+}
 // pinned host memory of the calling thread for small read-backs (nullptr on
 // failure); every use waits for its copy before the next
 void* ov_pinned_scratch();

@@ -1313,7 +1313,7 @@ static bool launch_multi(ov_state_impl* s, OvTree* t, const OvParams& P, const i
     OV_LAUNCHED();
     OV_TRY_CUDA(cudaGetLastError());
   }
-  cudaEventRecord(s->ev2, s->stream);
+  ov_mark(s, s->ev2);
   if (timed) {
     // the order for the next walk (after the timed kernel)
     const size_t nw = (size_t)warps;
@@ -1339,8 +1339,8 @@ bool ov_tree_walk_nodes(ov_state_impl* s, OvTree* t, const double* pos, bool own
   const int* order = own_tree ? t->perm.as<int>() : nullptr;
   int n_t = own_tree ? t->n_nodes : s->n;
   if (n_t == 0 || t->n_cells == 0) {
-    cudaEventRecord(s->ev1, s->stream);
-    cudaEventRecord(s->ev2, s->stream);
+    ov_mark(s, s->ev1);
+    ov_mark(s, s->ev2);
     OV_TRY_CUDA(cudaMemsetAsync(v_nl, 0, sizeof(double) * 3 * s->n, s->stream));
     OV_TRY_CUDA(cudaMemsetAsync(v_img, 0, sizeof(double) * 3 * s->n, s->stream));
     return true;
@@ -1354,8 +1354,8 @@ bool ov_tree_walk_nodes(ov_state_impl* s, OvTree* t, const double* pos, bool own
     n_t = std::min(k_count, n_t - lo);
     order += lo;
     if (n_t <= 0) {
-      cudaEventRecord(s->ev1, s->stream);
-      cudaEventRecord(s->ev2, s->stream);
+      ov_mark(s, s->ev1);
+      ov_mark(s, s->ev2);
       return true;
     }
   }
@@ -1387,7 +1387,7 @@ bool ov_tree_walk_nodes(ov_state_impl* s, OvTree* t, const double* pos, bool own
   const bool mixed = s->P.precision == OV_PREC_MIXED;
   unsigned combos = 0;
   if (image_combos(P, P.n_img, combos)) {
-    cudaEventRecord(s->ev1, s->stream);
+    ov_mark(s, s->ev1);
     P.near2 = s->P.near2;
     if (!launch_multi(s, t, P, order, s->status.as<int2>(), nullptr, pos, n_t, own_tree ? t->n_nodes : n_t, combos,
                       v_nl, v_img, ctr, own_tree))
@@ -1395,7 +1395,7 @@ bool ov_tree_walk_nodes(ov_state_impl* s, OvTree* t, const double* pos, bool own
     return true;
   }
   const TreeView tv = view_of(t);
-  cudaEventRecord(s->ev1, s->stream);
+  ov_mark(s, s->ev1);
   const int warps = (n_t + 31) / 32;
   const int blocks = (warps * 32 + 127) / 128;
   if (mixed) {
@@ -1408,7 +1408,7 @@ bool ov_tree_walk_nodes(ov_state_impl* s, OvTree* t, const double* pos, bool own
     OV_LAUNCHED();
   }
   OV_TRY_CUDA(cudaGetLastError());
-  cudaEventRecord(s->ev2, s->stream);
+  ov_mark(s, s->ev2);
   return true;
 }
 
