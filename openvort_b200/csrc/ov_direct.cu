@@ -211,8 +211,11 @@ static_assert(kCS == kTB, "every thread stages one segment (the ballot needs who
 // where that rule is applied.
 //
 // Shape measured on the 22.4k-point periodic tangle: 128 threads of 2
-// targets, at most 96 registers (5 resident blocks per SM), two records per
-// unrolled step.
+// targets, at most 96 registers (5 resident blocks per SM), a stretch of 16
+// records unrolled: 16.7 ms, against 17.7 with two records per step (the mask
+// positions of the pairs left to FP64 are constants only when unrolled) and
+// 17.2 with the FP64 formula inside the loop.  Bound by the FP32 pipe (two
+// thirds busy) and the latency of its chains at 20 warps per SM.
 constexpr int kPB = 128;            // threads per block
 constexpr int kPTgt = kPB * kTT;    // targets per block
 constexpr int kPSrc = 128;          // sources per shared-memory tile (kPSrc / 2 records)
@@ -254,26 +257,17 @@ __global__ void __launch_bounds__(kPB, OV_DIRECT_PAIRS_MIN_BLOCKS) k_direct_mixe
   for (int u = 0; u < kTT; ++u) acc[u][0] = acc[u][1] = acc[u][2] = 0;
   const double f4pi = P.f4pi;
   // FP64 evaluation of segment id at target u (skip rule of
-  // calculate_vs_shift, src/tangle.c:567-569, for the tangle itself), out of
-  // the way in IEEE operations: seg_vel64_nr inlined here costs the main loop
-  // registers (18.0 against 17.2 ms at 22.4k nodes)
+  // calculate_vs_shift, src/tangle.c:567-569, for the tangle itself)
   auto special = [&](int u, int id) {
-#pragma unroll
-    for (int v = 0; v < kTT; ++v) {
-      if (v != u) continue;
-      const int k = kk[v];
-      if (k < 0 || id < 0) return;
-      const int fw = S.fwd[id];
-      if (j == 0 && (id == k || fw == k)) return;
-      d3 r = ld3(pos, k);
-      if (j > 0) r = image_point(P, j - 1, r);
-      const double* sg = S.r1r2 + 6 * (size_t)id;
-      const d3 r1 = mk3(sg[0], sg[1], sg[2]), r2 = mk3(sg[3], sg[4], sg[5]);
-      const d3 vv = seg_vel64(f4pi, r1, r2, r);
-      acc[v][0] += vv.x;
-      acc[v][1] += vv.y;
-      acc[v][2] += vv.z;
-    }
+    const int k = u ? kk[1] : kk[0];
+    if (k < 0 || id < 0) return;
+    const int fw = S.fwd[id];
+    if (j == 0 && (id == k || fw == k)) return;
+    d3 r = ld3(pos, k);
+    if (j > 0) r = image_point(P, j - 1, r);
+    const double* sg = S.r1r2 + 6 * (size_t)id;
+    const d3 r1 = mk3(sg[0], sg[1], sg[2]), r2 = mk3(sg[3], sg[4], sg[5]);
+    add_target(acc, u, seg_vel64_nr(f4pi, r1, r2, r2 - r1, r));
   };
   const int s_lo = blockIdx.z * chunk, s_hi = min(n_src, s_lo + chunk);
   auto stage_one = [&](int m) -> SrcVals {
@@ -296,11 +290,8 @@ __global__ void __launch_bounds__(kPB, OV_DIRECT_PAIRS_MIN_BLOCKS) k_direct_mixe
     __syncthreads();
     // FP32 partial sums over 32 sources, each added into the FP64 sums
     for (int q0 = 0; q0 < kPSrc / 2; q0 += 16) {
-      f2 b[kTT][3];
-#pragma unroll
-      for (int k = 0; k < kTT; ++k) b[k][0] = b[k][1] = b[k][2] = f2_splat(0.f);
-#pragma unroll 2
-      for (int q = q0; q < q0 + 16; ++q) pair_interact<false>(sh[q], T, b, special);
+      f2 b[kTT][3], unused[kTT];
+      pair_stretch<false, false, 16>(sh + q0, T, b, unused, special);
 #pragma unroll
       for (int k = 0; k < kTT; ++k) {
 #pragma unroll
@@ -331,7 +322,9 @@ __global__ void __launch_bounds__(kPB, OV_DIRECT_PAIRS_MIN_BLOCKS) k_direct_mixe
 // whatever a block's extent and no key sort is needed.  Measured: on a
 // 4096-point ring an RK4 step takes less than the FP64 form's (the key sort
 // of k_direct_mixed_pairs costs more than its sum there); on the 22.4k-point
-// periodic tangle k_direct_mixed_pairs is faster (18.6 against 24.4 ms).
+// periodic tangle k_direct_mixed_pairs is faster (16.7 against 21.4 ms).
+// 12000 points, open: 0.34 ms, against 0.47 with the FP64 formula of the near
+// pairs inside the loop.
 static_assert(2 * kCH == kPSrc, "a chain tile is the two-source form's tile");
 
 #ifndef OV_DIRECT_CHAIN_MIN_BLOCKS
@@ -372,22 +365,15 @@ __global__ void __launch_bounds__(kPB, OV_DIRECT_CHAIN_MIN_BLOCKS) k_direct_mixe
   // near pairs in FP64, a large share of a small sum: refined reciprocals
   // (2000 open nodes 0.074 ms, against 0.100 with IEEE operations)
   auto special = [&](int u, int id) {
-#pragma unroll
-    for (int v = 0; v < kTT; ++v) {
-      if (v != u) continue;
-      const int k = kk[v];
-      if (k < 0 || id < 0) return;
-      const int fw = S.fwd[id];
-      if (j == 0 && (id == k || fw == k)) return;
-      d3 r = ld3(pos, k);
-      if (j > 0) r = image_point(P, j - 1, r);
-      const double* sg = S.r1r2 + 6 * (size_t)id;
-      const d3 r1 = mk3(sg[0], sg[1], sg[2]), r2 = mk3(sg[3], sg[4], sg[5]);
-      const d3 vv = seg_vel64_nr(f4pi, r1, r2, r2 - r1, r);
-      acc[v][0] += vv.x;
-      acc[v][1] += vv.y;
-      acc[v][2] += vv.z;
-    }
+    const int k = u ? kk[1] : kk[0];
+    if (k < 0 || id < 0) return;
+    const int fw = S.fwd[id];
+    if (j == 0 && (id == k || fw == k)) return;
+    d3 r = ld3(pos, k);
+    if (j > 0) r = image_point(P, j - 1, r);
+    const double* sg = S.r1r2 + 6 * (size_t)id;
+    const d3 r1 = mk3(sg[0], sg[1], sg[2]), r2 = mk3(sg[3], sg[4], sg[5]);
+    add_target(acc, u, seg_vel64_nr(f4pi, r1, r2, r2 - r1, r));
   };
   const int s_lo = blockIdx.z * chunk, s_hi = min(n_src, s_lo + chunk);
   // a source by slot for the two-source form (the tangle's own wrapped
@@ -467,7 +453,11 @@ __global__ void __launch_bounds__(kPB, OV_DIRECT_CHAIN_MIN_BLOCKS) k_direct_mixe
       f2 b[kTT][3];
 #pragma unroll
       for (int u = 0; u < kTT; ++u) b[u][0] = b[u][1] = b[u][2] = f2_splat(0.f);
-      for (int q = 0; 2 * q < n_irr; ++q) pair_interact<true>(sh_irr[q], T, b, special);
+      for (int q0 = 0; 2 * q0 < n_irr; q0 += 16) {
+        PairSpecials sp;
+        for (int q = 0; q < 16 && 2 * (q0 + q) < n_irr; ++q) sp.add(q, pair_interact<true>(sh_irr[q0 + q], T, b));
+        sp.run([&](int u, int h, int i) { special(u, pair_id(sh_irr[q0 + i], h)); });
+      }
 #pragma unroll
       for (int u = 0; u < kTT; ++u) {
 #pragma unroll
@@ -523,7 +513,6 @@ __global__ void __launch_bounds__(kPB) k_direct_mixed_points(OvParams P, SegTab 
   const int base = blockIdx.x * kPTgt;
   bool act[kTT];
   int kk[kTT];
-  d3 rr[kTT];
   PairTargets T;
 #pragma unroll
   for (int u = 0; u < kTT; ++u) {
@@ -531,7 +520,6 @@ __global__ void __launch_bounds__(kPB) k_direct_mixed_points(OvParams P, SegTab 
     act[u] = i < n_t;
     d3 r = act[u] ? ld3(tpos, i) : mk3(0, 0, 0);
     if (act[u] && j > 0) r = image_point(P, j - 1, r);
-    rr[u] = r;
     kk[u] = act[u] && j == 0 && tskip ? tskip[i] : -1;
     set_target(T, u, r.x, r.y, r.z);
   }
@@ -542,19 +530,15 @@ __global__ void __launch_bounds__(kPB) k_direct_mixed_points(OvParams P, SegTab 
   // FP64 evaluation of segment id at target u, with the skip rule of
   // calculate_vs_shift (src/tangle.c:567-569) for the tangle itself
   auto special = [&](int u, int id) {
-#pragma unroll
-    for (int v = 0; v < kTT; ++v) {
-      if (v != u) continue;
-      if (!act[v] || id < 0) return;
-      const int fw = S.fwd[id];
-      if (j == 0 && (id == kk[v] || fw == kk[v])) return;
-      const double* sg = S.r1r2 + 6 * (size_t)id;
-      const d3 r1 = mk3(sg[0], sg[1], sg[2]), r2 = mk3(sg[3], sg[4], sg[5]);
-      const d3 vv = seg_vel64(f4pi, r1, r2, rr[v]);
-      acc[v][0] += vv.x;
-      acc[v][1] += vv.y;
-      acc[v][2] += vv.z;
-    }
+    if (!(u ? act[1] : act[0]) || id < 0) return;
+    const int k = u ? kk[1] : kk[0];
+    const int fw = S.fwd[id];
+    if (j == 0 && (id == k || fw == k)) return;
+    const double* sg = S.r1r2 + 6 * (size_t)id;
+    const d3 r1 = mk3(sg[0], sg[1], sg[2]), r2 = mk3(sg[3], sg[4], sg[5]);
+    d3 r = ld3(tpos, base + threadIdx.x + kPB * u);
+    if (j > 0) r = image_point(P, j - 1, r);
+    add_target(acc, u, seg_vel64_nr(f4pi, r1, r2, r2 - r1, r));
   };
   const int s_lo = blockIdx.z * chunk, s_hi = min(n_src, s_lo + chunk);
   // sources in slot order; the tangle's own segments wrapped across a
@@ -578,10 +562,7 @@ __global__ void __launch_bounds__(kPB) k_direct_mixed_points(OvParams P, SegTab 
     __syncthreads();
     for (int q0 = 0; q0 < kPSrc / 2; q0 += 16) {
       f2 b[kTT][3], eb[kTT];
-#pragma unroll
-      for (int k = 0; k < kTT; ++k) b[k][0] = b[k][1] = b[k][2] = eb[k] = f2_splat(0.f);
-#pragma unroll 2
-      for (int q = q0; q < q0 + 16; ++q) pair_interact_impl<true, true>(sh[q], T, b, special, eb);
+      pair_stretch<true, true, 2>(sh + q0, T, b, eb, special);
 #pragma unroll
       for (int k = 0; k < kTT; ++k) {
         float lo, hi;

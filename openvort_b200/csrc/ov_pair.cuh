@@ -8,6 +8,8 @@
 
 #include <cuda_runtime.h>
 
+#include "ov_device.cuh"
+
 struct f2 {
   unsigned long long v;
 };
@@ -79,8 +81,7 @@ __device__ __forceinline__ f2 f2_rcp(f2 a) {
 // which is the reference's segment formula (src/tangle.c:486-517) and its
 // colinearity cut-off |cos - 1| < 1e-8, zero inside it.  Within 2.5e-3 of
 // the cut-off (the FP32 rounding bound of |R x d|^2, see seg_vel32), or
-// nearer than the source's far radius, the pair is left to the caller's
-// FP64 path.
+// nearer than the source's far radius, the pair is left to FP64.
 
 #ifndef OV_PAIR_TT
 #define OV_PAIR_TT 2
@@ -151,15 +152,22 @@ __device__ __forceinline__ void set_target(PairTargets& t, int k, double px, dou
 }
 
 // Two sources against the thread's targets: FP32 contributions (without the
-// kappa/4pi factor) into b[k] (low half: source 0, high half: source 1);
-// pairs needing FP64 call special(k, id).  The two-float form takes R as
+// kappa/4pi factor) into b[k] (low half: source 0, high half: source 1).
+// Returns the pairs left to FP64, bit 2 k + h for target k and source h: the
+// caller collects them over a stretch of records (PairSpecials) and evaluates
+// them after it, so the loop holds no FP64 code and every lane goes through
+// its own pairs at once instead of a warp stopping at each record where some
+// lane has one.  What an ordinary pair does not need (the selections, the
+// test of the cut-off's lower edge) stands behind one branch per target: with
+// it the loop is 31 packed operations, 6 approximations and 4 comparisons.
+// The two-float form takes R as
 // (a_hi - t_hi) + (a_lo - t_lo), which carries ~2 ulps of |R| itself
 // however far source and target are from the origin.  With kBound (two-
 // float form only) eb[k] also accumulates |d| / |R|^2 over the pairs
 // evaluated here in FP32, the quantity that bounds their rounding error.
-template <bool kTwo, bool kBound, class Special>
-__device__ __forceinline__ void pair_interact_impl(const PairSrc<kTwo>& src, const PairTargets& T,
-                                                   f2 (&b)[kTT][3], Special&& special, f2 (&eb)[kTT]) {
+template <bool kTwo, bool kBound>
+__device__ __forceinline__ unsigned pair_interact_impl(const PairSrc<kTwo>& src, const PairTargets& T,
+                                                       f2 (&b)[kTT][3], f2 (&eb)[kTT]) {
   static_assert(kTwo || !kBound, "the error bound needs |d|, staged in the two-float form");
   const float4 q0 = src.q[0], q1 = src.q[1], q2 = src.q[2], q3 = src.q[3], q4 = src.q[4], q5 = src.q[5];
   const f2 ax = f2_pack(q0.x, q0.y), ay = f2_pack(q0.z, q0.w), az = f2_pack(q1.x, q1.y);
@@ -175,6 +183,7 @@ __device__ __forceinline__ void pair_interact_impl(const PairSrc<kTwo>& src, con
     alz = f2_pack(q7.x, q7.y);
     dn = f2_pack(q7.z, q7.w);
   }
+  unsigned left = 0;
 #pragma unroll
   for (int k = 0; k < kTT; ++k) {
     f2 Rx = ax - T.x[k], Ry = ay - T.y[k], Rz = az - T.z[k];
@@ -195,36 +204,90 @@ __device__ __forceinline__ void pair_interact_impl(const PairSrc<kTwo>& src, con
     const f2 Cy = f2_fma(Rz, dx, Rx * ndz);
     const f2 Cz = f2_fma(Rx, dy, Ry * ndx);
     const f2 tc = f2_fma(Cz, Cz, f2_fma(Cy, Cy, Cx * Cx)) * (u * w);   // 1 - cos
-    float tc0, tc1, r20, r21, s0, s1;
+    float tc0, tc1, r20, r21;
     f2_unpack(tc, tc0, tc1);
     f2_unpack(R2, r20, r21);
-    f2_unpack(s, s0, s1);
     const bool far0 = r20 >= q5.x, far1 = r21 >= q5.y;
     const bool ok0 = far0 && tc0 > kColHi, ok1 = far1 && tc1 > kColHi;
-    // colinear (zero) and FP64 cases add nothing here
-    const f2 sk = f2_pack(ok0 ? s0 : 0.f, ok1 ? s1 : 0.f);
-    b[k][0] = f2_fma(Cx, sk, b[k][0]);
-    b[k][1] = f2_fma(Cy, sk, b[k][1]);
-    b[k][2] = f2_fma(Cz, sk, b[k][2]);
-    if constexpr (kBound) {
-      float i0, i1;
-      f2_unpack(ia * ia, i0, i1);
-      eb[k] = f2_fma(dn, f2_pack(ok0 ? i0 : 0.f, ok1 ? i1 : 0.f), eb[k]);
+    f2 si = s, i2 = s;
+    if constexpr (kBound) i2 = ia * ia;
+    if (!(ok0 && ok1)) {   // rare: a colinear (zero) or FP64 case, which adds nothing here
+      float s0, s1;
+      f2_unpack(s, s0, s1);
+      si = f2_pack(ok0 ? s0 : 0.f, ok1 ? s1 : 0.f);
+      if constexpr (kBound) {
+        float i0, i1;
+        f2_unpack(i2, i0, i1);
+        i2 = f2_pack(ok0 ? i0 : 0.f, ok1 ? i1 : 0.f);
+      }
+      if (!ok0 && !(far0 && tc0 < kColLo)) left |= 1u << (2 * k);
+      if (!ok1 && !(far1 && tc1 < kColLo)) left |= 2u << (2 * k);
     }
-    const bool sp0 = !ok0 && !(far0 && tc0 < kColLo);
-    const bool sp1 = !ok1 && !(far1 && tc1 < kColLo);
-    if (sp0 || sp1) {
-      if (sp0) special(k, __float_as_int(q5.z));
-      if (sp1) special(k, __float_as_int(q5.w));
-    }
+    b[k][0] = f2_fma(Cx, si, b[k][0]);
+    b[k][1] = f2_fma(Cy, si, b[k][1]);
+    b[k][2] = f2_fma(Cz, si, b[k][2]);
+    if constexpr (kBound) eb[k] = f2_fma(dn, i2, eb[k]);
+  }
+  return left;
+}
+
+template <bool kTwo>
+__device__ __forceinline__ unsigned pair_interact(const PairSrc<kTwo>& src, const PairTargets& T, f2 (&b)[kTT][3]) {
+  f2 unused[kTT];
+  return pair_interact_impl<kTwo, false>(src, T, b, unused);
+}
+
+// source slot h of a record
+template <bool kTwo>
+__device__ __forceinline__ int pair_id(const PairSrc<kTwo>& src, int h) {
+  return __float_as_int(h ? src.q[5].w : src.q[5].z);
+}
+
+// v added to target u's FP64 sums
+__device__ __forceinline__ void add_target(double (&acc)[kTT][3], int u, d3 v) {
+#pragma unroll
+  for (int k = 0; k < kTT; ++k) {
+    if (k != u) continue;
+    acc[k][0] += v.x;
+    acc[k][1] += v.y;
+    acc[k][2] += v.z;
   }
 }
 
-template <bool kTwo, class Special>
-__device__ __forceinline__ void pair_interact(const PairSrc<kTwo>& src, const PairTargets& T,
-                                              f2 (&b)[kTT][3], Special&& special) {
-  f2 unused[kTT];
-  pair_interact_impl<kTwo, false>(src, T, b, special, unused);
+// The pairs left to FP64 over up to 16 records (or chain positions)
+static_assert(kTT == 2, "four pairs per record");
+struct PairSpecials {
+  unsigned m[2] = {0, 0};
+  // left: pair bits of record i
+  __device__ __forceinline__ void add(int i, unsigned left) {
+    if (i < 8) m[0] |= left << (4 * i);
+    else m[1] |= left << (4 * (i - 8));
+  }
+  // eval(k, h, i) for every pair collected: target k, source h of record i
+  template <class Eval>
+  __device__ __forceinline__ void run(Eval&& eval) {
+#pragma unroll
+    for (int w = 0; w < 2; ++w) {
+      while (m[w]) {
+        const int b = __ffs(m[w]) - 1;
+        m[w] &= m[w] - 1;
+        eval((b >> 1) & 1, b & 1, 8 * w + (b >> 2));
+      }
+    }
+  }
+};
+
+// A stretch of 16 records: FP32 sums into b (and eb, with kBound), then the
+// pairs left to FP64 through special(u, id)
+template <bool kTwo, bool kBound, int kUnroll, class Special>
+__device__ __forceinline__ void pair_stretch(const PairSrc<kTwo>* sh, const PairTargets& T, f2 (&b)[kTT][3],
+                                             f2 (&eb)[kTT], Special&& special) {
+#pragma unroll
+  for (int k = 0; k < kTT; ++k) b[k][0] = b[k][1] = b[k][2] = eb[k] = f2_splat(0.f);
+  PairSpecials sp;
+#pragma unroll kUnroll
+  for (int q = 0; q < 16; ++q) sp.add(q, pair_interact_impl<kTwo, kBound>(sh[q], T, b, eb));
+  sp.run([&](int u, int h, int i) { special(u, pair_id(sh[i], h)); });
 }
 
 // ----------------------------------------------------------------------
@@ -306,8 +369,8 @@ __device__ __forceinline__ void chain_seg_set(ChainSeg& sg, const float (&dd)[2]
 
 // The kCH chained pairs of a staged tile against the thread's targets:
 // FP32 partial sums over 32 segments, each added (times f4pi) into acc;
-// pairs needing FP64 call special(u, slot).  Every thread of the warp runs
-// the same iterations.
+// pairs needing FP64 call special(u, slot) after each stretch of 16 positions
+// (PairSpecials).  Every thread of the warp runs the same iterations.
 template <bool kTwo, class Special>
 __device__ __forceinline__ void chain_sweep(const ChainNode<kTwo>* sh_node, const ChainSeg* sh_seg,
                                             const PairTargets& T, double (&acc)[kTT][3], double f4pi,
@@ -337,8 +400,10 @@ __device__ __forceinline__ void chain_sweep(const ChainNode<kTwo>* sh_node, cons
     f2 b[kTT][3];
 #pragma unroll
     for (int u = 0; u < kTT; ++u) b[u][0] = b[u][1] = b[u][2] = f2_splat(0.f);
+    PairSpecials sp;
 #pragma unroll kChainUnroll
     for (int i = i0; i < i0 + 16; ++i) {
+      unsigned left = 0;
       const ChainNode<kTwo> nd = sh_node[i + 1];
       const ChainSeg sg = sh_seg[i];
       const f2 nx = f2_pack(nd.x.x, nd.x.y), ny = f2_pack(nd.y.x, nd.y.y), nz = f2_pack(nd.z.x, nd.z.y);
@@ -385,17 +450,17 @@ __device__ __forceinline__ void chain_sweep(const ChainNode<kTwo>* sh_node, cons
         b[u][0] = f2_fma(Cx, sk, b[u][0]);
         b[u][1] = f2_fma(Cy, sk, b[u][1]);
         b[u][2] = f2_fma(Cz, sk, b[u][2]);
-        if (sp0 || sp1) {
-          if (sp0) special(u, sg.id[0]);
-          if (sp1) special(u, sg.id[1]);
-        }
+        if (sp0) left |= 1u << (2 * u);
+        if (sp1) left |= 2u << (2 * u);
         Rx[u] = Bx;
         Ry[u] = By;
         Rz[u] = Bz;
         R2[u] = B2;
         ia[u] = ib;
       }
+      sp.add(i - i0, left);
     }
+    sp.run([&](int u, int h, int i) { special(u, sh_seg[i0 + i].id[h]); });
 #pragma unroll
     for (int u = 0; u < kTT; ++u) {
 #pragma unroll
