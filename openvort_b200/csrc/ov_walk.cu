@@ -541,7 +541,7 @@ __device__ __forceinline__ void cell_mixed(const OvParams& P, const Cell* cp, fl
     // is g x P + m x Q + (m21 S, 0, 0), P = sum i3 R, Q = sum i5 R,
     // S = sum i3; since R_x and R_y are constant along a column,
     // P_x, P_y, Q_x, Q_y take each column's sums of i3 and i5 once.
-    f2 px = f2_splat(0.f), py = px, pz = px, qx = px, qy = px, qz = px, sv = px;
+    float Px, Py, Pz, Qx, Qy, Qz, Sv;
     // All 27 images accept (the usual case: the wrapped opening test
     // treats every image point like the target), or a product of per-axis
     // shift sets, and none but the tangle's own image is near: no per-image
@@ -573,42 +573,75 @@ __device__ __forceinline__ void cell_mixed(const OvParams& P, const Cell* cp, fl
             Fy[2] * Fy[2] >= fnear2 && Fz[0] * Fz[0] >= fnear2 && Fz[2] * Fz[2] >= fnear2;
     }
     if (all) {
-      // unrolled: the column offsets are chosen at compile time
+      // unrolled: the column offsets are chosen at compile time.  The sums
+      // over a shift along z are kept per shift, so R_z multiplies each once
+      // at the end, and column 8 goes by itself: its z shifts 0 and 1 as a
+      // pair, shift 2 alone.
+      f2 px = f2_splat(0.f), py = px, qx = px, qy = px, z3[3] = {px, px, px}, z5[3] = {px, px, px};
 #pragma unroll
-      for (int grp = 0; grp < 5; ++grp) {
-        const int xa = 2 * grp, xb = grp < 4 ? xa + 1 : xa;
+      for (int grp = 0; grp < 4; ++grp) {
+        const int xa = 2 * grp, xb = xa + 1;
         const int ixa = (xa * 11) >> 5, iya = xa - 3 * ixa;
         const int ixb = (xb * 11) >> 5, iyb = xb - 3 * ixb;
-        const float Xa = sel3f(ixa, Fx[0], Fx[1], Fx[2]), Xb = sel3f(ixb, Fx[0], Fx[1], Fx[2]);
-        const float Ya = sel3f(iya, Fy[0], Fy[1], Fy[2]), Yb = sel3f(iyb, Fy[0], Fy[1], Fy[2]);
-        const f2 X = f2_pack(Xa, Xb), Y = f2_pack(Ya, Yb);
+        const f2 X = f2_pack(Fx[ixa], Fx[ixb]), Y = f2_pack(Fy[iya], Fy[iyb]);
         const f2 XY2 = f2_fma(X, X, Y * Y);
-        // the last group holds column 8 twice: its second half is dropped
-        const f2 keep = f2_pack(1.f, grp < 4 ? 1.f : 0.f);
         f2 c3 = f2_splat(0.f), c5 = c3;
 #pragma unroll
         for (int iz = 0; iz < 3; ++iz) {
           const f2 Zs = f2_splat(Fz[iz]);
           f2 inv = f2_rsqrt(f2_fma(Zs, Zs, XY2));
-          if (grp == 4) inv = inv * keep;
           if (grp == 2 && iz == 1) inv = inv * f2_pack(near0 ? 0.f : 1.f, 1.f);
           const f2 inv2 = inv * inv;
           const f2 i3 = inv2 * inv;
-          const f2 i5 = (i3 * inv2) * Zs;
-          c3 = c3 + i3;
-          c5 = c5 + i5;
-          pz = f2_fma(i3, Zs, pz);
-          qz = f2_fma(i5, Zs, qz);
+          const f2 t5 = i3 * inv2;
+          c3 = iz ? c3 + i3 : i3;
+          c5 = iz ? f2_fma(t5, Zs, c5) : t5 * Zs;
+          z3[iz] = grp ? z3[iz] + i3 : i3;
+          z5[iz] = grp ? z5[iz] + t5 : t5;
         }
-        px = f2_fma(c3, X, px);
-        py = f2_fma(c3, Y, py);
-        qx = f2_fma(c5, X, qx);
-        qy = f2_fma(c5, Y, qy);
-        sv = sv + c3;
+        px = grp ? f2_fma(c3, X, px) : c3 * X;
+        py = grp ? f2_fma(c3, Y, py) : c3 * Y;
+        qx = grp ? f2_fma(c5, X, qx) : c5 * X;
+        qy = grp ? f2_fma(c5, Y, qy) : c5 * Y;
       }
+      const float X8 = Fx[2], Y8 = Fy[2], xy2 = fmaf(X8, X8, Y8 * Y8);
+      const f2 Z01 = f2_pack(Fz[0], Fz[1]);
+      const f2 inv = f2_rsqrt(f2_fma(Z01, Z01, f2_splat(xy2)));
+      const f2 inv2 = inv * inv;
+      const f2 i3 = inv2 * inv, t5 = i3 * inv2;
+      const float inv_2 = rsqrt_approx(fmaf(Fz[2], Fz[2], xy2)), i3_2 = (inv_2 * inv_2) * inv_2;
+      const float t5_2 = i3_2 * (inv_2 * inv_2);
+      float i3_0, i3_1, t5_0, t5_1, lo, hi;
+      f2_unpack(i3, i3_0, i3_1);
+      f2_unpack(t5, t5_0, t5_1);
+      const float c3 = (i3_0 + i3_1) + i3_2, c5 = fmaf(t5_2, Fz[2], fmaf(t5_1, Fz[1], t5_0 * Fz[0]));
+      f2_unpack(px, lo, hi);
+      Px = fmaf(c3, X8, lo + hi);
+      f2_unpack(py, lo, hi);
+      Py = fmaf(c3, Y8, lo + hi);
+      f2_unpack(qx, lo, hi);
+      Qx = fmaf(c5, X8, lo + hi);
+      f2_unpack(qy, lo, hi);
+      Qy = fmaf(c5, Y8, lo + hi);
+      f2_unpack(z3[0], lo, hi);
+      const float s0 = (lo + hi) + i3_0;
+      f2_unpack(z3[1], lo, hi);
+      const float s1 = (lo + hi) + i3_1;
+      f2_unpack(z3[2], lo, hi);
+      const float s2 = (lo + hi) + i3_2;
+      Sv = (s0 + s1) + s2;
+      Pz = fmaf(s2, Fz[2], fmaf(s1, Fz[1], s0 * Fz[0]));
+      f2_unpack(z5[0], lo, hi);
+      const float w0 = ((lo + hi) + t5_0) * Fz[0];
+      f2_unpack(z5[1], lo, hi);
+      const float w1 = ((lo + hi) + t5_1) * Fz[1];
+      f2_unpack(z5[2], lo, hi);
+      const float w2 = ((lo + hi) + t5_2) * Fz[2];
+      Qz = fmaf(w2, Fz[2], fmaf(w1, Fz[1], w0 * Fz[0]));
       if (near0)
         nl = nl + expansion64_at(cp, mk3(__dsub_rn(r.x, cx), __dsub_rn(r.y, cy), __dsub_rn(r.z, cz)));
     } else {
+    f2 px = f2_splat(0.f), py = px, pz = px, qx = px, qy = px, qz = px, sv = px;
 #pragma unroll 1
     for (int grp = 0; grp < 5; ++grp) {
       const int xa = 2 * grp, xb = grp < 4 ? xa + 1 : xa;
@@ -665,24 +698,24 @@ __device__ __forceinline__ void cell_mixed(const OvParams& P, const Cell* cp, fl
       qy = f2_fma(c5, Y, qy);
       sv = sv + c3;
     }
-    }
     float a0, a1;
     f2_unpack(px, a0, a1);
-    const float Px = a0 + a1;
+    Px = a0 + a1;
     f2_unpack(py, a0, a1);
-    const float Py = a0 + a1;
+    Py = a0 + a1;
     f2_unpack(pz, a0, a1);
-    const float Pz = a0 + a1;
+    Pz = a0 + a1;
     f2_unpack(qx, a0, a1);
-    const float Qx = a0 + a1;
+    Qx = a0 + a1;
     f2_unpack(qy, a0, a1);
-    const float Qy = a0 + a1;
+    Qy = a0 + a1;
     f2_unpack(qz, a0, a1);
-    const float Qz = a0 + a1;
+    Qz = a0 + a1;
     f2_unpack(sv, a0, a1);
-    const float S = a0 + a1;
+    Sv = a0 + a1;
+    }
     // g x P + m x Q + (m21 S, 0, 0), m = (m02, m12, m22)
-    ax = fmaf(g1, Pz, fmaf(-g2, Py, fmaf(m12, Qz, fmaf(-m22, Qy, m21 * S))));
+    ax = fmaf(g1, Pz, fmaf(-g2, Py, fmaf(m12, Qz, fmaf(-m22, Qy, m21 * Sv))));
     ay = fmaf(g2, Px, fmaf(-g0, Pz, fmaf(m22, Qx, -m02 * Qz)));
     az = fmaf(g0, Py, fmaf(-g1, Px, fmaf(m02, Qy, -m12 * Qx)));
   }
@@ -728,6 +761,8 @@ __device__ __forceinline__ void cell_fp64(const OvParams& P, const Cell* cp, dou
     }
   }
   if (all) {
+    // sums over a shift along z kept per shift, as in cell_mixed
+    double z3[3] = {0, 0, 0}, z5[3] = {0, 0, 0};
 #pragma unroll
     for (int xy = 0; xy < 9; ++xy) {
       const double X = Rx[xy / 3], Y = Ry[xy % 3];
@@ -740,18 +775,20 @@ __device__ __forceinline__ void cell_fp64(const OvParams& P, const Cell* cp, dou
         const double inv = rsqrt_nr(fma(Z, Z, XY2));
         const double inv2 = inv * inv;
         const double i3 = inv2 * inv;
-        const double i5 = (i3 * inv2) * Z;
-        c3 += i3;
-        c5 += i5;
-        pz = fma(i3, Z, pz);
-        qz = fma(i5, Z, qz);
+        const double t5 = i3 * inv2;
+        c3 = iz ? c3 + i3 : i3;
+        c5 = iz ? fma(t5, Z, c5) : t5 * Z;
+        z3[iz] = xy ? z3[iz] + i3 : i3;
+        z5[iz] = xy ? z5[iz] + t5 : t5;
       }
-      px = fma(c3, X, px);
-      py = fma(c3, Y, py);
-      qx = fma(c5, X, qx);
-      qy = fma(c5, Y, qy);
-      sv += c3;
+      px = xy ? fma(c3, X, px) : c3 * X;
+      py = xy ? fma(c3, Y, py) : c3 * Y;
+      qx = xy ? fma(c5, X, qx) : c5 * X;
+      qy = xy ? fma(c5, Y, qy) : c5 * Y;
     }
+    sv = (z3[0] + z3[1]) + z3[2];
+    pz = fma(z3[2], Rz[2], fma(z3[1], Rz[1], z3[0] * Rz[0]));
+    qz = fma(z5[2] * Rz[2], Rz[2], fma(z5[1] * Rz[1], Rz[1], (z5[0] * Rz[0]) * Rz[0]));
   } else {
 #pragma unroll 1
     for (int xy = 0; xy < 9; ++xy) {
@@ -789,20 +826,17 @@ __device__ __forceinline__ void cell_fp64(const OvParams& P, const Cell* cp, dou
                 fma(g[0], py, fma(-g[1], px, fma(m02, qy, -m12 * qx))));
 }
 
-// resident warps per SM the register allocation must allow.  At 16 neither
-// form spills (128 registers).  Measured, ms per launch at 1M / 200k / 22.4k
-// nodes for 12 / 16 / 20 (24) warps: mixed 31.5 / 6.04 / 1.07, 27.7 / 5.42 /
-// 0.94, 28.0 / 5.69 / 1.67; FP64 (16, 20, 24) 53.4 / 10.4 / 1.70, 52.9 / 10.6
-// / 1.99, 53.2 / 9.87 / 2.03.
+// resident warps per SM the register allocation must allow.  ms per launch for
+// 12 / 16 / 20 / 24 warps: mixed 1M nodes 31.5 / 27.7 / 28.0 before the sums
+// per z shift and the segments' queue (25.7 and 23.8 at 16 since); FP64 in one
+// part per group 1M 46.2 / 41.6 / 38.8 / 42.0, 200k 8.4 / 7.6 / 7.6 / 8.0, in
+// parts 60k 3.91 / 3.34 / 3.26.  20 warps spill some 90 bytes; the split form
+// stays at 16, where a wave holds fewer parts.
 // Blocks are one warp each: a block of four kept its place until its slowest
 // warp ended (200k nodes FP64, two parts, a first walk: 16.9 ms against 15.9;
 // 1M mixed 35.8 against 35.1).
-#ifndef OV_WALK_MULTI_MIN_WARPS_MIXED
-#define OV_WALK_MULTI_MIN_WARPS_MIXED 16
-#endif
-#ifndef OV_WALK_MULTI_MIN_WARPS_FP64
-#define OV_WALK_MULTI_MIN_WARPS_FP64 16
-#endif
+constexpr int kWalkWarps = 16;
+constexpr int kWalkWarpsFp64 = 20;
 
 // A group's walk split over `parts` warps (a power of two), for launches with
 // too few groups to fill the GPU.  Every part traverses the cells whose
@@ -824,14 +858,82 @@ struct WalkSplit {
   double* im;
 };
 
+__device__ __forceinline__ d3 shfl3(d3 v, int src) {
+  return mk3(__shfl_sync(0xffffffffu, v.x, src), __shfl_sync(0xffffffffu, v.y, src),
+             __shfl_sync(0xffffffffu, v.z, src));
+}
+
+// Pairs of cell and target waiting to be evaluated 32 at a time, one by each
+// lane of the warp, whichever lane's target they belong to.  A leaf is near 8
+// to 10 of a group's 32 targets and an accepted cell is one for 20 to 24 of
+// them, so evaluated at the visit they leave the other lanes idle.  A target's
+// pairs are taken in preorder and added in that order by its own lane, the
+// segments' sum apart from the cells', so the sums do not depend on the other
+// targets of the group.  Segments wait in both forms: 200k / 1M nodes mixed
+// 5.04 -> 4.62 / 25.7 -> 23.8 ms, FP64 10.0 -> 8.3 / 51.2 -> 43.5.  Cells wait
+// in the FP64 form, where their evaluation takes the FP64 pipe some 400
+// operations: 8.3 -> 7.6 / 43.5 -> 38.8; in the mixed form the queue costs more
+// than the idle lanes (23.8 -> 27.7).
+struct WalkQueue {
+  int cell[64];
+  unsigned mask[64];   // lane of the target << 27 | image mask
+};
+struct WalkBatch {
+  bool on;
+  int cell, own;   // own: lane of the target
+  unsigned mask;
+};
+
+// every lane with a mask adds the pair of cell q and its target; n < 32
+__device__ __forceinline__ void queue_put(WalkQueue& Q, int& n, int q, unsigned mask, int lane) {
+  const unsigned who = __ballot_sync(0xffffffffu, mask != 0);
+  if (mask) {
+    const int at = n + __popc(who & ((1u << lane) - 1u));
+    Q.cell[at] = q;
+    Q.mask[at] = mask | ((unsigned)lane << 27);
+  }
+  n += __popc(who);
+  __syncwarp();
+}
+
+// the first 32 entries (or all n), one per lane; of[l]: which of them are
+// of lane l's target, to be read after a __syncwarp()
+__device__ __forceinline__ WalkBatch queue_take(WalkQueue& Q, int& n, unsigned* of, int lane) {
+  const int cnt = min(n, 32);
+  WalkBatch e;
+  e.on = lane < cnt;
+  e.cell = e.on ? Q.cell[lane] : 0;
+  const unsigned m = e.on ? Q.mask[lane] : 0u;
+  e.own = e.on ? (int)(m >> 27) : lane;
+  e.mask = m & kAllImages;
+  const unsigned same = __match_any_sync(0xffffffffu, e.on ? e.own : 32 + lane);
+  of[lane] = 0;
+  const bool more = lane + 32 < n;
+  const int c1 = more ? Q.cell[lane + 32] : 0;
+  const unsigned m1 = more ? Q.mask[lane + 32] : 0u;
+  __syncwarp();
+  if (e.on && lane == __ffs(same) - 1) of[e.own] = same;
+  if (more) {
+    Q.cell[lane] = c1;
+    Q.mask[lane] = m1;
+  }
+  n -= cnt;
+  return e;
+}
+
 template <bool kMixed, bool kSplit>
-__global__ void __launch_bounds__(32, kMixed ? OV_WALK_MULTI_MIN_WARPS_MIXED : OV_WALK_MULTI_MIN_WARPS_FP64)
+__global__ void __launch_bounds__(32, kMixed || kSplit ? kWalkWarps : kWalkWarpsFp64)
     k_walk_multi(
     OvParams P, TreeView T, const int* __restrict__ order, const int2* __restrict__ status,
     const double* __restrict__ pos, int n_t, unsigned combos, ImageShortcut S, double near2,
     double* v_nl, double* v_img, unsigned long long* counters, const int* __restrict__ warp_perm,
     unsigned* __restrict__ warp_cost, WalkSplit W) {
   __shared__ unsigned sh_mask[kLevelSlots][32];
+  __shared__ WalkQueue leaves;                    // segments and the targets they are near
+  __shared__ WalkQueue cells;                     // accepted cells and their targets
+  __shared__ unsigned sh_of[32];                  // entries of each lane's target
+  __shared__ double sh_seg[kMixed ? 3 : 6][32];   // each lane's sums over segments
+  constexpr bool kQueueCells = !kMixed;
   const unsigned FULL = 0xffffffffu;
   const int lane = threadIdx.x;
   const long long t_start = clock64();
@@ -862,10 +964,73 @@ __global__ void __launch_bounds__(32, kMixed ? OV_WALK_MULTI_MIN_WARPS_MIXED : O
   d3 nl = mk3(0, 0, 0), im = mk3(0, 0, 0);
   unsigned n_p2p = 0, n_far = 0, n_iter = 0;
   int next = live ? 0 : T.n_cells;
+  int n_leaves = 0, n_cells = 0;   // entries waiting
+#pragma unroll
+  for (int c = 0; c < (kMixed ? 3 : 6); ++c) sh_seg[c][lane] = 0;
   __syncwarp();
   for (;;) {
     const int q = (int)__reduce_min_sync(FULL, (unsigned)next);
-    if (q >= T.n_cells) break;
+    const bool done = q >= T.n_cells;
+    if (kQueueCells && (n_cells >= 32 || (done && n_cells > 0))) {
+      const WalkBatch e = queue_take(cells, n_cells, sh_of, lane);
+      const d3 rt = shfl3(r, e.own);
+      d3 v = mk3(0, 0, 0), w = v;
+      if (e.on) {
+        const Cell* cp = T.cells + e.cell;
+        const double cx = cp->x[0], cy = cp->x[1], cz = cp->x[2];
+        if (kMixed)
+          cell_mixed(P, cp, __int_as_float(cp->a), cx, cy, cz, cp->thr, rt,
+                     mk3(__dsub_rn(cx, rt.x), __dsub_rn(cy, rt.y), __dsub_rn(cz, rt.z)), e.mask, near2, v);
+        else
+          cell_fp64(P, cp, cx, cy, cz, rt, e.mask, v, w);
+      }
+      __syncwarp();
+      for (unsigned of = sh_of[lane]; __any_sync(FULL, of != 0); of &= of - 1) {
+        const int src = of ? __ffs(of) - 1 : lane;
+        const d3 a = shfl3(v, src);
+        if (of) nl = nl + a;
+        if (!kMixed) {
+          const d3 b = shfl3(w, src);
+          if (of) im = im + b;
+        }
+      }
+      continue;
+    }
+    if (n_leaves >= 32 || (done && n_leaves > 0)) {
+      const WalkBatch e = queue_take(leaves, n_leaves, sh_of, lane);
+      const d3 rt = shfl3(r, e.own);
+      const int skip_t = __shfl_sync(FULL, skip, e.own);
+      d3 v = mk3(0, 0, 0), w = v;
+      if (e.on) {
+        const Cell* cp = T.cells + e.cell;
+        const int2 id = *reinterpret_cast<const int2*>(cp);
+        const d3 r1 = mk3(cp->x[0], cp->x[1], cp->x[2]), r2 = mk3(cp->y[0], cp->y[1], cp->y[2]);
+        if (kMixed && __popc(e.mask) >= kColumnImages)
+          p2p_mixed_columns(P, e.mask, rt, r1, r2, id.x, id.y, skip_t, near2, v, n_p2p);
+        else
+          p2p_images<kMixed>(P, e.mask, rt, r1, r2, id.x, id.y, skip_t, near2, v, w, n_p2p);
+      }
+      __syncwarp();
+      for (unsigned of = sh_of[lane]; __any_sync(FULL, of != 0); of &= of - 1) {
+        const int src = of ? __ffs(of) - 1 : lane;
+        const d3 a = shfl3(v, src);
+        if (of) {
+          sh_seg[0][lane] += a.x;
+          sh_seg[1][lane] += a.y;
+          sh_seg[2][lane] += a.z;
+        }
+        if constexpr (!kMixed) {
+          const d3 b = shfl3(w, src);
+          if (of) {
+            sh_seg[3][lane] += b.x;
+            sh_seg[4][lane] += b.y;
+            sh_seg[5][lane] += b.z;
+          }
+        }
+      }
+      continue;
+    }
+    if (done) break;
     const Cell* cp = T.cells + q;
     if (lane == 0 && q + 1 < T.n_cells) prefetch_l1(cp + 1);
     const int4 h = *reinterpret_cast<const int4*>(cp);
@@ -884,17 +1049,14 @@ __global__ void __launch_bounds__(32, kMixed ? OV_WALK_MULTI_MIN_WARPS_MIXED : O
         own_end = h.z;
       }
     }
-    unsigned p2p_mask = 0;   // images summing this cell's node range directly
+    unsigned p2p_mask = 0;    // images summing this cell's node range directly
+    unsigned leaf_mask = 0;   // images summing this leaf's segment
+    unsigned cell_mask = 0;   // images accepting this cell
     if (next == q) {
       const unsigned m = lvl_mask[32 * cell_ltop(h.w)];
       unsigned open = 0;
       if (kind == CELL_LEAF1) {
-        if (kMixed && __popc(m) >= kColumnImages)
-          p2p_mixed_columns(P, m, r, mk3(t0.y, t1.x, t1.y), mk3(cp->y[0], cp->y[1], cp->y[2]), h.x, h.y, skip,
-                            near2, nl, n_p2p);
-        else
-          p2p_images<kMixed>(P, m, r, mk3(t0.y, t1.x, t1.y), mk3(cp->y[0], cp->y[1], cp->y[2]), h.x,
-                             h.y, skip, near2, nl, im, n_p2p);
+        leaf_mask = h.y == -1 ? 0u : m;
       } else if (kind == CELL_LEAFN) {
         p2p_mask = mine ? m : 0;
       } else {
@@ -953,7 +1115,9 @@ __global__ void __launch_bounds__(32, kMixed ? OV_WALK_MULTI_MIN_WARPS_MIXED : O
         if (pass && mine) {
           n_far += __popc(pass);
           // expansion at every accepting image: R = r - L s - com, unwrapped
-          if (kMixed) {
+          if (kQueueCells) {
+            cell_mask = pass;
+          } else if (kMixed) {
             cell_mixed(P, cp, __int_as_float(h.x), cx, cy, cz, t0.x, r, mk3(dx, dy, dz), pass, near2, nl);
           } else {
             cell_fp64(P, cp, cx, cy, cz, r, pass, nl, im);
@@ -965,6 +1129,11 @@ __global__ void __launch_bounds__(32, kMixed ? OV_WALK_MULTI_MIN_WARPS_MIXED : O
       next = open ? q + 1 : max(h.z, q + 1);
     }
     ++n_iter;
+    if (kind == CELL_LEAF1) {
+      queue_put(leaves, n_leaves, q, leaf_mask, lane);
+      continue;
+    }
+    if (kQueueCells) queue_put(cells, n_cells, q, cell_mask, lane);
     // direct sums over a node range (grain leaves), shared by the warp
     if (__ballot_sync(FULL, p2p_mask != 0)) {
       const int2 rg = T.cell_range[q];
@@ -982,6 +1151,8 @@ __global__ void __launch_bounds__(32, kMixed ? OV_WALK_MULTI_MIN_WARPS_MIXED : O
       }
     }
   }
+  nl = nl + mk3(sh_seg[0][lane], sh_seg[1][lane], sh_seg[2][lane]);
+  if constexpr (!kMixed) im = im + mk3(sh_seg[3][lane], sh_seg[4][lane], sh_seg[5][lane]);
   if (kSplit) {
     if (i < n_t) {
       st3(W.nl + 3 * (size_t)part * n_t, i, nl);
@@ -1175,7 +1346,8 @@ static __global__ void k_curve_keys(OvParams P, const double* __restrict__ pts, 
   vals[i] = k;
 }
 
-constexpr int kMaxParts = 32;   // warps a group's walk is split over, at most
+constexpr int kMaxParts = 16;        // warps a group of nodes' walk is split over, at most
+constexpr int kMaxPointParts = 32;   // and a group of points'
 
 static bool read_counters(ov_state_impl* s, OvTree* t) {
   unsigned long long c[3] = {0, 0, 0};
@@ -1254,25 +1426,28 @@ static bool launch_multi(ov_state_impl* s, OvTree* t, const OvParams& P, const i
   static const int wave_mixed = walk_wave(k_walk_multi<true, true>);
   static const int wave_fp64 = walk_wave(k_walk_multi<false, true>);
   const int wave = mixed ? wave_mixed : wave_fp64;
-  // Parts per group: enough that the units make two waves, so the last wave's
-  // slow units are short.  Measured, ms per walk of a tangle stepped on, at 1
-  // / 2 / 4 / 8 / 16 parts, 26 images.  Mixed (a wave is 2368 warps), theta =
-  // 0.4: 22.4k nodes 3.07 / 2.03 / 1.54 / 1.25 / 1.35, 60k 4.36 / 3.16 / 3.08
-  // / 3.22 / 3.76, 200k 10.7 / 10.6 / 11.0 / 12.0 / 14.0.  FP64 (3552):
-  // 22.4k 7.12 / 4.9 / 3.4 / 2.6 / 2.4, 200k at theta = 0.5 14.1 / 12.6 /
-  // 12.6 / 13.1; a first walk, without times to order it by, takes 15.8 / 15.9
-  // / 16.7 / 17.8 there.
+  // Parts per group.  Nodes: enough that the units make two waves (of 2368
+  // warps), so the last wave's slow units are short, but no more than 16, as
+  // each part takes the decisions above the frontier again.  26 images, theta
+  // = 0.4, ms per walk of a tangle stepped on: 8 / 16 / 32 parts at 3000 nodes
+  // mixed 0.25 / 0.23 / 0.32, at 8000 0.37 / 0.34 / 0.65; targets of one, two
+  // and four waves at 22.4k 0.96 / 0.85 / 1.52, at 100k 4.06 / 3.48 / 3.56.
+  // Points are fewer and their groups wider: 5/6 of a wave, so that it is one
+  // wave whatever power of two the parts come to, and up to 32 parts: queries
+  // of 512 points over 20k nodes 0.74 ms, 16 parts 0.85; of 4096 over 50k 1.15
+  // ms in 16 parts, 1.29 in 32.
   int parts = 1;
   const int groups = (n_t + 31) / 32;
   const long long groups_rule = (n_rule + 31) / 32;
-  while (parts < kMaxParts && groups_rule * parts < 2LL * wave) parts *= 2;
+  const long long units = status ? 2LL * wave : 5LL * wave / 6;
+  while (parts < (status ? kMaxParts : kMaxPointParts) && groups_rule * parts < units) parts *= 2;
   // Frontier: a smaller one deals the work out more evenly, but its cells'
-  // decisions are taken again in every part.  1/64 of the cells, for few
-  // groups (16 parts and more) and for points, whose groups are wider, 1/256:
-  // mixed 22.4k nodes at 8 parts 1.25 ms against 1.39 at 1/128; FP64 3000
-  // nodes at 32 parts 0.49 ms against 0.81 at 1/64; 512 points over 50k nodes
-  // 2.4 ms a query.
-  const int frontier = std::max(1, t->n_cells / (status && parts < 16 ? 64 : 256));
+  // decisions are taken again in every part.  Nodes 1/32 of the cells, ms at
+  // 1/8, 1/16, 1/32, 1/64, 1/128: mixed 8000 nodes 0.34 (1/32), 0.35, 0.40;
+  // 22.4k 0.92, 0.76, 0.79, 0.85, 1.06; 60k 1.83, 1.88, 1.87, 2.09, 2.30; FP64
+  // 22.4k 1.29, 1.20, 1.17, 1.24, 1.48.  Points 1/96 (512 over 20k nodes 0.77
+  // at 1/64, 0.74, 0.75 at 1/128, 0.77 at 1/192).
+  const int frontier = std::max(1, t->n_cells / (status ? 32 : 96));
   // stretches of a quarter of the frontier (22.4k nodes FP64, 8 parts: 2.52
   // ms, against 2.66 with a sixteenth)
   int deal = 0;
