@@ -102,23 +102,26 @@ __device__ bool tangent_node(const OvParams& P, const Links& L, const double* po
   return ok;
 }
 
-// The direct sum's partials of target k: the tangle's own sum nl = part[0]
-// and the image sum img = sum_j part[j] in image order (src/tangle.c:627-638),
-// mirror images reflecting their velocity (src/tangle.c:633-634).  With source
-// splits, each image's partial sums are added split by split, in order.
+// The direct sum's partials of target k for image j (0: the tangle itself),
+// with source splits added split by split, in order; mirror images reflect
+// their velocity (src/tangle.c:633-634).
+__device__ __forceinline__ d3 image_sum(const OvParams& P, const double* __restrict__ part, int n_t, int splits, int k,
+                                        int j) {
+  const size_t img_stride = 3 * (size_t)n_t, split_stride = img_stride * (P.n_img + 1);
+  const double* p = part + (size_t)j * img_stride;
+  d3 v = ld3(p, k);
+  for (int z = 1; z < splits; ++z) v = v + ld3(p + z * split_stride, k);
+  const int face = j > 0 ? P.img[j - 1][3] : -1;
+  return face > -1 ? mirror_dir(v, face) : v;
+}
+
+// The tangle's own sum nl and the image sum img in image order
+// (src/tangle.c:627-638)
 __device__ __forceinline__ void sum_partials(const OvParams& P, const double* __restrict__ part, int n_t, int splits,
                                              int k, d3& nl, d3& img) {
-  const size_t img_stride = 3 * (size_t)n_t, split_stride = img_stride * (P.n_img + 1);
-  nl = ld3(part, k);
-  for (int z = 1; z < splits; ++z) nl = nl + ld3(part + z * split_stride, k);
+  nl = image_sum(P, part, n_t, splits, k, 0);
   img = mk3(0, 0, 0);
-  for (int j = 1; j <= P.n_img; ++j) {
-    d3 v = ld3(part + (size_t)j * img_stride, k);
-    for (int z = 1; z < splits; ++z) v = v + ld3(part + z * split_stride + (size_t)j * img_stride, k);
-    const int face = P.img[j - 1][3];
-    if (face > -1) v = mirror_dir(v, face);
-    img = img + v;
-  }
+  for (int j = 1; j <= P.n_img; ++j) img = img + image_sum(P, part, n_t, splits, k, j);
 }
 
 // velocity assembly of a non-EMPTY node (update_velocity, src/tangle.c:

@@ -22,6 +22,7 @@
 #include <vector>
 
 #include "ov_internal.h"
+#include "ov_node.cuh"
 
 namespace {
 
@@ -178,97 +179,121 @@ __global__ void k_rec_scatter(const int* __restrict__ nodes, int count, int n, c
   st3(v_img, k, ld3(img, i));
 }
 
-// the four links do_reconnection changed, as kernel arguments
-struct LinkPatch {
+// What a reconnection changes, as kernel arguments: four links; the segments
+// whose slot m's forward link was (sign -1) or is now (sign +1) f; and the
+// entries of the known list that sit out the rest of the pass.  No links: the
+// known nodes' epilogue alone.
+struct RecChange {
+  int n_links = 0, n_seg = 0, n_retired = 0;
   int slot[4];
   int2 link[4];
-};
-
-__global__ void k_rec_patch_links(LinkPatch L, int2* links, int n, int* flag) {
-  const int c = threadIdx.x;
-  if (c >= 4) return;
-  if (L.slot[c] < 0 || L.slot[c] >= n) {
-    atomicOr(flag, 1);
-    return;
-  }
-  links[L.slot[c]] = L.link[c];
-}
-
-// one segment change of a reconnection: slot m's forward link was (sign -1)
-// or is now (sign +1) f
-struct SegChange {
   int m[4], f[4];
   double sign[4];
+  int retired[10];
 };
 
-// v_nl and v_img of the listed nodes += the changed segments' fields, with
-// the skip rule of the tangle's own sum (src/tangle.c:614-616) and the
-// mirror reflection of each image's sum (src/tangle.c:633-634).  One warp
-// per node: lane 0 takes the tangle itself, the lanes share the images
-// (image j on lane j mod 32), and the image terms are added in a fixed
-// shuffle tree, so the result does not depend on scheduling.
-constexpr int kCorrectWarps = 4;
-__global__ void __launch_bounds__(32 * kCorrectWarps) k_rec_correct(OvParams P, SegChange C,
-                                                                   const int* __restrict__ nodes, int count,
-                                                                   int n, const double* __restrict__ pos,
-                                                                   double* v_nl, double* v_img, int* flag) {
+// A reconnection for every known node in one launch: the links patched;
+// v_nl and v_img += the changed segments' fields, with the skip rule of the
+// tangle's own sum (src/tangle.c:614-616) and the mirror reflection of each
+// image's sum (src/tangle.c:633-634); then update_velocity's epilogue, with
+// vels and vs (6 doubles per entry of the list) stored into pinned host
+// memory.  One warp per node: the lanes share the images (image j on lane j
+// mod 32) and the tangle itself (as image n_img), and the image terms are
+// added in a fixed shuffle tree, so the result does not depend on scheduling.
+// The
+// epilogue reads a free node's own links only, and every slot whose link
+// changes is a retired one, so block 0 patches the links meanwhile.  A retired
+// entry becomes -1.
+// Bound by latency: with the links, the sums, the epilogue and the packing in
+// four launches, an upload of the list and two copies back a reconnection took
+// 43 us of the pass (100k nodes, open, 85 reconnections), now 22.
+constexpr int kUpdateWarps = 4;
+__global__ void __launch_bounds__(32 * kUpdateWarps) k_rec_update(
+    OvParams P, RecChange C, double t, int* __restrict__ nodes, int count, int n, const double* __restrict__ pos,
+    int2* links, const int2* __restrict__ status, const double* __restrict__ tan, const double* __restrict__ nrm,
+    double* v_nl, double* v_img, volatile double* host, volatile int* host_flag, int* flag) {
   const int lane = threadIdx.x & 31;
-  const int i = blockIdx.x * kCorrectWarps + (threadIdx.x >> 5);
+  const int i = blockIdx.x * kUpdateWarps + (threadIdx.x >> 5);
+  // error bits: into the pass's flag, and a word the host sees
+  auto fail = [&](int bits) { *host_flag = atomicOr(flag, bits) | bits; };
+  bool ok = true;
+  for (int c = 0; c < C.n_links; ++c) ok = ok && C.slot[c] >= 0 && C.slot[c] < n;
+  for (int c = 0; c < C.n_seg; ++c) ok = ok && C.m[c] >= 0 && C.m[c] < n && C.f[c] >= 0 && C.f[c] < n;
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    const int before = *flag;
+    if (before) *host_flag = before;
+    if (!ok) fail(1);
+  }
+  if (!ok) return;
+  if (blockIdx.x == 0 && threadIdx.x < C.n_links) links[C.slot[threadIdx.x]] = C.link[threadIdx.x];
   if (i >= count) return;   // whole warp
   const int k = nodes[i];
-  bool ok = k >= 0 && k < n;
-  for (int c = 0; c < 4; ++c) ok = ok && C.m[c] >= 0 && C.m[c] < n && C.f[c] >= 0 && C.f[c] < n;
-  if (!ok) {
-    if (lane == 0) atomicOr(flag, 1);
+  bool out = false;
+  for (int c = 0; c < C.n_retired; ++c) out = out || C.retired[c] == i;
+  __syncwarp();
+  if (out || k < 0 || k >= n) {
+    if (lane == 0) {
+      if (k >= n) fail(1);
+      nodes[i] = -1;
+    }
     return;
   }
   const d3 r = ld3(pos, k);
-  d3 r1[4], r2[4];
-  for (int c = 0; c < 4; ++c) {
-    r1[c] = ld3(pos, C.m[c]);
-    r2[c] = pwrap(P, r1[c], ld3(pos, C.f[c]));
-  }
   d3 nl = mk3(0, 0, 0), im = mk3(0, 0, 0);
-  if (lane == 0)
-    for (int c = 0; c < 4; ++c)
-      if (k != C.m[c] && k != C.f[c]) nl = nl + seg_vel64(P.f4pi, r1[c], r2[c], r) * C.sign[c];
-  for (int j = lane; j < P.n_img; j += 32) {
-    const d3 t = image_point(P, j, r);
-    d3 v = mk3(0, 0, 0);
-    for (int c = 0; c < 4; ++c) v = v + seg_vel64(P.f4pi, r1[c], r2[c], t) * C.sign[c];
-    const int face = P.img[j][3];
-    if (face > -1) v = mirror_dir(v, face);
-    im = im + v;
+  if (C.n_seg > 0) {
+    d3 r1[4], r2[4];
+    for (int c = 0; c < 4; ++c) {
+      r1[c] = ld3(pos, C.m[c]);
+      r2[c] = pwrap(P, r1[c], ld3(pos, C.f[c]));
+    }
+    for (int j = lane; j <= P.n_img; j += 32) {
+      const bool own = j == P.n_img;
+      const d3 x = own ? r : image_point(P, j, r);
+      d3 v = mk3(0, 0, 0);
+      for (int c = 0; c < 4; ++c)
+        if (!own || (k != C.m[c] && k != C.f[c]))
+          v = v + seg_vel64(P.f4pi, r1[c], r2[c], x) * C.sign[c];
+      if (own) {
+        nl = v;
+        continue;
+      }
+      const int face = P.img[j][3];
+      if (face > -1) v = mirror_dir(v, face);
+      im = im + v;
+    }
+    const int at = P.n_img & 31;
+    nl = mk3(__shfl_sync(0xffffffffu, nl.x, at), __shfl_sync(0xffffffffu, nl.y, at),
+             __shfl_sync(0xffffffffu, nl.z, at));
+    for (int off = 16; off > 0; off >>= 1) {
+      im.x += __shfl_down_sync(0xffffffffu, im.x, off);
+      im.y += __shfl_down_sync(0xffffffffu, im.y, off);
+      im.z += __shfl_down_sync(0xffffffffu, im.z, off);
+    }
   }
-  for (int off = 16; off > 0; off >>= 1) {
-    im.x += __shfl_down_sync(0xffffffffu, im.x, off);
-    im.y += __shfl_down_sync(0xffffffffu, im.y, off);
-    im.z += __shfl_down_sync(0xffffffffu, im.z, off);
-  }
+  d3 v = mk3(0, 0, 0), vs = v;
   if (lane == 0) {
-    st3(v_nl, k, ld3(v_nl, k) + nl);
-    st3(v_img, k, ld3(v_img, k) + im);
+    if (!P.lia_only) {
+      nl = ld3(v_nl, k) + nl;
+      im = ld3(v_img, k) + im;
+      if (C.n_seg > 0) {
+        st3(v_nl, k, nl);
+        st3(v_img, k, im);
+      }
+    }
+    Links L{links, status};
+    const int err = epilogue_node(P, L, t, pos, k, ld3(tan, k), ld3(nrm, k), nl, im, v, vs);
+    if (err) fail(err);
+  }
+  const double a[6] = {v.x, v.y, v.z, vs.x, vs.y, vs.z};
+#pragma unroll
+  for (int c = 0; c < 6; ++c) {
+    const double x = __shfl_sync(0xffffffffu, a[c], 0);
+    if (lane == c) host[6 * (size_t)i + c] = x;
   }
 }
 
-// vels and vs of the listed nodes, packed 6 doubles per node for one copy
-__global__ void k_rec_pack(const int* __restrict__ nodes, int count, int n, const double* __restrict__ vels,
-                           const double* __restrict__ vs, double* out, int* flag) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= count) return;
-  const int k = nodes[i];
-  if (k < 0 || k >= n) {
-    atomicOr(flag, 1);
-    for (int c = 0; c < 6; ++c) out[6 * (size_t)i + c] = 0;
-    return;
-  }
-  st3(out + 6 * (size_t)i, 0, ld3(vels, k));
-  st3(out + 6 * (size_t)i + 3, 0, ld3(vs, k));
-}
-
-// Pinned host memory for the pass's per-reconnection copies (the known list
-// up, the known nodes' values and the error flag down), so each copy is one
-// asynchronous transfer rather than a staged pageable one.
+// Pinned host memory: the known list's upload, and the known nodes' values
+// and the error flag, which k_rec_update stores here itself.
 struct PinnedBuf {
   void* p = nullptr;
   size_t bytes = 0;
@@ -288,9 +313,9 @@ struct PinnedBuf {
 };
 
 struct RecState {
-  PinnedBuf h_list, h_vals;   // known list (ints), known values (6 doubles each) + flag
+  PinnedBuf h_list, h_vals;   // known list (ints); flag, known values (6 doubles each)
   ov_state_impl s;
-  DevBuf keys, keys2, ids, ids2, pairs, count, hist, scan_part, skip, pack;
+  DevBuf keys, keys2, ids, ids2, pairs, count, hist, scan_part, skip;
   DevBuf batch, pts, bnl, bimg, known;   // batched velocities
   DevBuf bound, two;                     // mixed form: error bounds, FP64 re-checks
 };
@@ -437,39 +462,36 @@ bool upload_for_pass(RecState& R, const tangle_state* t) {
 // on the current links, mirrored on the host: node k's values at
 // hv[6 * pos_of[k]].
 struct RecVel {
-  std::vector<int> known;        // slots with velocities on the device
+  std::vector<int> known;        // slots with velocities on the device, -1: retired
   std::vector<int> pos_of;       // slot -> index in known, -1 if not known
-  std::vector<double> hv;        // 6 per known node: vels, vs
+  const double* hv = nullptr;    // 6 per known node: vels, vs (pinned, written by k_rec_update)
   std::vector<double> bound;     // per known node: bound on |mixed - FP64| of its sums (0: FP64)
   double time = 0;
 };
 
-// epilogue of every known node and the copy of their vels and vs to the host
-bool refresh_known(RecState& R, RecVel& V) {
+// a change to the links, the known nodes' sums and values, and their host copy
+bool refresh_known(RecState& R, RecVel& V, const RecChange& C) {
   ov_state_impl* s = &R.s;
   const int cnt = (int)V.known.size();
-  if (cnt == 0) return true;
+  if (cnt == 0 && C.n_links == 0) return true;
+  constexpr size_t kHead = 64;   // the flag word, then the values
+  if (!R.h_vals.reserve(kHead + sizeof(double) * 6 * (size_t)cnt)) return false;
+  int* h_flag = R.h_vals.as<int>();
+  double* h_val = reinterpret_cast<double*>(R.h_vals.as<char>() + kHead);
+  *h_flag = 0;
   // the pass's error flag (zeroed at its start) accumulates every kernel's bits
-  int* flag = s->dflag.as<int>();
-  if (!ov_launch_epilogue_list(s->stream, s->P, s->links.as<int2>(), s->status.as<int2>(), V.time,
-                               s->pos.as<double>(), s->tan.as<double>(), s->nrm.as<double>(),
-                               s->v_nl.as<double>(), s->v_img.as<double>(), s->vels.as<double>(),
-                               s->vs.as<double>(), R.known.as<int>(), cnt, flag))
-    return false;
-  if (!R.pack.reserve(sizeof(double) * 6 * (size_t)cnt + 64)) return false;
-  k_rec_pack<<<(cnt + 255) / 256, 256, 0, s->stream>>>(R.known.as<int>(), cnt, s->n, s->vels.as<double>(),
-                                                       s->vs.as<double>(), R.pack.as<double>(), flag);
+  k_rec_update<<<std::max(1, (cnt + kUpdateWarps - 1) / kUpdateWarps), 32 * kUpdateWarps, 0, s->stream>>>(
+      s->P, C, V.time, R.known.as<int>(), cnt, s->n, s->pos.as<double>(), s->links.as<int2>(), s->status.as<int2>(),
+      s->tan.as<double>(), s->nrm.as<double>(), s->v_nl.as<double>(), s->v_img.as<double>(), h_val, h_flag,
+      s->dflag.as<int>());
   OV_LAUNCHED();
   OV_TRY_CUDA(cudaGetLastError());
-  // the values, then the flag, into pinned memory: one wait
-  const size_t vbytes = sizeof(double) * 6 * (size_t)cnt;
-  if (!R.h_vals.reserve(vbytes + 64)) return false;
-  int* h_flag = reinterpret_cast<int*>(R.h_vals.as<char>() + vbytes);
-  OV_TRY_CUDA(cudaMemcpyAsync(R.h_vals.p, R.pack.p, vbytes, cudaMemcpyDeviceToHost, s->stream));
-  OV_TRY_CUDA(cudaMemcpyAsync(h_flag, flag, sizeof(int), cudaMemcpyDeviceToHost, s->stream));
   OV_TRY_CUDA(cudaStreamSynchronize(s->stream));
-  V.hv.assign(R.h_vals.as<double>(), R.h_vals.as<double>() + 6 * (size_t)cnt);
-  return ov_flag_status(*h_flag, "update_velocity");
+  V.hv = h_val;
+  if (!*h_flag) return true;
+  int bits = 0;
+  OV_TRY_CUDA(cudaMemcpy(&bits, s->dflag.p, sizeof(int), cudaMemcpyDeviceToHost));
+  return ov_flag_status(bits, "update_velocity");
 }
 
 // the known list to the device (R.known), through pinned memory.  Every
@@ -518,7 +540,16 @@ bool compute_nodes(RecState& R, RecVel& V, const std::vector<int>& nodes, bool m
   ov_state_impl* s = &R.s;
   const int m = (int)nodes.size();
   if (m == 0) return true;
-  const int old = (int)V.known.size();
+  // the retired entries' places first
+  size_t live = 0;
+  for (size_t q = 0; q < V.known.size(); ++q) {
+    if (V.known[q] < 0) continue;
+    V.known[live] = V.known[q];
+    V.bound[live] = V.bound[q];
+    V.pos_of[V.known[q]] = (int)live++;
+  }
+  V.known.resize(live);
+  const int old = (int)live;
   for (int k : nodes) {
     V.pos_of[k] = (int)V.known.size();
     V.known.push_back(k);
@@ -532,7 +563,7 @@ bool compute_nodes(RecState& R, RecVel& V, const std::vector<int>& nodes, bool m
   OV_TRY_CUDA(cudaStreamSynchronize(s->stream));
   g_rec_stats.sums_s += secs_since(t0);
   g_rec_stats.nodes_summed += m;
-  return refresh_known(R, V);
+  return refresh_known(R, V, RecChange());
 }
 
 // Both nodes of a candidate again with FP64 sums on the current links (the
@@ -550,7 +581,7 @@ bool recheck_fp64(RecState& R, RecVel& V, int k, int l) {
   V.bound[V.pos_of[k]] = 0.0;
   V.bound[V.pos_of[l]] = 0.0;
   ++g_rec_stats.fp64_rechecks;
-  return refresh_known(R, V);
+  return refresh_known(R, V, RecChange());
 }
 
 }  // namespace
@@ -649,8 +680,8 @@ int ov_reconnect_vortices(struct tangle_state* tangle, double t, double rec_dist
     h_pwrap(tangle, tangle->vnodes[k].p, tangle->vnodes[l].p, w);
     for (int c = 0; c < 3; ++c) dx[c] = tangle->vnodes[k].p[c] - w[c];
     auto approach = [&](double& dot, double& scale) {
-      const double* hk = V.hv.data() + 6 * (size_t)V.pos_of[k];
-      const double* hl = V.hv.data() + 6 * (size_t)V.pos_of[l];
+      const double* hk = V.hv + 6 * (size_t)V.pos_of[k];
+      const double* hl = V.hv + 6 * (size_t)V.pos_of[l];
       dot = 0;
       double vk2 = 0, vl2 = 0;
       for (int c = 0; c < 3; ++c) {
@@ -674,8 +705,8 @@ int ov_reconnect_vortices(struct tangle_state* tangle, double t, double rec_dist
     // update_velocity of both nodes writes their vels and vs (as the
     // reference's does, src/vortex_dynamics.c:275-276)
     {
-      const double* hk = V.hv.data() + 6 * (size_t)V.pos_of[k];
-      const double* hl = V.hv.data() + 6 * (size_t)V.pos_of[l];
+      const double* hk = V.hv + 6 * (size_t)V.pos_of[k];
+      const double* hl = V.hv + 6 * (size_t)V.pos_of[l];
       for (int c = 0; c < 3; ++c) {
         tangle->vels[k].p[c] = hk[c];
         tangle->vs[k].p[c] = hk[3 + c];
@@ -693,15 +724,11 @@ int ov_reconnect_vortices(struct tangle_state* tangle, double t, double rec_dist
     old_fwd[0] = changed[0] == k ? knext : lnext;
     old_fwd[1] = changed[0] == k ? l : k;
     // the same links on the device
-    {
-      LinkPatch L;
-      for (int c = 0; c < 4; ++c) {
-        L.slot[c] = changed[c];
-        L.link[c] = make_int2(tangle->connections[changed[c]].forward, tangle->connections[changed[c]].reverse);
-      }
-      k_rec_patch_links<<<1, 32, 0, s->stream>>>(L, s->links.as<int2>(), s->n, s->dflag.as<int>());
-      OV_LAUNCHED();
-      if (!ov_cuda_ok(cudaGetLastError(), "k_rec_patch_links")) return -ov_last_error();
+    RecChange C;
+    C.n_links = 4;
+    for (int c = 0; c < 4; ++c) {
+      C.slot[c] = changed[c];
+      C.link[c] = make_int2(tangle->connections[changed[c]].forward, tangle->connections[changed[c]].reverse);
     }
     const int flag[10] = {k, tangle->connections[k].forward, tangle->connections[k].reverse, knext, kprev,
                           l, tangle->connections[l].forward, tangle->connections[l].reverse, lnext, lprev};
@@ -711,40 +738,22 @@ int ov_reconnect_vortices(struct tangle_state* tangle, double t, double rec_dist
     // nodes now flagged sit out the rest of the pass: no more velocities for
     // them (a node whose own links changed may even sit on a zero-length
     // segment, whose local term is not finite)
-    {
-      std::vector<int> keep;
-      std::vector<double> keep_bound;
-      keep.reserve(V.known.size());
-      keep_bound.reserve(V.known.size());
-      for (size_t q = 0; q < V.known.size(); ++q) {
-        const int x = V.known[q];
-        if (tangle->recalculate[x]) {
-          V.pos_of[x] = -3;   // retired
-        } else {
-          V.pos_of[x] = (int)keep.size();
-          keep.push_back(x);
-          keep_bound.push_back(V.bound[q]);
-        }
-      }
-      V.known.swap(keep);
-      V.bound.swap(keep_bound);
-      if (!upload_known(R, V)) return -ov_last_error();
+    for (int x : flag) {
+      const int q = V.pos_of[x];
+      if (q < 0) continue;
+      V.known[q] = -1;
+      V.pos_of[x] = -3;   // retired
+      C.retired[C.n_retired++] = q;
     }
     // every known node: the removed and added segments' fields
-    SegChange C;
-    C.m[0] = changed[0]; C.f[0] = old_fwd[0]; C.sign[0] = -1;
-    C.m[1] = changed[3]; C.f[1] = old_fwd[1]; C.sign[1] = -1;
-    C.m[2] = changed[0]; C.f[2] = tangle->connections[changed[0]].forward; C.sign[2] = 1;
-    C.m[3] = changed[3]; C.f[3] = tangle->connections[changed[3]].forward; C.sign[3] = 1;
-    const int cnt = (int)V.known.size();
-    if (cnt > 0 && !s->P.lia_only) {
-      k_rec_correct<<<(cnt + kCorrectWarps - 1) / kCorrectWarps, 32 * kCorrectWarps, 0, s->stream>>>(
-          s->P, C, R.known.as<int>(), cnt, s->n, s->pos.as<double>(), s->v_nl.as<double>(),
-          s->v_img.as<double>(), s->dflag.as<int>());
-      OV_LAUNCHED();
-      if (!ov_cuda_ok(cudaGetLastError(), "k_rec_correct")) return -ov_last_error();
+    if (!s->P.lia_only) {
+      C.n_seg = 4;
+      C.m[0] = changed[0]; C.f[0] = old_fwd[0]; C.sign[0] = -1;
+      C.m[1] = changed[3]; C.f[1] = old_fwd[1]; C.sign[1] = -1;
+      C.m[2] = changed[0]; C.f[2] = tangle->connections[changed[0]].forward; C.sign[2] = 1;
+      C.m[3] = changed[3]; C.f[3] = tangle->connections[changed[3]].forward; C.sign[3] = 1;
     }
-    if (!refresh_known(R, V)) return -ov_last_error();
+    if (!refresh_known(R, V, C)) return -ov_last_error();
   }
   if (!ov_cuda_ok(cudaStreamSynchronize(s->stream), "cudaStreamSynchronize")) return -ov_last_error();
   g_rec_stats.reconnections = nrecs;

@@ -447,6 +447,66 @@ def test_tree_sort_sizes_vs_oracle(ov, oracle, slots):
     st.close()
 
 
+@pytest.mark.parametrize("boundary", ["open", "periodic-6", "periodic-26"])
+def test_eval_points_counts_vs_oracle(ov, oracle, boundary):
+    """Direct sums at point counts around the widths of the blocks that add
+    the partial sums up (256 points a block with no images, 36 with six,
+    eight with 26), against the oracle."""
+    from openvort_b200.tangle import IMAGE_TABLES
+    t = G.random_ring_tangle(3, 8, 0.1, boundary=boundary, empty_slots=3)
+    p = Params(core_a=1e-8, dl_max=1e-3)
+    ov.configure(p, 0)
+    st = ov.DeviceState(t.copy())
+    for npts in (1, 7, 9, 35, 37, 255, 257):
+        pts = np.random.default_rng(npts).uniform(0, 0.1, size=(npts, 3))
+        want = oracle.segments_at(t, p, pts)
+        for sh, _ in IMAGE_TABLES[boundary]:
+            want = want + oracle.segments_at(t, p, pts - 0.1 * np.array(sh))
+        assert rel_err(st.eval_points(pts, method=0), want) < TOL_V64
+    st.close()
+
+
+@pytest.mark.parametrize("precision", [0, 1])
+@pytest.mark.parametrize("boundary", ["open", "periodic-26"])
+def test_reconnection_velocities_follow_the_links(ov, oracle, boundary, precision):
+    """The velocities a pass writes for the two nodes of each reconnection, at
+    its test, are those of the links the earlier reconnections left (the
+    oracle's update of the same tangle), for nodes whose tangent and normal
+    those did not touch."""
+    D = 0.05
+    p = Params(kappa=9.97e-4, core_a=1e-8, use_mf=1, alpha=0.1, alpha_p=0.01, dl_max=1e-3,
+               vn=Flow("simple", {"external_v": (0.1, 0.0, 0.0)}))
+    t = oracle.update_tangle(G.random_ring_tangle(17, 40, D, dl=D / 100, boundary=boundary), p)
+    lib = ov.load()
+    ov.configure(p, precision)
+    out = t.copy()
+    out.set_images_from_library(lib)
+    out.vels[:] = np.nan
+    out.recalc[:] = 0
+    pairs = np.zeros(2 * 100000, np.int32)
+    m = lib.ov_reconnect_candidates(out.ptr(), 2.5 * D / 100, 0.087, pairs.ctypes.data, 100000)
+    assert lib.ov_reconnect_vortices(out.ptr(), 0.0, 2.5 * D / 100, 0.087) > 3
+    cand = pairs[:2 * m].reshape(-1, 2)
+    # reconnections: pairs joined by the pass, in the order of k
+    joined = [(int(k), int(l)) for k, l in cand if l in out.links[k] and l not in t.links[k]]
+    compared = 0
+    now = t.copy()
+    for i, (k, l) in enumerate(joined):
+        if i < 40:
+            want = oracle.update_tangle(now, p)
+            at = [x for x in (k, l) if np.array_equal(want.tangents[x], t.tangents[x])
+                  and np.array_equal(want.normals[x], t.normals[x])]
+            compared += len(at)
+            if at:
+                assert rel_err(out.vels[at], want.vels[at]) < (TOL_V64 if precision == 0 else TOL_MIXED)
+        a, b = (k, l) if out.links[k, 0] == l else (l, k)   # a runs to b from now on
+        after_a, before_b = now.links[a, 0], now.links[b, 1]
+        now.links[a, 0], now.links[b, 1] = b, a
+        now.links[before_b, 0], now.links[after_a, 1] = after_a, before_b
+    assert np.array_equal(now.links, out.links)
+    assert compared > 10
+
+
 @pytest.mark.parametrize("boundary", ["open", "periodic-26", "periodic-z-open-xy"])
 @pytest.mark.parametrize("rings,grain", [(1, 1e-8), (12, 1e-8), (40, 3e-3)])
 def test_split_walk_vs_oracle(ov, oracle, boundary, rings, grain):
