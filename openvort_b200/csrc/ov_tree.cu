@@ -164,7 +164,7 @@ __global__ void k_keys(OvParams P, const double* __restrict__ pos, const int2* _
 // rank within the warp, keep the order stable with two block barriers.
 // With more than kRsFused tiles each block would read too many counts; the
 // offsets then come from three scan launches.  Tiles of 1024 keys up to 256k
-// keys, so a small sort fills the GPU: 22.4k keys take 4 + 3 us a pass on the
+// keys, so a small sort fills the GPU: 22.4k keys take 8 + 5 us a pass on the
 // device, against 22 + 10 with 4096-key tiles ranked 256 at a time and 9 more
 // for the scans.
 constexpr int kRsThreads = 256;
