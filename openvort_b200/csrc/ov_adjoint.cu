@@ -464,9 +464,8 @@ LocalP local_params(const OvParams& P) {
 // velocities at positions x (3n doubles, device) into v
 bool velocity_at(ov_adjoint* a, const double* x, double t, double* v) {
   ov_state_impl* s = &a->s;
-  return ov_geometry(s, x, a->tmp_dxi.as<double>(), a->tmp_tan.as<double>(), a->tmp_nrm.as<double>()) &&
-         ov_velocities(s, t, x, a->tmp_dxi.as<double>(), a->tmp_tan.as<double>(), a->tmp_nrm.as<double>(), v,
-                       a->tmp_vs.as<double>(), nullptr);
+  return ov_evaluate(s, t, x, a->tmp_dxi.as<double>(), a->tmp_tan.as<double>(), a->tmp_nrm.as<double>(), v,
+                     a->tmp_vs.as<double>(), kNoStage);
 }
 
 // nonlocal sums at positions x into vnl

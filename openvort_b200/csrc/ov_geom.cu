@@ -40,45 +40,13 @@ __global__ void k_tangents(OvParams P, Links L, const double* __restrict__ pos,
   st3(nrm, k, nn);
 }
 
-// dxi, tangents and normals of every slot in one launch: a node's stencil
-// takes the segment lengths it needs from the positions, in dxi_node's
-// operations, instead of waiting for a pass over dxi.  A node next to a pinned
-// one reads its neighbours' tangents and is left to k_tangents (pass 1).
+// dxi, tangents and normals of every slot in one launch (geometry_slot).
 // Bound by launches up to ~100k nodes and by HBM above: 1M nodes 54 us,
 // against 93 us in three launches.
 __global__ void __launch_bounds__(kThreads) k_geometry(OvParams P, Links L, const double* __restrict__ pos,
-                                                       double* dxi, double* tan, double* nrm, int n, int* flag) {
+                                                       OvGeomOut G, int n) {
   const int k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= n) return;
-  const int2 st = L.st[k];
-  if (st.x == OV_EMPTY) return;
-  const int2 lk = L.lk[k];
-  d3 t, nn;
-  if (st.x == OV_FREE && lk.x >= 0 && lk.y >= 0) {
-    const int ff = L.lk[lk.x].x, rr = L.lk[lk.y].y;
-    if (ff >= 0 && rr >= 0 && L.st[lk.x].x != OV_PINNED && L.st[lk.y].x != OV_PINNED) {
-      const d3 s0 = ld3(pos, k);
-      const d3 p[4] = {ld3(pos, ff), ld3(pos, lk.x), ld3(pos, lk.y), ld3(pos, rr)};
-      const double d0 = norm_ref(s0 - pwrap(P, s0, p[1])), d1 = norm_ref(p[1] - pwrap(P, p[1], p[0]));
-      const double dm1 = norm_ref(p[2] - pwrap(P, p[2], s0)), dm2 = norm_ref(p[3] - pwrap(P, p[3], p[2]));
-      const double x[4] = {d0 + d1, d0, -dm1, -(dm1 + dm2)};
-      stencil4(P, s0, p, x, t, nn);
-      dxi[k] = d0;
-      st3(tan, k, t);
-      st3(nrm, k, nn);
-      return;
-    }
-  }
-  double d;
-  if (!dxi_node(P, L, pos, k, d)) { atomicOr(flag, 1); return; }
-  dxi[k] = d;
-  if (near_pinned(L, k)) return;
-  auto arc = [&](int kk, int dist, double& out) {
-    return arc_length_of(L, [&](int i, double& l) { return dxi_node(P, L, pos, i, l); }, kk, dist, out);
-  };
-  if (!tangent_node(P, L, pos, k, arc, tan, t, nn)) { atomicOr(flag, 1); return; }
-  st3(tan, k, t);
-  st3(nrm, k, nn);
+  if (k < n) geometry_slot(P, L, pos, k, G);
 }
 
 // velocity assembly per node (update_velocity, src/tangle.c:583-684) from
@@ -152,7 +120,7 @@ bool ov_launch_geometry(cudaStream_t st, const OvParams& P, const int2* links, c
                         const double* pos, double* dxi, double* tan, double* nrm, int n, bool pinned, int* flag) {
   if (n <= 0) return true;
   Links L{links, status};
-  k_geometry<<<blocks_for(n), kThreads, 0, st>>>(P, L, pos, dxi, tan, nrm, n, flag);
+  k_geometry<<<blocks_for(n), kThreads, 0, st>>>(P, L, pos, OvGeomOut{dxi, tan, nrm, flag}, n);
   OV_LAUNCHED();
   if (pinned) {
     k_tangents<<<blocks_for(n), kThreads, 0, st>>>(P, L, pos, dxi, tan, nrm, nullptr, n, 1, flag);
@@ -185,15 +153,6 @@ bool ov_launch_epilogue(cudaStream_t st, const OvParams& P, const int2* links, c
   Links L{links, status};
   k_epilogue<<<blocks_for(k1 - k0), kThreads, 0, st>>>(P, L, t_dev, t0, pos, tan, nrm, sums, n_slots, stage, vels, vs,
                                                          k0, k1, flag);
-  OV_LAUNCHED();
-  OV_TRY_CUDA(cudaGetLastError());
-  return true;
-}
-
-bool ov_launch_euler(cudaStream_t st, const int2* status, const double* x0, const double* v,
-                     double h, double* xs, int n) {
-  if (n <= 0) return true;
-  k_euler<<<blocks_for(n), kThreads, 0, st>>>(status, x0, v, h, xs, n);
   OV_LAUNCHED();
   OV_TRY_CUDA(cudaGetLastError());
   return true;
@@ -304,10 +263,8 @@ bool ov_rk4(ov_state_impl* s, double t, double dt, int classic, bool have_stage1
   double* xs[3] = {s->spos.as<double>(), s->pos0.as<double>(), s->spos.as<double>()};
   if (!have_stage1 && !ov_rk4_stage_positions(s, 1, dt, classic)) return false;
   for (int q = 0; q < 3; ++q) {
-    if (!ov_geometry(s, xs[q], s->sdxi.as<double>(), s->stan.as<double>(), s->snrm.as<double>()))
-      return false;
-    if (!ov_velocities(s, ts[q], xs[q], s->sdxi.as<double>(), s->stan.as<double>(), s->snrm.as<double>(), ks[q],
-                       s->svs.as<double>(), nullptr, q < 2 ? OvStage{x0, h[q + 1], xs[q + 1]} : kNoStage))
+    if (!ov_evaluate(s, ts[q], xs[q], s->sdxi.as<double>(), s->stan.as<double>(), s->snrm.as<double>(), ks[q],
+                     s->svs.as<double>(), q < 2 ? OvStage{x0, h[q + 1], xs[q + 1]} : kNoStage))
       return false;
   }
   return ov_rk4_combine(s, dt);

@@ -117,6 +117,13 @@ struct OvSums {
   const double* part;
   int splits;
 };
+// where a kernel stores the geometry of the nodes (dxi null: nowhere)
+struct OvGeomOut {
+  double *dxi, *tan, *nrm;
+  int* flag;
+};
+constexpr OvGeomOut kNoGeom = {nullptr, nullptr, nullptr, nullptr};
+
 // the stage that follows an evaluation: xs = x0 + h v (xs null: none; xs must
 // not be the positions the evaluation reads)
 struct OvStage {
@@ -210,6 +217,9 @@ bool ov_geometry(ov_state_impl* s, const double* pos, double* dxi, double* tan, 
 bool ov_velocities(ov_state_impl* s, double t, const double* pos, const double* dxi,
                    const double* tan, const double* nrm, double* vels, double* vs,
                    OvTree* external_tree, const OvStage& stage = kNoStage);
+// both, at positions pos
+bool ov_evaluate(ov_state_impl* s, double t, const double* pos, double* dxi, double* tan, double* nrm, double* vels,
+                 double* vs, const OvStage& stage);
 // one RK4 step on the state's pos using the state's vels as k1 (have_stage1:
 // the evaluation of vels has already formed the first stage's positions, as
 // ov_rk4_first's stage).  After an error (the flag set) the positions stay.
@@ -247,8 +257,10 @@ bool ov_radix_sort_u64(uint64_t* ka, int* va, uint64_t* kb, int* vb, int n, int 
                        DevBuf& scan_part, cudaStream_t st);
 // direct sums for all nodes -> v_nl, v_img
 bool ov_direct_nodes(ov_state_impl* s, const double* pos, double* v_nl, double* v_img);
-// the same left as partials (in s->img_part) for the epilogue to add up
-bool ov_direct_partials(ov_state_impl* s, const double* pos, double* v_nl, double* v_img, OvSums* out);
+// the same left as partials (in s->img_part) for the epilogue to add up, and
+// the geometry of every slot where asked for (no pinned nodes)
+bool ov_direct_partials(ov_state_impl* s, const double* pos, double* v_nl, double* v_img, const OvGeomOut& geom,
+                        OvSums* out);
 // direct sums at arbitrary points (device arrays), sources = all segments or
 // the slot list `only`: out_nl = the tangle's own sum, out_img = image sum
 // (nullptr: no images)
@@ -264,9 +276,6 @@ bool ov_direct_points_scratch(cudaStream_t st, const OvParams& P, const double* 
                               const int2* links, const int2* status, int n, int npts,
                               const double* pts, const int* skip, double* seg, int* fwd,
                               double* part, double* out, double* img);
-// s->seg64 / s->segid: r1 and the wrapped r2 of every slot's forward
-// segment at positions pos, and the forward slot (-1: no segment)
-bool ov_segment_table(ov_state_impl* s, const double* pos);
 // out = a + b for n vectors of 3 doubles (device)
 bool ov_add3(cudaStream_t st, const double* a, const double* b, double* out, int n);
 
@@ -295,8 +304,6 @@ bool ov_launch_epilogue(cudaStream_t st, const OvParams& P, const int2* links, c
                         const double* t_dev, double t0, const double* pos, const double* tan,
                         const double* nrm, const OvSums& sums, int n_slots, const OvStage& stage, double* vels,
                         double* vs, int k0, int k1, int* flag);
-bool ov_launch_euler(cudaStream_t st, const int2* status, const double* x0, const double* v,
-                     double h, double* xs, int n);
 // flag given: nothing happens when it is set
 bool ov_launch_rk4_combine(cudaStream_t st, const int2* status, const double* k1, const double* k2,
                            const double* k3, const double* k4, double dt, double* x, int n,

@@ -102,6 +102,43 @@ __device__ bool tangent_node(const OvParams& P, const Links& L, const double* po
   return ok;
 }
 
+// dxi, tangent and normal of slot k: its stencil takes the segment lengths it
+// needs from the positions, in dxi_node's operations, instead of waiting for
+// a pass over dxi.  A node next to a pinned one reads its neighbours' tangents
+// and is left to k_tangents (pass 1, ov_geom.cu).
+__device__ __forceinline__ void geometry_slot(const OvParams& P, const Links& L, const double* __restrict__ pos, int k,
+                                              const OvGeomOut& G) {
+  const int2 st = L.st[k];
+  if (st.x == OV_EMPTY) return;
+  const int2 lk = L.lk[k];
+  d3 t, nn;
+  if (st.x == OV_FREE && lk.x >= 0 && lk.y >= 0) {
+    const int ff = L.lk[lk.x].x, rr = L.lk[lk.y].y;
+    if (ff >= 0 && rr >= 0 && L.st[lk.x].x != OV_PINNED && L.st[lk.y].x != OV_PINNED) {
+      const d3 s0 = ld3(pos, k);
+      const d3 p[4] = {ld3(pos, ff), ld3(pos, lk.x), ld3(pos, lk.y), ld3(pos, rr)};
+      const double d0 = norm_ref(s0 - pwrap(P, s0, p[1])), d1 = norm_ref(p[1] - pwrap(P, p[1], p[0]));
+      const double dm1 = norm_ref(p[2] - pwrap(P, p[2], s0)), dm2 = norm_ref(p[3] - pwrap(P, p[3], p[2]));
+      const double x[4] = {d0 + d1, d0, -dm1, -(dm1 + dm2)};
+      stencil4(P, s0, p, x, t, nn);
+      G.dxi[k] = d0;
+      st3(G.tan, k, t);
+      st3(G.nrm, k, nn);
+      return;
+    }
+  }
+  double d;
+  if (!dxi_node(P, L, pos, k, d)) { atomicOr(G.flag, 1); return; }
+  G.dxi[k] = d;
+  if (near_pinned(L, k)) return;
+  auto arc = [&](int kk, int dist, double& out) {
+    return arc_length_of(L, [&](int i, double& l) { return dxi_node(P, L, pos, i, l); }, kk, dist, out);
+  };
+  if (!tangent_node(P, L, pos, k, arc, G.tan, t, nn)) { atomicOr(G.flag, 1); return; }
+  st3(G.tan, k, t);
+  st3(G.nrm, k, nn);
+}
+
 // The direct sum's partials of target k for image j (0: the tangle itself),
 // with source splits added split by split, in order; mirror images reflect
 // their velocity (src/tangle.c:633-634).
