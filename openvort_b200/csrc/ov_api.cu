@@ -669,8 +669,9 @@ static bool bs_sums(ov_state_impl* s, const double* pos, OvTree* external_tree, 
 
 // The epilogue of an evaluation over every node.
 static bool finish_velocities(ov_state_impl* s, double t, const double* pos, const double* tan,
-                              const double* nrm, const OvStage& stage, double* vels, double* vs) {
-  if (!ov_epilogue(s, t, pos, tan, nrm, s->sums, stage, vels, vs, 0, s->n)) return false;
+                              const double* nrm, const OvStage& stage, double* vels, double* vs,
+                              bool early = false) {
+  if (!ov_epilogue(s, t, pos, tan, nrm, s->sums, stage, vels, vs, 0, s->n, early)) return false;
   ++s->pending;
   return true;
 }
@@ -684,13 +685,14 @@ bool ov_velocities(ov_state_impl* s, double t, const double* pos, const double* 
 
 // The geometry goes along with a small direct sum, which reads only the
 // positions: an RK4 step of a 256-node ring 78 us, against 99 with a launch of
-// its own.  Not with pinned nodes, which take a second pass.
+// its own.  Not with pinned nodes, which take a second pass.  The epilogue
+// follows early: 65 us.
 bool ov_evaluate(ov_state_impl* s, double t, const double* pos, double* dxi, double* tan, double* nrm, double* vels,
                  double* vs, const OvStage& stage) {
   const bool along = small_sum(s) && !s->P.lia_only && s->n_active > 0 && s->n_active == s->n_targets;
   if (!along && !ov_geometry(s, pos, dxi, tan, nrm)) return false;
   return bs_sums(s, pos, nullptr, 0, -1, along ? OvGeomOut{dxi, tan, nrm, s->dflag.as<int>()} : kNoGeom) &&
-         finish_velocities(s, t, pos, tan, nrm, stage, vels, vs);
+         finish_velocities(s, t, pos, tan, nrm, stage, vels, vs, along);
 }
 
 // ======================================================================

@@ -137,6 +137,7 @@ __global__ void __launch_bounds__(kTB) k_direct64_chain(OvParams P, int n_src, c
                                                         const int* __restrict__ tskip, int n_t,
                                                         double* __restrict__ part, int chunk, OvGeomOut G) {
   if constexpr (kGeom) {
+    follow_early();
     // one z beyond the source splits: the slots' geometry
     if (blockIdx.z == gridDim.z - 1) {
       const int k = blockIdx.x * kTB + threadIdx.x;
@@ -796,10 +797,15 @@ bool ov_direct_partials(ov_state_impl* s, const double* pos, double* v_nl, doubl
     const int chunk = source_chunk(s->n, (long long)bx * (nimg + 1), 32, &splits, 4, 64, res64);
     if (!s->img_part.reserve(sizeof(double) * 3 * (size_t)s->n * (nimg + 1) * splits)) return false;
     ov_mark(s, s->ev1);
-    auto kernel = geom.dxi ? k_direct64_chain<false, true> : k_direct64_chain<false>;
-    kernel<<<dim3(bx, nimg + 1, splits + (geom.dxi ? 1 : 0)), kTB, 0, s->stream>>>(
-        s->P, s->n, pos, s->links.as<int2>(), s->status.as<int2>(), nullptr, nullptr, s->n, s->img_part.as<double>(),
-        chunk, geom);
+    const dim3 grid(bx, nimg + 1, splits);
+    if (geom.dxi)
+      OV_TRY_CUDA(ov_launch_early(k_direct64_chain<false, true>, dim3(grid.x, grid.y, splits + 1), kTB, s->stream, s->P,
+                                  s->n, pos, s->links.as<int2>(), s->status.as<int2>(), nullptr, nullptr, s->n,
+                                  s->img_part.as<double>(), chunk, geom));
+    else
+      k_direct64_chain<false><<<grid, kTB, 0, s->stream>>>(s->P, s->n, pos, s->links.as<int2>(), s->status.as<int2>(),
+                                                           nullptr, nullptr, s->n, s->img_part.as<double>(), chunk,
+                                                           geom);
     OV_LAUNCHED();
     OV_TRY_CUDA(cudaGetLastError());
   }

@@ -59,6 +59,7 @@ __global__ void k_epilogue(OvParams P, Links L, const double* __restrict__ t_dev
                            const double* __restrict__ pos, const double* __restrict__ tan,
                            const double* __restrict__ nrm, OvSums S, int n_slots, OvStage G, double* vels,
                            double* vs_out, int k0, int k1, int* flag) {
+  follow_early();
   const int k = k0 + blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= k1) return;
   const double t = t_dev ? t0 + *t_dev : t0;
@@ -95,6 +96,7 @@ __global__ void k_rk4_combine(const int2* __restrict__ st, const double* __restr
                               const double* __restrict__ k2, const double* __restrict__ k3,
                               const double* __restrict__ k4, double dt, double* x, int n,
                               const int* __restrict__ flag) {
+  follow_early();
   int k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= n || st[k].x == OV_EMPTY || (flag && *flag)) return;
 #pragma unroll
@@ -148,20 +150,29 @@ bool ov_launch_geometry_list(cudaStream_t st, const OvParams& P, const int2* lin
 bool ov_launch_epilogue(cudaStream_t st, const OvParams& P, const int2* links, const int2* status,
                         const double* t_dev, double t0, const double* pos, const double* tan,
                         const double* nrm, const OvSums& sums, int n_slots, const OvStage& stage, double* vels,
-                        double* vs, int k0, int k1, int* flag) {
+                        double* vs, int k0, int k1, int* flag, bool early) {
   if (k1 <= k0) return true;
   Links L{links, status};
-  k_epilogue<<<blocks_for(k1 - k0), kThreads, 0, st>>>(P, L, t_dev, t0, pos, tan, nrm, sums, n_slots, stage, vels, vs,
-                                                         k0, k1, flag);
+  if (early)
+    OV_TRY_CUDA(ov_launch_early(k_epilogue, dim3(blocks_for(k1 - k0)), kThreads, st, P, L, t_dev, t0, pos, tan, nrm,
+                                sums, n_slots, stage, vels, vs, k0, k1, flag));
+  else
+    k_epilogue<<<blocks_for(k1 - k0), kThreads, 0, st>>>(P, L, t_dev, t0, pos, tan, nrm, sums, n_slots, stage, vels, vs,
+                                                           k0, k1, flag);
   OV_LAUNCHED();
   OV_TRY_CUDA(cudaGetLastError());
   return true;
 }
 
 bool ov_launch_rk4_combine(cudaStream_t st, const int2* status, const double* k1, const double* k2,
-                           const double* k3, const double* k4, double dt, double* x, int n, const int* flag) {
+                           const double* k3, const double* k4, double dt, double* x, int n, const int* flag,
+                           bool early) {
   if (n <= 0) return true;
-  k_rk4_combine<<<blocks_for(n), kThreads, 0, st>>>(status, k1, k2, k3, k4, dt, x, n, flag);
+  if (early)
+    OV_TRY_CUDA(ov_launch_early(k_rk4_combine, dim3(blocks_for(n)), kThreads, st, status, k1, k2, k3, k4, dt, x, n,
+                                flag));
+  else
+    k_rk4_combine<<<blocks_for(n), kThreads, 0, st>>>(status, k1, k2, k3, k4, dt, x, n, flag);
   OV_LAUNCHED();
   OV_TRY_CUDA(cudaGetLastError());
   return true;
@@ -191,10 +202,10 @@ bool ov_geometry(ov_state_impl* s, const double* pos, double* dxi, double* tan, 
 
 bool ov_epilogue(ov_state_impl* s, double t, const double* pos, const double* tan,
                  const double* nrm, const OvSums& sums, const OvStage& stage, double* vels,
-                 double* vs, int k0, int k1) {
+                 double* vs, int k0, int k1, bool early) {
   if (k1 <= k0) return true;
   return ov_launch_epilogue(s->stream, s->P, s->links.as<int2>(), s->status.as<int2>(), nullptr, t, pos, tan, nrm,
-                            sums, s->n, stage, vels, vs, k0, k1, s->dflag.as<int>());
+                            sums, s->n, stage, vels, vs, k0, k1, s->dflag.as<int>(), early);
 }
 
 bool ov_euler(ov_state_impl* s, double dt) {
@@ -242,7 +253,7 @@ bool ov_rk4_combine(ov_state_impl* s, double dt) {
   if (s->n == 0) return true;
   return ov_launch_rk4_combine(s->stream, s->status.as<int2>(), s->vels.as<double>(), s->k2.as<double>(),
                                s->k3.as<double>(), s->k4.as<double>(), dt, s->pos.as<double>(), s->n,
-                               s->dflag.as<int>());
+                               s->dflag.as<int>(), true);
 }
 
 bool ov_rk4_first(ov_state_impl* s, double dt, OvStage* stage) {

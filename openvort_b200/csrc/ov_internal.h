@@ -3,6 +3,8 @@
 // error channel and the kernel launchers.
 #pragma once
 
+#include <utility>
+
 #include <cuda_runtime.h>
 #include <stddef.h>
 #include <stdint.h>
@@ -283,7 +285,7 @@ bool ov_add3(cudaStream_t st, const double* a, const double* b, double* out, int
 // friction for slots k0 <= k < k1, and the following stage's positions
 bool ov_epilogue(ov_state_impl* s, double t, const double* pos, const double* tan,
                  const double* nrm, const OvSums& sums, const OvStage& stage,
-                 double* vels, double* vs, int k0, int k1);
+                 double* vels, double* vs, int k0, int k1, bool early = false);
 
 bool ov_state_reserve(ov_state_impl* s, int n);
 
@@ -299,15 +301,16 @@ bool ov_launch_geometry(cudaStream_t st, const OvParams& P, const int2* links, c
 bool ov_launch_geometry_list(cudaStream_t st, const OvParams& P, const int2* links, const int2* status,
                              const double* pos, double* dxi, double* tan, double* nrm, const int* idx, int n,
                              int* flag);
-// epilogue at time t0 + *t_dev (t_dev may be null: time t0)
+// epilogue at time t0 + *t_dev (t_dev may be null: time t0); early: by
+// ov_launch_early (not while the stream is captured)
 bool ov_launch_epilogue(cudaStream_t st, const OvParams& P, const int2* links, const int2* status,
                         const double* t_dev, double t0, const double* pos, const double* tan,
                         const double* nrm, const OvSums& sums, int n_slots, const OvStage& stage, double* vels,
-                        double* vs, int k0, int k1, int* flag);
+                        double* vs, int k0, int k1, int* flag, bool early = false);
 // flag given: nothing happens when it is set
 bool ov_launch_rk4_combine(cudaStream_t st, const int2* status, const double* k1, const double* k2,
                            const double* k3, const double* k4, double dt, double* x, int n,
-                           const int* flag = nullptr);
+                           const int* flag = nullptr, bool early = false);
 // error for flag bits h (false and the error set when any bit is set)
 bool ov_flag_status(int h, const char* where);
 
@@ -327,3 +330,30 @@ OvStatsAcc& ov_stats_tls();
 void ov_note_launch(int n);
 long long ov_launches();
 #define OV_LAUNCHED() ov_note_launch(1)
+
+#ifdef __CUDACC__
+// Launches a kernel that begins with follow_early(): its blocks may take
+// their places while the kernel before it in the stream still runs, and wait
+// there for its end, so the launch itself costs nothing between the two.  For
+// kernels of a few microseconds.
+template <class... P, class... A>
+inline cudaError_t ov_launch_early(void (*kernel)(P...), dim3 grid, int block, cudaStream_t st, A&&... args) {
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t c{};
+  c.gridDim = grid;
+  c.blockDim = dim3(block);
+  c.stream = st;
+  c.attrs = &at;
+  c.numAttrs = 1;
+  return cudaLaunchKernelEx(&c, kernel, std::forward<A>(args)...);
+}
+// Waits for the kernel before (all its writes are then visible) and lets the
+// one after take its places; first in the kernel, before any access to
+// memory.  Nothing happens where the launches are ordinary ones.
+__device__ __forceinline__ void follow_early() {
+  cudaGridDependencySynchronize();
+  cudaTriggerProgrammaticLaunchCompletion();
+}
+#endif
