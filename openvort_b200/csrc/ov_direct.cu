@@ -130,12 +130,12 @@ constexpr int kCS = 128;   // chained segments per shared-memory tile
 static_assert(kCS == kTS, "the chain sweep splits sources as k_direct64 does");
 
 template <bool kPoints, bool kGeom = false>
-__global__ void __launch_bounds__(kTB) k_direct64_chain(OvParams P, int n_src, const double* __restrict__ pos,
-                                                        const int2* __restrict__ links,
-                                                        const int2* __restrict__ status,
-                                                        const double* __restrict__ tpos,
-                                                        const int* __restrict__ tskip, int n_t,
-                                                        double* __restrict__ part, int chunk, OvGeomOut G) {
+__global__ void __launch_bounds__(kTB) k_direct64_chain(OvParams P, int n_src, const double* pos,
+                                                        const int2* links,
+                                                        const int2* status,
+                                                        const double* tpos,
+                                                        const int* tskip, int n_t,
+                                                        double* part, int chunk, OvGeomOut G) {
   if constexpr (kGeom) {
     follow_early();
     // one z beyond the source splits: the slots' geometry

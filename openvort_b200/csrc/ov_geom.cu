@@ -55,9 +55,9 @@ __global__ void __launch_bounds__(kThreads) k_geometry(OvParams P, Links L, cons
 // saved), and, when a stage follows, the node's position in it
 // (x0 + h v: euler_step2, src/vortex_dynamics.c:36-52)
 // time = t0 + (*t_dev when given: a graph replayed at advancing times)
-__global__ void k_epilogue(OvParams P, Links L, const double* __restrict__ t_dev, double t0,
-                           const double* __restrict__ pos, const double* __restrict__ tan,
-                           const double* __restrict__ nrm, OvSums S, int n_slots, OvStage G, double* vels,
+__global__ void k_epilogue(OvParams P, Links L, const double* t_dev, double t0,
+                           const double* pos, const double* tan,
+                           const double* nrm, OvSums S, int n_slots, OvStage G, double* vels,
                            double* vs_out, int k0, int k1, int* flag) {
   follow_early();
   const int k = k0 + blockIdx.x * blockDim.x + threadIdx.x;
@@ -92,10 +92,10 @@ __global__ void k_euler(const int2* __restrict__ st, const double* __restrict__ 
 }
 
 // x += dt/6 k1 + dt/3 k2 + dt/3 k3 + dt/6 k4 (src/vortex_dynamics.c:94-112)
-__global__ void k_rk4_combine(const int2* __restrict__ st, const double* __restrict__ k1,
-                              const double* __restrict__ k2, const double* __restrict__ k3,
-                              const double* __restrict__ k4, double dt, double* x, int n,
-                              const int* __restrict__ flag) {
+__global__ void k_rk4_combine(const int2* st, const double* k1,
+                              const double* k2, const double* k3,
+                              const double* k4, double dt, double* x, int n,
+                              const int* flag) {
   follow_early();
   int k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= n || st[k].x == OV_EMPTY || (flag && *flag)) return;

@@ -334,7 +334,8 @@ long long ov_launches();
 #ifdef __CUDACC__
 // Launches a kernel that begins with follow_early(): its blocks may take
 // their places while the kernel before it in the stream still runs, and wait
-// there for its end, so the launch itself costs nothing between the two.  For
+// there for its end, so the launch itself costs nothing between the two (a tree
+// build of 22.4k nodes, 27 launches: 0.231 ms, 0.176 so).  For
 // kernels of a few microseconds.
 template <class... P, class... A>
 inline cudaError_t ov_launch_early(void (*kernel)(P...), dim3 grid, int block, cudaStream_t st, A&&... args) {
@@ -351,7 +352,9 @@ inline cudaError_t ov_launch_early(void (*kernel)(P...), dim3 grid, int block, c
 }
 // Waits for the kernel before (all its writes are then visible) and lets the
 // one after take its places; first in the kernel, before any access to
-// memory.  Nothing happens where the launches are ordinary ones.
+// memory.  Such a kernel's pointers are not __restrict__: what the kernel
+// before writes is not constant while this one runs, and no load may be taken
+// ahead of the wait.  Nothing happens where the launches are ordinary ones.
 __device__ __forceinline__ void follow_early() {
   cudaGridDependencySynchronize();
   cudaTriggerProgrammaticLaunchCompletion();

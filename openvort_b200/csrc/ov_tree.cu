@@ -93,8 +93,9 @@ __device__ __forceinline__ void set_digit(uint64_t& hi, uint64_t& lo, int level,
 }
 
 // ---------------------------------------------------------------- 1. keys
-__global__ void k_keys(OvParams P, const double* __restrict__ pos, const int2* __restrict__ status,
+__global__ void k_keys(OvParams P, const double* pos, const int2* status,
                        int n, uint64_t* khi, uint64_t* klo, int* vals, int* term, int* counters, int* flag) {
+  follow_early();
   int k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= n) return;
   vals[k] = k;
@@ -173,8 +174,9 @@ constexpr int kRsFused = 256;
 constexpr int kRsSmall = 4, kRsLarge = 16;   // keys per thread
 
 template <int kItems>
-__global__ void __launch_bounds__(kRsThreads) k_rs_hist(const uint64_t* __restrict__ keys, int n, int shift,
+__global__ void __launch_bounds__(kRsThreads) k_rs_hist(const uint64_t* keys, int n, int shift,
                                                         unsigned* hist) {
+  follow_early();
   __shared__ unsigned h[256];
   h[threadIdx.x] = 0;
   __syncthreads();
@@ -189,17 +191,19 @@ __global__ void __launch_bounds__(kRsThreads) k_rs_hist(const uint64_t* __restri
 }
 
 // digit-major copy of the counts for the scans of a large sort
-__global__ void k_rs_transpose(const unsigned* __restrict__ hist, int tiles, unsigned* out) {
+__global__ void k_rs_transpose(const unsigned* hist, int tiles, unsigned* out) {
+  follow_early();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= 256 * tiles) return;
   out[(size_t)(i & 255) * tiles + (i >> 8)] = hist[i];
 }
 
 template <int kItems, bool kScanned>
-__global__ void __launch_bounds__(kRsThreads) k_rs_scatter(const uint64_t* __restrict__ kin,
-                                                           const int* __restrict__ vin, uint64_t* kout, int* vout,
-                                                           int n, int shift, const unsigned* __restrict__ hist,
+__global__ void __launch_bounds__(kRsThreads) k_rs_scatter(const uint64_t* kin,
+                                                           const int* vin, uint64_t* kout, int* vout,
+                                                           int n, int shift, const unsigned* hist,
                                                            int tiles) {
+  follow_early();
   __shared__ unsigned wcnt[kRsWarps][256];
   __shared__ unsigned offs[256];
   __shared__ unsigned wsum[kRsWarps];
@@ -310,8 +314,9 @@ __device__ __forceinline__ unsigned block_excl_scan(unsigned x, unsigned* sh, un
   return r;
 }
 
-__global__ void __launch_bounds__(kScanThreads) k_scan_sums(const unsigned* __restrict__ v, int m,
+__global__ void __launch_bounds__(kScanThreads) k_scan_sums(const unsigned* v, int m,
                                                             unsigned* sums) {
+  follow_early();
   __shared__ unsigned sh[33];
   const int i = blockIdx.x * kScanThreads + threadIdx.x;
   unsigned tot;
@@ -321,6 +326,7 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_sums(const unsigned* __re
 
 // one block: exclusive scan of nb block sums, 1024 at a time with a carry
 __global__ void __launch_bounds__(kScanThreads) k_scan_top(unsigned* sums, int nb) {
+  follow_early();
   __shared__ unsigned sh[33];
   unsigned carry = 0;
   for (int b0 = 0; b0 < nb; b0 += kScanThreads) {
@@ -333,7 +339,8 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_top(unsigned* sums, int n
 }
 
 __global__ void __launch_bounds__(kScanThreads) k_scan_apply(unsigned* v, int m,
-                                                             const unsigned* __restrict__ sums) {
+                                                             const unsigned* sums) {
+  follow_early();
   __shared__ unsigned sh[33];
   const int i = blockIdx.x * kScanThreads + threadIdx.x;
   const unsigned x = i < m ? v[i] : 0u;
@@ -343,8 +350,9 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_apply(unsigned* v, int m,
 }
 
 // gather the low key words and termination codes into sorted order
-__global__ void k_gather_lo(const int* __restrict__ perm, const uint64_t* __restrict__ klo_slot,
-                            const int* __restrict__ term_slot, uint64_t* klo, int* term, int n) {
+__global__ void k_gather_lo(const int* perm, const uint64_t* klo_slot,
+                            const int* term_slot, uint64_t* klo, int* term, int n) {
+  follow_early();
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   int s = perm[i];
@@ -354,8 +362,9 @@ __global__ void k_gather_lo(const int* __restrict__ perm, const uint64_t* __rest
 
 // order runs of equal high words by the low word (insertion sort; runs are
 // nodes closer than 2^-16 of the box, essentially always length 1)
-__global__ void k_fix_ties(const uint64_t* __restrict__ khi, uint64_t* klo, int* perm, int* term,
+__global__ void k_fix_ties(const uint64_t* khi, uint64_t* klo, int* perm, int* term,
                            int n) {
+  follow_early();
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   if (i > 0 && khi[i - 1] == khi[i]) return;
@@ -395,8 +404,9 @@ __device__ __forceinline__ int kdelta(const uint64_t* hi, const uint64_t* lo, in
   return 128 + __clz(i ^ j);
 }
 
-__global__ void k_karras(const uint64_t* __restrict__ hi, const uint64_t* __restrict__ lo, int n,
+__global__ void k_karras(const uint64_t* hi, const uint64_t* lo, int n,
                          BNode* nodes, int* leaf_parent) {
+  follow_early();
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n - 1) return;
   int d = (kdelta(hi, lo, n, i, i + 1) - kdelta(hi, lo, n, i, i - 1)) > 0 ? 1 : -1;
@@ -453,8 +463,9 @@ __device__ __forceinline__ void bnode_range(const BNode* nodes, int n, int b, in
   }
 }
 
-__global__ void k_classify(const BNode* __restrict__ nodes, const int* __restrict__ leaf_parent,
-                           const int* __restrict__ term, int n, CellInfo* info, unsigned* cnt) {
+__global__ void k_classify(const BNode* nodes, const int* leaf_parent,
+                           const int* term, int n, CellInfo* info, unsigned* cnt) {
+  follow_early();
   int b = blockIdx.x * blockDim.x + threadIdx.x;
   if (b >= 2 * n - 1) return;
   int first, last, dX, parent;
@@ -544,12 +555,13 @@ __device__ float mac_margin(const OvParams& P, double thr) {
   return __double2float_ru(E);
 }
 
-__global__ void k_write_cells(const BNode* __restrict__ nodes, const int* __restrict__ leaf_parent,
-                              const CellInfo* __restrict__ info, const unsigned* __restrict__ base,
-                              const uint64_t* __restrict__ khi, const uint64_t* __restrict__ klo,
-                              const double* __restrict__ nodes64, const int2* __restrict__ nodeids,
+__global__ void k_write_cells(const BNode* nodes, const int* leaf_parent,
+                              const CellInfo* info, const unsigned* base,
+                              const uint64_t* khi, const uint64_t* klo,
+                              const double* nodes64, const int2* nodeids,
                               OvParams P, int n, int big, Cell* cells, double* cell_lm, int2* cell_range,
-                              int* lists, int* list_counts, const int* __restrict__ flag, int* tail) {
+                              int* lists, int* list_counts, const int* flag, int* tail) {
+  follow_early();
   int b = blockIdx.x * blockDim.x + threadIdx.x;
   if (b >= 2 * n - 1) return;
   if (b == 0) {   // for the host's one read-back
@@ -614,8 +626,9 @@ __global__ void k_write_cells(const BNode* __restrict__ nodes, const int* __rest
 
 // ---------------------------------------------------------------- 5. nodes + moments
 // per sorted node: r1, wrapped r2 (src/tangle.c:519-528) and ids for the skip rule
-__global__ void k_nodes(OvParams P, const int* __restrict__ perm, const double* __restrict__ pos,
-                        const int2* __restrict__ links, int n, double* nodes64, int2* nodeids) {
+__global__ void k_nodes(OvParams P, const int* perm, const double* pos,
+                        const int2* links, int n, double* nodes64, int2* nodeids) {
+  follow_early();
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   int k = perm[i];
@@ -646,10 +659,11 @@ __device__ __forceinline__ void write_moments(Cell* c, d3 com, d3 g, double m21,
 // src/octree.c:237-266): com = (sum of positions) * (1/N); gam = sum of the
 // segment vectors; M = sum ds (x) (r - com).  Only the four entries of M the
 // expansion reads are kept.
-__global__ void k_moments_thread(const int* __restrict__ list, const int* __restrict__ list_count,
-                                 Cell* cells, const int2* __restrict__ cell_range,
-                                 const double* __restrict__ nodes64,
-                                 const int2* __restrict__ nodeids, double f4pi) {
+__global__ void k_moments_thread(const int* list, const int* list_count,
+                                 Cell* cells, const int2* cell_range,
+                                 const double* nodes64,
+                                 const int2* nodeids, double f4pi) {
+  follow_early();
   int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= *list_count) return;
   int c = list[t];
@@ -710,10 +724,11 @@ __device__ void moments_warp(int c, Cell* cells, const int2* __restrict__ cell_r
   if (tid == 0) write_moments(cells + c, com, mk3(a[0], a[1], a[2]), a[3], a[4], a[5], a[6], f4pi);
 }
 
-__global__ void k_moments_warp(const int* __restrict__ list, const int* __restrict__ list_count,
-                               Cell* cells, const int2* __restrict__ cell_range,
-                               const double* __restrict__ nodes64,
-                               const int2* __restrict__ nodeids, double f4pi) {
+__global__ void k_moments_warp(const int* list, const int* list_count,
+                               Cell* cells, const int2* cell_range,
+                               const double* nodes64,
+                               const int2* nodeids, double f4pi) {
+  follow_early();
   int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   if (w >= *list_count) return;
   moments_warp(list[w], cells, cell_range, nodes64, nodeids, f4pi);
@@ -767,8 +782,9 @@ __device__ __forceinline__ double chunk_sum(const double* __restrict__ part, int
 }
 
 __global__ void __launch_bounds__(kMomThreads) k_moments_chunk_pos(
-    const int* __restrict__ list, const int2* __restrict__ cell_range,
-    const double* __restrict__ nodes64, int chunk, int max_chunks, double* part) {
+    const int* list, const int2* cell_range,
+    const double* nodes64, int chunk, int max_chunks, double* part) {
+  follow_early();
   __shared__ double sh[(kMomThreads / 32) * 3];
   const int j = blockIdx.x, k = blockIdx.y;
   const int2 rg = cell_range[list[j]];
@@ -788,9 +804,10 @@ __global__ void __launch_bounds__(kMomThreads) k_moments_chunk_pos(
 }
 
 __global__ void __launch_bounds__(kMomThreads) k_moments_chunk_acc(
-    const int* __restrict__ list, const int2* __restrict__ cell_range,
-    const double* __restrict__ nodes64, const int2* __restrict__ nodeids, int chunk,
+    const int* list, const int2* cell_range,
+    const double* nodes64, const int2* nodeids, int chunk,
     int max_chunks, double* part) {
+  follow_early();
   __shared__ double sh[(kMomThreads / 32) * 7];
   __shared__ double sh_com[3];
   const int j = blockIdx.x, k = blockIdx.y;
@@ -820,9 +837,10 @@ __global__ void __launch_bounds__(kMomThreads) k_moments_chunk_acc(
 
 // one warp per list cell, a lane per sum: chunk sums in chunk order into the
 // cell record
-__global__ void k_moments_chunk_write(const int* __restrict__ list, const int* __restrict__ list_count,
-                                      Cell* cells, const int2* __restrict__ cell_range, int chunk,
-                                      int max_chunks, const double* __restrict__ part, double f4pi) {
+__global__ void k_moments_chunk_write(const int* list, const int* list_count,
+                                      Cell* cells, const int2* cell_range, int chunk,
+                                      int max_chunks, const double* part, double f4pi) {
+  follow_early();
   const int j = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   if (j >= *list_count) return;
   const int c = list[j];
@@ -872,11 +890,11 @@ static bool scan_excl(unsigned* v, int m, DevBuf& part, cudaStream_t st) {
   const int nb = (m + kScanThreads - 1) / kScanThreads;
   if (!part.reserve(sizeof(unsigned) * (size_t)nb)) return false;
   unsigned* sums = part.as<unsigned>();
-  k_scan_sums<<<nb, kScanThreads, 0, st>>>(v, m, sums);
+  OV_TRY_CUDA(ov_launch_early(k_scan_sums, dim3(nb), kScanThreads, st, v, m, sums));
   OV_LAUNCHED();
-  k_scan_top<<<1, kScanThreads, 0, st>>>(sums, nb);
+  OV_TRY_CUDA(ov_launch_early(k_scan_top, dim3(1), kScanThreads, st, sums, nb));
   OV_LAUNCHED();
-  k_scan_apply<<<nb, kScanThreads, 0, st>>>(v, m, sums);
+  OV_TRY_CUDA(ov_launch_early(k_scan_apply, dim3(nb), kScanThreads, st, v, m, sums));
   OV_LAUNCHED();
   return ov_cuda_ok(cudaGetLastError(), "scan");
 }
@@ -891,15 +909,17 @@ static bool rs_passes(uint64_t* ka, int* va, uint64_t* kb, int* vb, int n, int p
   unsigned* h = hist.as<unsigned>();
   for (int pass = 0; pass < passes; ++pass) {
     const int shift = 8 * pass;
-    k_rs_hist<kItems><<<tiles, kRsThreads, 0, st>>>(ka, n, shift, h);
+    OV_TRY_CUDA(ov_launch_early(k_rs_hist<kItems>, dim3(tiles), kRsThreads, st, ka, n, shift, h));
     OV_LAUNCHED();
     if (fused) {
-      k_rs_scatter<kItems, false><<<tiles, kRsThreads, 0, st>>>(ka, va, kb, vb, n, shift, h, tiles);
+      OV_TRY_CUDA(ov_launch_early((k_rs_scatter<kItems, false>), dim3(tiles), kRsThreads, st, ka, va, kb, vb, n, shift,
+                                  h, tiles));
     } else {
-      k_rs_transpose<<<tiles, 256, 0, st>>>(h, tiles, h + counts);
+      OV_TRY_CUDA(ov_launch_early(k_rs_transpose, dim3(tiles), 256, st, h, tiles, h + counts));
       OV_LAUNCHED();
       if (!scan_excl(h + counts, (int)counts, scan_part, st)) return false;
-      k_rs_scatter<kItems, true><<<tiles, kRsThreads, 0, st>>>(ka, va, kb, vb, n, shift, h + counts, tiles);
+      OV_TRY_CUDA(ov_launch_early((k_rs_scatter<kItems, true>), dim3(tiles), kRsThreads, st, ka, va, kb, vb, n, shift,
+                                  h + counts, tiles));
     }
     OV_LAUNCHED();
     OV_TRY_CUDA(cudaGetLastError());
@@ -961,8 +981,8 @@ bool ov_tree_build(ov_state_impl* s, const double* pos, OvTree* T, bool order_on
                 // box, cells per moment class (3), cells, the state's error flag
   OV_TRY_CUDA(cudaMemsetAsync(ctr, 0, sizeof(int) * 16, st));
   if (n > 0) {
-    k_keys<<<(n + 255) / 256, 256, 0, st>>>(s->P, pos, s->status.as<int2>(), n, khi, klo_slot, vals,
-                                             term_slot, ctr, s->dflag.as<int>());
+    OV_TRY_CUDA(ov_launch_early(k_keys, dim3((n + 255) / 256), 256, st, s->P, pos, s->status.as<int2>(), n, khi,
+                                klo_slot, vals, term_slot, ctr, s->dflag.as<int>()));
     OV_LAUNCHED();
     OV_TRY_CUDA(cudaGetLastError());
   }
@@ -980,10 +1000,10 @@ bool ov_tree_build(ov_state_impl* s, const double* pos, OvTree* T, bool order_on
   int* perm = T->perm.as<int>();
   if (n > 0) {
     OV_TRY_CUDA(cudaMemcpyAsync(perm, va, sizeof(int) * n, cudaMemcpyDeviceToDevice, st));
-    k_gather_lo<<<(n + 255) / 256, 256, 0, st>>>(perm, klo_slot, term_slot, klo, term, n);
+    OV_TRY_CUDA(ov_launch_early(k_gather_lo, dim3((n + 255) / 256), 256, st, perm, klo_slot, term_slot, klo, term, n));
     OV_LAUNCHED();
     if (na > 0) {
-      k_fix_ties<<<(na + 255) / 256, 256, 0, st>>>(ka, klo, perm, term, na);
+      OV_TRY_CUDA(ov_launch_early(k_fix_ties, dim3((na + 255) / 256), 256, st, ka, klo, perm, term, na));
       OV_LAUNCHED();
     }
     OV_TRY_CUDA(cudaGetLastError());
@@ -998,8 +1018,8 @@ bool ov_tree_build(ov_state_impl* s, const double* pos, OvTree* T, bool order_on
       !T->nodeids.reserve(sizeof(int2) * (size_t)(na > 0 ? na : 1)))
     return false;
   if (na > 0) {
-    k_nodes<<<(na + 255) / 256, 256, 0, st>>>(s->P, perm, pos, s->links.as<int2>(), na,
-                                               T->nodes64.as<double>(), T->nodeids.as<int2>());
+    OV_TRY_CUDA(ov_launch_early(k_nodes, dim3((na + 255) / 256), 256, st, s->P, perm, pos, s->links.as<int2>(), na,
+                                T->nodes64.as<double>(), T->nodeids.as<int2>()));
     OV_LAUNCHED();
     OV_TRY_CUDA(cudaGetLastError());
   }
@@ -1037,16 +1057,15 @@ bool ov_tree_build(ov_state_impl* s, const double* pos, OvTree* T, bool order_on
     if (!read_build(s, T, ctr, hc)) return false;
     T->n_cells = 1;
   } else {
-    k_karras<<<(na - 1 + 255) / 256, 256, 0, st>>>(hi_sorted, klo, na, bn, leaf_parent);
+    OV_TRY_CUDA(ov_launch_early(k_karras, dim3((na - 1 + 255) / 256), 256, st, hi_sorted, klo, na, bn, leaf_parent));
     OV_LAUNCHED();
     OV_TRY_CUDA(cudaMemsetAsync(base, 0, sizeof(unsigned) * (na + 1), st));
-    k_classify<<<(nbin + 255) / 256, 256, 0, st>>>(bn, leaf_parent, term, na, info, base);
+    OV_TRY_CUDA(ov_launch_early(k_classify, dim3((nbin + 255) / 256), 256, st, bn, leaf_parent, term, na, info, base));
     OV_LAUNCHED();
     if (!scan_excl(base, na + 1, T->scan_part, st)) return false;
-    k_write_cells<<<(nbin + 255) / 256, 256, 0, st>>>(bn, leaf_parent, info, base, hi_sorted, klo,
-                                                      T->nodes64.as<double>(), T->nodeids.as<int2>(),
-                                                      s->P, na, mom_big(na), cells, cell_lm, cell_range, lists,
-                                                      list_counts, s->dflag.as<int>(), ctr + 7);
+    OV_TRY_CUDA(ov_launch_early(k_write_cells, dim3((nbin + 255) / 256), 256, st, bn, leaf_parent, info, base,
+                                hi_sorted, klo, T->nodes64.as<double>(), T->nodeids.as<int2>(), s->P, na, mom_big(na),
+                                cells, cell_lm, cell_range, lists, list_counts, s->dflag.as<int>(), ctr + 7));
     OV_LAUNCHED();
     OV_TRY_CUDA(cudaGetLastError());
     if (!read_build(s, T, ctr, hc)) return false;
@@ -1055,14 +1074,14 @@ bool ov_tree_build(ov_state_impl* s, const double* pos, OvTree* T, bool order_on
     const int* lc = hc + 4;
     const double f4 = s->P.f4pi;
     if (lc[0] > 0) {
-      k_moments_thread<<<(lc[0] + 127) / 128, 128, 0, st>>>(lists, list_counts, cells, cell_range,
-                                                            T->nodes64.as<double>(), T->nodeids.as<int2>(), f4);
+      OV_TRY_CUDA(ov_launch_early(k_moments_thread, dim3((lc[0] + 127) / 128), 128, st, lists, list_counts, cells,
+                                  cell_range, T->nodes64.as<double>(), T->nodeids.as<int2>(), f4));
       OV_LAUNCHED();
     }
     if (lc[1] > 0) {
-      k_moments_warp<<<(lc[1] * 32 + 255) / 256, 256, 0, st>>>(lists + 2 * (size_t)na, list_counts + 1,
-                                                              cells, cell_range, T->nodes64.as<double>(),
-                                                              T->nodeids.as<int2>(), f4);
+      OV_TRY_CUDA(ov_launch_early(k_moments_warp, dim3((lc[1] * 32 + 255) / 256), 256, st, lists + 2 * (size_t)na,
+                                  list_counts + 1, cells, cell_range, T->nodes64.as<double>(), T->nodeids.as<int2>(),
+                                  f4));
       OV_LAUNCHED();
     }
     if (lc[2] > 0) {
@@ -1073,14 +1092,14 @@ bool ov_tree_build(ov_state_impl* s, const double* pos, OvTree* T, bool order_on
       const int* blist = lists + 4 * (size_t)na;
       double* part = T->mom_part.as<double>();
       const dim3 grid(lc[2], max_chunks);
-      k_moments_chunk_pos<<<grid, kMomThreads, 0, st>>>(blist, cell_range, T->nodes64.as<double>(), chunk,
-                                                         max_chunks, part);
+      OV_TRY_CUDA(ov_launch_early(k_moments_chunk_pos, dim3(grid), kMomThreads, st, blist, cell_range,
+                                  T->nodes64.as<double>(), chunk, max_chunks, part));
       OV_LAUNCHED();
-      k_moments_chunk_acc<<<grid, kMomThreads, 0, st>>>(blist, cell_range, T->nodes64.as<double>(),
-                                                         T->nodeids.as<int2>(), chunk, max_chunks, part);
+      OV_TRY_CUDA(ov_launch_early(k_moments_chunk_acc, dim3(grid), kMomThreads, st, blist, cell_range,
+                                  T->nodes64.as<double>(), T->nodeids.as<int2>(), chunk, max_chunks, part));
       OV_LAUNCHED();
-      k_moments_chunk_write<<<(lc[2] + 3) / 4, 128, 0, st>>>(blist, list_counts + 2, cells, cell_range,
-                                                                  chunk, max_chunks, part, f4);
+      OV_TRY_CUDA(ov_launch_early(k_moments_chunk_write, dim3((lc[2] + 3) / 4), 128, st, blist, list_counts + 2, cells,
+                                  cell_range, chunk, max_chunks, part, f4));
       OV_LAUNCHED();
     }
     OV_TRY_CUDA(cudaGetLastError());

@@ -1294,7 +1294,8 @@ static __global__ void k_drop_first(const int* __restrict__ perm, int nin, int n
 // bits (the time as an FP32 number, its sign and low 15 bits dropped), so two
 // passes of the radix sort order them
 constexpr int kCostBits = 16;
-static __global__ void k_cost_keys(const unsigned* __restrict__ cost, int n, uint64_t* keys, int* vals) {
+static __global__ void k_cost_keys(const unsigned* cost, int n, uint64_t* keys, int* vals) {
+  follow_early();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   keys[i] = 0xffffu - ((unsigned)__float_as_int((float)cost[i]) >> 15);
@@ -1308,8 +1309,9 @@ static __global__ void k_cost_keys(const unsigned* __restrict__ cost, int n, uin
 // order only decides which targets share a warp.  Value i of the sort is
 // slots[i] (or i).
 constexpr int kCurveBits = 10;
-static __global__ void k_curve_keys(OvParams P, const double* __restrict__ pts, const int* __restrict__ slots, int n,
+static __global__ void k_curve_keys(OvParams P, const double* pts, const int* slots, int n,
                                     uint64_t* keys, int* vals) {
+  follow_early();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const int k = slots ? slots[i] : i;
@@ -1495,8 +1497,8 @@ static bool launch_multi(ov_state_impl* s, OvTree* t, const OvParams& P, const i
     if (!t->wkeys.reserve(sizeof(uint64_t) * nw) || !t->wkeys2.reserve(sizeof(uint64_t) * nw) ||
         !t->wvals.reserve(sizeof(int) * nw) || !t->wvals2.reserve(sizeof(int) * nw))
       return false;
-    k_cost_keys<<<(warps + 255) / 256, 256, 0, s->stream>>>(wcost, warps, t->wkeys.as<uint64_t>(),
-                                                              t->wvals.as<int>());
+    OV_TRY_CUDA(ov_launch_early(k_cost_keys, dim3((warps + 255) / 256), 256, s->stream, wcost, warps,
+                                t->wkeys.as<uint64_t>(), t->wvals.as<int>()));
     OV_LAUNCHED();
     if (!ov_radix_sort_u64(t->wkeys.as<uint64_t>(), t->wvals.as<int>(), t->wkeys2.as<uint64_t>(),
                            t->wvals2.as<int>(), warps, kCostBits, t->whist, t->wscan, s->stream))
@@ -1575,7 +1577,7 @@ bool ov_tree_walk_nodes(ov_state_impl* s, OvTree* t, const double* pos, bool own
   const int blocks = (warps * 32 + 127) / 128;
   if (mixed) {
     k_walk_nodes<true><<<blocks, 128, 0, s->stream>>>(P, tv, order, s->status.as<int2>(), pos, n_t,
-                                                       v_nl, v_img, ctr);
+                                                        v_nl, v_img, ctr);
     OV_LAUNCHED();
   } else {
     k_walk_nodes<false><<<blocks, 128, 0, s->stream>>>(P, tv, order, s->status.as<int2>(), pos, n_t,
@@ -1616,7 +1618,8 @@ bool ov_tree_walk_points(ov_state_impl* s, OvTree* t, int npts, const double* pt
       if (!t->pkeys.reserve(sizeof(uint64_t) * 2 * np) || !t->pvals.reserve(sizeof(int) * 2 * np)) return false;
       uint64_t* keys = t->pkeys.as<uint64_t>();
       int* vals = t->pvals.as<int>();
-      k_curve_keys<<<(npts + 255) / 256, 256, 0, s->stream>>>(P, pts, nullptr, npts, keys, vals);
+      OV_TRY_CUDA(ov_launch_early(k_curve_keys, dim3((npts + 255) / 256), 256, s->stream, P, pts, nullptr, npts, keys,
+                                  vals));
       OV_LAUNCHED();
       if (!ov_radix_sort_u64(keys, vals, keys + np, vals + np, npts, 3 * kCurveBits, t->whist, t->wscan, s->stream))
         return false;
