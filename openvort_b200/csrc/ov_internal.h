@@ -334,9 +334,9 @@ long long ov_launches();
 #ifdef __CUDACC__
 // Launches a kernel that begins with follow_early(): its blocks may take
 // their places while the kernel before it in the stream still runs, and wait
-// there for its end, so the launch itself costs nothing between the two (a tree
-// build of 22.4k nodes, 27 launches: 0.231 ms, 0.176 so).  For
-// kernels of a few microseconds.
+// there for its end, so the launch itself costs nothing between the two (a
+// tree build of 22.4k nodes, 27 launches: 0.231 ms, 0.176 so).  For kernels of
+// a few microseconds.
 template <class... P, class... A>
 inline cudaError_t ov_launch_early(void (*kernel)(P...), dim3 grid, int block, cudaStream_t st, A&&... args) {
   cudaLaunchAttribute at{};

@@ -447,6 +447,32 @@ def test_tree_sort_sizes_vs_oracle(ov, oracle, slots):
     st.close()
 
 
+@pytest.mark.parametrize("precision", [0, 1])
+@pytest.mark.parametrize("nodes", [31, 127, 128, 129, 257])
+def test_small_runs_vs_oracle(ov, oracle, nodes, precision):
+    """Runs small enough that an evaluation's geometry goes along with its
+    direct sum, at slot counts around the blocks of 128, with EMPTY slots: two
+    RK4 steps against the oracle's.  FP64 to a few roundings of the positions;
+    mixed to its tolerance on the distance moved."""
+    from openvort_b200.tangle import ring_points
+    r = ring_points(np.array([0.05, 0.05, 0.05]), (0.3, 0.2, 0.9), 0.02, nodes)
+    t = G.rings_to_tangle([r], (0, 0, 0), (0.1, 0.1, 0.1), "periodic-6", empty_slots=3)
+    p = Params(core_a=1e-8, alpha=0.098, alpha_p=0.016, use_mf=1, dl_max=1e-2,
+               vn=Flow("simple", {"external_v": (0.5, 0, 0)}))
+    dt = 1e-6
+    want = oracle.update_tangle(t, p)
+    for i in range(2):
+        want = oracle.rk4_step(oracle.update_tangle(want, p), p, i * dt, dt)
+    ov.configure(p, precision)
+    got = t.copy()
+    st = ov.DeviceState(got)
+    st.run(0.0, dt, 2)
+    st.download(ov.OV_FIELD_POS)
+    st.close()
+    moved = np.abs(want.pos[t.active] - t.pos[t.active]).max() / np.abs(want.pos[t.active]).max()
+    assert pos_err(got.pos, want.pos, t.active) < 1e-14 + (TOL_MIXED * moved if precision else 0)
+
+
 @pytest.mark.parametrize("boundary", ["open", "periodic-6", "periodic-26"])
 def test_eval_points_counts_vs_oracle(ov, oracle, boundary):
     """Direct sums at point counts around the widths of the blocks that add
