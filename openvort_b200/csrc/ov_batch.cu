@@ -26,18 +26,27 @@ namespace {
 
 struct BatchView {
   const int* off;       // n_sys + 1 slot offsets
-  const int2* items;    // (system, first target slot), costliest first
+  const int4* items;    // (system, first target slot, share of the sources), costliest first
   const double* near2;  // per system: FP64 within this squared distance (mixed form)
   int n_items;
+  int splits;           // shares a system's sources are summed in
 };
+
+// The source slots of share z of a system's slots [s0, s1)
+__device__ __forceinline__ int2 source_share(const BatchView& B, int s0, int s1, int z) {
+  const int len = ((s1 - s0 + B.splits - 1) / B.splits + 31) / 32 * 32;
+  const int c0 = min(s1, s0 + z * len);
+  return make_int2(c0, min(s1, c0 + len));
+}
 
 // What a Biot-Savart kernel does with a target's sum (inactive targets:
 // EMPTY slots, whose sums are zero): v_nl for the per-node kernels that
-// follow.
+// follow, or share z's partial sums for the epilogue to add up.
 struct StoreSums {
   double* v_nl;
-  __device__ void operator()(const OvParams&, int k, bool act, d3 v) const {
-    st3(v_nl, k, act ? v : mk3(0, 0, 0));
+  size_t stride;   // doubles from one share to the next
+  __device__ void operator()(int z, int k, bool act, d3 v) const {
+    st3(v_nl + z * stride, k, act ? v : mk3(0, 0, 0));
   }
 };
 
@@ -48,7 +57,7 @@ struct StoreSums {
 // |R| < 1e-8 cut-off returns zero.
 // Bound by the FP64 pipe: 1.09 ms per sum for 256 systems (277k points),
 // against 2.4 ms with IEEE square roots and divisions per pair.
-template <int TB, int TS>
+template <int TB, int TS, bool kShares>
 __global__ void __launch_bounds__(TB) k_batch_bs64(OvParams P, BatchView B,
                                                    const double* __restrict__ pos,
                                                    const int2* __restrict__ links,
@@ -65,13 +74,14 @@ __global__ void __launch_bounds__(TB) k_batch_bs64(OvParams P, BatchView B,
     __syncthreads();
     const int it = sh_item;
     if (it >= B.n_items) return;   // uniform over the block
-    const int2 w = B.items[it];
+    const int4 w = B.items[it];
     const int s0 = B.off[w.x], s1 = B.off[w.x + 1];
+    const int2 src = kShares ? source_share(B, s0, s1, w.z) : make_int2(s0, s1);
     const int k = w.y + threadIdx.x;
     const bool act = k < s1 && status[k].x == OV_FREE;
     const d3 r = act ? ld3(pos, k) : mk3(0, 0, 0);
     d3 acc = mk3(0, 0, 0);
-    for (int base = s0; base < s1; base += TS) {
+    for (int base = src.x; base < src.y; base += TS) {
       __syncthreads();
       for (int q = threadIdx.x; q <= TS; q += TB) {
         const int m = base + q;
@@ -82,7 +92,7 @@ __global__ void __launch_bounds__(TB) k_batch_bs64(OvParams P, BatchView B,
       }
       for (int q = threadIdx.x; q < TS; q += TB) {
         const int m = base + q;
-        const int f = m < s1 && status[m].x != OV_EMPTY ? links[m].x : -1;
+        const int f = m < src.y && status[m].x != OV_EMPTY ? links[m].x : -1;
         const bool chained = f >= 0 && f == m + 1;
         const unsigned bits = __ballot_sync(0xffffffffu, chained);
         const unsigned rest = __ballot_sync(0xffffffffu, f >= 0 && !chained);
@@ -93,12 +103,12 @@ __global__ void __launch_bounds__(TB) k_batch_bs64(OvParams P, BatchView B,
       }
       __syncthreads();
       if (!act) continue;
-      chain64_sweep<false>(sh_node, sh_chain, sh_other, min(TS, s1 - base), -2, r, cut, acc, [&](int i) {
+      chain64_sweep<false>(sh_node, sh_chain, sh_other, min(TS, src.y - base), -2, r, cut, acc, [&](int i) {
         const d3 r1 = ld3(pos, base + i), r2 = ld3(pos, links[base + i].x);
         return seg_vel64_nr(1.0, r1, r2, r2 - r1, r, cut);
       });
     }
-    if (k < s1) out(P, k, act, acc * P.f4pi);
+    if (k < s1) out(kShares ? w.z : 0, k, act, acc * P.f4pi);
   }
 }
 
@@ -118,7 +128,7 @@ __global__ void __launch_bounds__(TB) k_batch_bs64(OvParams P, BatchView B,
 // partial sums over 32 sources are added into FP64 sums.  With open
 // boundaries the two segments the skip rule drops have an endpoint at the
 // target, so they are near and the FP64 cut-off returns zero for them.
-template <int TB, int TS, bool kTwo = (TB > 64)>
+template <int TB, int TS, bool kShares, bool kTwo = (TB > 64)>
 __global__ void __launch_bounds__(TB) k_batch_bs_mixed(OvParams P, BatchView B,
                                                        const double* __restrict__ pos,
                                                        const int2* __restrict__ links,
@@ -134,8 +144,9 @@ __global__ void __launch_bounds__(TB) k_batch_bs_mixed(OvParams P, BatchView B,
     __syncthreads();
     const int it = sh_item;
     if (it >= B.n_items) return;
-    const int2 w = B.items[it];
+    const int4 w = B.items[it];
     const int s0 = B.off[w.x], s1 = B.off[w.x + 1];
+    const int2 src = kShares ? source_share(B, s0, s1, w.z) : make_int2(s0, s1);
     const double near2 = B.near2[w.x];
     // two-float offsets from the item's first target; single-rounded ones
     // from its middle target
@@ -159,7 +170,7 @@ __global__ void __launch_bounds__(TB) k_batch_bs_mixed(OvParams P, BatchView B,
       add_target(acc, u, seg_vel64_nr(f4pi, r1, r2, r2 - r1, ld3(pos, k)));
     };
     auto stage_one = [&](int m) -> SrcVals {
-      if (m >= s1 || status[m].x == OV_EMPTY) return src_none();
+      if (m >= src.y || status[m].x == OV_EMPTY) return src_none();
       const int f = links[m].x;
       if (f < 0) return src_none();
       const d3 a = ld3(pos, m), bb = ld3(pos, f);
@@ -167,12 +178,12 @@ __global__ void __launch_bounds__(TB) k_batch_bs_mixed(OvParams P, BatchView B,
       const double far2 = fmax(16.0 * (dx * dx + dy * dy + dz * dz), near2);
       return src_from(a.x - O.x, a.y - O.y, a.z - O.z, dx, dy, dz, far2, m);
     };
-    for (int base = s0; base < s1; base += TS) {
+    for (int base = src.x; base < src.y; base += TS) {
       __syncthreads();
       for (int q = threadIdx.x; q < TS / 2; q += TB)
         stage_pair(sh[q], stage_one(base + 2 * q), stage_one(base + 2 * q + 1));
       __syncthreads();
-      const int nrec = (min(TS, s1 - base) + 1) / 2;   // records holding a source
+      const int nrec = (min(TS, src.y - base) + 1) / 2;   // records holding a source
       for (int q0 = 0; q0 < nrec; q0 += 16) {
         f2 bsum[kTT][3];
 #pragma unroll
@@ -196,7 +207,7 @@ __global__ void __launch_bounds__(TB) k_batch_bs_mixed(OvParams P, BatchView B,
 #pragma unroll
     for (int u = 0; u < kTT; ++u) {
       const int k = w.y + threadIdx.x + TB * u;
-      if (k < s1) out(P, k, kk[u] >= 0, mk3(acc[u][0], acc[u][1], acc[u][2]));
+      if (k < s1) out(kShares ? B.items[sh_item].z : 0, k, kk[u] >= 0, mk3(acc[u][0], acc[u][1], acc[u][2]));
     }
   }
 }
@@ -208,7 +219,7 @@ __global__ void __launch_bounds__(TB) k_batch_bs_mixed(OvParams P, BatchView B,
 // Two-float offsets from the coordinate origin (the systems span whole
 // rings, and a slot may be EMPTY); near pairs and pairs at the colinearity
 // cut-off in FP64, FP32 partial sums over 32 segments added into FP64 sums.
-template <int TB>
+template <int TB, bool kShares>
 __global__ void __launch_bounds__(TB) k_batch_bs_chain(OvParams P, BatchView B,
                                                        const double* __restrict__ pos,
                                                        const int2* __restrict__ links,
@@ -227,8 +238,9 @@ __global__ void __launch_bounds__(TB) k_batch_bs_chain(OvParams P, BatchView B,
     __syncthreads();
     const int it = sh_item;
     if (it >= B.n_items) return;
-    const int2 w = B.items[it];
+    const int4 w = B.items[it];
     const int s0 = B.off[w.x], s1 = B.off[w.x + 1];
+    const int2 src = kShares ? source_share(B, s0, s1, w.z) : make_int2(s0, s1);
     const double near2 = B.near2[w.x];
     int kk[kTT];
     PairTargets T;
@@ -250,7 +262,7 @@ __global__ void __launch_bounds__(TB) k_batch_bs_chain(OvParams P, BatchView B,
     };
     // the segment starting at slot m: forward slot (or -1), vector, far radius
     auto seg_of = [&](int m, double* d, double* far2) -> int {
-      if (m >= s1 || status[m].x == OV_EMPTY) return -1;
+      if (m >= src.y || status[m].x == OV_EMPTY) return -1;
       const int f = links[m].x;
       if (f < 0) return -1;
       const d3 a = ld3(pos, m), bb = ld3(pos, f);
@@ -260,7 +272,7 @@ __global__ void __launch_bounds__(TB) k_batch_bs_chain(OvParams P, BatchView B,
       *far2 = fmax(16.0 * (d[0] * d[0] + d[1] * d[1] + d[2] * d[2]), near2);
       return f;
     };
-    for (int sb = s0; sb < s1; sb += 2 * kCH) {
+    for (int sb = src.x; sb < src.y; sb += 2 * kCH) {
       __syncthreads();
       if (threadIdx.x == 0) sh_n_irr = 0;
       __syncthreads();
@@ -336,7 +348,7 @@ __global__ void __launch_bounds__(TB) k_batch_bs_chain(OvParams P, BatchView B,
 #pragma unroll
     for (int u = 0; u < kTT; ++u) {
       const int k = w.y + threadIdx.x + TB * u;
-      if (k < s1) out(P, k, kk[u] >= 0, mk3(acc[u][0], acc[u][1], acc[u][2]));
+      if (k < s1) out(kShares ? B.items[sh_item].z : 0, k, kk[u] >= 0, mk3(acc[u][0], acc[u][1], acc[u][2]));
     }
   }
 }
@@ -374,12 +386,16 @@ using BsKernel = void (*)(OvParams, BatchView, const double*, const int2*, const
 // the kernel shapes the autotuner chooses from
 struct Shape {
   int tb, ts;
-  BsKernel k64, kmixed;
+  BsKernel k64[2], kmixed[2];   // sources in one share, in several
 };
-#define OV_SHAPE(TB, TS) {TB, TS, k_batch_bs64<TB, TS>, k_batch_bs_mixed<TB, TS>}
+#define OV_SHAPE(TB, TS) \
+  {TB, TS, {k_batch_bs64<TB, TS, false>, k_batch_bs64<TB, TS, true>}, \
+   {k_batch_bs_mixed<TB, TS, false>, k_batch_bs_mixed<TB, TS, true>}}
 // sources_per_tile 0: the mixed form in chain order (tiles of 128 segments);
 // the FP64 form as with 128
-#define OV_SHAPE_CHAIN(TB) {TB, 0, k_batch_bs64<TB, 128>, k_batch_bs_chain<TB>}
+#define OV_SHAPE_CHAIN(TB) \
+  {TB, 0, {k_batch_bs64<TB, 128, false>, k_batch_bs64<TB, 128, true>}, \
+   {k_batch_bs_chain<TB, false>, k_batch_bs_chain<TB, true>}}
 const Shape kShapes[] = {
     OV_SHAPE(64, 64),  OV_SHAPE(64, 128),  OV_SHAPE(64, 256),  OV_SHAPE(128, 64), OV_SHAPE(128, 128),
     OV_SHAPE(128, 256), OV_SHAPE(256, 64), OV_SHAPE(256, 128), OV_SHAPE(256, 256), OV_SHAPE_CHAIN(64),
@@ -406,7 +422,7 @@ struct ov_batch {
   std::vector<int> off;    // host copy of the offsets
   std::vector<int> order;  // systems by decreasing slot count
   DevBuf d_off, d_items, d_near2, d_work, d_time;
-  int items_tb = 0, n_items = 0;
+  int items_tb = 0, n_items = 0, splits = 1;
   int shape = 4;           // kShapes index (128 targets, 128 sources)
   int blocks_per_sm = 0;
   double tuned_ms = 0;
@@ -419,36 +435,56 @@ struct ov_batch {
 
 namespace {
 
-bool build_items(ov_batch* b, int tb) {
-  if (b->items_tb == tb) return true;
-  std::vector<int2> items;
-  for (int s : b->order)
-    for (int t0 = b->off[s]; t0 < b->off[s + 1]; t0 += tb) items.push_back(make_int2(s, t0));
-  b->n_items = (int)items.size();
-  if (!b->d_items.reserve(sizeof(int2) * std::max<size_t>(1, items.size()))) return false;
-  if (!items.empty())
-    OV_TRY_CUDA(cudaMemcpy(b->d_items.p, items.data(), sizeof(int2) * items.size(),
-                           cudaMemcpyHostToDevice));
-  b->items_tb = tb;
-  return true;
-}
-
 // SMs x resident blocks per SM of each kernel shape and form, looked up on
 // first use (before any graph capture: ov_batch_run calls it first)
 int g_sms = 0;
 int g_occ[kNumShapes][2] = {};
 
+bool count_sms() {
+  if (g_sms) return true;
+  int dev = 0, sms = 0;
+  OV_TRY_CUDA(cudaGetDevice(&dev));
+  OV_TRY_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+  g_sms = std::max(1, sms);
+  return true;
+}
+
+// Work items of `tb` targets.  An ensemble with fewer blocks of 128 targets
+// than twice the places for them (10 per SM) has its systems' sources summed
+// in shares, as one block over all the sources of its largest system would
+// decide the time: 8 systems of 64 to 2047 nodes 0.059 ms a sum (mixed) and
+// 0.046 (FP64), against 0.225 and 0.231 in one share; 64 systems 0.22 and
+// 0.31, against 0.29 and 0.44; from 256 systems on one share.  The shares
+// depend on the ensemble alone, so the sums do not depend on the kernel's
+// shape.  One share has kernels of its own (with the share's bounds in them
+// they take up to 2% longer).
+constexpr int kMaxShares = 16;
+bool build_items(ov_batch* b, int tb) {
+  if (b->items_tb == tb) return true;
+  if (!count_sms()) return false;
+  long long blocks = 0;
+  for (int s = 0; s < b->n_sys; ++s) blocks += (b->off[s + 1] - b->off[s] + 127) / 128;
+  b->splits = (int)std::min<long long>(kMaxShares, std::max(1LL, 20LL * g_sms / std::max(1LL, blocks)));
+  if (b->splits > 1 && !b->s.img_part.reserve(sizeof(double) * 3 * (size_t)b->s.n * b->splits)) return false;
+  std::vector<int4> items;
+  for (int s : b->order)
+    for (int t0 = b->off[s]; t0 < b->off[s + 1]; t0 += tb)
+      for (int z = 0; z < b->splits; ++z) items.push_back(make_int4(s, t0, z, 0));
+  b->n_items = (int)items.size();
+  if (!b->d_items.reserve(sizeof(int4) * std::max<size_t>(1, items.size()))) return false;
+  if (!items.empty())
+    OV_TRY_CUDA(cudaMemcpy(b->d_items.p, items.data(), sizeof(int4) * items.size(),
+                           cudaMemcpyHostToDevice));
+  b->items_tb = tb;
+  return true;
+}
+
 bool prepare_shape(int shape, bool mixed) {
-  if (!g_sms) {
-    int dev = 0;
-    OV_TRY_CUDA(cudaGetDevice(&dev));
-    OV_TRY_CUDA(cudaDeviceGetAttribute(&g_sms, cudaDevAttrMultiProcessorCount, dev));
-    if (g_sms <= 0) g_sms = 1;
-  }
+  if (!count_sms()) return false;
   int& occ = g_occ[shape][mixed ? 1 : 0];
   const Shape& sh = kShapes[shape];
   if (!occ) {
-    OV_TRY_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, mixed ? sh.kmixed : sh.k64, sh.tb, 0));
+    OV_TRY_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, (mixed ? sh.kmixed : sh.k64)[0], sh.tb, 0));
     if (occ < 1) occ = 1;
   }
   return true;
@@ -461,22 +497,24 @@ int grid_for(const ov_batch* b, bool mixed) {
   return std::max(1, std::min(b->n_items, g_sms * per_sm));
 }
 
-// the Biot-Savart sum of every system at positions pos -> v_nl; work: a
-// zeroed counter
 // targets per work item of a kernel shape and form
 int item_targets(int shape, bool mixed) { return kShapes[shape].tb * (mixed ? kTT : 1); }
 
-bool launch_bs(ov_batch* b, const double* pos, double* v_nl, int* work) {
+// the Biot-Savart sum of every system at positions pos -> sums_of(b); work: a
+// zeroed counter
+
+bool launch_bs(ov_batch* b, const double* pos, int* work) {
   const Shape& sh = kShapes[b->shape];
   const bool mixed = b->s.P.precision == OV_PREC_MIXED;
   if (!build_items(b, item_targets(b->shape, mixed))) return false;
   if (b->n_items == 0) return true;
-  BatchView B{b->d_off.as<int>(), b->d_items.as<int2>(), b->d_near2.as<double>(), b->n_items};
-  BsKernel k = mixed ? sh.kmixed : sh.k64;
+  BatchView B{b->d_off.as<int>(), b->d_items.as<int4>(), b->d_near2.as<double>(), b->n_items, b->splits};
+  double* out = b->splits > 1 ? b->s.img_part.as<double>() : b->s.v_nl.as<double>();
+  BsKernel k = (mixed ? sh.kmixed : sh.k64)[b->splits > 1 ? 1 : 0];
   if (!g_occ[b->shape][mixed ? 1 : 0] && !prepare_shape(b->shape, mixed)) return false;
   const int grid = grid_for(b, mixed);
   k<<<grid, sh.tb, 0, b->s.stream>>>(b->s.P, B, pos, b->s.links.as<int2>(), b->s.status.as<int2>(),
-                                     StoreSums{v_nl}, work);
+                                     StoreSums{out, 3 * (size_t)b->s.n}, work);
   OV_LAUNCHED();
   OV_TRY_CUDA(cudaGetLastError());
   return true;
@@ -493,6 +531,12 @@ bool launch_near2(ov_batch* b, const double* pos) {
   return true;
 }
 
+// where launch_bs leaves the sums
+OvSums sums_of(ov_batch* b) {
+  if (b->splits > 1) return OvSums{nullptr, nullptr, b->s.img_part.as<double>(), b->splits};
+  return OvSums{b->s.v_nl.as<double>(), nullptr, nullptr, 0};
+}
+
 // geometry + Biot-Savart + epilogue at positions pos (time t0 + *t_dev)
 bool enqueue_eval(ov_batch* b, const double* pos, double* dxi, double* tan, double* nrm, double* vels,
                   double* vs, const double* t_dev, double t0, int* work, const OvStage& stage, cudaEvent_t e0,
@@ -504,11 +548,11 @@ bool enqueue_eval(ov_batch* b, const double* pos, double* dxi, double* tan, doub
     return false;
   if (!s->P.lia_only) {
     if (e0) OV_TRY_CUDA(cudaEventRecord(e0, s->stream));
-    if (!launch_bs(b, pos, s->v_nl.as<double>(), work)) return false;
+    if (!launch_bs(b, pos, work)) return false;
     if (e1) OV_TRY_CUDA(cudaEventRecord(e1, s->stream));
   }
   return ov_launch_epilogue(s->stream, s->P, s->links.as<int2>(), s->status.as<int2>(), t_dev, t0, pos,
-                            tan, nrm, OvSums{s->v_nl.as<double>(), nullptr, nullptr, 0}, s->n, stage, vels, vs, 0,
+                            tan, nrm, sums_of(b), s->n, stage, vels, vs, 0,
                             s->n, flag);
 }
 
@@ -554,7 +598,7 @@ bool time_bs(ov_batch* b, double* ms_out) {
   if (!launch_near2(b, s->pos.as<double>())) return false;
   OV_TRY_CUDA(cudaMemsetAsync(b->d_work.p, 0, sizeof(int), s->stream));
   OV_TRY_CUDA(cudaEventRecord(b->ev_bs[0], s->stream));
-  if (!launch_bs(b, s->pos.as<double>(), s->v_nl.as<double>(), b->d_work.as<int>())) return false;
+  if (!launch_bs(b, s->pos.as<double>(), b->d_work.as<int>())) return false;
   OV_TRY_CUDA(cudaEventRecord(b->ev_bs[1], s->stream));
   OV_TRY_CUDA(cudaStreamSynchronize(s->stream));
   float ms = 0;
@@ -692,7 +736,7 @@ void ov_batch_destroy(ov_batch* b) {
   for (DevBuf* d : bufs) d->release();
   DevBuf* sb[] = {&b->s.pos, &b->s.links, &b->s.status, &b->s.dxi, &b->s.tan, &b->s.nrm, &b->s.vels,
                   &b->s.vs, &b->s.pos0, &b->s.spos, &b->s.sdxi, &b->s.stan, &b->s.snrm, &b->s.svs,
-                  &b->s.k2, &b->s.k3, &b->s.k4, &b->s.v_nl, &b->s.v_img, &b->s.dflag};
+                  &b->s.k2, &b->s.k3, &b->s.k4, &b->s.v_nl, &b->s.v_img, &b->s.img_part, &b->s.dflag};
   for (DevBuf* d : sb) d->release();
   if (b->s.stream) cudaStreamDestroy(b->s.stream);
   ov_events_release(&b->s);
@@ -827,7 +871,7 @@ int ov_batch_autotune(ov_batch* b, ov_batch_tuning* out) {
       for (int rep = 0; ok && rep < 3; ++rep) {
         ok = ov_cuda_ok(cudaMemsetAsync(b->d_work.p, 0, sizeof(int), s->stream), "cudaMemsetAsync") &&
              ov_cuda_ok(cudaEventRecord(b->ev_bs[0], s->stream), "cudaEventRecord") &&
-             launch_bs(b, s->pos.as<double>(), s->v_nl.as<double>(), b->d_work.as<int>()) &&
+             launch_bs(b, s->pos.as<double>(), b->d_work.as<int>()) &&
              ov_cuda_ok(cudaEventRecord(b->ev_bs[1], s->stream), "cudaEventRecord") &&
              ov_cuda_ok(cudaStreamSynchronize(s->stream), "cudaStreamSynchronize");
         float ms = 0;

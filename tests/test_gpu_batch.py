@@ -204,3 +204,27 @@ def test_batch_rejects_bad_ensembles(ov, ensemble, monkeypatch):
     assert not lib.ov_batch_create(per.ptr(), 1, two.ctypes.data)
     assert lib.ov_last_error() == ov._lib.OV_ERR_INVALID
     lib.ov_clear_error()
+
+
+@pytest.mark.parametrize("sizes", [(64,), (65, 31, 130), (300, 64, 33)])
+def test_small_ensembles_in_source_shares_vs_oracle(ov, sizes):
+    """Ensembles whose systems' sources are summed in several shares (of at
+    least 32 slots, some of them empty), at slot counts around the shares'
+    edges: velocities of both forms against the oracle on each system alone."""
+    from openvort_b200.tangle import ring_points
+    systems = [[ring_points(np.array([0.0, 0.0, 0.01 * i]), (0.3, 0.2, 0.9), 0.01, n)] for i, n in enumerate(sizes)]
+    half = 0.09
+    t = G.rings_to_tangle([r for s in systems for r in s], (-half,) * 3, (half,) * 3, "open")
+    off = np.concatenate([[0], np.cumsum(sizes)]).astype(np.int32)
+    orc = Oracle()
+    for precision, tol in ((ov.OV_PREC_FP64, TOL_V64), (ov.OV_PREC_MIXED, TOL_MIXED)):
+        ov.configure(PARAMS, precision)
+        b = ov.DeviceBatch(t.copy(), off)
+        for tb, ts in ((64, 64), (64, 256), (128, 128), (128, 0)):
+            b.set_tuning(tb, ts)
+            b.update(0.0)
+            b.download()
+            for s, rings in enumerate(systems):
+                ref = orc.update_tangle(system_tangle(rings), PARAMS, 0.0)
+                assert rel_err(b.t.vels[off[s]:off[s + 1]], ref.vels) < tol, (s, tb, ts)
+        b.close()
