@@ -166,10 +166,11 @@ __global__ void __launch_bounds__(kTB) k_direct64_chain(OvParams P, int n_src, c
   for (int sb = s_lo; sb < s_hi; sb += kCS) {
     __syncthreads();
     // nodes sb .. sb + kCS (positions; a slot beyond the range or EMPTY is
-    // used by no chained segment)
+    // used by no chained segment and staged as zero, as chain64_sweep needs a
+    // finite value in each)
     for (int i = threadIdx.x; i <= kCS; i += kTB) {
       const int m = sb + i;
-      const d3 p = m < n_src ? ld3(pos, m) : mk3(0, 0, 0);
+      const d3 p = m < n_src && status[m].x != OV_EMPTY ? ld3(pos, m) : mk3(0, 0, 0);
       sh_node[i][0] = p.x;
       sh_node[i][1] = p.y;
       sh_node[i][2] = p.z;

@@ -1,0 +1,166 @@
+"""GPU: EMPTY slots may hold anything.
+
+A tangle grows by realloc, so the position of an EMPTY slot can be any bit
+pattern.  Every entry point must give the live nodes the same values whatever
+the EMPTY slots hold: each call with NaN (of either sign), an infinity or 1e300
+in the holes against the same call with the box centre.  FP64 bit for bit;
+the mixed sums in slot order add their unchained segments in no fixed order (two
+runs of the same input differ by 1e-11), so the mixed form to its tolerance."""
+import ctypes as C
+
+import numpy as np
+import pytest
+
+from cases import rel_err
+from openvort_b200 import geometry as G
+from openvort_b200._lib import Vec3d
+from openvort_b200.tangle import Flow, Params
+
+pytestmark = pytest.mark.gpu
+
+VALUES = [np.nan, -np.nan, np.inf, 1e300]
+IDS = ["nan", "-nan", "inf", "1e300"]
+D, DT, TOL_MIXED = 0.1, 1e-6, 1e-5
+PARAMS = dict(kappa=9.97e-4, core_a=1e-8, alpha=0.098, alpha_p=0.016, use_mf=1, dl_max=1e-3, bh_theta=0.5,
+              vn=Flow("simple", {"external_v": (0.5, 0, 0)}))
+
+
+@pytest.fixture(scope="module")
+def ov():
+    import openvort_b200 as ov
+    lib = ov.load()
+    assert lib.ov_init(0) == 0, lib.ov_last_error_message()
+    yield ov
+    ov.configure(Params(**PARAMS), ov.OV_PREC_FP64)
+
+
+def same(a, b, precision):
+    if not np.all(np.isfinite(a)):
+        return False
+    return np.array_equal(a, b) if precision == 0 else rel_err(b, a) < TOL_MIXED
+
+
+def holed(t, value):
+    """t with `value` at its EMPTY slots"""
+    out = t.copy()
+    out.pos[~t.active] = value
+    assert (~t.active).sum() >= 7
+    return out
+
+
+# around the block of 128 slots whose small sums take the geometry along; more
+# than the interactions of such a sum; Barnes-Hut
+@pytest.mark.parametrize("value", VALUES, ids=IDS)
+@pytest.mark.parametrize("precision", [0, 1])
+@pytest.mark.parametrize("boundary,rings,use_bh", [("open", 2, 0), ("periodic-26", 4, 0), ("periodic-26", 40, 0),
+                                                   ("periodic-26", 12, 1)])
+def test_updates_runs_and_points(ov, boundary, rings, use_bh, precision, value):
+    t = G.random_ring_tangle(5 + rings, rings, D, boundary=boundary, empty_slots=7)
+    p = Params(use_bh=use_bh, **PARAMS)
+    pts = np.random.default_rng(1).uniform(0, D, size=(40, 3))
+    got = []
+    for hole in (D / 2, value):
+        ov.configure(p, precision)
+        h = holed(t, hole)
+        ov.update_tangle(h, 0.0)
+        res = [h.vels[t.active], h.vs[t.active], h.tangents[t.active], h.normals[t.active]]
+        ov.rk4_step(h, 0.0, DT)
+        res.append(h.pos[t.active])
+        st = ov.DeviceState(holed(t, hole))
+        st.run(0.0, DT, 2)
+        st.download()
+        res += [st.t.pos[t.active], st.t.vels[t.active], st.eval_points(pts, method=0), st.eval_points(pts, method=1)]
+        st.close()
+        lib = ov.load()
+        h = holed(t, hole)
+        v = lib.calculate_vs(h.ptr(), Vec3d((C.c_double * 3)(*pts[0])), -1)
+        res.append(np.array(v.p[:]))
+        k = int(np.nonzero(t.active)[0][3])
+        ov.update_tangle(h, 0.0)
+        lib.update_velocity(h.ptr(), k, 0.0, None)
+        ov.check(lib)
+        res.append(h.vels[k])
+        got.append(res)
+    for i, (a, b) in enumerate(zip(*got)):
+        assert same(a, b, precision), i
+
+
+@pytest.mark.parametrize("value", VALUES, ids=IDS)
+@pytest.mark.parametrize("systems", [3, 400])
+def test_fp64_ensembles(ov, systems, value):
+    """Few systems (their sources summed in shares) and many."""
+    t, off = holed_ensemble(systems)
+    assert_same_ensemble(ov, t, off, value, ov.OV_PREC_FP64, [(128, 128), (64, 0)])
+
+
+def holed_ensemble(systems):
+    """ring pairs of 5 .. 140 nodes a ring, with EMPTY slots at the front, in
+    the middle and at the end of each system"""
+    rng = np.random.default_rng(systems)
+    parts, off = [], [0]
+    for _ in range(systems):
+        rings = [G.ring_points(rng.uniform(-0.02, 0.02, 3), rng.normal(size=3), rng.uniform(5e-3, 1e-2),
+                               int(rng.integers(5, 140))) for _ in range(2)]
+        parts.append(rings)
+    pos, fwd, rev, status = [], [], [], []
+    for rings in parts:
+        n0 = off[-1]
+        at = n0 + 2
+        for r in rings:
+            n, i = len(r), np.arange(len(r))
+            pos += [np.zeros((2, 3)), r]
+            fwd += [[-1, -1], at + (i + 1) % n]
+            rev += [[-1, -1], at + (i - 1) % n]
+            status += [[-1, -1], np.zeros(n, int)]
+            at += n + 2
+        pos.append(np.zeros((1, 3)))
+        fwd.append([-1])
+        rev.append([-1])
+        status.append([-1])
+        off.append(at - 1)
+    from openvort_b200.tangle import HostTangle
+    cat = lambda x: np.concatenate(x).astype(np.int32)
+    t = HostTangle(np.concatenate(pos), cat(fwd), cat(rev), cat(status), None, (-0.05,) * 3, (0.05,) * 3, "open")
+    return t, off
+
+
+def assert_same_ensemble(ov, t, off, value, precision, shapes):
+    act = t.active
+    for shape in shapes:
+        got = []
+        for hole in (0.0, value):
+            ov.configure(Params(**PARAMS), precision)
+            b = ov.DeviceBatch(holed(t, hole), off)
+            b.set_tuning(*shape)
+            b.update(0.0)
+            b.download()
+            res = [b.t.vels[act].copy()]
+            b.run(0.0, DT, 2)
+            b.download()
+            got.append(res + [b.t.pos[act].copy()])
+            b.close()
+        for x, y in zip(*got):
+            assert same(x, y, precision), shape
+
+
+@pytest.mark.parametrize("value", VALUES, ids=IDS)
+@pytest.mark.parametrize("precision", [0, 1])
+@pytest.mark.parametrize("boundary", ["open", "periodic-26"])
+def test_reconnection(ov, boundary, precision, value):
+    side = 0.05
+    t = G.random_ring_tangle(17, 40, side, dl=side / 100, boundary=boundary, empty_slots=9)
+    p = Params(**PARAMS)
+    lib = ov.load()
+    got = []
+    for hole in (side / 2, value):
+        ov.configure(p, precision)
+        h = holed(t, hole)
+        ov.update_tangle(h, 0.0)
+        h.recalc[:] = 0
+        n = lib.ov_reconnect_vortices(h.ptr(), 0.0, 2.5 * side / 100, 0.087)
+        ov.check(lib)
+        assert n > 3
+        got.append(h)
+    a, b = got
+    assert np.array_equal(a.links, b.links) and np.array_equal(a.recalc, b.recalc)
+    assert same(a.vels[t.active], b.vels[t.active], precision)
