@@ -245,7 +245,9 @@ __global__ void __launch_bounds__(kVT) k_bs_vjp_targets(double f4pi, ColCut cut,
   for (int base = s_lo; base < s_hi; base += kVT) {
     __syncthreads();
     for (int i = threadIdx.x; i <= kVT; i += kVT) {
-      const d3 p = base + i < n ? ld3(pos, base + i) : mk3(0, 0, 0);
+      const int j = base + i;
+      // an EMPTY slot may hold anything, and a pair left out is multiplied by zero
+      const d3 p = j < n && status[j].x != OV_EMPTY ? ld3(pos, j) : mk3(0, 0, 0);
       nd[i][0] = p.x; nd[i][1] = p.y; nd[i][2] = p.z;
     }
     const int m = base + threadIdx.x;
@@ -305,7 +307,8 @@ __global__ void __launch_bounds__(kVT) k_bs_vjp_segments(double f4pi, ColCut cut
                                                          const int2* __restrict__ status,
                                                          const double* __restrict__ gnl, double* xbar,
                                                          int n, int chunk) {
-  __shared__ double sh[kVT][6];   // target position and its cotangent (zero: no target)
+  __shared__ double sh[kVT][6];          // target position and its cotangent
+  __shared__ unsigned sh_target[kVT / 32];   // slots that are targets
   const int t_lo = blockIdx.y * chunk, t_hi = min(n, t_lo + chunk);   // this block's targets
   const int m = blockIdx.x * kVT + threadIdx.x;
   int f = -1;
@@ -317,14 +320,17 @@ __global__ void __launch_bounds__(kVT) k_bs_vjp_segments(double f4pi, ColCut cut
     __syncthreads();
     const int k = base + threadIdx.x;
     const bool t_ok = k < t_hi && status[k].x == OV_FREE;
-    const d3 r = k < t_hi ? ld3(pos, k) : mk3(0, 0, 0);
+    const d3 r = t_ok ? ld3(pos, k) : mk3(0, 0, 0);
     const d3 g = t_ok ? ld3(gnl, k) : mk3(0, 0, 0);
+    const unsigned targets = __ballot_sync(0xffffffffu, t_ok);
+    if ((threadIdx.x & 31) == 0) sh_target[threadIdx.x >> 5] = targets;
     sh[threadIdx.x][0] = r.x; sh[threadIdx.x][1] = r.y; sh[threadIdx.x][2] = r.z;
     sh[threadIdx.x][3] = g.x; sh[threadIdx.x][4] = g.y; sh[threadIdx.x][5] = g.z;
     __syncthreads();
     if (f < 0) continue;
     const int cnt = min(kVT, t_hi - base);
     for (int i0 = 0; i0 < cnt; i0 += kVGroup) {
+      const unsigned tb = sh_target[i0 >> 5] >> (i0 & 31);
       bool slow[kVGroup], any = false;
 #pragma unroll
       for (int q = 0; q < kVGroup; ++q) {
@@ -335,7 +341,7 @@ __global__ void __launch_bounds__(kVT) k_bs_vjp_segments(double f4pi, ColCut cut
         const double ia = rsqrt_nr(R2), ib = rsqrt_nr(Rp2);
         const double u = ia * ib, den = fma(dot3(R, Rp), u, 1.0);
         const int c = vjp_case(cut, R2, Rp2, den);
-        const bool on = i0 + q < cnt;
+        const bool on = (tb >> q) & 1u;
         slow[q] = on && c == 2;
         any = any || slow[q];
         const VjpCoef o = vjp_coef(R, Rp, R2, Rp2, ia, ib, u, den, g, on && c == 1);
@@ -616,6 +622,11 @@ ov_adjoint* ov_adjoint_create(const struct tangle_state* t) {
   a->hdr.vnodes = nullptr;
   a->n = t->N;
   bool ok = ov_upload_tangle(&a->s, t) && reserve_all(a);
+  // stage positions of EMPTY slots are never written: keep them defined
+  for (DevBuf& y : a->y)
+    ok = ok && ov_cuda_ok(cudaMemcpyAsync(y.p, a->s.pos.p, sizeof(double) * 3 * (size_t)a->n, cudaMemcpyDeviceToDevice,
+                                          a->s.stream),
+                          "cudaMemcpyAsync");
   if (ok) {
     // the normal-fluid vector of vn_conf when it is "simple"
     if (a->s.P.vn.kind == OVF_SIMPLE)

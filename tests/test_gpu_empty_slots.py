@@ -164,3 +164,33 @@ def test_reconnection(ov, boundary, precision, value):
     a, b = got
     assert np.array_equal(a.links, b.links) and np.array_equal(a.recalc, b.recalc)
     assert same(a.vels[t.active], b.vels[t.active], precision)
+
+
+@pytest.mark.parametrize("value", VALUES, ids=IDS)
+@pytest.mark.parametrize("nodes", [30, 127, 301])
+def test_adjoint(ov, nodes, value):
+    """Velocity, its vector-Jacobian product and the gradient through four
+    steps, two from a checkpoint.  The pair passes add with atomics, in no fixed
+    order: some hundred roundings of partial sums up to a few ten times the
+    result, so 1e-12 of the largest entry."""
+    from openvort_b200.adjoint import Adjoint
+    rng = np.random.default_rng(nodes)
+    rings = [G.ring_points(c, rng.normal(size=3), 1e-2, n)
+             for c, n in (((0, 0, 0), nodes // 3), ((5e-3, 0, 0), nodes - nodes // 3))]
+    t = G.rings_to_tangle(rings, (-0.05,) * 3, (0.05,) * 3, "open", empty_slots=9)
+    act = t.active
+    g = np.where(act[:, None], rng.normal(size=(t.n, 3)), 0.0)
+    vn = np.array([0.2, 0.0, 0.1])
+    got = []
+    for hole in (0.0, value):
+        ov.configure(Params(**PARAMS), ov.OV_PREC_FP64)
+        h = holed(t, hole)
+        a = Adjoint(h)
+        x_bar, vn_bar = a.velocity_vjp(h.pos, g, vn)
+        res = [a.velocity(h.pos, vn)[act], x_bar[act], vn_bar]
+        res.append(a.forward(h.pos, vn, 0.0, DT, 4, every=2)[act])
+        x_bar, vn_bar = a.backward(g)
+        got.append(res + [x_bar[act], vn_bar])
+        a.close()
+    for i, (a, b) in enumerate(zip(*got)):
+        assert np.all(np.isfinite(b)) and np.abs(a - b).max() <= 1e-12 * np.abs(a).max(), i
