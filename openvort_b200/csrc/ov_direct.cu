@@ -766,7 +766,7 @@ bool ov_direct_partials(ov_state_impl* s, const double* pos, double* v_nl, doubl
       ov_mark(s, s->ev1);
       ov_mark(s, s->ev2);
       OV_TRY_CUDA(cudaMemsetAsync(v_nl, 0, sizeof(double) * 3 * s->n, s->stream));
-      OV_TRY_CUDA(cudaMemsetAsync(v_img, 0, sizeof(double) * 3 * s->n, s->stream));
+      if (v_img) OV_TRY_CUDA(cudaMemsetAsync(v_img, 0, sizeof(double) * 3 * s->n, s->stream));
       return true;
     }
     const int bx = (n_t + kPTgt - 1) / kPTgt;

@@ -194,3 +194,22 @@ def test_adjoint(ov, nodes, value):
         a.close()
     for i, (a, b) in enumerate(zip(*got)):
         assert np.all(np.isfinite(b)) and np.abs(a - b).max() <= 1e-12 * np.abs(a).max(), i
+
+
+@pytest.mark.parametrize("precision", [0, 1])
+def test_adjoint_without_nodes(ov, precision):
+    """Slots that are all EMPTY: nothing moves, and the gradient passes through."""
+    from openvort_b200.adjoint import Adjoint
+    from openvort_b200.tangle import HostTangle
+    n = 6
+    none = -np.ones(n, np.int32)
+    t = HostTangle(np.ones((n, 3)), none, none, none, none, (-0.05,) * 3, (0.05,) * 3, "open")
+    ov.configure(Params(**PARAMS), precision)
+    a = Adjoint(t)
+    g = np.random.default_rng(2).normal(size=(n, 3))
+    assert np.array_equal(a.forward(t.pos, np.zeros(3), 0.0, DT, 3, every=2), t.pos)
+    x_bar, vn_bar = a.backward(g)
+    assert np.array_equal(x_bar, g) and np.all(vn_bar == 0)
+    x_bar, vn_bar = a.velocity_vjp(t.pos, g, np.zeros(3))
+    assert np.all(x_bar == 0) and np.all(vn_bar == 0)
+    a.close()
