@@ -193,9 +193,11 @@ __host__ __device__ __forceinline__ ColCut col_cut_of(double col) {
 // surely inside (the segment adds nothing), above kEndWord + 1 surely
 // outside, and at these two words the reference's own square root decides.
 // A node's own two segments end at the node itself and are inside.
-constexpr int kEndWord = 0x3c9cd2b2;
-__device__ __forceinline__ bool end_inside(double R2) { return __double2hiint(R2) < kEndWord; }
-__device__ __forceinline__ bool end_near(double R2) { return __double2hiint(R2) <= kEndWord + 1; }
+// |R|^2 is not negative, so the words compare as unsigned, where a NaN of
+// either sign is outside.
+constexpr unsigned kEndWord = 0x3c9cd2b2;
+__device__ __forceinline__ bool end_inside(double R2) { return (unsigned)__double2hiint(R2) < kEndWord; }
+__device__ __forceinline__ bool end_near(double R2) { return (unsigned)__double2hiint(R2) <= kEndWord + 1; }
 
 // The reference's segment formula without IEEE square roots and divisions:
 // with u = 1/(|R||R'|) from two refined reciprocal square roots,
