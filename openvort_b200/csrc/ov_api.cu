@@ -459,7 +459,7 @@ static void state_release(ov_state_impl* s) {
   DevBuf* bufs[] = {&s->pos, &s->links, &s->status, &s->dxi, &s->tan, &s->nrm, &s->vels, &s->vs,
                     &s->pos0, &s->spos, &s->sdxi, &s->stan, &s->snrm, &s->svs, &s->k2, &s->k3,
                     &s->k4, &s->v_nl, &s->v_img, &s->img_part, &s->seg64, &s->segid, &s->dflag,
-                    &s->xown};
+                    &s->xown, &s->walk_part, &s->pkeys, &s->pvals, &s->phist, &s->pscan};
   for (DevBuf* b : bufs) b->release();
   ov_tree_release(&s->tree);
   if (s->stream) cudaStreamDestroy(s->stream);
@@ -980,9 +980,13 @@ ov_state_impl& tls_state() {
   return *s;
 }
 
-// The device-side tree behind an opaque struct octree*.
+// The device-side tree behind an opaque struct octree*.  Threads may query one
+// tree at the same time: update_velocity and update_velocities walk it with
+// the calling thread's state and only read it; octree_get_vs uses the tree's
+// own, one call at a time (they would follow one another on its stream anyway).
 struct TreeHandle {
   ov_state_impl st;   // its own node snapshot, stream and buffers
+  std::mutex get_vs;
 };
 }  // namespace
 
@@ -1201,6 +1205,7 @@ void octree_get_vs(const struct octree* tree, const struct vec3d* r, double reso
   if (!res) return;
   memset(res, 0, sizeof(*res));
   if (!tree || !r) return;
+  std::lock_guard<std::mutex> lock(const_cast<struct octree*>(tree)->h.get_vs);
   ov_state_impl* s = const_cast<ov_state_impl*>(&tree->h.st);
   s->P.precision = g_precision;
   DevBuf q;

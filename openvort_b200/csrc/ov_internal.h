@@ -101,8 +101,6 @@ struct OvTree {
   DevBuf scan_part;     // block sums of the exclusive scans
   DevBuf mom_part;      // per-chunk partial moments of the largest cells
   DevBuf walk_order;    // the walk's target list when nodes lie outside the root box
-  DevBuf walk_part;     // partial sums of a walk split over several warps per group
-  DevBuf pkeys, pvals;  // point queries: sort keys and order
   // the multi-image walk's units (groups of 32 targets, or their parts) by
   // decreasing time in the last walk (wvals after the sort), their times,
   // and the sort's buffers
@@ -165,6 +163,10 @@ struct ov_state_impl {
   DevBuf pos0, spos, sdxi, stan, snrm, svs, k2, k3, k4;
   // Biot-Savart outputs: primary sum and image sum per slot
   DevBuf v_nl, v_img;
+  // what a tree walk writes besides its results: several threads may walk one
+  // tree at a time, each with its own state, so none of it is the tree's
+  DevBuf walk_part;                    // partial sums of a walk split over several warps per group
+  DevBuf pkeys, pvals, phist, pscan;   // point queries: sort keys and order, the sort's counts
   // direct-sum per-image partials and segment table
   DevBuf img_part, seg64, segid;
   OvSums sums = {nullptr, nullptr, nullptr, 0};   // of the evaluation under way

@@ -878,8 +878,8 @@ void ov_tree_release(OvTree* t) {
   DevBuf* bufs[] = {&t->keys, &t->keys_alt, &t->vals, &t->vals_alt, &t->stop, &t->hist,
                     &t->perm, &t->bnode, &t->cstart_cnt, &t->cbase, &t->cell_of, &t->cells,
                     &t->cell_lm, &t->cell_range, &t->nodes64, &t->nodeids, &t->nodes32, &t->counters,
-                    &t->scratch, &t->scan_part, &t->mom_part, &t->walk_order, &t->walk_part, &t->pkeys,
-                    &t->pvals, &t->warp_cost, &t->wkeys, &t->wkeys2, &t->wvals, &t->wvals2, &t->whist, &t->wscan};
+                    &t->scratch, &t->scan_part, &t->mom_part, &t->walk_order, &t->warp_cost,
+                    &t->wkeys, &t->wkeys2, &t->wvals, &t->wvals2, &t->whist, &t->wscan};
   for (DevBuf* b : bufs) b->release();
   t->n_nodes = t->n_cells = t->built = t->n_perm_warps = 0;
 }

@@ -1351,10 +1351,9 @@ static __global__ void k_curve_keys(OvParams P, const double* pts, const int* sl
 constexpr int kMaxParts = 16;        // warps a group of nodes' walk is split over, at most
 constexpr int kMaxPointParts = 32;   // and a group of points'
 
-static bool read_counters(ov_state_impl* s, OvTree* t) {
+static bool read_counters(ov_state_impl* s, const unsigned long long* ctr) {
   unsigned long long c[3] = {0, 0, 0};
-  OV_TRY_CUDA(cudaMemcpyAsync(c, t->counters.as<char>() + 64, sizeof(c), cudaMemcpyDeviceToHost,
-                              s->stream));
+  OV_TRY_CUDA(cudaMemcpyAsync(c, ctr, sizeof(c), cudaMemcpyDeviceToHost, s->stream));
   OV_TRY_CUDA(cudaStreamSynchronize(s->stream));
   OvStatsAcc& st = ov_stats_tls();
   st.interactions = (double)c[0];
@@ -1459,8 +1458,8 @@ static bool launch_multi(ov_state_impl* s, OvTree* t, const OvParams& P, const i
   WalkSplit W{parts, frontier, deal, skip, nullptr, nullptr};
   if (split) {
     const size_t per = 3 * (size_t)n_t * parts;
-    if (!t->walk_part.reserve(sizeof(double) * (mixed ? 1 : 2) * per)) return false;
-    W.nl = t->walk_part.as<double>();
+    if (!s->walk_part.reserve(sizeof(double) * (mixed ? 1 : 2) * per)) return false;
+    W.nl = s->walk_part.as<double>();
     W.im = mixed ? nullptr : W.nl + per;
   }
   // Longest first: the launch runs the warps' units (groups of 32 targets,
@@ -1476,8 +1475,6 @@ static bool launch_multi(ov_state_impl* s, OvTree* t, const OvParams& P, const i
   if (timed) {
     if (!t->warp_cost.reserve(sizeof(unsigned) * (size_t)warps)) return false;
     wcost = t->warp_cost.as<unsigned>();
-  } else {
-    t->n_perm_warps = 0;
   }
   auto kernel = split ? (mixed ? k_walk_multi<true, true> : k_walk_multi<false, true>)
                       : (mixed ? k_walk_multi<true, false> : k_walk_multi<false, false>);
@@ -1597,7 +1594,7 @@ bool ov_tree_walk_points(ov_state_impl* s, OvTree* t, int npts, const double* pt
     if (out_img) OV_TRY_CUDA(cudaMemsetAsync(out_img, 0, sizeof(double) * 3 * npts, s->stream));
     return true;
   }
-  unsigned long long* ctr = reinterpret_cast<unsigned long long*>(t->counters.as<char>() + 64);
+  unsigned long long* ctr = s->evctr.as<unsigned long long>() + 3 * s->pending;
   OV_TRY_CUDA(cudaMemsetAsync(ctr, 0, 24, s->stream));
   OvParams P = t->P;
   P.n_img = s->P.n_img;
@@ -1615,20 +1612,20 @@ bool ov_tree_walk_points(ov_state_impl* s, OvTree* t, int npts, const double* pt
     const int* order = nullptr;
     if (npts > 32) {
       const size_t np = (size_t)npts;
-      if (!t->pkeys.reserve(sizeof(uint64_t) * 2 * np) || !t->pvals.reserve(sizeof(int) * 2 * np)) return false;
-      uint64_t* keys = t->pkeys.as<uint64_t>();
-      int* vals = t->pvals.as<int>();
+      if (!s->pkeys.reserve(sizeof(uint64_t) * 2 * np) || !s->pvals.reserve(sizeof(int) * 2 * np)) return false;
+      uint64_t* keys = s->pkeys.as<uint64_t>();
+      int* vals = s->pvals.as<int>();
       OV_TRY_CUDA(ov_launch_early(k_curve_keys, dim3((npts + 255) / 256), 256, s->stream, P, pts, nullptr, npts, keys,
                                   vals));
       OV_LAUNCHED();
-      if (!ov_radix_sort_u64(keys, vals, keys + np, vals + np, npts, 3 * kCurveBits, t->whist, t->wscan, s->stream))
+      if (!ov_radix_sort_u64(keys, vals, keys + np, vals + np, npts, 3 * kCurveBits, s->phist, s->pscan, s->stream))
         return false;
       order = vals;
     }
     P.precision = OV_PREC_FP64;
     if (!launch_multi(s, t, P, order, nullptr, skip, pts, npts, npts, combos, out_nl, out_img, ctr, false))
       return false;
-    return read_counters(s, t);
+    return read_counters(s, ctr);
   }
   const int warps = (npts + 31) / 32;
   const int blocks = (warps * 32 + 127) / 128;
@@ -1644,7 +1641,7 @@ bool ov_tree_walk_points(ov_state_impl* s, OvTree* t, int npts, const double* pt
     OV_LAUNCHED();
   }
   OV_TRY_CUDA(cudaGetLastError());
-  return read_counters(s, t);
+  return read_counters(s, ctr);
 }
 
 // ---------------------------------------------------------------- shards
