@@ -84,6 +84,7 @@ struct OvTree {
   int n_nodes = 0;      // active (non-EMPTY) nodes
   int n_drop_root = 0;  // active nodes outside the root box (sorted last)
   int n_cells = 0;
+  int has_ranges = 0;   // some cell sums a node range (LEAFN, OPEN_P2P)
   int built = 0;
   int flag_seen = 0;    // the state's error flag when the build was read back
   double theta = 0;     // theta used for thr

@@ -593,6 +593,7 @@ __global__ void k_write_cells(const BNode* nodes, const int* leaf_parent,
     c.a = first;
     c.b = last - first + 1;
   }
+  if (ci.kind == CELL_LEAFN || ci.kind == CELL_OPEN_P2P) tail[2] = 1;
   cell_range[idx] = make_int2(first, last - first + 1);
   if (ci.mac_level >= 0) {
     // replay the descent to the tested level to get the reference's box
@@ -978,7 +979,7 @@ bool ov_tree_build(ov_state_impl* s, const double* pos, OvTree* T, bool order_on
   int* term = vals_alt + n;
   int* ctr = T->counters.as<int>();
   int hc[16];   // the device counters: active nodes, depth error, deepest level, nodes outside the
-                // box, cells per moment class (3), cells, the state's error flag
+                // box, cells per moment class (3), cells, the state's error flag, cells with a node range
   OV_TRY_CUDA(cudaMemsetAsync(ctr, 0, sizeof(int) * 16, st));
   if (n > 0) {
     OV_TRY_CUDA(ov_launch_early(k_keys, dim3((n + 255) / 256), 256, st, s->P, pos, s->status.as<int2>(), n, khi,
@@ -988,7 +989,7 @@ bool ov_tree_build(ov_state_impl* s, const double* pos, OvTree* T, bool order_on
   }
   const int na = s->n_active;   // as counted by the upload
   T->n_nodes = na;
-  T->n_drop_root = T->flag_seen = 0;
+  T->n_drop_root = T->flag_seen = T->has_ranges = 0;
   // radix sort over the high word (8 passes of 8 bits), stable; vals_alt's
   // second half holds the sorted term codes, so the values alternate with a
   // separate scratch.  The sorted data ends back in khi / vals.
@@ -1071,6 +1072,7 @@ bool ov_tree_build(ov_state_impl* s, const double* pos, OvTree* T, bool order_on
     if (!read_build(s, T, ctr, hc)) return false;
     T->n_cells = hc[7];
     T->flag_seen = hc[8];
+    T->has_ranges = hc[9];
     const int* lc = hc + 4;
     const double f4 = s->P.f4pi;
     if (lc[0] > 0) {

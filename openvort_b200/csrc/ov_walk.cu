@@ -867,9 +867,11 @@ __device__ __forceinline__ d3 shfl3(d3 v, int src) {
 // lane of the warp, whichever lane's target they belong to.  A leaf is near 8
 // to 10 of a group's 32 targets and an accepted cell is one for 20 to 24 of
 // them, so evaluated at the visit they leave the other lanes idle.  A target's
-// pairs are taken in preorder and added in that order by its own lane, the
-// segments' sum apart from the cells', so the sums do not depend on the other
-// targets of the group.  Segments wait in both forms: 200k / 1M nodes mixed
+// pairs are taken in preorder and added in that order by its own lane.  When a
+// queue's are depends on the other targets of the group, so each queue's pairs
+// have a sum of their own, to which nothing else is added, and a target's sums
+// do not depend on its group.  A grain leaf's node range waits with the
+// segments where cells wait.  Segments wait in both forms: 200k / 1M nodes mixed
 // 5.04 -> 4.62 / 25.7 -> 23.8 ms, FP64 10.0 -> 8.3 / 51.2 -> 43.5.  Cells wait
 // in the FP64 form, where their evaluation takes the FP64 pipe some 400
 // operations: 8.3 -> 7.6 / 43.5 -> 38.8; in the mixed form the queue costs more
@@ -921,7 +923,10 @@ __device__ __forceinline__ WalkBatch queue_take(WalkQueue& Q, int& n, unsigned* 
   return e;
 }
 
-template <bool kMixed, bool kSplit>
+// kRanges: the tree has grain leaves of several nodes.  The FP64 form has
+// kernels of its own without them: with the loop over a node range they take
+// 2% longer over trees that have none (200k nodes 7.93 ms, against 7.74).
+template <bool kMixed, bool kSplit, bool kRanges>
 __global__ void __launch_bounds__(32, kMixed || kSplit ? kWalkWarps : kWalkWarpsFp64)
     k_walk_multi(
     OvParams P, TreeView T, const int* __restrict__ order, const int2* __restrict__ status,
@@ -933,7 +938,7 @@ __global__ void __launch_bounds__(32, kMixed || kSplit ? kWalkWarps : kWalkWarps
   __shared__ WalkQueue cells;                     // accepted cells and their targets
   __shared__ unsigned sh_of[32];                  // entries of each lane's target
   __shared__ double sh_seg[kMixed ? 3 : 6][32];   // each lane's sums over segments
-  constexpr bool kQueueCells = !kMixed;
+  constexpr bool kQueueCells = !kMixed, kQueueRanges = kQueueCells && kRanges;
   const unsigned FULL = 0xffffffffu;
   const int lane = threadIdx.x;
   const long long t_start = clock64();
@@ -1003,12 +1008,30 @@ __global__ void __launch_bounds__(32, kMixed || kSplit ? kWalkWarps : kWalkWarps
       d3 v = mk3(0, 0, 0), w = v;
       if (e.on) {
         const Cell* cp = T.cells + e.cell;
-        const int2 id = *reinterpret_cast<const int2*>(cp);
-        const d3 r1 = mk3(cp->x[0], cp->x[1], cp->x[2]), r2 = mk3(cp->y[0], cp->y[1], cp->y[2]);
-        if (kMixed && __popc(e.mask) >= kColumnImages)
-          p2p_mixed_columns(P, e.mask, rt, r1, r2, id.x, id.y, skip_t, near2, v, n_p2p);
-        else
-          p2p_images<kMixed>(P, e.mask, rt, r1, r2, id.x, id.y, skip_t, near2, v, w, n_p2p);
+        const int4 eh = *reinterpret_cast<const int4*>(cp);
+        int2 id = make_int2(eh.x, eh.y);
+        d3 r1 = mk3(cp->x[0], cp->x[1], cp->x[2]), r2 = mk3(cp->y[0], cp->y[1], cp->y[2]);
+        int j = 0, end = 1;
+        auto load = [&]() {
+          const double* nd = T.nodes64 + 6 * (size_t)j;
+          id = T.nodeids[j];
+          r1 = mk3(nd[0], nd[1], nd[2]);
+          r2 = mk3(nd[3], nd[4], nd[5]);
+        };
+        if (kQueueRanges && cell_kind(eh.w) != CELL_LEAF1) {
+          const int2 rg = T.cell_range[e.cell];
+          j = max(rg.x, 0);
+          end = min(rg.x + rg.y, T.n_nodes);
+          if (j < end) load();
+        }
+        while (j < end) {
+          if (kMixed && __popc(e.mask) >= kColumnImages)
+            p2p_mixed_columns(P, e.mask, rt, r1, r2, id.x, id.y, skip_t, near2, v, n_p2p);
+          else
+            p2p_images<kMixed>(P, e.mask, rt, r1, r2, id.x, id.y, skip_t, near2, v, w, n_p2p);
+          if (!kQueueRanges || ++j >= end) break;
+          load();
+        }
       }
       __syncwarp();
       for (unsigned of = sh_of[lane]; __any_sync(FULL, of != 0); of &= of - 1) {
@@ -1134,8 +1157,10 @@ __global__ void __launch_bounds__(32, kMixed || kSplit ? kWalkWarps : kWalkWarps
       continue;
     }
     if (kQueueCells) queue_put(cells, n_cells, q, cell_mask, lane);
-    // direct sums over a node range (grain leaves), shared by the warp
-    if (__ballot_sync(FULL, p2p_mask != 0)) {
+    // direct sums over a node range (grain leaves)
+    if (kQueueRanges) {
+      if (kind == CELL_LEAFN || kind == CELL_OPEN_P2P) queue_put(leaves, n_leaves, q, p2p_mask, lane);
+    } else if (kRanges && __ballot_sync(FULL, p2p_mask != 0)) {   // shared by the warp
       const int2 rg = T.cell_range[q];
       const int end = min(rg.x + rg.y, T.n_nodes);
       for (int j = max(rg.x, 0); j < end; ++j) {
@@ -1424,8 +1449,8 @@ static bool launch_multi(ov_state_impl* s, OvTree* t, const OvParams& P, const i
   const bool mixed = P.precision == OV_PREC_MIXED;
   const ImageShortcut sc = image_shortcut(P, combos);
   const TreeView tv = view_of(t);
-  static const int wave_mixed = walk_wave(k_walk_multi<true, true>);
-  static const int wave_fp64 = walk_wave(k_walk_multi<false, true>);
+  static const int wave_mixed = walk_wave(k_walk_multi<true, true, true>);
+  static const int wave_fp64 = walk_wave(k_walk_multi<false, true, true>);
   const int wave = mixed ? wave_mixed : wave_fp64;
   // Parts per group.  Nodes: enough that the units make two waves (of 2368
   // warps), so the last wave's slow units are short, but no more than 16, as
@@ -1476,8 +1501,12 @@ static bool launch_multi(ov_state_impl* s, OvTree* t, const OvParams& P, const i
     if (!t->warp_cost.reserve(sizeof(unsigned) * (size_t)warps)) return false;
     wcost = t->warp_cost.as<unsigned>();
   }
-  auto kernel = split ? (mixed ? k_walk_multi<true, true> : k_walk_multi<false, true>)
-                      : (mixed ? k_walk_multi<true, false> : k_walk_multi<false, false>);
+  auto kernel = split ? (mixed         ? k_walk_multi<true, true, true>
+                         : t->has_ranges ? k_walk_multi<false, true, true>
+                                         : k_walk_multi<false, true, false>)
+                      : (mixed         ? k_walk_multi<true, false, true>
+                         : t->has_ranges ? k_walk_multi<false, false, true>
+                                         : k_walk_multi<false, false, false>);
   kernel<<<warps, 32, 0, s->stream>>>(P, tv, order, status, pos, n_t, combos, sc, P.near2, v_nl, v_img, ctr, wperm,
                                       wcost, W);
   OV_LAUNCHED();

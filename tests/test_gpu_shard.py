@@ -160,3 +160,25 @@ def test_more_ranks_than_nodes(ov):
         assert np.array_equal(st.t.pos[t.active], ref.t.pos[t.active])
         st.close()
     ref.close()
+
+
+@pytest.mark.parametrize("precision", [0, 1])
+@pytest.mark.parametrize("rings", [20, 250])
+def test_sharded_steps_with_leaves_of_several_nodes(ov, rings, precision):
+    """A grain of 3e-3 leaves several nodes in a box, which are summed as node
+    ranges among the accepted cells: 3 ranks, whose groups of 32 targets are not
+    those of one run, still equal it bit for bit, with the walk split over many
+    warps and over few."""
+    t = G.random_ring_tangle(23, rings, 0.1, boundary="periodic-26", empty_slots=5)
+    p = Params(core_a=1e-8, alpha=0.098, alpha_p=0.016, use_mf=1, dl_max=1e-3, use_bh=1, bh_theta=0.5,
+               bh_grain=3e-3, vn=Flow("simple", {"external_v": (0.5, 0, 0)}))
+    ov.configure(p, precision)
+    ref = ov.DeviceState(t.copy())
+    ref.run(0.0, DT, 1)
+    ref.download()
+    act = t.active
+    for st in run_ranks(ov, t, 3, 1):
+        assert np.array_equal(st.t.pos[act], ref.t.pos[act])
+        assert np.array_equal(st.t.vels[act], ref.t.vels[act])
+        st.close()
+    ref.close()
