@@ -133,7 +133,6 @@ namespace {
 thread_local int tl_err = OV_OK;
 thread_local char tl_msg[512] = "";
 thread_local OvStatsAcc tl_stats = {0, 0, 0, 0, 0, 0, 0};
-thread_local ov_state_impl* tl_last_state = nullptr;
 int g_precision = OV_PREC_FP64;
 int g_rk4_classic = 0;
 // FP64 near field of the mixed form, in units of global_dl_max: at 8 (and
@@ -436,7 +435,7 @@ void* ov_pinned_scratch() {
 bool ov_state_reserve(ov_state_impl* s, int n) {
   if (!s->stream) {
     OV_TRY_CUDA(cudaStreamCreateWithFlags(&s->stream, cudaStreamNonBlocking));
-    if (!s->dflag.reserve(64) || !s->evctr.reserve(sizeof(unsigned long long) * 3 * kEvalSlots) || !use_slot(s, 0, true))
+    if (!s->dflag.reserve(64) || !s->evctr.reserve(sizeof(unsigned long long) * 3 * (kEvalSlots + 1)) || !use_slot(s, 0, true))
       return false;
     OV_TRY_CUDA(cudaMemsetAsync(s->dflag.p, 0, 64, s->stream));
   }
@@ -614,7 +613,6 @@ bool ov_eval_collect(ov_state_impl* s, const char* where) {
     s->acc_cells += tl_stats.cell_interactions;
     s->acc_warp_iter += tl_stats.warp_iterations;
   }
-  if (pending > 0 && !use_slot(s, 0, true)) return false;   // the timed one's, for ov_get_last_stats
   return ov_flag_status(*flag, where);
 }
 
@@ -639,7 +637,6 @@ static int max_pending(const ov_state_impl* s) {
 // geometry along where asked for.
 static bool bs_sums(ov_state_impl* s, const double* pos, OvTree* external_tree, int k0, int k_count,
                     const OvGeomOut& geom = kNoGeom) {
-  tl_last_state = s;
   if (s->pending >= max_pending(s) && !ov_eval_collect(s, "update_velocities")) return false;
   tl_stats = OvStatsAcc{0, 0, 0, 0, 0, 0, 0};
   if (!use_slot(s, s->pending, s->pending == 0 || !small_sum(s))) return false;
@@ -881,7 +878,6 @@ int ov_state_shard_end(ov_state* st, int q, double t, double dt) {
   if (!shard_ready(s, q)) return tl_err;
   const ShardStage g = shard_stage(s, q, t, dt);
   if (!s->P.lia_only && !ov_shard_unpack(s, s->xbuf, s->xbytes / sizeof(double))) return tl_err;
-  tl_last_state = s;
   if (!finish_velocities(s, g.t, g.pos, g.tan, g.nrm, kNoStage, g.vels, g.vs)) return tl_err;
   if (q == 3 && !ov_rk4_combine(s, dt)) return tl_err;
   if (!ov_eval_collect(s, "update_velocities")) return tl_err;
@@ -950,20 +946,14 @@ int ov_state_eval_points(ov_state* st, int npts, const double* pts, const int* s
 int ov_get_last_stats(ov_eval_stats* out) {
   if (!out) return OV_ERR_INVALID;
   memset(out, 0, sizeof(*out));
-  ov_state_impl* s = tl_last_state;
+  // of the last evaluation that was waited for (ov_eval_collect), its
+  // counters and times alike
   out->interactions = tl_stats.interactions;
   out->cell_interactions = tl_stats.cell_interactions;
   out->cells = tl_stats.cells;
-  if (s && s->stream) {
-    cudaStreamSynchronize(s->stream);
-    float a = 0, b = 0;
-    if (cudaEventElapsedTime(&a, s->ev0, s->ev1) == cudaSuccess) out->build_ms = a;
-    if (cudaEventElapsedTime(&b, s->ev1, s->ev2) == cudaSuccess) out->eval_ms = b;
-    // an event not recorded yet fails the query above; drop that error so
-    // it is not reported by the next launch check
-    (void)cudaGetLastError();
-    out->total_ms = out->build_ms + out->eval_ms;
-  }
+  out->build_ms = tl_stats.build_ms;
+  out->eval_ms = tl_stats.eval_ms;
+  out->total_ms = tl_stats.total_ms;
   return OV_OK;
 }
 

@@ -155,7 +155,7 @@ struct ov_state_impl {
   // and takes their times, counters and error flags
   OvEvalSlot slots[kEvalSlots];
   int pending = 0;
-  DevBuf evctr;         // walk counters, 3 per slot
+  DevBuf evctr;         // walk counters, 3 per slot, and a point query's after them
   // slot-indexed (AoS, 3 doubles per vector, as struct vec3d)
   DevBuf pos, links, status, dxi, tan, nrm, vels, vs;
   // RK4 scratch (two stage positions: an evaluation reads one while its

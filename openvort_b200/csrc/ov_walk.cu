@@ -1516,7 +1516,7 @@ static bool launch_multi(ov_state_impl* s, OvTree* t, const OvParams& P, const i
     OV_LAUNCHED();
     OV_TRY_CUDA(cudaGetLastError());
   }
-  ov_mark(s, s->ev2);
+  if (status) ov_mark(s, s->ev2);   // of an evaluation; a point query is none
   if (timed) {
     // the order for the next walk (after the timed kernel)
     const size_t nw = (size_t)warps;
@@ -1623,7 +1623,7 @@ bool ov_tree_walk_points(ov_state_impl* s, OvTree* t, int npts, const double* pt
     if (out_img) OV_TRY_CUDA(cudaMemsetAsync(out_img, 0, sizeof(double) * 3 * npts, s->stream));
     return true;
   }
-  unsigned long long* ctr = s->evctr.as<unsigned long long>() + 3 * s->pending;
+  unsigned long long* ctr = s->evctr.as<unsigned long long>() + 3 * kEvalSlots;
   OV_TRY_CUDA(cudaMemsetAsync(ctr, 0, 24, s->stream));
   OvParams P = t->P;
   P.n_img = s->P.n_img;
