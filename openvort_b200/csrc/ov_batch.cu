@@ -149,8 +149,17 @@ __global__ void __launch_bounds__(TB) k_batch_bs_mixed(OvParams P, BatchView B,
     const int2 src = kShares ? source_share(B, s0, s1, w.z) : make_int2(s0, s1);
     const double near2 = B.near2[w.x];
     // two-float offsets from the item's first target; single-rounded ones
-    // from its middle target
-    const d3 O = ld3(pos, kTwo ? w.y : w.y + min(TB * kTT, s1 - w.y) / 2);
+    // from its middle target; where that slot is EMPTY, and may hold anything,
+    // from the next live one (or the one before)
+    const int mid = kTwo ? w.y : w.y + min(TB * kTT, s1 - w.y) / 2;
+    d3 O = ld3(pos, mid);
+    if (status[mid].x == OV_EMPTY) {
+      int o = mid;
+      while (o < s1 && status[o].x == OV_EMPTY) ++o;
+      if (o == s1)
+        for (o = mid; o > s0 && status[o].x == OV_EMPTY;) --o;
+      O = status[o].x != OV_EMPTY ? ld3(pos, o) : mk3(0, 0, 0);
+    }
     int kk[kTT];
     PairTargets T;
     double acc[kTT][3];

@@ -93,6 +93,15 @@ def test_fp64_ensembles(ov, systems, value):
     assert_same_ensemble(ov, t, off, value, ov.OV_PREC_FP64, [(128, 128), (64, 0)])
 
 
+@pytest.mark.parametrize("value", VALUES, ids=IDS)
+@pytest.mark.parametrize("systems", [3, 400])
+def test_mixed_ensembles(ov, systems, value):
+    """Every kind of mixed kernel: offsets from the first target, from the
+    middle one, and in chain order."""
+    t, off = holed_ensemble(systems)
+    assert_same_ensemble(ov, t, off, value, ov.OV_PREC_MIXED, [(128, 128), (256, 64), (64, 64), (64, 256), (128, 0)])
+
+
 def holed_ensemble(systems):
     """ring pairs of 5 .. 140 nodes a ring, with EMPTY slots at the front, in
     the middle and at the end of each system"""
