@@ -247,7 +247,8 @@ __global__ void __launch_bounds__(kVT) k_bs_vjp_targets(double f4pi, ColCut cut,
     for (int i = threadIdx.x; i <= kVT; i += kVT) {
       const int j = base + i;
       // an EMPTY slot may hold anything, and a pair left out is multiplied by zero
-      const d3 p = j < n && status[j].x != OV_EMPTY ? ld3(pos, j) : mk3(0, 0, 0);
+      d3 p = j < n ? ld3(pos, j) : mk3(0, 0, 0);
+      if (j < n && status[j].x == OV_EMPTY) p = mk3(0, 0, 0);
       nd[i][0] = p.x; nd[i][1] = p.y; nd[i][2] = p.z;
     }
     const int m = base + threadIdx.x;
@@ -329,8 +330,9 @@ __global__ void __launch_bounds__(kVT) k_bs_vjp_segments(double f4pi, ColCut cut
     __syncthreads();
     if (f < 0) continue;
     const int cnt = min(kVT, t_hi - base);
+    unsigned tb = 0;
     for (int i0 = 0; i0 < cnt; i0 += kVGroup) {
-      const unsigned tb = sh_target[i0 >> 5] >> (i0 & 31);
+      tb = i0 & 31 ? tb >> kVGroup : sh_target[i0 >> 5];
       bool slow[kVGroup], any = false;
 #pragma unroll
       for (int q = 0; q < kVGroup; ++q) {

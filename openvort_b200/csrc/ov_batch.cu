@@ -85,7 +85,8 @@ __global__ void __launch_bounds__(TB) k_batch_bs64(OvParams P, BatchView B,
       __syncthreads();
       for (int q = threadIdx.x; q <= TS; q += TB) {
         const int m = base + q;
-        const d3 a = m < s1 && status[m].x != OV_EMPTY ? ld3(pos, m) : mk3(0, 0, 0);
+        d3 a = m < s1 ? ld3(pos, m) : mk3(0, 0, 0);
+        if (m < s1 && status[m].x == OV_EMPTY) a = mk3(0, 0, 0);
         sh_node[q][0] = a.x;
         sh_node[q][1] = a.y;
         sh_node[q][2] = a.z;

@@ -170,7 +170,8 @@ __global__ void __launch_bounds__(kTB) k_direct64_chain(OvParams P, int n_src, c
     // finite value in each)
     for (int i = threadIdx.x; i <= kCS; i += kTB) {
       const int m = sb + i;
-      const d3 p = m < n_src && status[m].x != OV_EMPTY ? ld3(pos, m) : mk3(0, 0, 0);
+      d3 p = m < n_src ? ld3(pos, m) : mk3(0, 0, 0);
+      if (m < n_src && status[m].x == OV_EMPTY) p = mk3(0, 0, 0);
       sh_node[i][0] = p.x;
       sh_node[i][1] = p.y;
       sh_node[i][2] = p.z;
