@@ -106,7 +106,7 @@ __global__ void __launch_bounds__(TB) k_batch_bs64(OvParams P, BatchView B,
       if (!act) continue;
       chain64_sweep<false>(sh_node, sh_chain, sh_other, min(TS, src.y - base), -2, r, cut, acc, [&](int i) {
         const d3 r1 = ld3(pos, base + i), r2 = ld3(pos, links[base + i].x);
-        return seg_vel64_nr(1.0, r1, r2, r2 - r1, r, cut);
+        return seg_vel64_nr(1.0, r1, r2, r, cut);
       });
     }
     if (k < s1) out(kShares ? w.z : 0, k, act, acc * P.f4pi);
@@ -177,7 +177,7 @@ __global__ void __launch_bounds__(TB) k_batch_bs_mixed(OvParams P, BatchView B,
       const int k = u ? kk[1] : kk[0];
       if (k < 0 || id < 0) return;
       const d3 r1 = ld3(pos, id), r2 = ld3(pos, links[id].x);
-      add_target(acc, u, seg_vel64_nr(f4pi, r1, r2, r2 - r1, ld3(pos, k)));
+      add_target(acc, u, seg_vel64_nr(f4pi, r1, r2, ld3(pos, k)));
     };
     auto stage_one = [&](int m) -> SrcVals {
       if (m >= src.y || status[m].x == OV_EMPTY) return src_none();
@@ -268,7 +268,7 @@ __global__ void __launch_bounds__(TB) k_batch_bs_chain(OvParams P, BatchView B,
       const int k = u ? kk[1] : kk[0];
       if (k < 0 || id < 0) return;
       const d3 r1 = ld3(pos, id), r2 = ld3(pos, links[id].x);
-      add_target(acc, u, seg_vel64_nr(f4pi, r1, r2, r2 - r1, ld3(pos, k)));
+      add_target(acc, u, seg_vel64_nr(f4pi, r1, r2, ld3(pos, k)));
     };
     // the segment starting at slot m: forward slot (or -1), vector, far radius
     auto seg_of = [&](int m, double* d, double* far2) -> int {

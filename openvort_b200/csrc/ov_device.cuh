@@ -130,10 +130,9 @@ __device__ __forceinline__ d3 mirror_dir(d3 v, int face) {
 // ----------------------------------------------------------------------
 // straight-segment Biot-Savart (segment_field1, src/tangle.c:486-514)
 
-// FP64, the reference's formula and cut-offs: zero when either endpoint is
-// closer than 1e-8 or R, R' are colinear to 1e-8.
-__device__ __forceinline__ d3 seg_vel64(double f4pi, d3 r1, d3 r2, d3 r, double col = 1e-8) {
-  d3 R = r1 - r, Rp = r2 - r;
+// FP64, the reference's formula and cut-offs from R = r1 - r and R' = r2 - r:
+// zero when either endpoint is closer than 1e-8 or R, R' are colinear to 1e-8.
+__device__ __forceinline__ d3 seg_vel64_of(double f4pi, d3 R, d3 Rp, double col) {
   double R2 = dot3(R, R), Rp2 = dot3(Rp, Rp);
   double lR = sqrt(R2), lRp = sqrt(Rp2);
   double RRp = dot3(R, Rp);
@@ -149,6 +148,9 @@ __device__ __forceinline__ d3 seg_vel64(double f4pi, d3 r1, d3 r2, d3 r, double 
   }
   double s = f4pi * (lR + lRp) / (p * (p + RRp));
   return cross3(R, Rp) * s;
+}
+__device__ __forceinline__ d3 seg_vel64(double f4pi, d3 r1, d3 r2, d3 r, double col = 1e-8) {
+  return seg_vel64_of(f4pi, r1 - r, r2 - r, col);
 }
 
 // 1/sqrt(x) and 1/x in FP64 from the hardware approximations
@@ -202,14 +204,11 @@ __device__ __forceinline__ bool end_near(double R2) { return (unsigned)__double2
 // The reference's segment formula without IEEE square roots and divisions:
 // with u = 1/(|R||R'|) from two refined reciprocal square roots,
 //   f (|R| + |R'|) / (|R||R'| (|R||R'| + R.R')) = f (1/|R| + 1/|R'|) u / (1 + R.R' u).
-// R' = R + d (d = r2 - r1, staged per segment) differs from r2 - r by an ulp
-// of |R'|.  Where a cut-off is too close to call (end_near, ColCut) the
-// reference's own operations decide (seg_vel64), so every cut-off decision is
-// the reference's.
-__device__ __forceinline__ d3 seg_vel64_nr(double f4pi, d3 r1, d3 r2, d3 d, d3 r,
-                                           ColCut cut = col_cut_of(1e-8)) {
-  const d3 R = r1 - r;
-  const d3 Rp = R + d;
+// Where a cut-off is too close to call (end_near, ColCut) slow() decides in
+// the reference's own operations (seg_vel64), so every cut-off decision is the
+// reference's.
+template <class Slow>
+__device__ __forceinline__ d3 seg_vel64_nr_of(double f4pi, d3 R, d3 Rp, const ColCut& cut, Slow&& slow) {
   const double R2 = dot3(R, R), Rp2 = dot3(Rp, Rp), RRp = dot3(R, Rp);
   if (end_inside(R2) || end_inside(Rp2)) return mk3(0, 0, 0);
   const bool near = end_near(R2) || end_near(Rp2);
@@ -218,7 +217,15 @@ __device__ __forceinline__ d3 seg_vel64_nr(double f4pi, d3 r1, d3 r2, d3 d, d3 r
   const double den = fma(RRp, u, 1.0);
   if (!near && den < cut.lo) return cross3(R, Rp) * (f4pi * (ia + ib) * (u * rcp_nr(den)));
   if (!near && den > cut.hi) return mk3(0, 0, 0);
-  return seg_vel64(f4pi, r1, r2, r, cut.col);
+  return slow();
+}
+// R' is r2 - r itself, as the reference forms it: R + (r2 - r1) carries an ulp
+// of |R|, which at a target 1e-7 from the far end of a segment of 2.5e-3 is
+// 1e-12 of |R'|.
+__device__ __forceinline__ d3 seg_vel64_nr(double f4pi, d3 r1, d3 r2, d3 r,
+                                           const ColCut& cut = col_cut_of(1e-8)) {
+  const d3 R = r1 - r, Rp = r2 - r;
+  return seg_vel64_nr_of(f4pi, R, Rp, cut, [&] { return seg_vel64_of(f4pi, R, Rp, cut.col); });
 }
 
 // The chain sweep: cnt staged slots, the segment from node i to node i + 1

@@ -59,7 +59,7 @@ __global__ void __launch_bounds__(kTB) k_direct64(OvParams P, SegTab S, int n_sr
                                                   const int2* __restrict__ tstatus,
                                                   const int* __restrict__ tskip, int n_t,
                                                   double* __restrict__ part, int chunk) {
-  __shared__ double sh_r[kTS][9];   // r1, wrapped r2, d = r2 - r1
+  __shared__ double sh_r[kTS][6];   // r1, wrapped r2
   __shared__ int sh_id[kTS][2];
   const int j = blockIdx.y;  // 0: the tangle itself, j >= 1: image j-1
   const int k = blockIdx.x * kTB + threadIdx.x;
@@ -87,8 +87,6 @@ __global__ void __launch_bounds__(kTB) k_direct64(OvParams P, SegTab S, int n_sr
         const double* src = S.r1r2 + 6 * id;
 #pragma unroll
         for (int c = 0; c < 6; ++c) sh_r[q][c] = src[c];
-#pragma unroll
-        for (int c = 0; c < 3; ++c) sh_r[q][6 + c] = src[3 + c] - src[c];
       }
       sh_id[q][0] = id;
       sh_id[q][1] = fw;
@@ -101,8 +99,7 @@ __global__ void __launch_bounds__(kTB) k_direct64(OvParams P, SegTab S, int n_sr
       // skip rule of calculate_vs_shift (src/tangle.c:567-569)
       if (fw == -1 || id == skip || fw == skip) continue;
       d3 v = seg_vel64_nr(f4pi, mk3(sh_r[q][0], sh_r[q][1], sh_r[q][2]),
-                          mk3(sh_r[q][3], sh_r[q][4], sh_r[q][5]),
-                          mk3(sh_r[q][6], sh_r[q][7], sh_r[q][8]), r, cut);
+                          mk3(sh_r[q][3], sh_r[q][4], sh_r[q][5]), r, cut);
       ax += v.x; ay += v.y; az += v.z;
     }
   }
@@ -204,7 +201,7 @@ __global__ void __launch_bounds__(kTB) k_direct64_chain(OvParams P, int n_src, c
                              if (sb + i == skip || sh_fwd[i] == skip) return mk3(0, 0, 0);
                              const d3 r1 = mk3(sh_node[i][0], sh_node[i][1], sh_node[i][2]);
                              const d3 r2 = mk3(sh_end[i][0], sh_end[i][1], sh_end[i][2]);
-                             return seg_vel64_nr(1.0, r1, r2, r2 - r1, r, cut);
+                             return seg_vel64_nr(1.0, r1, r2, r, cut);
                            });
   }
   if (k < n_t) {
@@ -280,8 +277,11 @@ __global__ void __launch_bounds__(kPB, OV_DIRECT_PAIRS_MIN_BLOCKS) k_direct_mixe
     d3 r = ld3(pos, k);
     if (j > 0) r = image_point(P, j - 1, r);
     const double* sg = S.r1r2 + 6 * (size_t)id;
-    const d3 r1 = mk3(sg[0], sg[1], sg[2]), r2 = mk3(sg[3], sg[4], sg[5]);
-    add_target(acc, u, seg_vel64_nr(f4pi, r1, r2, r2 - r1, r));
+    // R' as R + d: right to an ulp of |R|, far below the form's own error, and
+    // with r2 - r the kernel spills (68.9 against 67.9 ms an RK4 step)
+    const d3 r1 = mk3(sg[0], sg[1], sg[2]), r2 = mk3(sg[3], sg[4], sg[5]), R = r1 - r;
+    add_target(acc, u, seg_vel64_nr_of(f4pi, R, R + (r2 - r1), col_cut_of(1e-8),
+                                       [&] { return seg_vel64(f4pi, r1, r2, r); }));
   };
   const int s_lo = blockIdx.z * chunk, s_hi = min(n_src, s_lo + chunk);
   auto stage_one = [&](int m) -> SrcVals {
@@ -387,7 +387,7 @@ __global__ void __launch_bounds__(kPB, OV_DIRECT_CHAIN_MIN_BLOCKS) k_direct_mixe
     if (j > 0) r = image_point(P, j - 1, r);
     const double* sg = S.r1r2 + 6 * (size_t)id;
     const d3 r1 = mk3(sg[0], sg[1], sg[2]), r2 = mk3(sg[3], sg[4], sg[5]);
-    add_target(acc, u, seg_vel64_nr(f4pi, r1, r2, r2 - r1, r));
+    add_target(acc, u, seg_vel64_nr(f4pi, r1, r2, r));
   };
   const int s_lo = blockIdx.z * chunk, s_hi = min(n_src, s_lo + chunk);
   // a source by slot for the two-source form (the tangle's own wrapped
@@ -557,7 +557,7 @@ __global__ void __launch_bounds__(kPB) k_direct_mixed_points(OvParams P, SegTab 
     const d3 r1 = mk3(sg[0], sg[1], sg[2]), r2 = mk3(sg[3], sg[4], sg[5]);
     d3 r = ld3(tpos, base + kTT * threadIdx.x + u);
     if (j > 0) r = image_point(P, j - 1, r);
-    add_target(acc, u, seg_vel64_nr(f4pi, r1, r2, r2 - r1, r));
+    add_target(acc, u, seg_vel64_nr(f4pi, r1, r2, r));
   };
   const int s_lo = blockIdx.z * chunk, s_hi = min(n_src, s_lo + chunk);
   // sources in slot order; the tangle's own segments wrapped across a

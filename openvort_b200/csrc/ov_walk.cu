@@ -116,7 +116,7 @@ __device__ __forceinline__ void p2p_one(const OvParams& P, d3 r1, d3 r2, d3 rp, 
       return;
     }
   }
-  const d3 v = seg_vel64_nr(P.f4pi, r1, r2, r2 - r1, rp);
+  const d3 v = seg_vel64_nr(P.f4pi, r1, r2, rp);
   ax += v.x; ay += v.y; az += v.z;
 }
 
@@ -261,7 +261,7 @@ __device__ __forceinline__ float sel3f(int i, float a, float b, float c) {
 // calls' register saves made the mixed walk 52.1 ms per launch at 1M points
 // against 37.9 ms.
 __device__ __forceinline__ d3 seg64_at(double f4pi, d3 r1, d3 r2, d3 t) {
-  return seg_vel64_nr(f4pi, r1, r2, r2 - r1, t);
+  return seg_vel64_nr(f4pi, r1, r2, t);
 }
 __device__ __forceinline__ d3 expansion64_at(const Cell* cp, d3 R) { return expansion64(cp->y, cp->m, R); }
 
@@ -376,7 +376,7 @@ __device__ __forceinline__ void p2p_images(const OvParams& P, unsigned mask, d3 
     }
     // the reference's formula with Newton-refined reciprocals (its own
     // operations near the cut-offs), as the FP64 direct sum
-    const d3 v = seg_vel64_nr(P.f4pi, r1, r2, ds, t);
+    const d3 v = seg_vel64_nr(P.f4pi, r1, r2, t);
     if (c == kPrimary) nl = nl + v;
     else im = im + v;
   }
