@@ -355,9 +355,9 @@ inline cudaError_t ov_launch_early(void (*kernel)(P...), dim3 grid, int block, c
 }
 // Waits for the kernel before (all its writes are then visible) and lets the
 // one after take its places; first in the kernel, before any access to
-// memory.  Such a kernel's pointers are not __restrict__: what the kernel
-// before writes is not constant while this one runs, and no load may be taken
-// ahead of the wait.  Nothing happens where the launches are ordinary ones.
+// memory.  Neither such a kernel's pointers nor those of the device functions
+// it calls are __restrict__: what the kernel before writes is not constant
+// while this one runs, and no load may be taken ahead of the wait.  Nothing happens where the launches are ordinary ones.
 __device__ __forceinline__ void follow_early() {
   cudaGridDependencySynchronize();
   cudaTriggerProgrammaticLaunchCompletion();

@@ -106,7 +106,7 @@ __device__ bool tangent_node(const OvParams& P, const Links& L, const double* po
 // needs from the positions, in dxi_node's operations, instead of waiting for
 // a pass over dxi.  A node next to a pinned one reads its neighbours' tangents
 // and is left to k_tangents (pass 1, ov_geom.cu).
-__device__ __forceinline__ void geometry_slot(const OvParams& P, const Links& L, const double* __restrict__ pos, int k,
+__device__ __forceinline__ void geometry_slot(const OvParams& P, const Links& L, const double* pos, int k,
                                               const OvGeomOut& G) {
   const int2 st = L.st[k];
   if (st.x == OV_EMPTY) return;
@@ -142,7 +142,7 @@ __device__ __forceinline__ void geometry_slot(const OvParams& P, const Links& L,
 // The direct sum's partials of target k for image j (0: the tangle itself),
 // with source splits added split by split, in order; mirror images reflect
 // their velocity (src/tangle.c:633-634).
-__device__ __forceinline__ d3 image_sum(const OvParams& P, const double* __restrict__ part, int n_t, int splits, int k,
+__device__ __forceinline__ d3 image_sum(const OvParams& P, const double* part, int n_t, int splits, int k,
                                         int j) {
   const size_t img_stride = 3 * (size_t)n_t, split_stride = img_stride * (P.n_img + 1);
   const double* p = part + (size_t)j * img_stride;
@@ -154,7 +154,7 @@ __device__ __forceinline__ d3 image_sum(const OvParams& P, const double* __restr
 
 // The tangle's own sum nl and the image sum img in image order
 // (src/tangle.c:627-638)
-__device__ __forceinline__ void sum_partials(const OvParams& P, const double* __restrict__ part, int n_t, int splits,
+__device__ __forceinline__ void sum_partials(const OvParams& P, const double* part, int n_t, int splits,
                                              int k, d3& nl, d3& img) {
   nl = image_sum(P, part, n_t, splits, k, 0);
   img = mk3(0, 0, 0);

@@ -691,9 +691,9 @@ __global__ void k_moments_thread(const int* list, const int* list_count,
 
 // same, one warp per cell (17 .. mom_big nodes): lane-strided sums, then a
 // butterfly over the warp
-__device__ void moments_warp(int c, Cell* cells, const int2* __restrict__ cell_range,
-                             const double* __restrict__ nodes64,
-                             const int2* __restrict__ nodeids, double f4pi) {
+__device__ void moments_warp(int c, Cell* cells, const int2* cell_range,
+                             const double* nodes64,
+                             const int2* nodeids, double f4pi) {
   const int tid = threadIdx.x & 31;
   const int start = cell_range[c].x, count = cell_range[c].y;
   double s[3] = {0, 0, 0};
@@ -774,7 +774,7 @@ __device__ __forceinline__ void block_sum(double (&v)[kN], double* sh) {
 }
 
 // sum q (0 .. 9) of list cell j over its chunks, in chunk order
-__device__ __forceinline__ double chunk_sum(const double* __restrict__ part, int j, int max_chunks, int nch, int q) {
+__device__ __forceinline__ double chunk_sum(const double* part, int j, int max_chunks, int nch, int q) {
   const double* p = part + (size_t)j * max_chunks * 10 + q;
   double s = 0;
 #pragma unroll 8
