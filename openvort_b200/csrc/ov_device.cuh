@@ -235,11 +235,12 @@ __device__ __forceinline__ d3 seg_vel64_nr(double f4pi, d3 r1, d3 r2, d3 r,
 // reference forms it (src/tangle.c:490-491).  A segment then costs 32 FP64
 // operations: R, |R|^2, R.R' 9; the reciprocals 5 and 3; the weight 5; cross
 // product and sum 9; the cut-off 1.  Slots whose segment does not run to the
-// next slot have their bit in `other` and take other_seg(i), in place, so the
-// terms are added in slot order whatever the staging.  kSkip: segments from
-// or to node `skip` (an index into the staged nodes) are left out.  Every
-// staged node must be finite, whether or not a segment uses it: a segment left
-// out still adds its cross product times zero.
+// next slot have their bit in `other` and take other_seg(i).  Terms are added
+// in slot order but for these and the ones too close to a cut-off, which follow
+// their group of kChainGroup slots, counted from the start of the tile.  kSkip:
+// segments from or to node `skip` (an index into the staged nodes) are left
+// out.  Every staged node must be finite, whether or not a segment uses it: a
+// segment left out still adds its cross product times zero.
 // Groups of kChainGroup segments are summed without a branch (a segment left
 // out has weight zero), so their dependency chains overlap; the segments the
 // reference's own operations decide follow the group.  Groups of 1 / 2 / 4:

@@ -15,8 +15,8 @@
 // Mixed form (k_direct_mixed_pairs): sources staged two by two as FP32
 // offsets from the block's first target (the subtraction done in FP64,
 // rounded once) and evaluated two per f32x2 instruction (ov_pair.cuh); near
-// or borderline-colinear pairs fall back to seg_vel64 from the FP64 table;
-// sums accumulate in FP64.
+// or borderline-colinear pairs take the FP64 form from the FP64 table after
+// each stretch of 32 sources; sums accumulate in FP64.
 #include <algorithm>
 
 #include "ov_internal.h"
@@ -789,8 +789,8 @@ bool ov_direct_partials(ov_state_impl* s, const double* pos, double* v_nl, doubl
     }
     OV_LAUNCHED();
     OV_TRY_CUDA(cudaGetLastError());
-    // k_direct_mixed_pairs wrote part[j][k] for slots k in the sorted set only;
-    // EMPTY slots are never read by the epilogue, but zero them for hygiene
+    // k_direct_mixed_pairs wrote part[j][k] for slots k in the sorted set only:
+    // the partials of EMPTY slots, and what is added up from them, are undefined
   } else {
     const int bx = (s->n + kTB - 1) / kTB;
     static const int res64 = resident_blocks(k_direct64_chain<false>, kTB);
@@ -832,8 +832,8 @@ bool ov_direct_points(ov_state_impl* s, const double* pos, int npts, const doubl
   if (npts <= 0) return true;
   int nimg = out_img ? s->P.n_img : 0;
   int n_src = only ? n_only : s->n;
-  // few points over many sources: split the sources so the GPU fills, about
-  // four waves of the kernel's 7 resident blocks per SM
+  // few points over many sources: split the sources so the GPU fills, some 32
+  // blocks per SM, in whole waves of the resident ones
   const int bx = (npts + kTB - 1) / kTB;
   int splits = 1;
   static const int res64 = resident_blocks(k_direct64_chain<true>, kTB);

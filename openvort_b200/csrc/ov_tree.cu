@@ -105,7 +105,6 @@ __global__ void k_keys(OvParams P, const double* pos, const int2* status,
     term[k] = -1;
     return;
   }
-  atomicAdd(&counters[0], 1);
   const int nch = P.quadtree ? 4 : 8;
   const double px = pos[3 * k], py = pos[3 * k + 1], pz = pos[3 * k + 2];
   double lo[3] = {P.lo[0], P.lo[1], P.lo[2]}, hi[3] = {P.hi[0], P.hi[1], P.hi[2]};
@@ -154,7 +153,6 @@ __global__ void k_keys(OvParams P, const double* pos, const int2* status,
   khi[k] = h;
   klo[k] = l;
   term[k] = tl | (tk << 8);
-  atomicMax(&counters[2], tl);
 }
 
 // ---------------------------------------------------------------- 2. sort
@@ -978,8 +976,8 @@ bool ov_tree_build(ov_state_impl* s, const double* pos, OvTree* T, bool order_on
   int* vals_alt = T->vals_alt.as<int>();
   int* term = vals_alt + n;
   int* ctr = T->counters.as<int>();
-  int hc[16];   // the device counters: active nodes, depth error, deepest level, nodes outside the
-                // box, cells per moment class (3), cells, the state's error flag, cells with a node range
+  int hc[16];   // the device counters: 1 depth error, 3 nodes outside the box, 4-6 cells per moment
+                // class, 7 cells, 8 the state's error flag, 9 cells with a node range
   OV_TRY_CUDA(cudaMemsetAsync(ctr, 0, sizeof(int) * 16, st));
   if (n > 0) {
     OV_TRY_CUDA(ov_launch_early(k_keys, dim3((n + 255) / 256), 256, st, s->P, pos, s->status.as<int2>(), n, khi,

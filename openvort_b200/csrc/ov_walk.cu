@@ -374,8 +374,8 @@ __device__ __forceinline__ void p2p_images(const OvParams& P, unsigned mask, d3 
       nl = nl + seg64_at(P.f4pi, r1, r2, t);
       continue;
     }
-    // the reference's formula with Newton-refined reciprocals (its own
-    // operations near the cut-offs), as the FP64 direct sum
+    // the reference's formula with refined reciprocals (its own operations
+    // near the cut-offs), as the FP64 direct sum
     const d3 v = seg_vel64_nr(P.f4pi, r1, r2, t);
     if (c == kPrimary) nl = nl + v;
     else im = im + v;
@@ -982,21 +982,15 @@ __global__ void __launch_bounds__(32, kMixed || kSplit ? kWalkWarps : kWalkWarps
       d3 v = mk3(0, 0, 0), w = v;
       if (e.on) {
         const Cell* cp = T.cells + e.cell;
-        const double cx = cp->x[0], cy = cp->x[1], cz = cp->x[2];
-        if (kMixed)
-          cell_mixed(P, cp, __int_as_float(cp->a), cx, cy, cz, cp->thr, rt,
-                     mk3(__dsub_rn(cx, rt.x), __dsub_rn(cy, rt.y), __dsub_rn(cz, rt.z)), e.mask, near2, v);
-        else
-          cell_fp64(P, cp, cx, cy, cz, rt, e.mask, v, w);
+        cell_fp64(P, cp, cp->x[0], cp->x[1], cp->x[2], rt, e.mask, v, w);
       }
       __syncwarp();
       for (unsigned of = sh_of[lane]; __any_sync(FULL, of != 0); of &= of - 1) {
         const int src = of ? __ffs(of) - 1 : lane;
-        const d3 a = shfl3(v, src);
-        if (of) nl = nl + a;
-        if (!kMixed) {
-          const d3 b = shfl3(w, src);
-          if (of) im = im + b;
+        const d3 a = shfl3(v, src), b = shfl3(w, src);
+        if (of) {
+          nl = nl + a;
+          im = im + b;
         }
       }
       continue;
@@ -1138,13 +1132,10 @@ __global__ void __launch_bounds__(32, kMixed || kSplit ? kWalkWarps : kWalkWarps
         if (pass && mine) {
           n_far += __popc(pass);
           // expansion at every accepting image: R = r - L s - com, unwrapped
-          if (kQueueCells) {
+          if (kQueueCells)
             cell_mask = pass;
-          } else if (kMixed) {
+          else
             cell_mixed(P, cp, __int_as_float(h.x), cx, cy, cz, t0.x, r, mk3(dx, dy, dz), pass, near2, nl);
-          } else {
-            cell_fp64(P, cp, cx, cy, cz, r, pass, nl, im);
-          }
         }
       }
       if (open) lvl_mask[32 * (cell_lbot(h.w) + 1)] = open;
@@ -1331,19 +1322,16 @@ static __global__ void k_cost_keys(const unsigned* cost, int n, uint64_t* keys, 
 // "Programming the Hilbert curve", AIP Conf. Proc. 707, 2004: the transform
 // of the axes into the curve's transposed index).  Points outside the box,
 // whose coordinates clamp, and NaN, which converts to 0, sort somewhere: the
-// order only decides which targets share a warp.  Value i of the sort is
-// slots[i] (or i).
+// order only decides which targets share a warp.
 constexpr int kCurveBits = 10;
-static __global__ void k_curve_keys(OvParams P, const double* pts, const int* slots, int n,
-                                    uint64_t* keys, int* vals) {
+static __global__ void k_curve_keys(OvParams P, const double* pts, int n, uint64_t* keys, int* vals) {
   follow_early();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
-  const int k = slots ? slots[i] : i;
   unsigned x[3];
 #pragma unroll
   for (int a = 0; a < 3; ++a) {
-    const double f = (pts[3 * (size_t)k + a] - P.lo[a]) / P.L[a] * (1 << kCurveBits);
+    const double f = (pts[3 * (size_t)i + a] - P.lo[a]) / P.L[a] * (1 << kCurveBits);
     x[a] = (unsigned)fmin(fmax(f, 0.0), (double)((1 << kCurveBits) - 1));
   }
   for (unsigned q = 1u << (kCurveBits - 1); q > 1; q >>= 1) {
@@ -1370,7 +1358,7 @@ static __global__ void k_curve_keys(OvParams P, const double* pts, const int* sl
 #pragma unroll
     for (int a = 0; a < 3; ++a) key = (key << 1) | (((x[a] ^ t) >> b) & 1u);
   keys[i] = key;
-  vals[i] = k;
+  vals[i] = i;
 }
 
 constexpr int kMaxParts = 16;        // warps a group of nodes' walk is split over, at most
@@ -1474,8 +1462,12 @@ static bool launch_multi(ov_state_impl* s, OvTree* t, const OvParams& P, const i
   // 22.4k 1.29, 1.20, 1.17, 1.24, 1.48.  Points 1/96 (512 over 20k nodes 0.77
   // at 1/64, 0.74, 0.75 at 1/128, 0.77 at 1/192).
   const int frontier = std::max(1, t->n_cells / (status ? 32 : 96));
-  // stretches of a quarter of the frontier (22.4k nodes FP64, 8 parts: 2.52
-  // ms, against 2.66 with a sixteenth)
+  // Stretches of a quarter of the frontier.  Chosen when a walk evaluated its
+  // leaves and cells at the visit (22.4k nodes FP64, 8 parts: 2.52 ms, against
+  // 2.66 with a sixteenth).  With the queues a sixteenth is the faster one:
+  // theta = 0.4, FP64 1.14 ms against 1.21 now and mixed 0.78 against 0.92 at
+  // 22.4k nodes, 3.46 / 3.53 and 2.29 / 2.34 at 59k, 0.58 / 0.60 and 0.35 /
+  // 0.34 at 7.9k.  It would change the order of the sums and is not taken here.
   int deal = 0;
   while ((8 << deal) <= frontier) ++deal;
   const bool split = parts > 1 || !status;
@@ -1633,10 +1625,10 @@ bool ov_tree_walk_points(ov_state_impl* s, OvTree* t, int npts, const double* pt
   unsigned combos = 0;
   // One traversal per point for all its images, the points in Hilbert order
   // of the box so a warp's 32 are close together: 4096 probes of a 50k-node
-  // tangle with 26 images take 2.9 ms, against 129 ms with one walk per image
-  // and the points as given.  FP64 in the mixed form too (a query's cost is
-  // its traversal).  A table with mirrors, or an opening angle other than the
-  // tree's, takes the walk per image.
+  // tangle with 26 images take 1.06 ms with the build, against 129 ms with one
+  // walk per image and the points as given.  FP64 in the mixed form too (a
+  // query's cost is its traversal).  A table with mirrors, or an opening angle
+  // other than the tree's, takes the walk per image.
   if (use_thr && image_combos(P, out_img ? P.n_img : 0, combos)) {
     const int* order = nullptr;
     if (npts > 32) {
@@ -1644,7 +1636,7 @@ bool ov_tree_walk_points(ov_state_impl* s, OvTree* t, int npts, const double* pt
       if (!s->pkeys.reserve(sizeof(uint64_t) * 2 * np) || !s->pvals.reserve(sizeof(int) * 2 * np)) return false;
       uint64_t* keys = s->pkeys.as<uint64_t>();
       int* vals = s->pvals.as<int>();
-      OV_TRY_CUDA(ov_launch_early(k_curve_keys, dim3((npts + 255) / 256), 256, s->stream, P, pts, nullptr, npts, keys,
+      OV_TRY_CUDA(ov_launch_early(k_curve_keys, dim3((npts + 255) / 256), 256, s->stream, P, pts, npts, keys,
                                   vals));
       OV_LAUNCHED();
       if (!ov_radix_sort_u64(keys, vals, keys + np, vals + np, npts, 3 * kCurveBits, s->phist, s->pscan, s->stream))
