@@ -7,6 +7,7 @@ in the holes against the same call with the box centre.  FP64 bit for bit;
 the mixed sums in slot order add their unchained segments in no fixed order (two
 runs of the same input differ by 1e-11), so the mixed form to its tolerance."""
 import ctypes as C
+import dataclasses
 
 import numpy as np
 import pytest
@@ -222,3 +223,49 @@ def test_adjoint_without_nodes(ov, precision):
     x_bar, vn_bar = a.velocity_vjp(t.pos, g, np.zeros(3))
     assert np.all(x_bar == 0) and np.all(vn_bar == 0)
     a.close()
+
+
+@pytest.mark.parametrize("value", VALUES, ids=IDS)
+def test_walls_pinned_nodes_and_remesh(ov, value):
+    """Mirror images with pinned nodes (the second geometry pass, the walk per
+    image), and the passes that change a tangle: remeshing takes EMPTY slots for
+    new nodes, boundary enforcement and small-loop removal visit all slots."""
+    from cases import load
+    lib = ov.load()
+    wall, pw, _, _ = load("wall_half_ring")
+    got = []
+    for hole in (D / 2, value):
+        res = []
+        for use_bh in (0, 1):
+            ov.configure(dataclasses.replace(pw, use_bh=use_bh, bh_theta=0.5), 0)
+            h = with_holes(wall, hole)
+            ov.update_tangle(h, 0.0)
+            res.append(h.vels[h.active].copy())
+            ov.rk4_step(h, 0.0, 1e-7)
+            res.append(h.pos[h.active].copy())
+        ov.configure(Params(**PARAMS), 0)
+        h = holed(G.random_ring_tangle(8, 6, D, boundary="periodic-26", empty_slots=40), hole)
+        ov.update_tangle(h, 0.0)
+        live = np.nonzero(h.active)[0]
+        h.pos[live[::9]] = 0.5 * (h.pos[live[::9]] + h.pos[h.links[live[::9], 0]])
+        ov.update_tangle(h, 0.0)
+        seg = np.median(h.dxi[h.active])
+        changes = lib.ov_remesh(h.ptr(), 0.6 * seg, 1.4 * seg, None)
+        ov.check(lib)
+        assert changes > 3
+        lib.ov_enforce_boundaries(h.ptr())
+        lib.ov_eliminate_small_loops(h.ptr(), 5)
+        ov.check(lib)
+        ov.update_tangle(h, 0.0)
+        got.append(res + [h.stat[:, 0].copy(), h.links[h.active].copy(), h.pos[h.active].copy(), h.vels[h.active].copy()])
+    for i, (a, b) in enumerate(zip(*got)):
+        assert np.all(np.isfinite(b)) and np.array_equal(a, b), i
+
+
+def with_holes(t, value):
+    """t with three EMPTY slots behind its nodes"""
+    from openvort_b200.tangle import HostTangle
+    none = np.full(3, -1, np.int32)
+    return HostTangle(np.concatenate([t.pos, np.full((3, 3), value)]), np.concatenate([t.links[:, 0], none]),
+                      np.concatenate([t.links[:, 1], none]), np.concatenate([t.stat[:, 0], none]),
+                      np.concatenate([t.stat[:, 1], none]), t.box_lo, t.box_hi, t.boundary)
